@@ -1,12 +1,12 @@
-// Residual-window flush, single-token append, and store -> dense dequantization.
+// Residual-window flush and single-token append.
 //
-// Flush is one launch: the first n_k CTAs each take one key tile
+// Flush is one launch.  flush16_kernel below serves the usual shapes; any other takes flush_kv_kernel: the first n_k CTAs each take one key tile
 // [G tokens x D channels] of one (b, kvh): the tile is staged in shared memory
 // with 16-byte row loads, then one thread per channel reduces min/max down its
 // column, quantizes it and writes the packed row straight into the store (the
 // transpose never touches global memory).  The remaining CTAs quantize value
 // rows (G contiguous channels of one token) with G/8 lanes per row.
-#include "mz_quant_math.cuh"
+#include "mz_quant16.cuh"
 #include "mz_store.cuh"
 
 namespace {
@@ -208,6 +208,254 @@ __global__ void __launch_bounds__(256) flush_kv_kernel(const FlushParams p) {
   else flush_value_rows_generic<DT>(p);
 }
 
+// ---- head_dim 64 / 128, groups of 32 / 64 / 128 that divide it: the packed quantizer (mz_quant16.cuh).
+//
+// Bound by instruction issue (HBM traffic is 2.6 bytes per value at 4 bits): the point of the layout is that every
+// step works on two values per register and that nothing is staged that can stay in registers.
+//   keys    a thread owns two neighbouring channels (the two halves of a register) of TPT tokens, so the loads of a
+//           warp are whole 128-byte rows and the transpose happens in the packing; the parts of a channel meet in
+//           shared memory for the min / max, one thread per channel then prepares the row (metadata, reciprocal,
+//           thresholds) and the finished codes go through shared memory into whole-line stores
+//   values  a thread owns 16 channels of one row (two 16-byte loads), G / 16 lanes per row, shuffles for min / max
+struct Flush16Params {
+  mz_kv_store s;
+  int n_tiles;               // key tiles per pair
+  int v_first, n_vtokens;    // value tokens: window rows [v_first, v_first + n_vtokens)
+  float eps;
+  const uint16_t* thr_k; const uint16_t* thr_v;
+  const uint16_t* ctab_k; const uint16_t* ctab_v; int ctab_k_n, ctab_v_n;
+  unsigned n_k_blocks, tiles;       // key CTAs; key tiles in all
+  unsigned v_blocks_per_pair;
+};
+
+template <int DT, int BITS, int TPT>
+__device__ __forceinline__ void flush16_keys(const Flush16Params& p, uint8_t* smem) {
+  using P = mzq::P2<DT>;
+  constexpr bool WIDE = BITS > 4;
+  constexpr int NT = WIDE ? 1 : (1 << BITS) - 1;
+  constexpr int CB = TPT * BITS / 8;                      // packed bytes of one channel in one thread
+  const mz_kv_store& s = p.s;
+  const int G = s.group, D = s.head_dim, QB = G * BITS / 8;
+  const int pairs = D >> 1, parts = G / TPT, tt = pairs * parts, per_cta = 256 / tt, rows = per_cta * D;
+  const int tid = threadIdx.x;
+  const int local = tid / tt, part = (tid % tt) / pairs, cp = tid % pairs;
+  // shared memory: partial min / max, row constants, thresholds (or the wide rows' constants), code tile
+  uint32_t* red = (uint32_t*)smem;                        // [per_cta][parts][2][pairs]
+  float* s_inv = (float*)(red + 512);                     // [rows]
+  float* s_span = s_inv + 256;                            // [rows], negative: special row
+  uint16_t* s_lo = (uint16_t*)(s_span + 256);             // [rows]
+  uint32_t* s_thr = (uint32_t*)(s_lo + 256);              // [NT][rows / 2] pairs, or floats [8][rows]
+  uint8_t* s_code = (uint8_t*)(s_thr + (WIDE ? 8 * 256 : NT * 128));   // even channels, then odd ones, padded rows
+  const int stride = QB + 8;
+  const unsigned tile0 = blockIdx.x * per_cta;
+  auto locate = [&](unsigned tile, int& j, int& h, int& b) {
+    j = tile % p.n_tiles; tile /= p.n_tiles;
+    h = tile % s.kv_heads; b = tile / s.kv_heads;
+  };
+  const bool live = tile0 + local < p.tiles;
+  uint32_t x[TPT];
+  const uint16_t* src = nullptr;
+  if (live) {
+    int j, h, b;
+    locate(tile0 + local, j, h, b);
+    src = (const uint16_t*)s.res_k + b * s.res_stride_b + h * s.res_stride_h + (long long)(s.res_start + j * G + part * TPT) * s.res_stride_t + 2 * cp;
+    uint32_t mn = P::INF2, mx = P::INF2 | 0x80008000u;
+#pragma unroll
+    for (int i = 0; i < TPT; ++i) x[i] = *(const uint32_t*)(src + i * s.res_stride_t);
+#pragma unroll
+    for (int i = 0; i < TPT; ++i) { mn = P::mn(mn, x[i]); mx = P::mx(mx, x[i]); }
+    red[((local * parts + part) * 2) * pairs + cp] = mn;
+    red[((local * parts + part) * 2 + 1) * pairs + cp] = mx;
+  }
+  __syncthreads();
+  if (tid < rows && tile0 + tid / D < p.tiles) {
+    const int l = tid / D, d = tid % D;
+    const uint16_t* r16 = (const uint16_t*)(red + l * parts * 2 * pairs);
+    float mn = mz_u16_to_float(r16[d], DT), mx = mz_u16_to_float(r16[D + d], DT);
+    for (int k = 1; k < parts; ++k) {
+      mn = fminf(mn, mz_u16_to_float(r16[2 * k * D + d], DT));
+      mx = fmaxf(mx, mz_u16_to_float(r16[(2 * k + 1) * D + d], DT));
+    }
+    mzq::RowHead<DT> head;
+    head.set(mn, mx, p.eps);
+    s_inv[tid] = head.inv_span;
+    s_span[tid] = head.special ? -1.0f : head.span;
+    s_lo[tid] = (uint16_t)(P::pack(head.lo, head.lo) & 0xffffu);
+    if constexpr (WIDE) {
+      mzq::WideRow<DT> w;
+      w.set(mz_u16_to_float((uint16_t)head.anchor_bits, DT), (float)((1 << BITS) - 1), MzType<DT>::round(p.eps));
+      float* f = (float*)s_thr + tid;
+      f[0] = w.anchor; f[256] = w.zero_code; f[512] = w.steps_up; f[768] = w.steps_dn;
+      f[1024] = w.room_up; f[1280] = w.room_dn; f[1536] = w.inv_up; f[1792] = w.inv_dn;
+    } else {
+      const uint16_t* t = p.thr_k + ((size_t)(head.special ? 0 : head.anchor_bits) << BITS);
+      uint16_t* o = (uint16_t*)s_thr + tid;
+      if constexpr (BITS == 4) {
+        const uint4 a = *(const uint4*)t, b = *(const uint4*)(t + 8);
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int k = 0; k < NT; ++k) o[k * 256] = (uint16_t)(w[k >> 1] >> ((k & 1) * 16));
+      } else {
+#pragma unroll
+        for (int k = 0; k < NT; ++k) o[k * 256] = t[k];
+      }
+    }
+    int j, h, b;
+    locate(tile0 + l, j, h, b);
+    const long long grp = s.k_groups + j;
+    if (MZ_IN_BOUNDS((grp + 1) * D - 1, s.km_stride_h, 2)) {
+      const long long m = b * s.km_stride_b + h * s.km_stride_h + grp * D + d;
+      mz_store_from_float(s.k_mn, m, head.lo, s.meta_dtype);
+      mz_store_from_float(s.k_scale, m, head.span, s.meta_dtype);
+    }
+  }
+  __syncthreads();
+  if (live) {
+    const int row = local * D + 2 * cp;
+    const uint32_t lo2 = *(const uint32_t*)(s_lo + row);
+    const float2 inv = *(const float2*)(s_inv + row), span = *(const float2*)(s_span + row);
+    uint8_t* dst = s_code + (size_t)(local * pairs + cp) * stride + part * CB;
+    uint8_t* dst_odd = dst + (size_t)per_cta * pairs * stride;
+    if (span.x < 0.f || span.y < 0.f) {
+      // a row outside the packed path's domain: value by value
+#pragma unroll 1
+      for (int c = 0; c < 2; ++c) {
+        float mn = INFINITY, mx = -INFINITY;
+        const uint16_t* r16 = (const uint16_t*)(red + local * parts * 2 * pairs);
+        for (int k = 0; k < parts; ++k) {
+          mn = fminf(mn, mz_u16_to_float(r16[2 * k * D + 2 * cp + c], DT));
+          mx = fmaxf(mx, mz_u16_to_float(r16[(2 * k + 1) * D + 2 * cp + c], DT));
+        }
+        MzQuantRow<DT> r;
+        r.setup(mn, mx, BITS, s.alpha_key, p.eps, p.ctab_k, p.ctab_k_n);
+#pragma unroll 1
+        for (int t0 = 0; t0 < TPT; t0 += 8) {
+          unsigned long long word = 0;
+#pragma unroll 1
+          for (int k = 0; k < 8; ++k)
+            word |= ((unsigned long long)r.code(mz_u16_to_float(src[(t0 + k) * s.res_stride_t + c], DT))) << (k * BITS);
+          for (int k = 0; k < BITS; ++k) (c ? dst_odd : dst)[(t0 >> 3) * BITS + k] = (uint8_t)(word >> (8 * k));
+        }
+      }
+    } else if constexpr (!WIDE) {
+      mzq::Thresholds<DT, BITS> th;
+#pragma unroll
+      for (int k = 0; k < NT; ++k) th.T[k] = s_thr[k * 128 + (row >> 1)];
+#pragma unroll
+      for (int t0 = 0; t0 < TPT; t0 += 16) {
+        unsigned long long ca = 0, cb = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t xx[4] = {x[t0 + 4 * q], x[t0 + 4 * q + 1], x[t0 + 4 * q + 2], x[t0 + 4 * q + 3]};
+          uint32_t u[4];
+          mzq::units_of<DT, 4>(xx, lo2, inv.x, inv.y, span.x, span.y, u);
+          // four codes of each channel in the two halves
+          const uint32_t acc = th.template codes<0>(u[0]) | th.template codes<BITS>(u[1]) |
+                               th.template codes<2 * BITS>(u[2]) | th.template codes<3 * BITS>(u[3]);
+          ca |= (unsigned long long)(acc & 0xffffu) << (4 * BITS * q);
+          cb |= (unsigned long long)(acc >> 16) << (4 * BITS * q);
+        }
+        uint8_t* da = dst + t0 * BITS / 8;
+        uint8_t* db = dst_odd + t0 * BITS / 8;
+        if (BITS == 4) { *(unsigned long long*)da = ca; *(unsigned long long*)db = cb; }
+        else if (BITS == 2) { *(uint32_t*)da = (uint32_t)ca; *(uint32_t*)db = (uint32_t)cb; }
+        else {
+#pragma unroll
+          for (int k = 0; k < BITS; ++k) {
+            *(uint16_t*)(da + 2 * k) = (uint16_t)(ca >> (16 * k));
+            *(uint16_t*)(db + 2 * k) = (uint16_t)(cb >> (16 * k));
+          }
+        }
+      }
+    } else {
+      mzq::WideRow<DT> ra, rb;
+      const float* f = (const float*)s_thr + row;
+      ra = {f[0], f[256], f[512], f[768], f[1024], f[1280], f[1536], f[1792]};
+      rb = {f[1], f[257], f[513], f[769], f[1025], f[1281], f[1537], f[1793]};
+#pragma unroll
+      for (int t0 = 0; t0 < TPT; t0 += 8) {
+        unsigned long long ca = 0, cb = 0;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const uint32_t xx[4] = {x[t0 + 4 * q], x[t0 + 4 * q + 1], x[t0 + 4 * q + 2], x[t0 + 4 * q + 3]};
+          uint32_t u[4];
+          mzq::units_of<DT, 4>(xx, lo2, inv.x, inv.y, span.x, span.y, u);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint32_t one = P::ONE | (P::ONE << 16);
+            // a NaN value has code 0
+            const uint32_t nn = P::ge(u[k], 0u);
+            const uint32_t c = mzq::wide_codes<DT>(P::mn(P::mx(u[k], 0u), one), ra, rb, (float)((1 << BITS) - 1), p.ctab_k) & nn;
+            ca |= (unsigned long long)(c & 0xffffu) << (BITS * (4 * q + k));
+            cb |= (unsigned long long)(c >> 16) << (BITS * (4 * q + k));
+          }
+        }
+        uint8_t* da = dst + (t0 >> 3) * BITS;
+        uint8_t* db = dst_odd + (t0 >> 3) * BITS;
+        if (BITS == 8) { *(unsigned long long*)da = ca; *(unsigned long long*)db = cb; }
+        else {
+#pragma unroll
+          for (int k = 0; k < BITS; ++k) { da[k] = (uint8_t)(ca >> (8 * k)); db[k] = (uint8_t)(cb >> (8 * k)); }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // code tile -> store: the D rows of a tile are contiguous there
+  const int words = D * QB / 4, wpr = QB / 4;
+  for (int l = 0; l < per_cta && tile0 + l < p.tiles; ++l) {
+    int j, h, b;
+    locate(tile0 + l, j, h, b);
+    const long long grp = s.k_groups + j;
+    if (!MZ_IN_BOUNDS((grp + 1) * D * QB - 1, s.pk_stride_h, 1)) continue;
+    uint32_t* out = (uint32_t*)(s.packed_k + b * s.pk_stride_b + h * s.pk_stride_h + grp * D * QB);
+    for (int i = tid; i < words; i += 256) {
+      const int d = i / wpr, w = i % wpr;
+      out[i] = *(const uint32_t*)(s_code + (size_t)((d & 1) * per_cta * pairs + l * pairs + (d >> 1)) * stride + 4 * w);
+    }
+  }
+}
+
+template <int DT, int BITS>
+__device__ __forceinline__ void flush16_values(const Flush16Params& p) {
+  const mz_kv_store& s = p.s;
+  const int G = s.group, D = s.head_dim, NG = D / G, QB = G * BITS / 8, lpr = G >> 4;
+  const unsigned blk = blockIdx.x - p.n_k_blocks;
+  const unsigned pair = blk / p.v_blocks_per_pair, chunk = blk % p.v_blocks_per_pair;
+  const int b = pair / s.kv_heads, h = pair % s.kv_heads;
+  const int r = chunk * (256 / lpr) + threadIdx.x / lpr, sub = threadIdx.x % lpr;   // row inside the pair: token * NG + group
+  const bool live = r < p.n_vtokens * NG;
+  const int t = live ? r / NG : 0, grp = live ? r % NG : 0;
+  uint32_t x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (live) {
+    const uint16_t* src = (const uint16_t*)s.res_v + b * s.res_stride_b + h * s.res_stride_h +
+                          (long long)(s.res_start + p.v_first + t) * s.res_stride_t + grp * G + sub * 8;
+    const uint4 a = *(const uint4*)src, c = *(const uint4*)(src + lpr * 8);
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = c.x; x[5] = c.y; x[6] = c.z; x[7] = c.w;
+  }
+  mzq::RowHead<DT> head;
+  unsigned long long word[2];
+  mzq::quantize_row16<DT, BITS>(x, lpr, s.alpha_value, p.eps, p.thr_v, p.ctab_v, p.ctab_v_n, head, word);
+  if (!live) return;
+  const long long row = (long long)(s.v_tokens + t) * NG + grp;
+  if (!MZ_IN_BOUNDS((row + 1) * QB - 1, s.pv_stride_h, 3) || !MZ_IN_BOUNDS(row, s.vm_stride_h, 4)) return;
+  uint8_t* dst = s.packed_v + b * s.pv_stride_b + h * s.pv_stride_h + row * QB + sub * BITS;
+  mz_store_octet(dst, word[0], BITS);
+  mz_store_octet(dst + lpr * BITS, word[1], BITS);
+  if (sub == 0) {
+    const long long m = b * s.vm_stride_b + h * s.vm_stride_h + row;
+    mz_store_from_float(s.v_mn, m, head.lo, s.meta_dtype);
+    mz_store_from_float(s.v_scale, m, head.span, s.meta_dtype);
+  }
+}
+
+template <int DT, int BITS, int TPT>
+__global__ void __launch_bounds__(256) flush16_kernel(const Flush16Params p) {
+  extern __shared__ __align__(16) uint8_t s_flush[];
+  if (blockIdx.x < p.n_k_blocks) flush16_keys<DT, BITS, TPT>(p, s_flush);
+  else flush16_values<DT, BITS>(p);
+}
+
 __global__ void append_kv_kernel(const mz_kv_store s, const uint16_t* __restrict__ k_new, const uint16_t* __restrict__ v_new,
                                  long long nsb, long long nsh) {
   // launched as a programmatic dependent: nothing is read or written before the previous kernel has completed,
@@ -276,6 +524,56 @@ __global__ void __launch_bounds__(256) dequant_values_kernel(const mz_kv_store s
 }
 
 bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
+
+bool flush16_serves(const mz_kv_store& s, const FlushParams& p) {
+  return (s.head_dim == 64 || s.head_dim == 128) && (s.group == 32 || s.group == 64 || s.group == 128) && s.head_dim % s.group == 0 &&
+         p.k_vec && ((uintptr_t)s.packed_k & 3) == 0 && ((s.pk_stride_b | s.pk_stride_h) & 3) == 0 && p.n_vtokens < (1 << 28);
+}
+template <int DT, int BITS>
+int launch_flush16(const Flush16Params& p, unsigned blocks, cudaStream_t st) {
+  const int per_cta = 256 / ((p.s.head_dim / 2) * (p.s.group / (p.s.group == 128 ? 32 : 16)));
+  const size_t smem = 2048 + 2 * 1024 + 512 + (BITS > 4 ? 8192 : ((1 << BITS) - 1) * 512) +
+                      (size_t)per_cta * p.s.head_dim * (p.s.group * BITS / 8 + 8);
+  if (p.s.group == 128) flush16_kernel<DT, BITS, 32><<<blocks, 256, smem, st>>>(p);
+  else flush16_kernel<DT, BITS, 16><<<blocks, 256, smem, st>>>(p);
+  MZ_LAUNCH_CHECK("flush16");
+  return MZ_OK;
+}
+template <int DT>
+int launch_flush16_bits(const Flush16Params& p, unsigned blocks, cudaStream_t st) {
+  switch (p.s.bits) {
+    case 1: return launch_flush16<DT, 1>(p, blocks, st);
+    case 2: return launch_flush16<DT, 2>(p, blocks, st);
+    case 3: return launch_flush16<DT, 3>(p, blocks, st);
+    case 4: return launch_flush16<DT, 4>(p, blocks, st);
+    case 5: return launch_flush16<DT, 5>(p, blocks, st);
+    case 6: return launch_flush16<DT, 6>(p, blocks, st);
+    case 7: return launch_flush16<DT, 7>(p, blocks, st);
+    default: return launch_flush16<DT, 8>(p, blocks, st);
+  }
+}
+// *done = 0 when the thresholds table is not available: the caller takes the per-value kernel
+int flush16(const mz_kv_store& s, const FlushParams& f, cudaStream_t st, int* done) {
+  Flush16Params p;
+  p.s = s; p.n_tiles = f.n_tiles; p.v_first = f.v_first; p.n_vtokens = f.n_vtokens; p.eps = f.eps;
+  p.ctab_k = f.ctab_k; p.ctab_k_n = f.ctab_k_n; p.ctab_v = f.ctab_v; p.ctab_v_n = f.ctab_v_n;
+  p.thr_k = p.thr_v = nullptr;
+  int rc;
+  if (s.bits <= 4) {
+    if ((rc = mz_get_unit_thresholds(s.kv_dtype, s.bits, s.alpha_key, f.eps, &p.thr_k))) return rc;
+    if ((rc = mz_get_unit_thresholds(s.kv_dtype, s.bits, s.alpha_value, f.eps, &p.thr_v))) return rc;
+    if (!p.thr_k || !p.thr_v) return MZ_OK;
+  }
+  const int tpt = s.group == 128 ? 32 : 16, per_cta = 256 / ((s.head_dim / 2) * (s.group / tpt));
+  const long long pairs = (long long)s.batch * s.kv_heads, tiles = pairs * p.n_tiles;
+  const int rows_per_cta = 256 / (s.group / 16);
+  p.v_blocks_per_pair = (unsigned)(((long long)p.n_vtokens * (s.head_dim / s.group) + rows_per_cta - 1) / rows_per_cta);
+  const long long kb = (tiles + per_cta - 1) / per_cta, vb = pairs * p.v_blocks_per_pair;
+  if (tiles >= (1LL << 31) || kb + vb >= (1LL << 31)) return MZ_OK;
+  p.tiles = (unsigned)tiles; p.n_k_blocks = (unsigned)kb;
+  *done = 1;
+  return s.kv_dtype == MZ_BF16 ? launch_flush16_bits<MZ_BF16>(p, (unsigned)(kb + vb), st) : launch_flush16_bits<MZ_F16>(p, (unsigned)(kb + vb), st);
+}
 }  // namespace
 
 extern "C" int mz_flush_kv_parts(const mz_kv_store* s, int n_key_tokens, int value_first, int n_value_tokens, float eps,
@@ -302,6 +600,10 @@ extern "C" int mz_flush_kv_parts(const mz_kv_store* s, int n_key_tokens, int val
   p.v_fast = pow2(g.G) && g.G >= 8 && g.G <= 256 && g.D % 8 == 0;
   p.k_vec = g.D % 8 == 0 && s->res_stride_t % 8 == 0 && s->res_stride_h % 8 == 0 && s->res_stride_b % 8 == 0 &&
             (uintptr_t)s->res_k % 16 == 0 && (uintptr_t)s->res_v % 16 == 0;
+  if (flush16_serves(*s, p)) {
+    int done = 0;
+    if ((rc = flush16(*s, p, (cudaStream_t)stream, &done)) || done) return rc;
+  }
   const int rows_per_cta = p.v_fast ? 256 / (g.G / 8) : 8;
   const long long vb = (p.v_rows + rows_per_cta - 1) / rows_per_cta;
   MZ_REQUIRE(kb + vb < (1LL << 31), "flush too large");

@@ -1,0 +1,43 @@
+"""GPU: the packed quantizer, the dense read-back, the fp32 quantizer and the alpha statistics against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import bits16
+
+pytestmark = pytest.mark.gpu
+
+
+def _block(oracle, B, KVH, S, D, dtype, seed):
+    """K / V with rows at the edges of the quantizer: constant, one-sided (anchor 0 and 1), tiny."""
+    k, v, _ = oracle.synth_kv(B, KVH, S, D, KVH, seed=seed)
+    k, v = k.float().clamp(-6e4, 6e4), v.float()
+    k[0, 0, :, 0], k[0, 0, :, 1], k[0, 0, :, 2] = 1.5, k[0, 0, :, 1].abs() + 0.1, -k[0, 0, :, 2].abs() - 0.1
+    k[0, 0, :, 3] *= 1e-4
+    v[0, 0, 1], v[0, 0, 2], v[0, 0, 3] = -2.0, v[0, 0, 2].abs() + 0.1, -v[0, 0, 3].abs() - 0.1
+    if dtype == torch.float16:       # a zero range is NaN in the reference at fp16
+        k[0, 0, :, 0] += torch.arange(S) % 2
+        v[0, 0, 1] += torch.arange(D) % 2
+    return k.to(dtype), v.to(dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D,group", [(64, 32), (64, 64), (128, 32), (128, 64), (128, 128)])
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 5, 7, 8])
+def test_flush_and_read_back(oracle, bits, D, group, dtype):
+    import muzero_b200 as mz
+    S = 128 + 3 * group + 5
+    k, v = _block(oracle, 1, 3, S, D, dtype, seed=bits + group)
+    ref = oracle.OracleCacheLayer(bits=bits, group=group, residual=128)
+    ref.append(k, v)
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=group, residual_length=128)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda().transpose(1, 2).contiguous().transpose(1, 2), v.cuda().transpose(1, 2).contiguous().transpose(1, 2),
+                 {"materialize_full_kv": False})
+    assert [layer._selected_alpha_key, layer._selected_alpha_value] == [ref.alpha_key, ref.alpha_value]
+    for mine, theirs in ((layer._key_mn, ref.k_mn), (layer._key_scale, ref.k_scale), (layer._value_mn, ref.v_mn),
+                         (layer._value_scale, ref.v_scale)):
+        assert np.array_equal(bits16(mine), bits16(theirs))
+    assert torch.equal(layer._packed_key_q.cpu(), ref.packed_k)
+    assert torch.equal(layer._packed_value_q.cpu(), ref.packed_v)
