@@ -75,6 +75,20 @@ int mz_dequantize_rows(const uint8_t* packed, const void* mn, const void* scale,
                        void* out, int out_dtype, void* stream);
 
 /*
+ * Statistics of a 16-bit block x[B,H,S,D] (shape[4], element strides[3] of the first three dimensions, innermost
+ * contiguous) from which the compander alpha is chosen.  want & 1: stats[0..2] = the 50 / 95 / 99 % order statistics
+ * of |x| over at most max_points strided samples (rank max(1, floor(p * n))); want & 2: stats[3] = mean over all
+ * groups of |zero anchor - 0.5|.  keys = 1: groups run along tokens, 0: along channels (both zero-padded to whole
+ * groups).  rows_order: element order that the sample strides through: 1 = the rows of the key store (whole groups
+ * only), 0 = natural with channels padded to whole groups (keys = 0), -1 = natural.  `stats` is on the device; so
+ * is `workspace`, zeroed by the caller once and kept for one stream (each call leaves it as it found it).
+ * Replaces: the torch statistics of select_alpha, muzero/quantizer.py:29-112.
+ */
+int mz_alpha_stats(const void* block, int dtype, const int* shape, const long long* strides, int group, int keys,
+                   int rows_order, int max_points, int want, void* workspace, float* stats, void* stream);
+size_t mz_alpha_stats_workspace_bytes(void);
+
+/*
  * The quantized store of one layer plus its dense residual window.
  * Layouts (reference: muzero/cache/layer.py:271-301):
  *   packed_k [B,KVH,k_group_cap,D,QB] u8     row = G consecutive tokens of one channel

@@ -28,7 +28,8 @@ from ..config import MuZeroConfig
 from ..kernels import _cabi
 from ..kernels._cabi import KVStore, MuZeroKernelError, check, dtype_code, stream_ptr
 from ..kernels.loader import ensure_expand_table, load_mu_zero_cuda_extension
-from ..quantizer import _magnitude_ratios, _anchor_offset, alpha_from_stats, select_alpha_key_block
+from ..quantizer import (_anchor_offset, _magnitude_ratios, _on_device, _statistics_needed, alpha_from_stats, device_alphas,
+                         select_alpha_key_block)
 from .policy import grown_capacity, plan_flush, residual_capacity
 
 _STORE_ATTRS = ("_packed_key_q", "_key_mn", "_key_scale", "_packed_value_q", "_value_mn", "_value_scale")
@@ -308,10 +309,18 @@ class MuZeroCacheLayer:
     def _ensure_alpha(self, n_flush: int, n_values: Optional[int] = None) -> None:
         n_values = n_flush if n_values is None else n_values
         g, bits, mp = self.q_group_size, self.nbits, self.cfg.stats_max_points
-        if self._selected_alpha_key is None and n_flush > 0:
+        want_k = self._selected_alpha_key is None and n_flush > 0
+        want_v = self._selected_alpha_value is None and n_values > 0
+        if want_k and want_v and _on_device(self.keys) and _on_device(self.values):
+            # both choices from one read-back
+            self._selected_alpha_key, self._selected_alpha_value = device_alphas(
+                [(self.keys[:, :, :n_flush], "key", 1), (self.values[:, :, :n_values], "value", 0)], bits=bits, q_group_size=g,
+                max_points=mp)
+            return
+        if want_k:
             self._selected_alpha_key = select_alpha_key_block(self.keys[:, :, :n_flush], bits=bits, q_group_size=g,
                                                               max_points=mp)
-        if self._selected_alpha_value is None and n_values > 0:
+        if want_v:
             self._selected_alpha_value = _select_alpha_value_block(self.values[:, :, :n_values], bits=bits, group=g,
                                                                    d_pad=self.v_head_dim_padded, max_points=mp)
 
@@ -625,8 +634,10 @@ def _side_stream(device: torch.device) -> "torch.cuda.Stream":
 def _select_alpha_value_block(block: torch.Tensor, *, bits: int, group: int, d_pad: int, max_points: int) -> float:
     """``select_alpha(rows, kind="value")`` for the rows [B*KVH*S*NG, G] of a value block
     [B,KVH,S,D] (channels zero-padded to ``d_pad``), sampling through index arithmetic."""
-    if bits == 4:
+    if not _statistics_needed(bits, "value"):
         return 2.0
+    if _on_device(block):
+        return device_alphas([(block, "value", 0)], bits=bits, q_group_size=group, max_points=max_points)[0]
     b, h, s, d = block.shape
     total = b * h * s * d_pad
     if total > max_points:

@@ -23,6 +23,7 @@ EXPORTS = (
     "mz_flush_kv", "mz_append_kv", "mz_dequantize_kv", "mz_decode_workspace_bytes", "mz_decode_attention",
     "mz_decode_attention_partial", "mz_lse_merge", "mz_qk_logits", "mz_av_output", "mz_decode_attention_static",
     "mz_decode_step", "mz_decode_step_workspace_bytes", "mz_flush_kv_parts", "mz_decode_workspace_bound", "mz_decode_attention_partial_packed", "mz_lse_merge_packed", "mz_store_gather_batch", "mz_debug_force_kernel", "mz_bounds_violations",
+    "mz_alpha_stats", "mz_alpha_stats_workspace_bytes",
 )
 
 
@@ -110,6 +111,10 @@ def load_library() -> ctypes.CDLL:
     lib.mz_debug_force_kernel.restype = c_int
     lib.mz_bounds_violations.argtypes = [ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(c_int), c_int]
     lib.mz_bounds_violations.restype = ctypes.c_longlong
+    lib.mz_alpha_stats.argtypes = [c_void_p, c_int, POINTER(c_int), POINTER(c_longlong), c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                   c_void_p, c_void_p]
+    lib.mz_alpha_stats_workspace_bytes.argtypes = []
+    lib.mz_alpha_stats_workspace_bytes.restype = c_size_t
     lib.mz_qk_logits.argtypes = [POINTER(KVStore), c_void_p, c_longlong, c_longlong, c_int, c_float, c_void_p, c_int, c_void_p]
     lib.mz_av_output.argtypes = [POINTER(KVStore), c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p]
     _lib = lib

@@ -8,12 +8,15 @@ Alpha selection is a one-time statistic per layer and stays in torch.
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional
 
 import torch
 import torch.nn.functional as F
 
-from .kernels.loader import MuZeroKernelError, mu_zero_dequantize_cuda, mu_zero_quantize_cuda
+from .kernels._cabi import check, dtype_code, stream_ptr
+from .kernels.loader import (MuZeroKernelError, load_mu_zero_cuda_extension, mu_zero_dequantize_cuda,
+                             mu_zero_quantize_cuda)
 
 _TINY = 1e-8
 
@@ -38,6 +41,83 @@ def alpha_from_stats(*, bits: int, kind: str, tail_ratio: float, concentration_r
     if bits == 3 and tail_ratio > 2.3 and anchor_offset > 0.12:
         return 4.0
     return 2.0
+
+
+def _statistics_needed(bits: int, kind: str) -> int:
+    """Which statistics the decision table reads for (bits, kind): 1 = magnitude ratios, 2 = anchor offset.  Most
+    code widths have one alpha whatever the data is."""
+    if kind == "key":
+        return {1: 3, 8: 1}.get(bits, 0)
+    return 3 if bits >= 8 else 1 if bits == 3 else 0
+
+
+def _anchor_decides(bits: int, kind: str, tail: float, conc: float) -> bool:
+    """Whether the anchor offset can still change the choice once the magnitude ratios are known."""
+    if not _statistics_needed(bits, kind):
+        return False
+    a, b = (alpha_from_stats(bits=bits, kind=kind, tail_ratio=tail, concentration_ratio=conc, anchor_offset=off)
+            for off in (0.0, 0.5))
+    return a != b
+
+
+_stat_workspaces: dict = {}
+
+
+def _stat_workspace(device: torch.device) -> torch.Tensor:
+    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    ws = _stat_workspaces.get(key)
+    if ws is None:
+        if len(_stat_workspaces) >= 64:      # streams come and go
+            _stat_workspaces.clear()
+        ws = torch.zeros(load_mu_zero_cuda_extension().mz_alpha_stats_workspace_bytes(), dtype=torch.uint8, device=device)
+        _stat_workspaces[key] = ws
+    return ws
+
+
+def device_alphas(requests: list, *, bits: int, q_group_size: int, max_points: int) -> list:
+    """Alphas of 16-bit CUDA blocks [B,H,S,D] (innermost contiguous): ``requests`` holds (block, kind, sample order)
+    with the orders of ``mz_alpha_stats``.  The statistics of all requests are read back with one copy."""
+    lib = load_mu_zero_cuda_extension()
+    out: list = [None] * len(requests)
+    stats: list = [None] * len(requests)
+
+    def launch(todo: list) -> None:
+        dev = requests[todo[0][0]][0].device
+        buf = torch.empty((len(todo), 4), dtype=torch.float32, device=dev)
+        ws, st = _stat_workspace(dev), stream_ptr(dev)
+        with torch.cuda.device(dev):
+            for row, (i, want) in enumerate(todo):
+                block, kind, order = requests[i]
+                check(lib.mz_alpha_stats(block.data_ptr(), dtype_code(block.dtype), (ctypes.c_int * 4)(*block.shape),
+                                         (ctypes.c_longlong * 3)(*block.stride()[:3]), q_group_size, int(kind == "key"), order,
+                                         max_points, want, ws.data_ptr(), buf.data_ptr() + 16 * row, st), "mz_alpha_stats")
+        for (i, want), got in zip(todo, buf.tolist()):
+            stats[i] = (got[:3] if want & 1 else stats[i][:3]) + [got[3] if want & 2 else None]
+
+    todo = []
+    for i, (_, kind, _) in enumerate(requests):
+        want = _statistics_needed(bits, kind)
+        if want:
+            todo.append((i, want))
+        else:
+            out[i] = alpha_from_stats(bits=bits, kind=kind, tail_ratio=0.0, concentration_ratio=0.0, anchor_offset=0.0)
+    while todo:
+        launch(todo)
+        again = []
+        for i, _ in todo:
+            kind = requests[i][1]
+            p50, p95, p99, off = stats[i]
+            tail, conc = p99 / max(p95, _TINY), p95 / max(p50, _TINY)
+            if off is None and _anchor_decides(bits, kind, tail, conc):
+                again.append((i, 2))
+            else:
+                out[i] = alpha_from_stats(bits=bits, kind=kind, tail_ratio=tail, concentration_ratio=conc, anchor_offset=off or 0.0)
+        todo = again
+    return out
+
+
+def _on_device(block: torch.Tensor) -> bool:
+    return block.is_cuda and block.dtype in (torch.bfloat16, torch.float16) and block.dim() == 4 and block.stride(-1) == 1
 
 
 def _magnitude_ratios(sample: torch.Tensor) -> tuple[float, float]:
@@ -67,11 +147,15 @@ def _anchor_offset(groups: torch.Tensor) -> float:
 
 def select_alpha(tensor: torch.Tensor, *, bits: int, q_group_size: int, kind: str,
                  max_points: int = 65536) -> float:
-    """Log-compander alpha for ``tensor`` ([N,G] rows or [B,H,S,D]); always 2.0 for 4 bits."""
-    if bits == 4:
+    """Log-compander alpha for ``tensor`` ([N,G] rows or [B,H,S,D]); always 2.0 where the decision table has one value."""
+    if not _statistics_needed(bits, kind):
         return 2.0
+    if _on_device(tensor) and (kind == "key" or tensor.shape[3] % q_group_size == 0):
+        return device_alphas([(tensor, kind, -1)], bits=bits, q_group_size=q_group_size, max_points=max_points)[0]
     work = tensor.float()
     tail, conc = _magnitude_ratios(_strided_sample(work.reshape(-1), max_points))
+    if not _anchor_decides(bits, kind, tail, conc):
+        return alpha_from_stats(bits=bits, kind=kind, tail_ratio=tail, concentration_ratio=conc, anchor_offset=0.0)
     if work.dim() == 2:
         rows, width = work.shape
         if width != q_group_size:
@@ -94,8 +178,10 @@ def select_alpha_key_block(block: torch.Tensor, *, bits: int, q_group_size: int,
     [B,KVH,nsg*G,D], without materialising the transposed rows: the strided sample is
     gathered through the row index arithmetic and the group min/max reduce over the token axis.
     """
-    if bits == 4:
+    if not _statistics_needed(bits, "key"):
         return 2.0
+    if _on_device(block):
+        return device_alphas([(block, "key", 1)], bits=bits, q_group_size=q_group_size, max_points=max_points)[0]
     b, h, s, d = block.shape
     g = q_group_size
     nsg = s // g

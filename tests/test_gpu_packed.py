@@ -41,3 +41,17 @@ def test_flush_and_read_back(oracle, bits, D, group, dtype):
         assert np.array_equal(bits16(mine), bits16(theirs))
     assert torch.equal(layer._packed_key_q.cpu(), ref.packed_k)
     assert torch.equal(layer._packed_value_q.cpu(), ref.packed_v)
+
+
+@pytest.mark.parametrize("power,shift,group", [(1, 0.0, 64), (3, 0.0, 32), (1, 1.0, 64)])
+def test_alpha_statistics(oracle, power, shift, group):
+    from muzero_b200.quantizer import device_alphas, select_alpha
+    k, _ = _block(oracle, 2, 3, 4 * group, 128, torch.bfloat16, seed=group)
+    k = (k.float() ** power + shift).to(torch.bfloat16)
+    for bits in (1, 3, 8):
+        want = [oracle.select_alpha_oracle(oracle.key_rows(k, group), bits=bits, group=group, kind="key", max_points=5000),
+                oracle.select_alpha_oracle(oracle.value_rows(k, group), bits=bits, group=group, kind="value", max_points=5000)]
+        assert device_alphas([(k.cuda(), "key", 1), (k.cuda(), "value", 0)], bits=bits, q_group_size=group, max_points=5000) == want
+        for kind in ("key", "value"):
+            assert select_alpha(k.cuda(), bits=bits, q_group_size=group, kind=kind) == \
+                oracle.select_alpha_oracle(k, bits=bits, group=group, kind=kind)
