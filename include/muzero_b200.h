@@ -157,6 +157,15 @@ int mz_dequantize_kv(const mz_kv_store* store, int g0, int g1, void* out_k,
                      int t0, int t1, void* out_v, int out_dtype, float eps, void* stream);
 
 /*
+ * The whole cache as dense tensors in one launch: the packed prefix dequantized as by mz_dequantize_kv, followed by
+ * the residual window (values: its rows from v_tokens - k_groups * group on).  out_k [B,KVH,k_groups*G+res_len,D],
+ * out_v [B,KVH,k_groups*G+res_len,D], contiguous, out_dtype.
+ * Replaces: the dequantization and the concatenation of update() for callers without the fused decode path,
+ * muzero/cache/layer.py:303-345,440-459.
+ */
+int mz_materialize_kv(const mz_kv_store* store, void* out_k, void* out_v, int out_dtype, float eps, void* stream);
+
+/*
  * Re-indexes a whole layer cache along the batch in one launch: entry i of dst takes entry index[i] of
  * src (index: int64 on the device), for the valid part of all eight tensors (packed codes and metadata
  * of keys and values, residual window).  dst has the same shape parameters, its own buffers with the

@@ -499,6 +499,20 @@ class MuZeroCacheLayer:
 
     # ------------------------------------------------------ cache management
     def _full_kv(self) -> tuple[torch.Tensor, torch.Tensor]:
+        if self._key_group_count and self._value_storage_len:
+            # prefix and window written side by side in one launch
+            self._require_device_path()
+            ensure_expand_table(self.nbits, self._selected_alpha_key, self.device)
+            ensure_expand_table(self.nbits, self._selected_alpha_value, self.device)
+            s = self._store_struct()
+            shape = (s.batch, s.kv_heads, s.k_groups * s.group + s.res_len, self.k_head_dim)
+            k = torch.empty(shape, dtype=self.dtype, device=self.device)
+            v = torch.empty(shape, dtype=self.dtype, device=self.device)
+            with torch.cuda.device(self.device):
+                check(load_mu_zero_cuda_extension().mz_materialize_kv(
+                    ctypes.byref(s), k.data_ptr(), v.data_ptr(), dtype_code(self.dtype), self.amax_eps, stream_ptr(self.device)),
+                    "mz_materialize_kv")
+            return k, v
         k = torch.cat([self._dequantize_key_prefix(), self.keys], dim=2) if self._key_group_count else self.keys
         v = torch.cat([self._dequantize_value_prefix(), self.values], dim=2) if self._value_storage_len else self.values
         return k, v

@@ -475,54 +475,6 @@ __global__ void append_kv_kernel(const mz_kv_store s, const uint16_t* __restrict
   ((uint16_t*)s.res_v)[dst] = v_new[src];
 }
 
-// store -> dense.  Keys: thread = (octet of tokens, channel) with channel fastest so that
-// the 8 writes of a warp are contiguous; values: thread = (token, group, octet of channels).
-__global__ void __launch_bounds__(256) dequant_keys_kernel(const mz_kv_store s, int g0, int g1, int QB, float eps,
-                                                           const float* __restrict__ table, void* __restrict__ out, int out_dt) {
-  const int G = s.group, D = s.head_dim, octs = (G + 7) >> 3, top = (1 << s.bits) - 1;
-  const long long per_bh = (long long)(g1 - g0) * octs * D;
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= per_bh * s.batch * s.kv_heads) return;
-  const int d = (int)(i % D); i /= D;
-  const int oct = (int)(i % octs); i /= octs;
-  const int g = g0 + (int)(i % (g1 - g0)); i /= (g1 - g0);
-  const int h = (int)(i % s.kv_heads);
-  const int b = (int)(i / s.kv_heads);
-  const long long m = b * s.km_stride_b + h * s.km_stride_h + (long long)g * D + d;
-  const MzRowParams r = mz_row_params(mz_load_as_float(s.k_mn, m, s.meta_dtype), mz_load_as_float(s.k_scale, m, s.meta_dtype), top, eps);
-  const uint8_t* row = s.packed_k + b * s.pk_stride_b + h * s.pk_stride_h + ((long long)g * D + d) * QB;
-  const long long S = (long long)(g1 - g0) * G;
-  const long long o0 = (((long long)b * s.kv_heads + h) * S + (long long)(g - g0) * G + oct * 8) * D + d;
-  const int n = min(8, G - oct * 8);
-  for (int k = 0; k < n; ++k) {
-    const int q = mz_extract_code(row, oct * 8 + k, s.bits, QB);
-    mz_store_from_float(out, o0 + (long long)k * D, mz_dequant_exact(r, q, table, top + 1), out_dt);
-  }
-}
-
-__global__ void __launch_bounds__(256) dequant_values_kernel(const mz_kv_store s, int t0, int t1, int QB, int NG, float eps,
-                                                             const float* __restrict__ table, void* __restrict__ out, int out_dt) {
-  const int G = s.group, D = s.head_dim, octs = (G + 7) >> 3, top = (1 << s.bits) - 1;
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)s.batch * s.kv_heads * (t1 - t0) * NG * octs;
-  if (i >= total) return;
-  const int oct = (int)(i % octs); i /= octs;
-  const int grp = (int)(i % NG); i /= NG;
-  const int t = t0 + (int)(i % (t1 - t0)); i /= (t1 - t0);
-  const int h = (int)(i % s.kv_heads);
-  const int b = (int)(i / s.kv_heads);
-  const long long m = b * s.vm_stride_b + h * s.vm_stride_h + (long long)t * NG + grp;
-  const MzRowParams r = mz_row_params(mz_load_as_float(s.v_mn, m, s.meta_dtype), mz_load_as_float(s.v_scale, m, s.meta_dtype), top, eps);
-  const uint8_t* row = s.packed_v + b * s.pv_stride_b + h * s.pv_stride_h + ((long long)t * NG + grp) * QB;
-  const long long o0 = (((long long)b * s.kv_heads + h) * (t1 - t0) + (t - t0)) * D;
-  for (int k = 0; k < 8; ++k) {
-    const int idx = oct * 8 + k, c = grp * G + idx;
-    if (idx >= G || c >= D) break;
-    const int q = mz_extract_code(row, idx, s.bits, QB);
-    mz_store_from_float(out, o0 + c, mz_dequant_exact(r, q, table, top + 1), out_dt);
-  }
-}
-
 bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
 bool flush16_serves(const mz_kv_store& s, const FlushParams& p) {
@@ -644,33 +596,5 @@ extern "C" int mz_append_kv(const mz_kv_store* s, const void* k_new, const void*
   cfg.numAttrs = 1;
   MZ_CUDA(cudaLaunchKernelEx(&cfg, append_kv_kernel, *s, (const uint16_t*)k_new, (const uint16_t*)v_new, nsb, nsh));
   MZ_LAUNCH_CHECK("append_kv");
-  return MZ_OK;
-}
-
-extern "C" int mz_dequantize_kv(const mz_kv_store* s, int g0, int g1, void* out_k, int t0, int t1, void* out_v, int out_dtype,
-                                float eps, void* stream) {
-  MZ_RANGE("mz_dequantize_kv");
-  int rc = mz_check_store_basic(s);
-  if (rc) return rc;
-  if ((rc = mz_check_store_quantized(s))) return rc;
-  MZ_REQUIRE(mz_dtype_ok(out_dtype), "bad out_dtype");
-  const MzStoreGeom g = mz_geom(*s);
-  cudaStream_t st = (cudaStream_t)stream;
-  if (out_k && g1 > g0) {
-    MZ_REQUIRE(g0 >= 0 && g1 <= s->k_groups, "key group range [%d,%d) outside [0,%d)", g0, g1, s->k_groups);
-    const float* table;
-    if ((rc = mz_get_expand_table(g.bits, s->alpha_key, &table))) return rc;
-    const long long n = (long long)g.B * g.KVH * (g1 - g0) * ((g.G + 7) / 8) * g.D;
-    dequant_keys_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(*s, g0, g1, g.QB, eps, table, out_k, out_dtype);
-    MZ_LAUNCH_CHECK("dequant_keys");
-  }
-  if (out_v && t1 > t0) {
-    MZ_REQUIRE(t0 >= 0 && t1 <= s->v_tokens, "value token range [%d,%d) outside [0,%d)", t0, t1, s->v_tokens);
-    const float* table;
-    if ((rc = mz_get_expand_table(g.bits, s->alpha_value, &table))) return rc;
-    const long long n = (long long)g.B * g.KVH * (t1 - t0) * g.NG * ((g.G + 7) / 8);
-    dequant_values_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(*s, t0, t1, g.QB, g.NG, eps, table, out_v, out_dtype);
-    MZ_LAUNCH_CHECK("dequant_values");
-  }
   return MZ_OK;
 }

@@ -41,6 +41,9 @@ def test_flush_and_read_back(oracle, bits, D, group, dtype):
         assert np.array_equal(bits16(mine), bits16(theirs))
     assert torch.equal(layer._packed_key_q.cpu(), ref.packed_k)
     assert torch.equal(layer._packed_value_q.cpu(), ref.packed_v)
+    full_k, full_v = layer._full_kv()
+    assert np.array_equal(bits16(full_k), bits16(torch.cat([ref.key_prefix(dtype), ref.keys], dim=2)))
+    assert np.array_equal(bits16(full_v), bits16(torch.cat([ref.value_prefix(dtype), ref.values], dim=2)))
 
 
 @pytest.mark.parametrize("power,shift,group", [(1, 0.0, 64), (3, 0.0, 32), (1, 1.0, 64)])
