@@ -3,8 +3,10 @@
 // Fast path (G a power of two, 8..256): G/8 lanes own one row, each lane owns
 // 8 consecutive values = one 16-byte load of 16-bit input and exactly `bits`
 // packed bytes; the row min/max is a shuffle reduction over those lanes.
+// 16-bit rows of 16 to 256 values take the packed quantizer (mz_quant16.cuh), 16 values per lane.
 // Any other G takes the warp-per-row kernel.
-#include "mz_quant_math.cuh"
+#include "mz_quant16.cuh"
+#include "mz_quant_f32.cuh"
 
 namespace {
 
@@ -49,16 +51,61 @@ __global__ void __launch_bounds__(256) quantize_rows_octet_kernel(
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
   }
   if (!live) return;
-  MzQuantRow<DT> r;
-  r.setup(mn, mx, bits, alpha, eps, ctab, ctab_n);
   unsigned long long word = 0;
+  float lo, span;
+  if (DT == MZ_F32) {
+    mzq::F32Row r;
+    r.set(mn, mx, bits, alpha, eps);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) word |= ((unsigned long long)r.code(v[i])) << (i * bits);
+    for (int i = 0; i < 8; ++i) word |= ((unsigned long long)r.code(v[i], mn, mx, bits, alpha, eps)) << (i * bits);
+    lo = r.lo; span = r.span;
+  } else {
+    MzQuantRow<DT> r;
+    r.setup(mn, mx, bits, alpha, eps, ctab, ctab_n);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) word |= ((unsigned long long)r.code(v[i])) << (i * bits);
+    lo = r.lo; span = r.span;
+  }
   mz_store_octet(packed + row * (long long)(lpr * bits) + sub * bits, word, bits);
   if (sub == 0) {
-    mz_store_from_float(mn_out, row, r.lo, meta_dtype);
-    mz_store_from_float(scale_out, row, r.span, meta_dtype);
+    mz_store_from_float(mn_out, row, lo, meta_dtype);
+    mz_store_from_float(scale_out, row, span, meta_dtype);
   }
+}
+
+// 16-bit rows, 16 values per lane (chunks sub and sub + lpr of eight)
+template <int DT, int BITS>
+__global__ void __launch_bounds__(256) quantize_rows16_kernel(const uint16_t* __restrict__ x, long long n_rows, int group, float alpha,
+                                                              float eps, uint8_t* __restrict__ packed, void* __restrict__ mn_out,
+                                                              void* __restrict__ scale_out, int meta_dtype, const uint16_t* __restrict__ thr,
+                                                              const uint16_t* __restrict__ ctab, int ctab_n) {
+  const int lpr = group >> 4, sub = threadIdx.x % lpr;
+  const long long row = (long long)blockIdx.x * (256 / lpr) + threadIdx.x / lpr;
+  const bool live = row < n_rows;
+  uint32_t v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (live) {
+    const uint16_t* src = x + row * group + sub * 8;
+    const uint4 a = *(const uint4*)src, c = *(const uint4*)(src + lpr * 8);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+  }
+  mzq::RowHead<DT> head;
+  unsigned long long word[2];
+  mzq::quantize_row16<DT, BITS>(v, lpr, alpha, eps, thr, ctab, ctab_n, head, word);
+  if (!live) return;
+  uint8_t* dst = packed + row * (long long)(group * BITS / 8) + sub * BITS;
+  mz_store_octet(dst, word[0], BITS);
+  mz_store_octet(dst + lpr * BITS, word[1], BITS);
+  if (sub == 0) {
+    mz_store_from_float(mn_out, row, head.lo, meta_dtype);
+    mz_store_from_float(scale_out, row, head.span, meta_dtype);
+  }
+}
+template <int DT, int BITS>
+void launch_rows16(const void* x, long long n_rows, int group, float alpha, float eps, uint8_t* packed, void* mn, void* scale, int meta_dtype,
+                   const uint16_t* thr, const uint16_t* ctab, int ctab_n, cudaStream_t st) {
+  const int rows_per_cta = 256 / (group >> 4);
+  quantize_rows16_kernel<DT, BITS><<<(unsigned)((n_rows + rows_per_cta - 1) / rows_per_cta), 256, 0, st>>>(
+      (const uint16_t*)x, n_rows, group, alpha, eps, packed, mn, scale, meta_dtype, thr, ctab, ctab_n);
 }
 
 // any G <= 1024: one warp per row, codes staged in shared memory
@@ -121,6 +168,29 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(
   }
 }
 
+// groups of whole octets: one octet per thread, packed bytes and outputs as vectors
+template <int OUT>
+__global__ void __launch_bounds__(256) dequantize_octets_kernel(
+    const uint8_t* __restrict__ packed, const void* __restrict__ mn, const void* __restrict__ scale, int meta_dtype,
+    long long n_oct, int octets, int bits, float eps, const float* __restrict__ table, void* __restrict__ out) {
+  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= n_oct) return;
+  const long long row = n_oct < (1LL << 31) ? (long long)((unsigned)gid / (unsigned)octets) : gid / octets;
+  const int top = (1 << bits) - 1;
+  const MzRowParams r = mz_row_params(mz_load_as_float(mn, row, meta_dtype), mz_load_as_float(scale, row, meta_dtype), top, eps);
+  const unsigned long long w = mz_load_octet(packed + gid * bits, bits);
+  float v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = mz_dequant_exact(r, (int)(w >> (i * bits)) & top, table, top + 1);
+  if (OUT == MZ_F32) {
+    ((float4*)out)[2 * gid] = make_float4(v[0], v[1], v[2], v[3]);
+    ((float4*)out)[2 * gid + 1] = make_float4(v[4], v[5], v[6], v[7]);
+  } else {
+    using P = mzq::P2<OUT == MZ_F32 ? MZ_BF16 : OUT>;
+    ((uint4*)out)[gid] = make_uint4(P::pack(v[0], v[1]), P::pack(v[2], v[3]), P::pack(v[4], v[5]), P::pack(v[6], v[7]));
+  }
+}
+
 bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
 template <int DT>
@@ -133,6 +203,26 @@ int launch_quantize(const void* x, long long n_rows, int group, int bits, float 
     if (rc != MZ_OK) return rc;
   }
   const bool aligned = ((uintptr_t)x % 16 == 0) && ((uintptr_t)packed % 8 == 0);
+  const uint16_t* thr = nullptr;
+  if (DT != MZ_F32 && pow2(group) && group >= 16 && group <= 256 && aligned) {
+    int rc = mz_get_unit_thresholds(DT, bits, alpha, eps, &thr);
+    if (rc != MZ_OK) return rc;
+    if (bits > 4 || thr) {
+      constexpr int T = DT == MZ_F32 ? MZ_BF16 : DT;       // never instantiated for fp32 rows' launch
+      switch (bits) {
+        case 1: launch_rows16<T, 1>(x, n_rows, group, alpha, eps, packed, mn, scale, meta_dtype, thr, ctab, ctab_n, st); break;
+        case 2: launch_rows16<T, 2>(x, n_rows, group, alpha, eps, packed, mn, scale, meta_dtype, thr, ctab, ctab_n, st); break;
+        case 3: launch_rows16<T, 3>(x, n_rows, group, alpha, eps, packed, mn, scale, meta_dtype, thr, ctab, ctab_n, st); break;
+        case 4: launch_rows16<T, 4>(x, n_rows, group, alpha, eps, packed, mn, scale, meta_dtype, thr, ctab, ctab_n, st); break;
+        case 5: launch_rows16<T, 5>(x, n_rows, group, alpha, eps, packed, mn, scale, meta_dtype, thr, ctab, ctab_n, st); break;
+        case 6: launch_rows16<T, 6>(x, n_rows, group, alpha, eps, packed, mn, scale, meta_dtype, thr, ctab, ctab_n, st); break;
+        case 7: launch_rows16<T, 7>(x, n_rows, group, alpha, eps, packed, mn, scale, meta_dtype, thr, ctab, ctab_n, st); break;
+        default: launch_rows16<T, 8>(x, n_rows, group, alpha, eps, packed, mn, scale, meta_dtype, thr, ctab, ctab_n, st); break;
+      }
+      MZ_LAUNCH_CHECK("quantize_rows16");
+      return MZ_OK;
+    }
+  }
   if (pow2(group) && group >= 8 && group <= 256 && aligned) {
     const int rows_per_cta = 256 / (group / 8);
     const long long blocks = (n_rows + rows_per_cta - 1) / rows_per_cta;
@@ -182,6 +272,12 @@ extern "C" int mz_dequantize_rows(const uint8_t* packed, const void* mn, const v
   const long long threads = n_rows * ((group + 7) / 8);
   const long long blocks = (threads + 255) / 256;
   MZ_REQUIRE(blocks < (1LL << 31), "problem too large");
+  if (group % 8 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)packed % 8 == 0) {
+    auto kern = out_dtype == MZ_F32 ? dequantize_octets_kernel<MZ_F32> : out_dtype == MZ_F16 ? dequantize_octets_kernel<MZ_F16> : dequantize_octets_kernel<MZ_BF16>;
+    kern<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(packed, mn, scale, meta_dtype, threads, group / 8, bits, eps, table, out);
+    MZ_LAUNCH_CHECK("dequantize_octets");
+    return MZ_OK;
+  }
   dequantize_rows_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(packed, mn, scale, meta_dtype, n_rows, group, bits,
                                                                            eps, table, out, out_dtype);
   MZ_LAUNCH_CHECK("dequantize_rows");

@@ -23,7 +23,7 @@ EXPORTS = (
     "mz_flush_kv", "mz_append_kv", "mz_dequantize_kv", "mz_decode_workspace_bytes", "mz_decode_attention",
     "mz_decode_attention_partial", "mz_lse_merge", "mz_qk_logits", "mz_av_output", "mz_decode_attention_static",
     "mz_decode_step", "mz_decode_step_workspace_bytes", "mz_flush_kv_parts", "mz_decode_workspace_bound", "mz_decode_attention_partial_packed", "mz_lse_merge_packed", "mz_store_gather_batch", "mz_debug_force_kernel", "mz_bounds_violations",
-    "mz_alpha_stats", "mz_alpha_stats_workspace_bytes", "mz_materialize_kv",
+    "mz_alpha_stats", "mz_alpha_stats_workspace_bytes", "mz_materialize_kv", "mz_roundtrip_kv",
 )
 
 
@@ -112,6 +112,8 @@ def load_library() -> ctypes.CDLL:
     lib.mz_bounds_violations.argtypes = [ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(c_int), c_int]
     lib.mz_bounds_violations.restype = ctypes.c_longlong
     lib.mz_materialize_kv.argtypes = [POINTER(KVStore), c_void_p, c_void_p, c_int, c_float, c_void_p]
+    lib.mz_roundtrip_kv.argtypes = [c_void_p, c_int, POINTER(c_int), POINTER(c_longlong), c_int, c_int, c_float, c_float, c_int, c_int,
+                                    c_void_p, c_void_p]
     lib.mz_alpha_stats.argtypes = [c_void_p, c_int, POINTER(c_int), POINTER(c_longlong), c_int, c_int, c_int, c_int, c_int, c_void_p,
                                    c_void_p, c_void_p]
     lib.mz_alpha_stats_workspace_bytes.argtypes = []

@@ -15,7 +15,7 @@ import torch
 import torch.nn.functional as F
 
 from .kernels._cabi import check, dtype_code, stream_ptr
-from .kernels.loader import (MuZeroKernelError, load_mu_zero_cuda_extension, mu_zero_dequantize_cuda,
+from .kernels.loader import (MuZeroKernelError, ensure_expand_table, load_mu_zero_cuda_extension, mu_zero_dequantize_cuda,
                              mu_zero_quantize_cuda)
 
 _TINY = 1e-8
@@ -231,6 +231,26 @@ def dequantize_rows(packed_q: torch.Tensor, mn: torch.Tensor, scale: torch.Tenso
     return out
 
 
+def _fused_roundtrip_serves(t: torch.Tensor, g: int, kind: str) -> bool:
+    """The shapes of ``mz_roundtrip_kv``; others go through rows."""
+    b, h, s, d = t.shape
+    unit = 1 if kind == "key" else 7
+    return (_on_device(t) and t.numel() > 0 and d in (64, 128) and g in (32, 64, 128) and d % g == 0 and s < 1 << 27
+            and (kind == "value" or s % g == 0) and not any(x & unit for x in t.stride()[:3])
+            and t.data_ptr() % (4 if kind == "key" else 16) == 0)
+
+
+def _fused_roundtrip(t: torch.Tensor, bits: int, g: int, alpha: float, amax_dtype: torch.dtype, amax_eps: float, kind: str):
+    out = torch.empty(t.shape, dtype=t.dtype, device=t.device)
+    ensure_expand_table(bits, alpha, t.device)
+    with torch.cuda.device(t.device):
+        check(load_mu_zero_cuda_extension().mz_roundtrip_kv(
+            t.data_ptr(), dtype_code(t.dtype), (ctypes.c_int * 4)(*t.shape), (ctypes.c_longlong * 3)(*t.stride()[:3]), g, bits,
+            float(alpha), float(amax_eps), dtype_code(amax_dtype), int(kind == "key"), out.data_ptr(), stream_ptr(t.device)),
+            "mz_roundtrip_kv")
+    return out
+
+
 def roundtrip(key: torch.Tensor, value: torch.Tensor, *, bits: int = 4, q_group_size: int = 64,
               alpha_key: Optional[float] = None, alpha_value: Optional[float] = None,
               amax_dtype: torch.dtype = torch.float16, amax_eps: float = 1e-8):
@@ -241,6 +261,9 @@ def roundtrip(key: torch.Tensor, value: torch.Tensor, *, bits: int = 4, q_group_
     if alpha_value is None:
         alpha_value = select_alpha(value, bits=bits, q_group_size=g, kind="value")
 
+    if all(_fused_roundtrip_serves(t, g, kind) for t, kind in ((key, "key"), (value, "value"))):
+        return tuple(_fused_roundtrip(t, bits, g, alpha, amax_dtype, amax_eps, kind)
+                     for t, alpha, kind in ((key, alpha_key, "key"), (value, alpha_value, "value")))
     b, h, s, d = key.shape
     nsg = s // g
     rows = key.reshape(b, h, nsg, g, d).transpose(3, 4).contiguous().reshape(-1, g).float()
