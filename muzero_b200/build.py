@@ -19,7 +19,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libmuzero_b200.so")
 BOUNDS_LIB_PATH = os.path.join(LIB_DIR, "libmuzero_b200_bounds.so")
-SOURCES = ["mz_tables.cu", "mz_thresholds.cu", "mz_alpha.cu", "mz_rows.cu", "mz_flush.cu", "mz_dense.cu", "mz_roundtrip.cu", "mz_decode.cu", "mz_decode_generic.cu", "mz_decode_tiles.cu", "mz_decode_mma.cu", "mz_decode_umma.cu", "mz_qkav.cu", "mz_decode_static.cu", "mz_step.cu", "mz_manage.cu"]
+SOURCES = ["mz_tables.cu", "mz_thresholds.cu", "mz_alpha.cu", "mz_rows.cu", "mz_flush.cu", "mz_dense.cu", "mz_roundtrip.cu", "mz_decode.cu", "mz_decode_generic.cu", "mz_decode_tiles.cu", "mz_decode_mma.cu", "mz_decode_mma_flat.cu", "mz_decode_mma_b1.cu", "mz_decode_mma_b2.cu", "mz_decode_mma_b3.cu", "mz_decode_mma_b4.cu", "mz_decode_mma_b8.cu", "mz_decode_mma_wide.cu", "mz_combine.cu", "mz_decode_umma.cu", "mz_qkav.cu", "mz_decode_static.cu", "mz_step.cu", "mz_manage.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC", "--fmad=true", "-Xptxas", "-v",

@@ -109,15 +109,22 @@ int make_plan(const mz_decode_args* a, Plan* plan, bool need_tables) {
   p.table_k = p.table_v = nullptr;
   p.lut = nullptr;
   p.hetero = 0;
+  p.cluster = 0;
+  p.o = MzDecodeOut{};
+  p.new_k = p.new_v = nullptr;
+  p.new_sb = p.new_sh = 0;
   const int force = kernel_override();
-  plan->tiles = force != 1 && mz_decode_tiles_supported(p);
-  if (v_lead > 0 && !plan->tiles)
+  // 1 = tcgen05, 2 = tensor cores (mma.sync), 3 = SIMT tiles, 0 = shape-generic
+  const int which = force == 1 ? 0 : force == 4 && mz_decode_umma_supported(p) ? 1 : force != 2 && mz_decode_mma_supported(p) ? 2
+                    : mz_decode_tiles_supported(p) ? 3 : 0;
+  plan->tiles = which != 0;
+  if (v_lead > 0 && which != 3)
     return mz_fail(MZ_ERR_UNSUPPORTED, "a value prefix ahead of the key prefix is served by the tiled kernel only (head_dim 128, group 32/64/128)");
   if (plan->tiles) {
     p.tp2 = MzTilesPlan{};
     p.slots_a = 0;
-    if (force == 4 && mz_decode_umma_supported(p)) rc = mz_plan_umma(p, a->splits, sm_count(), &plan->slots);
-    else if (force != 2 && mz_decode_mma_supported(p)) rc = mz_plan_mma(p, a->splits, sm_count(), &plan->slots);
+    if (which == 1) rc = mz_plan_umma(p, a->splits, sm_count(), &plan->slots);
+    else if (which == 2) rc = mz_plan_mma(p, a->splits, sm_count(), &plan->slots);
     else rc = mz_plan_tiles(p, a->splits, sm_count(), &plan->slots);
     if (rc) return rc;
     p.splits = 0;
@@ -147,7 +154,7 @@ int make_plan(const mz_decode_args* a, Plan* plan, bool need_tables) {
 }
 
 // launches the main kernel of an existing plan (the workspace is checked here)
-int launch_partials(const mz_decode_args* a, Plan* plan, cudaStream_t st) {
+int launch_partials(const mz_decode_args* a, Plan* plan, const MzDecodeOut& o, cudaStream_t st) {
   if (a->workspace == nullptr || a->workspace_bytes < plan->ws_bytes)
     return mz_fail(MZ_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", plan->ws_bytes, a->workspace_bytes);
   MZ_REQUIRE((uintptr_t)a->workspace % 16 == 0, "workspace must be 16-byte aligned");
@@ -156,19 +163,16 @@ int launch_partials(const mz_decode_args* a, Plan* plan, cudaStream_t st) {
   p.part.l = p.part.m + plan->slots;
   p.part.acc = p.part.l + plan->slots;
   p.part.slots = (long long)plan->slots;
+  p.o = o;
   if (!plan->tiles) return mz_launch_decode_generic(p, st);
   if (p.tp.kind == 2) return mz_launch_decode_umma(p, st);
-  return p.tp.kind == 1 ? mz_launch_decode_mma(p, st) : mz_launch_decode_tiles(p, st);
+  return p.tp.kind == 0 ? mz_launch_decode_tiles(p, st) : mz_launch_decode_mma(p, st);
 }
 
-int run_partials(const mz_decode_args* a, Plan* plan, cudaStream_t st) {
-  int rc = make_plan(a, plan, true);
-  if (rc) return rc;
-  return launch_partials(a, plan, st);
-}
 
 int finish(const Plan& plan, const MzDecodeOut& o, cudaStream_t st) {
   const MzDecodeParams& p = plan.p;
+  if (p.cluster > 0) return MZ_OK;        // the kernel merged and wrote the result itself
   if (plan.tiles) return mz_combine_tiles(p, o, st);
   const int D = p.s.head_dim;
   const int threads = D >= 128 ? 128 : ((D + 31) / 32) * 32;
@@ -176,6 +180,13 @@ int finish(const Plan& plan, const MzDecodeOut& o, cudaStream_t st) {
   lse_combine_kernel<<<(unsigned)(p.s.batch * p.H), threads, 0, st>>>(v, p.splits, D, o);
   MZ_LAUNCH_CHECK("lse_combine");
   return MZ_OK;
+}
+
+int run(const mz_decode_args* a, const MzDecodeOut& o, cudaStream_t st) {
+  Plan plan;
+  int rc = make_plan(a, &plan, true);
+  if (rc == MZ_OK) rc = launch_partials(a, &plan, o, st);
+  return rc ? rc : finish(plan, o, st);
 }
 }  // namespace
 
@@ -186,7 +197,8 @@ int mz_decode_plan_info(const mz_decode_args* args, size_t* ws_bytes, int* needs
   int rc = make_plan(args, &plan, false);
   if (rc) return rc;
   *ws_bytes = plan.ws_bytes;
-  *needs_tables = plan.tiles ? 0 : 1;
+  // the promise is made for the shapes of the tiled kernels, whichever of them runs
+  *needs_tables = plan.tiles && mz_decode_tiles_supported(plan.p) ? 0 : 1;
   return MZ_OK;
 }
 
@@ -195,11 +207,16 @@ int mz_decode_plan(const mz_decode_args* a, MzDecodePlan* plan) {
   MZ_REQUIRE(a != nullptr && a->out != nullptr && mz_dtype_ok(a->out_dtype), "bad output");
   return make_plan(a, plan, true);
 }
-int mz_decode_run_plan(const mz_decode_args* a, MzDecodePlan* plan, cudaStream_t st) {
-  int rc = launch_partials(a, plan, st);
-  if (rc) return rc;
+bool mz_decode_takes_new_token(const MzDecodePlan& plan, const void* k_new, const void* v_new, long long nsb, long long nsh) {
+  return plan.tiles && plan.p.tp.kind == 1 && (((uintptr_t)k_new | (uintptr_t)v_new) & 15) == 0 && ((nsb | nsh) & 7) == 0;
+}
+int mz_decode_run_plan(const mz_decode_args* a, MzDecodePlan* plan, const void* k_new, const void* v_new, long long nsb, long long nsh,
+                       cudaStream_t st) {
+  MzDecodeParams& p = plan->p;
+  p.new_k = k_new; p.new_v = v_new; p.new_sb = nsb; p.new_sh = nsh;
   const MzDecodeOut o = {a->out, a->out_dtype, nullptr, nullptr, nullptr, 0, 0};
-  return finish(*plan, o, st);
+  int rc = launch_partials(a, plan, o, st);
+  return rc ? rc : finish(*plan, o, st);
 }
 
 extern "C" int mz_debug_force_kernel(int which) {
@@ -235,36 +252,24 @@ extern "C" size_t mz_decode_workspace_bytes(const mz_decode_args* args) {
 
 extern "C" int mz_decode_attention(const mz_decode_args* a, void* stream) {
   MZ_RANGE("mz_decode_attention");
-  Plan plan;
-  cudaStream_t st = (cudaStream_t)stream;
   MZ_REQUIRE(a != nullptr && a->out != nullptr && mz_dtype_ok(a->out_dtype), "bad output");
-  int rc = run_partials(a, &plan, st);
-  if (rc) return rc;
   const MzDecodeOut o = {a->out, a->out_dtype, nullptr, nullptr, nullptr, 0, 0};
-  return finish(plan, o, st);
+  return run(a, o, (cudaStream_t)stream);
 }
 
 extern "C" int mz_decode_attention_partial(const mz_decode_args* a, float* m, float* l, float* acc, void* stream) {
   MZ_RANGE("mz_decode_attention_partial");
-  Plan plan;
-  cudaStream_t st = (cudaStream_t)stream;
-  MZ_REQUIRE(m && l && acc, "NULL partial output");
-  int rc = run_partials(a, &plan, st);
-  if (rc) return rc;
+  MZ_REQUIRE(a != nullptr && m && l && acc, "NULL partial output");
   const MzDecodeOut o = {nullptr, MZ_F32, m, l, acc, a->store.head_dim, 1};
-  return finish(plan, o, st);
+  return run(a, o, (cudaStream_t)stream);
 }
 
 extern "C" int mz_decode_attention_partial_packed(const mz_decode_args* a, float* records, void* stream) {
   MZ_RANGE("mz_decode_attention_partial_packed");
-  Plan plan;
-  cudaStream_t st = (cudaStream_t)stream;
-  MZ_REQUIRE(records != nullptr, "NULL partial output");
-  int rc = run_partials(a, &plan, st);
-  if (rc) return rc;
+  MZ_REQUIRE(a != nullptr && records != nullptr, "NULL partial output");
   const int D = a->store.head_dim;
   const MzDecodeOut o = {nullptr, MZ_F32, records + D, records + D + 1, records, D + 2, D + 2};
-  return finish(plan, o, st);
+  return run(a, o, (cudaStream_t)stream);
 }
 
 namespace {

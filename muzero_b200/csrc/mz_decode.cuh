@@ -26,7 +26,7 @@ struct MzTilesPlan {
   int packed_tiles, dense_tokens, cost_q, cost_d;
   long long pair_cost, total_cost;   // packed_tiles*cost_q + dense_tiles*cost_d ; pairs * pair_cost (< 2^31)
   unsigned cost_quot, cost_rem;      // total_cost / total_warps and the remainder
-  // which main kernel the plan is for (0: SIMT tiled kernel, 1: tensor-core kernel) and, for the latter,
+  // which main kernel the plan is for (0: SIMT tiled, 1: tensor-core, 2: tcgen05, 3: unrolled tensor-core kernel) and, for these,
   // its per-warp staging size and the shared-window addresses of its two buffer pools
   int kind;
   unsigned stage_bytes, low_base, high_base;
@@ -55,6 +55,15 @@ __host__ __device__ inline void mz_warp_tiles(const MzTilesPlan& t, long long g,
   *f1 = mz_tiles_before(t, mz_cost_at(t, g + 1));
 }
 
+// where a call's result goes: normalised output, or the merged (m, l, acc) triple.  The triple is addressed
+// with strides so that it can be written as separate arrays (acc_stride = D, ml_stride = 1) or as one packed
+// record per row, [acc[D], m, l] (acc_stride = ml_stride = D + 2, m = acc + D, l = acc + D + 1).
+struct MzDecodeOut {
+  void* out; int out_dt;
+  float* m; float* l; float* acc;
+  long long acc_stride, ml_stride;
+};
+
 struct MzDecodeParams {
   mz_kv_store s;
   int H, gqa, splits;
@@ -80,15 +89,12 @@ struct MzDecodeParams {
   // tensor-core kernel, one launch over two plans: CTAs [0, hetero) work on plan `tp` (packed tiles only), the
   // rest on plan `tp2` (residual tiles only, records from slots_a on).  0 = one plan per launch.
   int hetero;
-};
-
-// where a call's result goes: normalised output, or the merged (m, l, acc) triple.  The triple is addressed
-// with strides so that it can be written as separate arrays (acc_stride = D, ml_stride = 1) or as one packed
-// record per row, [acc[D], m, l] (acc_stride = ml_stride = D + 2, m = acc + D, l = acc + D + 1).
-struct MzDecodeOut {
-  void* out; int out_dt;
-  float* m; float* l; float* acc;
-  long long acc_stride, ml_stride;
+  // tensor-core kernel, cluster mode: CTAs per pair (0 = flat partition and merge kernel); the kernel writes `o` itself
+  int cluster;
+  MzDecodeOut o;
+  // tensor-core kernel: the window's newest token, still in the caller's tensors [B,KVH,1,D] (nullptr: none); the kernel
+  // uses it from there and stores it into the window
+  const void* new_k; const void* new_v; long long new_sb, new_sh;
 };
 
 // A validated call: which kernel runs, its parameters, the partial records and scratch bytes it needs.
@@ -100,7 +106,11 @@ struct MzDecodePlan {
 };
 // validation + planning of mz_decode_attention(a), and the launches of an existing plan
 int mz_decode_plan(const mz_decode_args* a, MzDecodePlan* plan);
-int mz_decode_run_plan(const mz_decode_args* a, MzDecodePlan* plan, cudaStream_t st);
+// k_new / v_new (with their strides): the newest token of the window, if the kernel shall take it from there
+int mz_decode_run_plan(const mz_decode_args* a, MzDecodePlan* plan, const void* k_new, const void* v_new, long long nsb, long long nsh,
+                       cudaStream_t st);
+// whether the plan's kernel can take the newest token from the caller's tensors
+bool mz_decode_takes_new_token(const MzDecodePlan& plan, const void* k_new, const void* v_new, long long nsb, long long nsh);
 
 // generic kernel: any bits / group / head_dim<=512 / gqa<=16
 int mz_launch_decode_generic(const MzDecodeParams& p, cudaStream_t st);
@@ -112,12 +122,24 @@ int mz_plan_tiles(MzDecodeParams& p, int splits_request, int sm_count, size_t* s
 int mz_launch_decode_tiles(const MzDecodeParams& p, cudaStream_t st);
 int mz_combine_tiles(const MzDecodeParams& p, const MzDecodeOut& o, cudaStream_t st);
 
-// tensor-core kernel: head_dim 128, group 64, 2- or 4-bit codes, gqa in {1,2,4}; shares the partition,
-// the partial records and the merge kernel with the tiled kernel
+// tensor-core kernel: head_dim 64 / 128, group 32 / 64 / 128, any code width, up to 8 query heads per kv head; shares the
+// partition, the partial records and the merge kernel with the tiled kernel
 bool mz_decode_mma_supported(const MzDecodeParams& p);
 int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slots);
 int mz_launch_decode_mma(const MzDecodeParams& p, cudaStream_t st);
+bool mz_decode_flat_supported(const MzDecodeParams& p);
+int mz_plan_flat(MzDecodeParams& p, int splits_request, int sm_count, size_t* slots);
+int mz_launch_decode_flat(const MzDecodeParams& p, cudaStream_t st);
 int mz_smem_window_base();
+const unsigned* mz_mma_lookup_entries(int bits, float alpha_key, float alpha_value);
+// one instance of the tensor-core kernel: its function and the shared-memory sizes its configuration needs
+struct MzMmaKernel { const void* fn; unsigned ri_bytes, a_bytes, p_bytes, table_bytes; int max_warps; };
+bool mz_mma_kernel_b1(int D, int G, int nt, MzMmaKernel* k);
+bool mz_mma_kernel_b2(int D, int G, int nt, MzMmaKernel* k);
+bool mz_mma_kernel_b3(int D, int G, int nt, MzMmaKernel* k);
+bool mz_mma_kernel_b4(int D, int G, int nt, MzMmaKernel* k);
+bool mz_mma_kernel_b8(int D, int G, int nt, MzMmaKernel* k);
+bool mz_mma_kernel_wide(int D, int G, int nt, MzMmaKernel* k);
 
 // tcgen05 kernel (A operand in tensor memory): the packed tiles of head_dim 128 / group 64 / 2- or 4-bit caches;
 // the residual tiles go to the mma.sync kernel in a companion launch

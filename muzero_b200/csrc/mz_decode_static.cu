@@ -43,7 +43,7 @@ extern "C" int mz_decode_attention_static(const mz_decode_args* args, void* stre
   if (rc) return rc;
   if (needs_tables)
     return mz_fail(MZ_ERR_UNSUPPORTED,
-                   "this shape runs on the shape-generic kernel, whose lookup tables are allocated on first use; "
+                   "this shape may run on the shape-generic kernel, whose lookup tables are allocated on first use; "
                    "mz_decode_attention_static serves head_dim 128, group 32/64/128, 1/2/4/8 query heads per kv head");
   if (need > (size_t)MZ_STATIC_SCRATCH_BYTES)
     return mz_fail(MZ_ERR_WORKSPACE, "request needs %zu bytes of scratch, the static array holds %u; lower `splits` or the batch",

@@ -555,213 +555,6 @@ __global__ void __launch_bounds__(Cfg<BITS, G, GQA>::MAX_WARPS * 32, 1) decode_t
   write_partial();
 }
 
-// ---- merge of the records of one (batch, kv head) pair: one CTA per pair, one warp-quad (128
-// threads) per query head.  The warps of the main kernel that hold records of the pair are found from
-// the partition functions the main kernel uses: warp g owns the tiles whose start cost lies in
-// [cost(g), cost(g+1)), and cost(g) is within [g*quot, g*(quot+1)), so every contributor lies in the
-// candidate range [c_lo/(quot+1) - 1, (c_hi-1)/quot + 1], c_lo..c_hi being the pair's cost interval.
-// All threads test candidates at once; the list keeps the candidates' order (a fixed merge order).
-// WIDE (many records per pair, few pairs): one CTA per (pair, head); its four warp-quads each merge every
-// fourth chunk of records and the four partial states are merged in a fixed order at the end.
-constexpr int kMaxCombineSlots = 4096;
-// The workers of plan `tp` that can hold records of `pair` lie in [first, last] (a superset; see above).
-struct WorkerRange { long long first, last; };
-__device__ __forceinline__ WorkerRange candidate_workers(const MzTilesPlan& tp, int pair) {
-  WorkerRange r = {0, -1};
-  if (tp.total_warps <= 0) return r;
-  const unsigned quot = tp.cost_quot ? tp.cost_quot : 1u;
-  const unsigned c_lo = (unsigned)pair * (unsigned)tp.pair_cost, c_hi = c_lo + (unsigned)tp.pair_cost;
-  r.first = (long long)(c_lo / (quot + 1u)) - 1;
-  r.last = (long long)((c_hi - 1u) / quot) + 1;
-  if (r.first < 0 || tp.cost_quot == 0) r.first = 0;
-  if (r.last > tp.total_warps - 1 || tp.cost_quot == 0) r.last = tp.total_warps - 1;   // more workers than cost units: test them all
-  return r;
-}
-// record index of worker gw's segment for `pair` (first_record = index of the plan's first record), or -1
-__device__ __forceinline__ long long record_of(const MzTilesPlan& tp, long long gw, int pair, long long first_record) {
-  const int T = tp.tiles_per_pair;
-  const long long lo = (long long)pair * T, hi = lo + T;
-  long long f0, f1;
-  mz_warp_tiles(tp, gw, &f0, &f1);
-  if (!(f0 < hi && f1 > lo && f0 < f1)) return -1;
-  return first_record + gw * tp.max_segs + (pair - (int)((unsigned)f0 / (unsigned)T));
-}
-template <bool WIDE>
-__global__ void __launch_bounds__(512, 4) combine_tiles_kernel(const MzDecodeParams p, const MzDecodeOut o) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a dependent waits for this grid's completion itself
-  __shared__ int s_slot[kMaxCombineSlots];     // record of candidate i, or -1
-  __shared__ float s_part[WIDE ? 4 : 1][WIDE ? 130 : 1];
-  const int pair = WIDE ? blockIdx.x / p.gqa : blockIdx.x;
-  const int gqa = p.gqa;
-  // candidates of the main plan, then of the residual-tile plan of the tcgen05 route (its records follow)
-  const WorkerRange ra = candidate_workers(p.tp, pair), rb = candidate_workers(p.tp2, pair);
-  const long long cand_a = ra.last - ra.first + 1, cand_b = rb.last - rb.first + 1;
-  const long long cand = cand_a + cand_b;
-  const long long first_b = p.slots_a / gqa;
-  const bool listed = cand <= kMaxCombineSlots &&
-                      first_b + (long long)p.tp.total_warps * p.tp.max_segs + (long long)p.tp2.total_warps * p.tp2.max_segs < (1LL << 31);
-  if (listed) {
-    for (int i = threadIdx.x; i < cand; i += blockDim.x)
-      s_slot[i] = (int)(i < cand_a ? record_of(p.tp, ra.first + i, pair, 0) : record_of(p.tp2, rb.first + (i - cand_a), pair, first_b));
-  }
-  // everything above is arithmetic on the plans; the records themselves are the main kernels' output
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  __syncthreads();
-  const int n = (int)cand;
-  // more candidates than the list holds (a huge explicit split count): every thread walks them itself
-  auto for_each_slot = [&](auto&& fn) {
-    for (long long gw = ra.first; gw <= ra.last; ++gw) {
-      const long long rec = record_of(p.tp, gw, pair, 0);
-      if (rec >= 0) fn(rec);
-    }
-    for (long long gw = rb.first; gw <= rb.last; ++gw) {
-      const long long rec = record_of(p.tp2, gw, pair, first_b);
-      if (rec >= 0) fn(rec);
-    }
-  };
-  const int quad = threadIdx.x >> 7, quads = blockDim.x >> 7;
-  for (int h = WIDE ? blockIdx.x % gqa : quad; h < gqa; h += WIDE ? gqa : quads) {
-    const int d = threadIdx.x & 127;
-    float mx = -INFINITY, lsum = 0.f, a = 0.f;
-    if (listed) {
-      // four records at a time: their loads are independent and in flight together; the running
-      // maximum is carried along (one pass)
-      for (int i0 = WIDE ? 4 * quad : 0; i0 < n; i0 += WIDE ? 4 * quads : 4) {
-        float mi[4], li[4], ai[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int sl = i0 + j < n ? s_slot[i0 + j] : -1;
-          const bool on = sl >= 0;
-          const long long slot = on ? (long long)sl * gqa + h : 0;
-          mi[j] = on ? p.part.m[slot] : -INFINITY;
-          li[j] = on ? p.part.l[slot] : 0.f;
-          ai[j] = on ? p.part.acc[slot * D + d] : 0.f;
-        }
-        const float m_new = fmaxf(fmaxf(mx, fmaxf(mi[0], mi[1])), fmaxf(mi[2], mi[3]));
-        const float keep = mx > -INFINITY ? __expf(mx - m_new) : 0.f;
-        lsum *= keep; a *= keep;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float wgt = mi[j] > -INFINITY ? __expf(mi[j] - m_new) : 0.f;
-          lsum = fmaf(li[j], wgt, lsum);
-          a = fmaf(ai[j], wgt, a);
-        }
-        mx = m_new;
-      }
-      if (WIDE) {
-        // the quads' states, merged in quad order by quad 0
-        s_part[quad][d] = a;
-        if (d == 0) { s_part[quad][128] = mx; s_part[quad][129] = lsum; }
-        __syncthreads();
-        if (quad != 0) continue;      // WIDE visits one head per CTA: nothing follows for these threads
-        float m_all = -INFINITY;
-        for (int k = 0; k < quads; ++k) m_all = fmaxf(m_all, s_part[k][128]);
-        lsum = 0.f; a = 0.f;
-        for (int k = 0; k < quads; ++k) {
-          const float mk = s_part[k][128];
-          const float wgt = mk > -INFINITY ? __expf(mk - m_all) : 0.f;
-          lsum = fmaf(s_part[k][129], wgt, lsum);
-          a = fmaf(s_part[k][d], wgt, a);
-        }
-        mx = m_all;
-      }
-    } else if (!WIDE || quad == 0) {
-      for_each_slot([&](long long sl) { mx = fmaxf(mx, p.part.m[sl * gqa + h]); });
-      for_each_slot([&](long long sl) {
-        const long long slot = sl * gqa + h;
-        const float mi = p.part.m[slot];
-        const float wgt = mi > -INFINITY ? __expf(mi - mx) : 0.f;
-        lsum = fmaf(p.part.l[slot], wgt, lsum);
-        a = fmaf(p.part.acc[slot * D + d], wgt, a);
-      });
-    } else {
-      continue;
-    }
-    const long long row = (long long)pair * gqa + h;
-    if (o.out) mz_store_from_float(o.out, row * D + d, a / fmaxf(lsum, 1e-20f), o.out_dt);
-    else {
-      o.acc[row * o.acc_stride + d] = a;
-      if (d == 0) { o.m[row * o.ml_stride] = mx; o.l[row * o.ml_stride] = lsum; }
-    }
-  }
-}
-
-// The common case (a handful of records per pair): one WARP per (pair, head), no shared memory and no block
-// barrier.  Each lane finds one candidate's record before the wait (pure arithmetic), then up to eight records
-// are loaded at once (their m / l words and one float4 of acc per lane) and merged in candidate order; the
-// records of a second plan (residual tiles of a split launch) follow those of the first.
-__global__ void __launch_bounds__(256) combine_tiles_warp_kernel(const MzDecodeParams p, const MzDecodeOut o) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a dependent waits for this grid's completion itself
-  const int lane = threadIdx.x & 31;
-  const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const long long rows = (long long)p.s.batch * p.H;
-  const int gqa = p.gqa;
-  const int pair = (int)(row / gqa), h = (int)(row % gqa);
-  const bool live = row < rows;
-  const WorkerRange ca = live ? candidate_workers(p.tp, pair) : WorkerRange{0, -1};
-  const WorkerRange cb = live ? candidate_workers(p.tp2, pair) : WorkerRange{0, -1};
-  const long long first_b = p.slots_a / gqa;
-  // first chunk of candidates of each plan (one per lane); nearly always the only chunk
-  long long rec_a = -1, rec_b = -1;
-  if (ca.first + lane <= ca.last) rec_a = record_of(p.tp, ca.first + lane, pair, 0);
-  if (cb.first + lane <= cb.last) rec_b = record_of(p.tp2, cb.first + lane, pair, first_b);
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (!live) return;
-  float mx = -INFINITY, lsum = 0.f;
-  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto merge_chunk = [&](long long my_rec) {
-    unsigned todo = __ballot_sync(0xffffffffu, my_rec >= 0);
-    while (todo) {
-      float mi[8], li[8];
-      float4 ai[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const bool on = todo != 0;
-        const int src = on ? __ffs(todo) - 1 : 0;
-        if (on) todo &= todo - 1;
-        const long long rec = __shfl_sync(0xffffffffu, my_rec, src);
-        const long long slot = on ? rec * gqa + h : 0;
-        mi[j] = on ? p.part.m[slot] : -INFINITY;
-        li[j] = on ? p.part.l[slot] : 0.f;
-        ai[j] = on ? *((const float4*)(p.part.acc + slot * D) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      float m_new = mx;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) m_new = fmaxf(m_new, mi[j]);
-      const float keep = mx > -INFINITY ? __expf(mx - m_new) : 0.f;
-      lsum *= keep; a.x *= keep; a.y *= keep; a.z *= keep; a.w *= keep;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float wgt = mi[j] > -INFINITY ? __expf(mi[j] - m_new) : 0.f;
-        lsum = fmaf(li[j], wgt, lsum);
-        a.x = fmaf(ai[j].x, wgt, a.x); a.y = fmaf(ai[j].y, wgt, a.y);
-        a.z = fmaf(ai[j].z, wgt, a.z); a.w = fmaf(ai[j].w, wgt, a.w);
-      }
-      mx = m_new;
-    }
-  };
-  for (long long base = ca.first; base <= ca.last; base += 32) {
-    if (base != ca.first) rec_a = base + lane <= ca.last ? record_of(p.tp, base + lane, pair, 0) : -1;
-    merge_chunk(rec_a);
-  }
-  for (long long base = cb.first; base <= cb.last; base += 32) {
-    if (base != cb.first) rec_b = base + lane <= cb.last ? record_of(p.tp2, base + lane, pair, first_b) : -1;
-    merge_chunk(rec_b);
-  }
-  const int d = 4 * lane;
-  if (o.out) {
-    const float den = fmaxf(lsum, 1e-20f);
-    mz_store_from_float(o.out, row * D + d, a.x / den, o.out_dt);
-    mz_store_from_float(o.out, row * D + d + 1, a.y / den, o.out_dt);
-    mz_store_from_float(o.out, row * D + d + 2, a.z / den, o.out_dt);
-    mz_store_from_float(o.out, row * D + d + 3, a.w / den, o.out_dt);
-  } else {
-    float* dst = o.acc + row * o.acc_stride + d;
-    dst[0] = a.x; dst[1] = a.y; dst[2] = a.z; dst[3] = a.w;
-    if (lane == 0) { o.m[row * o.ml_stride] = mx; o.l[row * o.ml_stride] = lsum; }
-  }
-}
-
 template <int BITS, int G, int GQA>
 int launch_one(const MzDecodeParams& p, cudaStream_t st) {
   auto kern = decode_tiles_kernel<BITS, G, GQA>;
@@ -910,34 +703,4 @@ int mz_launch_decode_tiles(const MzDecodeParams& p, cudaStream_t st) {
     case 8: return mzt::launch_group<8>(p, st);
   }
   return mz_fail(MZ_ERR_UNSUPPORTED, "bits %d", p.s.bits);
-}
-
-int mz_combine_tiles(const MzDecodeParams& p, const MzDecodeOut& o, cudaStream_t st) {
-  if (p.tp.max_segs < 1) return mz_fail(MZ_ERR_ARG, "bad plan");
-  // programmatic dependent launch: the merge grid may start while the main kernel drains; it finds its
-  // records (pure arithmetic) and then waits for the main grid's results (griddepcontrol.wait)
-  cudaLaunchConfig_t cfg = {};
-  // many records per pair and few pairs: one CTA per (pair, head) with the records split over its quads
-  const long long pairs = (long long)p.s.batch * p.s.kv_heads;
-  const bool wide = p.tp.total_warps / pairs >= 24 && pairs * p.gqa <= 4096;
-  cfg.gridDim = dim3((unsigned)(wide ? pairs * p.gqa : pairs));
-  cfg.blockDim = dim3(wide ? 512 : 128 * (p.gqa < 4 ? p.gqa : 4));
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  // one plan and a few records per pair (workers per pair below 8): the warp-per-row kernel
-  const bool per_warp = !wide && (p.tp2.total_warps == 0 || p.hetero > 0) && p.tp.total_warps / pairs < 8;
-  if (per_warp) {
-    cfg.blockDim = dim3(256);
-    cfg.gridDim = dim3((unsigned)((pairs * p.gqa + 7) / 8));
-  }
-  if (per_warp) MZ_CUDA(cudaLaunchKernelEx(&cfg, mzt::combine_tiles_warp_kernel, p, o));
-  else if (wide) MZ_CUDA(cudaLaunchKernelEx(&cfg, mzt::combine_tiles_kernel<true>, p, o));
-  else MZ_CUDA(cudaLaunchKernelEx(&cfg, mzt::combine_tiles_kernel<false>, p, o));
-  MZ_LAUNCH_CHECK("combine_tiles");
-  return MZ_OK;
 }

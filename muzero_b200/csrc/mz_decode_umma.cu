@@ -598,7 +598,8 @@ int launch_gqa(const MzDecodeParams& p, cudaStream_t st) {
 
 
 bool mz_decode_umma_supported(const MzDecodeParams& p) {
-  return mz_decode_mma_supported(p) && p.s.k_groups > 0;
+  return mz_decode_mma_supported(p) && p.s.head_dim == 128 && p.s.group == 64 && (p.s.bits == 2 || p.s.bits == 4) &&
+         (p.gqa == 1 || p.gqa == 2 || p.gqa == 4) && p.s.k_groups > 0;
 }
 
 // Plan of the packed tiles for the tcgen05 kernel (p.tp, workers = warpgroups) and, when there is a residual
@@ -657,7 +658,7 @@ int mz_plan_umma(MzDecodeParams& p, int splits_request, int sm_count, size_t* sl
     // the residual tiles alone, as a plan of the mma.sync kernel: the same arithmetic with zero packed tiles
     MzDecodeParams q = p;
     q.s.k_groups = 0;
-    int rc = mz_plan_mma(q, splits_request > 0 ? 1 : 0, sm_count, &slots_b);
+    int rc = mz_plan_mma(q, splits_request > 0 ? splits_request : -1, sm_count, &slots_b);
     if (rc) return rc;
     p.tp2 = q.tp;
   }

@@ -155,4 +155,29 @@ __device__ __forceinline__ void row_constants(float lo, float span, int& zc, flo
   if (zc == 0) Bdn = Bup;
   if (zc == TOP) Bup = Bdn;
 }
+// ---- row constants: Bdn = clamp(-lo, 0, span) is the part of the range below zero, Bup the part above, A the value of the
+// zero code (0 when the range straddles zero).  The zero code is rint(RN(RN(-lo / span) * TOP)) as the dequantizer has it.
+// The quotient is correctly rounded by Markstein's final step (IBM J. Res. Dev. 34(1), 1990: with y = RN(1/s) and q within
+// an ulp of b/s, q + (b - q s) y rounds to RN(b/s)); that is branch-free, where the IEEE division costs a range test and a
+// slow path per row.  Ties matter: 16-bit extremes often give a quotient that lies exactly on a code boundary.
+// Spans from 2^125 on would flush the reciprocal: `wild` asks for the division.
+__device__ __forceinline__ void row_split(float lo, float span, float top, float& A, float& bup, float& bdn, int& zc, bool& wild) {
+  span = fmaxf(span, 1e-8f);
+  bdn = fminf(fmaxf(-lo, 0.0f), span);
+  bup = span - bdn;
+  A = lo + bdn;
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(span));
+  y = fmaf(fmaf(-span, y, 1.0f), y, y);
+  const float q0 = bdn * y;
+  const float q = fmaf(fmaf(-q0, span, bdn), y, q0);
+  zc = __float_as_int(__fmul_rn(q, top) + 12582912.0f) & 0xff;
+  wild |= !(span < 4e37f);
+  bup = fminf(bup, 65504.f);
+  bdn = fminf(bdn, 65504.f);
+}
+__device__ __forceinline__ int exact_zero_code(float lo, float span, float top) {
+  const float anchor = fminf(fmaxf(__fdiv_rn(__fsub_rn(0.0f, lo), fmaxf(span, 1e-8f)), 0.0f), 1.0f);
+  return __float2int_rn(__fmul_rn(anchor, top));
+}
 }  // namespace mzm
