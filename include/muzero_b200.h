@@ -139,6 +139,16 @@ int mz_flush_kv_parts(const mz_kv_store* store, int n_key_tokens, int value_firs
                       void* stream);
 
 /*
+ * mz_flush_kv_parts, and in the same launch the rows that stay dense are copied to a new window (kv_dtype, element
+ * strides as given, room for res_len - n_key_tokens rows): key row n_key_tokens becomes its row 0, and the value rows
+ * from value_first + n_value_tokens (not below n_key_tokens) on move by the same distance.  A prompt block is quantized
+ * straight from the caller's tensors and only its tail gets a buffer of its own this way.
+ * Replaces: the copies of _append_dense / compress_residual_prefix, muzero/cache/layer.py:135-217.
+ */
+int mz_flush_kv_move(const mz_kv_store* store, int n_key_tokens, int value_first, int n_value_tokens, void* dst_k, void* dst_v,
+                     long long dst_stride_b, long long dst_stride_h, long long dst_stride_t, float eps, void* stream);
+
+/*
  * Appends one token per (b,kvh) to the residual window at index res_start+res_len:
  * k_new,v_new [B,KVH,1,D] with element strides (new_stride_b,new_stride_h).
  * Replaces: the two single-token buffer copies of _append_dense, muzero/cache/layer.py:183-193.

@@ -16,7 +16,7 @@ from typing import Optional
 
 import torch
 
-from ..kernels._cabi import DecodeArgs, MuZeroKernelError, check, dtype_code, last_error, stream_ptr
+from ..kernels._cabi import DecodeArgs, MuZeroKernelError, check, dtype_code, last_error, on_device, stream_ptr
 from ..kernels.loader import load_mu_zero_cuda_extension
 
 _MU_ZERO_DECODE_STATS = defaultdict(int)
@@ -33,9 +33,11 @@ def get_mu_zero_decode_stats() -> dict[str, int]:
 
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """One reusable scratch buffer per (device, stream); grows, never shrinks."""
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, stream_ptr(device))
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
+        if len(_workspaces) >= 64:      # streams come and go
+            _workspaces.clear()
         buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
         _workspaces[key] = buf
     return buf
@@ -56,8 +58,7 @@ def build_decode_args(layer, query: torch.Tensor, scaling: float, attention_mask
         raise MuZeroKernelError(f"query dtype {query.dtype} differs from cache dtype {layer.dtype}")
     if query.stride(-1) != 1:
         query = query.contiguous()
-    a = DecodeArgs()
-    a.store = layer._store_struct()
+    a, total = layer._decode_args()
     a.q_heads = query.shape[1]
     a.query = query.data_ptr()
     a.q_stride_b, a.q_stride_h = query.stride(0), query.stride(1)
@@ -70,7 +71,7 @@ def build_decode_args(layer, query: torch.Tensor, scaling: float, attention_mask
             mask = mask.to(query.dtype)
         if mask.dtype not in (torch.float32, torch.float16, torch.bfloat16):
             mask = mask.to(torch.float32)
-        total = a.store.k_groups * a.store.group + a.store.res_len + (1 if step else 0)
+        total += 1 if step else 0
         if mask.dim() != 4 or mask.shape[1] != 1 or mask.shape[2] != 1 or mask.shape[-1] < total:
             raise MuZeroKernelError(f"attention_mask must be [B,1,1,>={total}], got {tuple(mask.shape)}")
         if mask.stride(-1) != 1:
@@ -84,8 +85,12 @@ def build_decode_args(layer, query: torch.Tensor, scaling: float, attention_mask
         a.out = out.data_ptr()
         a.out_dtype = dtype_code(out.dtype)
     lib = load_mu_zero_cuda_extension()
-    if bound:
-        need = lib.mz_decode_workspace_bound(ctypes.byref(a))
+    if bound or (splits == 0 and not step):
+        # one size for any number of cached tokens: asked once per layer and head count, not per call
+        sized = layer._ws_bound
+        if sized is None or sized[0] != (a.store.batch, a.q_heads):
+            sized = layer._ws_bound = ((a.store.batch, a.q_heads), lib.mz_decode_workspace_bound(ctypes.byref(a)))
+        need = sized[1]
     elif step:
         need = lib.mz_decode_step_workspace_bytes(ctypes.byref(a), int(step[0]), int(step[1]))
     else:
@@ -108,11 +113,10 @@ def decode_attention(layer, query: torch.Tensor, scaling: float, attention_mask:
         kvh = layer.keys.shape[1]
         if not (d == 128 and layer.q_group_size in (32, 64, 128) and h % kvh == 0 and h // kvh in (1, 2, 4, 8)):
             return _decode_attention_unaligned(layer, query, scaling, attention_mask, out_dtype or query.dtype)
-    out = torch.empty((b, 1, h, d), dtype=out_dtype or query.dtype, device=query.device)
+    out = query.new_empty((b, 1, h, d)) if out_dtype is None else torch.empty((b, 1, h, d), dtype=out_dtype, device=query.device)
     args = build_decode_args(layer, query, scaling, attention_mask, out, splits=splits)
-    with torch.cuda.device(query.device):
-        check(load_mu_zero_cuda_extension().mz_decode_attention(ctypes.byref(args), stream_ptr(query.device)),
-              "mz_decode_attention")
+    check(on_device(query.device, load_mu_zero_cuda_extension().mz_decode_attention, ctypes.byref(args), stream_ptr(query.device)),
+          "mz_decode_attention")
     return out
 
 

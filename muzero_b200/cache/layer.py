@@ -26,7 +26,7 @@ import torch
 
 from ..config import MuZeroConfig
 from ..kernels import _cabi
-from ..kernels._cabi import KVStore, MuZeroKernelError, check, dtype_code, stream_ptr
+from ..kernels._cabi import DecodeArgs, KVStore, MuZeroKernelError, check, dtype_code, on_device, stream_ptr
 from ..kernels.loader import ensure_expand_table, load_mu_zero_cuda_extension
 from ..quantizer import (_anchor_offset, _magnitude_ratios, _on_device, _statistics_needed, alpha_from_stats, device_alphas,
                          select_alpha_key_block)
@@ -65,7 +65,8 @@ class MuZeroCacheLayer:
         self._window_stale = False     # decode_step moved the window; the views are rebuilt on first use
         self._window_len = 0           # residual tokens after the last one-call decode step
         self._step_args = None         # C argument block kept across steady-state decode steps
-        self._step_base = 0            # _res_start at the time the block was built
+        self._ws_bound = None          # ((batch, query heads), workspace bytes)
+        self._arg_base = None          # C argument block with the buffers' pointers and strides (see _decode_args)
         self._step_ws_bound = 0
         self._key_buffer = None
         self._value_buffer = None
@@ -173,6 +174,28 @@ class MuZeroCacheLayer:
             s.res_start, s.res_len = 0, k.shape[2]
         return s
 
+    def _decode_args(self) -> tuple[DecodeArgs, int]:
+        """A C argument block for the current state, and the number of keys it covers.  Pointers and strides live as long
+        as the buffers do, so a block that holds them is kept and copied; a call fills in the counters."""
+        kb, pk = self._key_buffer, self._bufs.get("pk")
+        if kb is None:
+            a = DecodeArgs()
+            a.store = self._store_struct()
+            return a, a.store.k_groups * a.store.group + a.store.res_len
+        alphas = (self._selected_alpha_key, self._selected_alpha_value)
+        base = self._arg_base
+        if base is None or base[1] is not kb or base[2] is not pk or base[3] != alphas:
+            a = DecodeArgs()
+            a.store = self._store_struct()
+            a.store.res_k, a.store.res_v = kb.data_ptr(), self._value_buffer.data_ptr()
+            base = self._arg_base = (a, kb, pk, alphas)
+        a = DecodeArgs.from_buffer_copy(base[0])
+        st = a.store
+        st.k_groups, st.v_tokens = self._key_group_count, self._value_storage_len
+        st.res_start = self._res_start
+        st.res_len = self._window_len if self._window_stale else int(self._keys.shape[2])
+        return a, st.k_groups * self.q_group_size + st.res_len
+
     # ----------------------------------------------------------- dense window
     def _rehome_residual(self, min_tokens: int) -> None:
         """Puts the residual window at the front of a buffer with room for ``min_tokens``."""
@@ -188,6 +211,7 @@ class MuZeroCacheLayer:
                 kb[:, :, :cur].copy_(self.keys)
                 vb[:, :, lead:cur].copy_(self.values)
             self._key_buffer, self._value_buffer, self._buffer_capacity = kb, vb, cap
+            self._arg_base = None
         elif self._res_start > 0 and cur:
             src_k, src_v = self.keys, self.values
             if self._res_start < cur:          # overlapping move
@@ -215,10 +239,9 @@ class MuZeroCacheLayer:
             if self.device.type == "cuda" and key_states.stride(-1) == 1 and value_states.stride(-1) == 1 \
                     and key_states.stride()[:2] == value_states.stride()[:2]:
                 s = self._store_struct()
-                with torch.cuda.device(self.device):
-                    check(load_mu_zero_cuda_extension().mz_append_kv(
-                        ctypes.byref(s), key_states.data_ptr(), value_states.data_ptr(), key_states.stride(0),
-                        key_states.stride(1), stream_ptr(self.device)), "mz_append_kv")
+                check(on_device(self.device, load_mu_zero_cuda_extension().mz_append_kv, ctypes.byref(s), key_states.data_ptr(),
+                                value_states.data_ptr(), key_states.stride(0), key_states.stride(1), stream_ptr(self.device)),
+                      "mz_append_kv")
             else:
                 pos = self._res_start + cur
                 self._key_buffer[:, :, pos:pos + 1].copy_(key_states)
@@ -229,7 +252,7 @@ class MuZeroCacheLayer:
             return
         self.keys = torch.cat([self.keys, key_states], dim=-2)
         self.values = torch.cat([self.values, value_states], dim=-2)
-        self._key_buffer = self._value_buffer = None
+        self._key_buffer = self._value_buffer = self._arg_base = None
         self._buffer_capacity = 0
         self._res_start = 0
         if self._value_lead:                   # keep keys and values addressable as one window
@@ -241,19 +264,11 @@ class MuZeroCacheLayer:
         n_values = n if n_values is None else n_values
         if n <= 0 and n_values <= 0:
             return
-        lead = self._value_lead + n_values - n
-        if self._key_buffer is not None:
-            self._res_start += n
-            self._value_lead = lead
-            a, cur = self._res_start, int(self.keys.shape[2]) - n
-            self.keys = self._key_buffer[:, :, a:a + cur]
-            self.values = self._value_buffer[:, :, a + lead:a + cur]
-        else:
-            # aliased prefill block: keep only the tail, in a buffer of its own
-            self.keys = self.keys[:, :, n:]
-            self.values = self.values[:, :, n_values:]
-            self._value_lead = lead
-            self._rehome_residual(int(self.keys.shape[2]) + 1)
+        self._res_start += n
+        self._value_lead += n_values - n
+        a, cur = self._res_start, int(self.keys.shape[2]) - n
+        self.keys = self._key_buffer[:, :, a:a + cur]
+        self.values = self._value_buffer[:, :, a + self._value_lead:a + cur]
 
     # ----------------------------------------------------------------- store
     def _ensure_store(self, groups: int, tokens: int) -> None:
@@ -286,7 +301,7 @@ class MuZeroCacheLayer:
             for name in ("pv", "vmn", "vsc"):
                 new[name][:, :, :vt].copy_(self._bufs[name][:, :, :vt])
         self._bufs = new
-        self._step_args = None
+        self._step_args = self._arg_base = None
         self._refresh_views()
 
     def _refresh_views(self) -> None:
@@ -302,7 +317,7 @@ class MuZeroCacheLayer:
     def _adopt_store(self, tensors: dict[str, torch.Tensor]) -> None:
         """Replaces the store by exact-size tensors (after batch reindexing / device moves)."""
         self._bufs = {k: v.contiguous() for k, v in tensors.items()}
-        self._step_args = None
+        self._step_args = self._arg_base = None
         self._refresh_views()
 
     # ------------------------------------------------------------------ alpha
@@ -311,6 +326,10 @@ class MuZeroCacheLayer:
         g, bits, mp = self.q_group_size, self.nbits, self.cfg.stats_max_points
         want_k = self._selected_alpha_key is None and n_flush > 0
         want_v = self._selected_alpha_value is None and n_values > 0
+        if want_k and not _statistics_needed(bits, "key"):       # one alpha whatever the data is
+            self._selected_alpha_key, want_k = 2.0, False
+        if want_v and not _statistics_needed(bits, "value"):
+            self._selected_alpha_value, want_v = 2.0, False
         if want_k and want_v and _on_device(self.keys) and _on_device(self.values):
             # both choices from one read-back
             self._selected_alpha_key, self._selected_alpha_value = device_alphas(
@@ -342,14 +361,27 @@ class MuZeroCacheLayer:
         if self._value_lead and self._key_buffer is None:
             self._rehome_residual(int(self.keys.shape[2]) + 1)      # one window for keys and values
         s = self._store_struct()
-        with torch.cuda.device(self.device):
-            # value rows are addressed inside the key window: they start `_value_lead` rows in
-            check(load_mu_zero_cuda_extension().mz_flush_kv_parts(ctypes.byref(s), n, self._value_lead, nv, self.amax_eps,
-                                                                  stream_ptr(self.device)), "mz_flush_kv_parts")
+        lib, st = load_mu_zero_cuda_extension(), stream_ptr(self.device)
+        # value rows are addressed inside the key window: they start `_value_lead` rows in
+        if self._key_buffer is None:
+            # a prompt block: what stays dense moves into a window of the layer's own, in the same launch
+            cur, lead = s.res_len - n, self._value_lead + nv - n
+            cap = residual_capacity(cur + 1, self.residual_length, g)
+            kb = torch.empty((s.batch, s.kv_heads, cap, self.k_head_dim), dtype=self.dtype, device=self.device)
+            vb = torch.empty_like(kb)
+            sb, sh, srow, _ = kb.stride()
+            check(on_device(self.device, lib.mz_flush_kv_move, ctypes.byref(s), n, self._value_lead, nv, kb.data_ptr(), vb.data_ptr(),
+                            sb, sh, srow, self.amax_eps, st), "mz_flush_kv_move")
+            self._key_buffer, self._value_buffer, self._buffer_capacity, self._res_start = kb, vb, cap, 0
+            self._value_lead, self._arg_base = lead, None
+            self.keys, self.values = kb[:, :, :cur], vb[:, :, lead:cur]
+        else:
+            check(on_device(self.device, lib.mz_flush_kv_parts, ctypes.byref(s), n, self._value_lead, nv, self.amax_eps, st),
+                  "mz_flush_kv_parts")
+            self._drop_residual_prefix(n, nv)
         self._key_group_count += n // g
         self._value_storage_len += nv
         self._refresh_views()
-        self._drop_residual_prefix(n, nv)
 
     # ---------------------------------------------------------------- dequant
     def _dequantize(self, g0: int, g1: int, t0: int, t1: int, want_k: bool, want_v: bool):
@@ -437,14 +469,13 @@ class MuZeroCacheLayer:
             self.update(key_states, value_states, {"materialize_full_kv": False})
             return decode_attention(self, query, scaling, attention_mask)
         b, h, _, d = query.shape
-        out = torch.empty((b, 1, h, d), dtype=query.dtype, device=query.device)
+        out = query.new_empty((b, 1, h, d))
         lib = load_mu_zero_cuda_extension()
         args = self._step_args
         if attention_mask is not None or args is None or query.stride(-1) != 1 or query.dtype != self.dtype:
             # (re)build the argument block: pointers, strides and counters of the current state.  With a mask
             # the block is built per call (the mask tensor may be converted and has to stay alive).
             args = build_decode_args(self, query, scaling, attention_mask, out, step=(self.residual_length, unit), bound=True)
-            self._step_base = self._res_start
             self._step_ws_bound = args.workspace_bytes
             self._step_args = args if attention_mask is None else None
         else:
@@ -454,17 +485,16 @@ class MuZeroCacheLayer:
             args.out, args.out_dtype = out.data_ptr(), dtype_code(out.dtype)
             ws = _workspace(query.device, self._step_ws_bound)
             args.workspace, args.workspace_bytes = ws.data_ptr(), ws.numel()
-        with torch.cuda.device(self.device):
-            rc = lib.mz_decode_step(
-                ctypes.byref(args), key_states.data_ptr(), value_states.data_ptr(), key_states.stride(0), key_states.stride(1),
-                self.residual_length, unit, int(self._bufs["pk"].shape[2]) if self._bufs else 0,
-                self._buffer_capacity - self._step_base, self.amax_eps, stream_ptr(self.device))
+        rc = on_device(
+            self.device, lib.mz_decode_step, ctypes.byref(args), key_states.data_ptr(), value_states.data_ptr(), key_states.stride(0),
+            key_states.stride(1), self.residual_length, unit, self._bufs["pk"].shape[2] if self._bufs else 0,
+            self._buffer_capacity, self.amax_eps, stream_ptr(self.device))
         if rc != 0:
             self._step_args = None                # nothing moved (the library commits counters last); rebuild next time
             check(rc, "mz_decode_step")
         st = args.store
         flushed = st.k_groups != self._key_group_count
-        self._res_start = self._step_base + st.res_start     # the block's window starts at its own pointer
+        self._res_start = st.res_start
         self._key_group_count, self._value_storage_len = st.k_groups, st.v_tokens
         self._window_len = st.res_len
         self.cumulative_length += 1
@@ -507,11 +537,9 @@ class MuZeroCacheLayer:
             s = self._store_struct()
             shape = (s.batch, s.kv_heads, s.k_groups * s.group + s.res_len, self.k_head_dim)
             k = torch.empty(shape, dtype=self.dtype, device=self.device)
-            v = torch.empty(shape, dtype=self.dtype, device=self.device)
-            with torch.cuda.device(self.device):
-                check(load_mu_zero_cuda_extension().mz_materialize_kv(
-                    ctypes.byref(s), k.data_ptr(), v.data_ptr(), dtype_code(self.dtype), self.amax_eps, stream_ptr(self.device)),
-                    "mz_materialize_kv")
+            v = torch.empty_like(k)
+            check(on_device(self.device, load_mu_zero_cuda_extension().mz_materialize_kv, ctypes.byref(s), k.data_ptr(), v.data_ptr(),
+                            dtype_code(self.dtype), self.amax_eps, stream_ptr(self.device)), "mz_materialize_kv")
             return k, v
         k = torch.cat([self._dequantize_key_prefix(), self.keys], dim=2) if self._key_group_count else self.keys
         v = torch.cat([self._dequantize_value_prefix(), self.values], dim=2) if self._value_storage_len else self.values
@@ -544,7 +572,7 @@ class MuZeroCacheLayer:
             # also with zero residual tokens (residual_length=0 right after a flush): the window's shape
             # carries the batch size, and its old buffers belong to the old batch
             self.keys, self.values = fn(self.keys).contiguous(), fn(self.values).contiguous()
-            self._key_buffer = self._value_buffer = None
+            self._key_buffer = self._value_buffer = self._arg_base = None
             self._buffer_capacity, self._res_start = 0, 0
         if self._bufs and (self._key_group_count or self._value_storage_len):
             kg, vt = self._key_group_count, self._value_storage_len
@@ -573,7 +601,7 @@ class MuZeroCacheLayer:
         vb = torch.empty((n, kvh, cap, self.v_head_dim), dtype=self.dtype, device=self.device)
         new = {name: torch.empty((n, *t.shape[1:]), dtype=t.dtype, device=self.device) for name, t in self._bufs.items()}
         self._bufs, self._key_buffer, self._value_buffer, self._res_start = new, kb, vb, 0
-        self._step_args = None
+        self._step_args = self._arg_base = None
         self._keys, self._values = kb[:, :, :cur], vb[:, :, :cur]
         self._window_stale = False
         dst = self._store_struct()
@@ -584,7 +612,7 @@ class MuZeroCacheLayer:
                 "mz_store_gather_batch")
         if int(status.item()):
             self._bufs, self._key_buffer, self._value_buffer, self._res_start, self._keys, self._values = old
-            self._step_args = None
+            self._step_args = self._arg_base = None
             self._refresh_views()
             raise MuZeroKernelError("batch index out of range")
         del old

@@ -11,8 +11,16 @@
 
 namespace {
 
+// the rows of the window that a flush leaves dense, copied to a new window (dst_k == nullptr: not asked for)
+struct MoveParams {
+  uint16_t* dst_k; uint16_t* dst_v;
+  long long sb, sh, st;      // element strides of the new window
+  int k_first, v_first;      // first key / value row that stays; key row k_first becomes row 0 of the new window
+};
+
 struct FlushParams {
   mz_kv_store s;
+  MoveParams mv;
   int n_tiles;               // key tiles (groups of G tokens) to flush, from the window's first token
   int v_first, n_vtokens;    // value tokens to flush: window rows [v_first, v_first + n_vtokens)
   int QB, NG;
@@ -226,6 +234,8 @@ struct Flush16Params {
   const uint16_t* ctab_k; const uint16_t* ctab_v; int ctab_k_n, ctab_v_n;
   unsigned n_k_blocks, tiles;       // key CTAs; key tiles in all
   unsigned v_blocks_per_pair;
+  unsigned n_v_blocks, mv_per_pair;   // value CTAs; CTAs per pair of the rows that stay
+  MoveParams mv;
 };
 
 template <int DT, int BITS, int TPT>
@@ -449,11 +459,36 @@ __device__ __forceinline__ void flush16_values(const Flush16Params& p) {
   }
 }
 
+// rows that stay dense: 16 bytes of the key row and of the value row per thread
+__device__ __forceinline__ void move_rows16(const mz_kv_store& s, const MoveParams& m, unsigned blk, unsigned per_pair) {
+  const unsigned pair = blk / per_pair;
+  const int vpr = s.head_dim >> 3, i = (int)(blk % per_pair) * 256 + threadIdx.x, row = m.k_first + i / vpr, c = (i % vpr) * 8;
+  if (row >= s.res_len) return;
+  const int b = pair / s.kv_heads, h = pair % s.kv_heads;
+  const long long src = b * s.res_stride_b + h * s.res_stride_h + (long long)(s.res_start + row) * s.res_stride_t + c;
+  const long long dst = b * m.sb + h * m.sh + (long long)(row - m.k_first) * m.st + c;
+  *(uint4*)(m.dst_k + dst) = *(const uint4*)((const uint16_t*)s.res_k + src);
+  if (row >= m.v_first) *(uint4*)(m.dst_v + dst) = *(const uint4*)((const uint16_t*)s.res_v + src);
+}
+
 template <int DT, int BITS, int TPT>
 __global__ void __launch_bounds__(256) flush16_kernel(const Flush16Params p) {
   extern __shared__ __align__(16) uint8_t s_flush[];
   if (blockIdx.x < p.n_k_blocks) flush16_keys<DT, BITS, TPT>(p, s_flush);
-  else flush16_values<DT, BITS>(p);
+  else if (blockIdx.x < p.n_k_blocks + p.n_v_blocks) flush16_values<DT, BITS>(p);
+  else move_rows16(p.s, p.mv, blockIdx.x - p.n_k_blocks - p.n_v_blocks, p.mv_per_pair);
+}
+
+__global__ void __launch_bounds__(256) move_rows_kernel(const mz_kv_store s, const MoveParams m) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int D = s.head_dim, nk = s.res_len - m.k_first;
+  if (i >= (long long)s.batch * s.kv_heads * nk * D) return;
+  const int d = (int)(i % D), row = (int)(i / D % nk) + m.k_first;
+  const long long pair = i / D / nk;
+  const long long src = (pair / s.kv_heads) * s.res_stride_b + (pair % s.kv_heads) * s.res_stride_h + (long long)(s.res_start + row) * s.res_stride_t + d;
+  const long long dst = (pair / s.kv_heads) * m.sb + (pair % s.kv_heads) * m.sh + (long long)(row - m.k_first) * m.st + d;
+  m.dst_k[dst] = ((const uint16_t*)s.res_k)[src];
+  if (row >= m.v_first) m.dst_v[dst] = ((const uint16_t*)s.res_v)[src];
 }
 
 __global__ void append_kv_kernel(const mz_kv_store s, const uint16_t* __restrict__ k_new, const uint16_t* __restrict__ v_new,
@@ -521,16 +556,18 @@ int flush16(const mz_kv_store& s, const FlushParams& f, cudaStream_t st, int* do
   const int rows_per_cta = 256 / (s.group / 16);
   p.v_blocks_per_pair = (unsigned)(((long long)p.n_vtokens * (s.head_dim / s.group) + rows_per_cta - 1) / rows_per_cta);
   const long long kb = (tiles + per_cta - 1) / per_cta, vb = pairs * p.v_blocks_per_pair;
-  if (tiles >= (1LL << 31) || kb + vb >= (1LL << 31)) return MZ_OK;
-  p.tiles = (unsigned)tiles; p.n_k_blocks = (unsigned)kb;
+  p.mv = f.mv;
+  p.mv_per_pair = f.mv.dst_k ? (unsigned)(((s.res_len - f.mv.k_first) * (s.head_dim / 8) + 255) / 256) : 0;
+  const long long mb = pairs * p.mv_per_pair;
+  if (tiles >= (1LL << 31) || kb + vb + mb >= (1LL << 31)) return MZ_OK;
+  p.tiles = (unsigned)tiles; p.n_k_blocks = (unsigned)kb; p.n_v_blocks = (unsigned)vb;
   *done = 1;
-  return s.kv_dtype == MZ_BF16 ? launch_flush16_bits<MZ_BF16>(p, (unsigned)(kb + vb), st) : launch_flush16_bits<MZ_F16>(p, (unsigned)(kb + vb), st);
+  return s.kv_dtype == MZ_BF16 ? launch_flush16_bits<MZ_BF16>(p, (unsigned)(kb + vb + mb), st) : launch_flush16_bits<MZ_F16>(p, (unsigned)(kb + vb + mb), st);
 }
 }  // namespace
 
-extern "C" int mz_flush_kv_parts(const mz_kv_store* s, int n_key_tokens, int value_first, int n_value_tokens, float eps,
-                                 void* stream) {
-  MZ_RANGE("mz_flush_kv_parts");
+namespace {
+int flush(const mz_kv_store* s, int n_key_tokens, int value_first, int n_value_tokens, float eps, const MoveParams& mv, void* stream) {
   int rc = mz_check_store_basic(s);
   if (rc) return rc;
   if ((rc = mz_check_store_quantized(s))) return rc;
@@ -544,7 +581,7 @@ extern "C" int mz_flush_kv_parts(const mz_kv_store* s, int n_key_tokens, int val
   const MzStoreGeom g = mz_geom(*s);
   FlushParams p;
   p.s = *s; p.n_tiles = n_key_tokens / g.G; p.v_first = value_first; p.n_vtokens = n_value_tokens;
-  p.QB = g.QB; p.NG = g.NG; p.eps = eps;
+  p.QB = g.QB; p.NG = g.NG; p.eps = eps; p.mv = mv;
   if ((rc = mz_get_compand_table(g.kv_dt, s->alpha_key, &p.ctab_k, &p.ctab_k_n))) return rc;
   if ((rc = mz_get_compand_table(g.kv_dt, s->alpha_value, &p.ctab_v, &p.ctab_v_n))) return rc;
   const long long kb = (long long)g.B * g.KVH * p.n_tiles;
@@ -552,7 +589,8 @@ extern "C" int mz_flush_kv_parts(const mz_kv_store* s, int n_key_tokens, int val
   p.v_fast = pow2(g.G) && g.G >= 8 && g.G <= 256 && g.D % 8 == 0;
   p.k_vec = g.D % 8 == 0 && s->res_stride_t % 8 == 0 && s->res_stride_h % 8 == 0 && s->res_stride_b % 8 == 0 &&
             (uintptr_t)s->res_k % 16 == 0 && (uintptr_t)s->res_v % 16 == 0;
-  if (flush16_serves(*s, p)) {
+  const bool mv_vec = !mv.dst_k || ((((uintptr_t)mv.dst_k | (uintptr_t)mv.dst_v) & 15) == 0 && ((mv.sb | mv.sh | mv.st) & 7) == 0);
+  if (mv_vec && flush16_serves(*s, p)) {
     int done = 0;
     if ((rc = flush16(*s, p, (cudaStream_t)stream, &done)) || done) return rc;
   }
@@ -571,7 +609,29 @@ extern "C" int mz_flush_kv_parts(const mz_kv_store* s, int n_key_tokens, int val
     flush_kv_kernel<MZ_F16><<<(unsigned)(kb + vb), 256, smem, st>>>(p);
   }
   MZ_LAUNCH_CHECK("flush_kv");
+  if (mv.dst_k && s->res_len > mv.k_first) {
+    const long long n = (long long)g.B * g.KVH * (s->res_len - mv.k_first) * g.D;
+    MZ_REQUIRE((n + 255) / 256 < (1LL << 31), "window too large");
+    move_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(*s, mv);
+    MZ_LAUNCH_CHECK("move_rows");
+  }
   return MZ_OK;
+}
+}  // namespace
+
+extern "C" int mz_flush_kv_parts(const mz_kv_store* s, int n_key_tokens, int value_first, int n_value_tokens, float eps,
+                                 void* stream) {
+  MZ_RANGE("mz_flush_kv_parts");
+  return flush(s, n_key_tokens, value_first, n_value_tokens, eps, MoveParams{}, stream);
+}
+
+extern "C" int mz_flush_kv_move(const mz_kv_store* s, int n_key_tokens, int value_first, int n_value_tokens, void* dst_k, void* dst_v,
+                                long long dst_stride_b, long long dst_stride_h, long long dst_stride_t, float eps, void* stream) {
+  MZ_RANGE("mz_flush_kv_move");
+  MZ_REQUIRE(s != nullptr && dst_k && dst_v && dst_stride_t >= s->head_dim, "bad destination window");
+  const MoveParams mv = {(uint16_t*)dst_k, (uint16_t*)dst_v, dst_stride_b, dst_stride_h, dst_stride_t, n_key_tokens, value_first + n_value_tokens};
+  MZ_REQUIRE(n_key_tokens + n_value_tokens > 0 && mv.v_first >= mv.k_first, "nothing to flush, or values behind the keys");
+  return flush(s, n_key_tokens, value_first, n_value_tokens, eps, mv, stream);
 }
 
 extern "C" int mz_flush_kv(const mz_kv_store* s, int n_tokens, float eps, void* stream) {

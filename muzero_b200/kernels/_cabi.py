@@ -23,7 +23,7 @@ EXPORTS = (
     "mz_flush_kv", "mz_append_kv", "mz_dequantize_kv", "mz_decode_workspace_bytes", "mz_decode_attention",
     "mz_decode_attention_partial", "mz_lse_merge", "mz_qk_logits", "mz_av_output", "mz_decode_attention_static",
     "mz_decode_step", "mz_decode_step_workspace_bytes", "mz_flush_kv_parts", "mz_decode_workspace_bound", "mz_decode_attention_partial_packed", "mz_lse_merge_packed", "mz_store_gather_batch", "mz_debug_force_kernel", "mz_bounds_violations",
-    "mz_alpha_stats", "mz_alpha_stats_workspace_bytes", "mz_materialize_kv", "mz_roundtrip_kv",
+    "mz_alpha_stats", "mz_alpha_stats_workspace_bytes", "mz_materialize_kv", "mz_roundtrip_kv", "mz_flush_kv_move",
 )
 
 
@@ -90,6 +90,8 @@ def load_library() -> ctypes.CDLL:
                                        c_void_p, c_int, c_void_p]
     lib.mz_flush_kv.argtypes = [POINTER(KVStore), c_int, c_float, c_void_p]
     lib.mz_flush_kv_parts.argtypes = [POINTER(KVStore), c_int, c_int, c_int, c_float, c_void_p]
+    lib.mz_flush_kv_move.argtypes = [POINTER(KVStore), c_int, c_int, c_int, c_void_p, c_void_p, c_longlong, c_longlong, c_longlong, c_float,
+                                     c_void_p]
     lib.mz_append_kv.argtypes = [POINTER(KVStore), c_void_p, c_void_p, c_longlong, c_longlong, c_void_p]
     lib.mz_dequantize_kv.argtypes = [POINTER(KVStore), c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_float, c_void_p]
     lib.mz_decode_workspace_bytes.argtypes = [POINTER(DecodeArgs)]
@@ -143,7 +145,17 @@ def dtype_code(dt: torch.dtype) -> int:
 
 
 def stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Handle of the calling thread's current stream (without building a Stream object: 0.1 instead of 2.3 us)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+def on_device(device: torch.device, fn, *args):
+    """``fn(*args)`` with ``device`` current; the context manager only where another device is."""
+    if device.index is None or device.index == torch.cuda.current_device():
+        return fn(*args)
+    with torch.cuda.device(device):
+        return fn(*args)
 
 
 def require_cuda(*tensors: torch.Tensor) -> None:
