@@ -75,10 +75,11 @@ __device__ __forceinline__ void build_rows(const Warp<BITS, G, GQA>& w, const ui
         dst[1] = fmaf(u[1] < 0.f ? Bdn : Bup, u[1], A);
       }
     } else {
-      const float inv_a = 1.0f / alpha;
+      // value of code e, n = e - zc: (A - cup) + cup * 2^(n kup) from the zero code on, (A + cdn) - cdn * 2^(-n kdn) below
       const int up = max(TOP - zc, 1), dn = max(zc, 1);
-      *(float4*)dst = make_float4(A, Bup * inv_a, Bdn * inv_a, lg2a / (float)up);
-      *(float4*)(dst + 4) = make_float4(lg2a / (float)dn, __int_as_float(zc), 0.f, 0.f);
+      const float inv_a = __fdividef(1.0f, alpha), cup = Bup * inv_a, cdn = Bdn * inv_a;
+      *(float4*)dst = make_float4(8388608.0f + (float)zc, __fdividef(lg2a, (float)up), -__fdividef(lg2a, (float)dn), cup);
+      *(float4*)(dst + 4) = make_float4(-cdn, A - cup, A + cdn, 0.f);
     }
   }
 }

@@ -136,8 +136,8 @@ __device__ __forceinline__ unsigned long long load_codes(const uint8_t* row, int
 // N codes -> N values.  `rb` is the shared-window address of the expansion rows of the current
 // unrolled block (256-byte aligned), `lane_off` (< 256, multiple of ROW_BYTES) the byte offset of
 // this lane's row inside a step, IMM the byte offset of the step.
-// BOOKS: the row is a codebook.  Otherwise it holds {A, Bup, Bdn, kup, kdn, zero_code, -, -}:
-// value = A + Bup*(2^(n*kup)-1) above the zero code, A - Bdn*(2^(n*kdn)-1) below it.
+// BOOKS: the row is a codebook.  Otherwise it holds {2^23 + zero code, kup, -kdn, cup, -cdn, A - cup, A + cdn, -}:
+// value = (A - cup) + cup * 2^(n kup) from the zero code on, (A + cdn) - cdn * 2^(-n kdn) below it (n = code - zero code).
 template <int BITS, bool BOOKS, bool PRMT, int N, int IMM>
 __device__ __forceinline__ void expand(unsigned long long codes, uint32_t rb, uint32_t lane_off, float (&v)[N]) {
   constexpr unsigned MASK = (1u << BITS) - 1u;
@@ -163,13 +163,16 @@ __device__ __forceinline__ void expand(unsigned long long codes, uint32_t rb, ui
   } else {
     const float4 a = lds_f32x4<IMM>(rb + lane_off);
     const float4 b = lds_f32x4<IMM + 16>(rb + lane_off);
-    const int zc = __float_as_int(b.y);
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-      const int c = (int)((codes >> (BITS * k)) & MASK);
-      const int n = c - zc;
-      const float e = n >= 0 ? ex2f((float)n * a.w) : ex2f((float)(-n) * b.x);
-      v[k] = n >= 0 ? fmaf(a.y, e - 1.0f, a.x) : fmaf(-a.z, e - 1.0f, a.x);
+      // 2^23 + code as a float: the code's bits under the exponent of 2^23 (one byte permute for 8 bits)
+      uint32_t f;
+      if (BITS == 8) f = prmt(k < 4 ? (uint32_t)codes : (uint32_t)(codes >> 32), 0x4B000000u, 0x7440u | (uint32_t)(k & 3));
+      else f = ((uint32_t)(codes >> (BITS * k)) & MASK) | 0x4B000000u;
+      const float n = __uint_as_float(f) - a.x;
+      const bool up = n >= 0.0f;
+      const float x = ex2f(n * (up ? a.y : a.z));
+      v[k] = fmaf(x, up ? a.w : b.x, up ? b.y : b.z);
     }
   }
 }
