@@ -231,9 +231,10 @@ __device__ __forceinline__ void fill_tables(uint32_t table, const uint32_t* __re
 
 // ---- wide codes: (v - A) / span of code e.  Row constants {zc, kup, kdn, cup, cdn}: above the zero code
 // cup * (2^(n kup) - 1), below it cdn * (2^(n kdn) - 1) with n = |e - zc| and cdn < 0.
-struct WideRow { float zc, kup, kdn, cup, cdn; };
-__device__ __forceinline__ float wide_value(float e, const WideRow& r) {
-  const float n = e - r.zc;
+struct WideRow { float zc, kup, kdn, cup, cdn; };        // zc: 2^23 + zero code
+// f: 2^23 + code
+__device__ __forceinline__ float wide_value(float f, const WideRow& r) {
+  const float n = f - r.zc;
   const bool up = n >= 0.0f;
   const float x = ex2f(fabsf(n) * (up ? r.kup : r.kdn));
   return (x - 1.0f) * (up ? r.cup : r.cdn);
@@ -291,9 +292,9 @@ __device__ __forceinline__ void wide_side(uint32_t buf, uint32_t ri, int g, int 
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
               uint32_t e;
-              if (BITS == 8) e = ((i < 4 ? w[s].x : w[s].y) >> (8 * (i & 3))) & 0xffu;
-              else e = (uint32_t)((((unsigned long long)w[s].y << 32) | w[s].x) >> (i * bits)) & ((1u << bits) - 1u);
-              v[s] = wide_value((float)e, r[s]);
+              if (BITS == 8) e = prmt(i < 4 ? w[s].x : w[s].y, 0x4B000000u, 0x7440u | (uint32_t)(i & 3));
+              else e = ((uint32_t)((((unsigned long long)w[s].y << 32) | w[s].x) >> (i * bits)) & ((1u << bits) - 1u)) | 0x4B000000u;
+              v[s] = wide_value(__uint_as_float(e), r[s]);
             }
             split_pair(v[0], v[1], hi[rr], lo[rr]);
             split_pair(v[2], v[3], hi[2 + rr], lo[2 + rr]);
@@ -701,7 +702,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         const int blk = values ? (pos >> 4) * NG + grp : pos >> 4;
         const uint32_t at = L.ri + (blk * 4 + ((pos >> 2) & 3)) * 128 + (pos & 3) * 16;
         const float inv = __fdividef(inv_alpha, span);
-        sts128(at, make_uint4(__float_as_uint((float)zc), __float_as_uint(__fdividef(lg, (float)max(top - zc, 1))),
+        sts128(at, make_uint4(__float_as_uint(8388608.0f + (float)zc), __float_as_uint(__fdividef(lg, (float)max(top - zc, 1))),
                               __float_as_uint(__fdividef(lg, (float)max(zc, 1))), __float_as_uint(bup * inv)));
         const float sp = fminf(span, 65504.f);
         sts128(at + 64, make_uint4(__float_as_uint(-bdn * inv), h2_bits(__floats2half2_rn(sp, sp)), 0u, 0u));
