@@ -12,17 +12,19 @@
 // Both contractions run on the tensor cores (mma.sync m16n8k16, fp16 operands, fp32 accumulate):
 //   * the A operand holds table values; one code = 32 bits of a shared-memory lookup that returns the
 //     fp16 pair (u+, u-), which is one A-fragment register (the reduction index is doubled: one slot for
-//     the part above the zero code, one for the part below it).  3 and 4 bits look up one code per load; 1 and
-//     2 bits look up two neighbouring codes at once with a 64-bit load
+//     the part above the zero code, one for the part below it)
 //   * the table is replicated once per lane, so no lookup pattern can cause a bank conflict, and it sits
 //     at shared-window address 65536 with a stride of 256 bytes, so that the address of a lookup is one byte
-//     permute: byte 1 of the address <- (zc, code or pair of codes)
+//     permute: byte 1 of the address <- (zc, sub-bin, code)
 //   * the B operand holds the folded query (keys) or folded probabilities (values); its 8 columns are
-//     4 heads x {product rounded to fp16, its exact fp16 remainder (+ the remainder of the probability)};
+//     4 heads x {product rounded to fp16, its exact fp16 remainder (+ the remainders of the constant and of the
+//     probability)};
 //     5 to 8 heads per kv head use a second set of 8 columns on the same A fragments
 //   * the idle half of a table entry (u- of a code above the zero code, u+ of one below) carries the fp16
-//     remainder of the active half, pre-scaled by the nominal ratio of the two side constants of the
-//     zero-code bin, which recovers most of the table's own fp16 rounding
+//     remainder of the active half, pre-scaled by the nominal ratio of the two side constants, which recovers most
+//     of the table's own fp16 rounding.  The ratio is nominal for the zero anchor's bin: one zero code at 4 bits,
+//     a fourth / an eighth of one at 3 / 2 bits (1 bit has end bins only, where it is exact).  With the constants as
+//     value + remainder the result is within about 1e-5 of the fp32 evaluation (norms)
 //   * M rows are tokens (keys) or channels (values), permuted so that one load of packed codes
 //     feeds a thread's rows of all M tiles.
 // Codes of 5 to 8 bits have no table (2^16 entries): their value (v - A) / span is computed per code (one ex2) and
@@ -45,7 +47,6 @@ constexpr uint32_t WIDE_ROW = 32;           // row constants of a wide code: 8 w
 template <int BITS, int D_, int G_, int NT_>
 struct Cfg {
   static constexpr bool WIDE = BITS == 0 || BITS > 4;
-  static constexpr bool PAIRED = BITS == 1 || BITS == 2;       // one 64-bit lookup per two codes
   static constexpr int D = D_, G = G_, NT = NT_;
   static constexpr int NG = D / G;            // value groups of a token
   static constexpr int CPL = G / 8;           // consecutive positions of a row per lane
@@ -53,14 +54,13 @@ struct Cfg {
   static constexpr int NB = D / 8;            // reduction blocks of 8 rows per tile side (both sides have D rows)
   static constexpr int MAXW = NT == 1 ? 12 : 8;
   static constexpr int NE = 1 << (WIDE ? 1 : BITS);
-  // table: entries in 256-byte slots.  Single codes: keys' copies in the lower, values' in the upper half of a slot;
-  // pairs: a slot is one table's entry, the values' table follows the keys'
-  static constexpr int ENTRIES = WIDE ? 0 : (PAIRED ? NE * NE * NE : NE * NE);
-  static constexpr int ZSHIFT = PAIRED ? 2 * BITS : BITS;      // position of the zero code in the index byte
-  static constexpr uint32_t TABLE_BYTES = ENTRIES * 256u * (PAIRED ? 2 : 1);
+  // table: entries (zero code, sub-bin, code) in 256-byte slots, keys' copies in the lower, values' in the upper half
+  static constexpr int SUB = WIDE ? 0 : kSubBits[BITS];
+  static constexpr int ENTRIES = WIDE ? 0 : NE * NE << SUB;
+  static constexpr uint32_t TABLE_BYTES = ENTRIES * 256u;
   // row constants, and the folded-query source (the block loops are not unrolled over it)
   static constexpr uint32_t Q_BYTES = NT * NB * 64;
-  static constexpr uint32_t RI_BYTES = D * (WIDE ? WIDE_ROW : 8) + Q_BYTES;
+  static constexpr uint32_t RI_BYTES = D * (WIDE ? WIDE_ROW : 10) + Q_BYTES;       // table path: constants (8), zero-code byte, padding
   static constexpr uint32_t A_BYTES = D * 4;
   static constexpr uint32_t P_BYTES = G * 16 * NT;             // probabilities: [G/8][4 x 8 NT] half2
 };
@@ -68,20 +68,16 @@ struct Layout { uint32_t kbuf, vbuf, ri, a, pbuf, q; };
 
 // One B-operand register of a lane: x * B for the pair B = (Bup, Bdn).  mask = 0 (even column): the fp16
 // product; mask = all ones (odd column): what that rounding dropped, exactly.
-__device__ __forceinline__ uint32_t fold_pair(__half2 x, uint32_t B, uint32_t mask) {
+// `lo` is the remainder of the constants, `xm` = x in the odd columns, else 0.
+__device__ __forceinline__ uint32_t fold_pair(__half2 x, __half2 xm, uint32_t B, uint32_t lo, uint32_t mask) {
   const uint32_t h = h2_bits(__hmul2(x, bits_h2(B))) & mask;
-  return h2_bits(__hfma2(x, bits_h2(B), __hneg2(bits_h2(h))));
+  return h2_bits(__hfma2(xm, bits_h2(lo), __hfma2(x, bits_h2(B), __hneg2(bits_h2(h)))));
 }
 
 // table lookups: the table never changes after the fill, so the compiler may move them freely
 __device__ __forceinline__ uint32_t tab32(uint32_t a) {
   uint32_t v;
   asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ uint2 tab64(uint32_t a) {
-  uint2 v;
-  asm("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
   return v;
 }
 __device__ __forceinline__ uint32_t pack_u16(uint32_t lo, uint32_t hi) { return prmt(lo, hi, 0x5410u); }
@@ -142,10 +138,10 @@ struct Quad<3, CPL> {
     }
   }
 };
-// 2-bit codes: a nibble is the pair of positions (2m, 2m + 1) of M tile m
+// 2-bit codes: 8 positions = 16 bits; byte 2 slot + h of c[k] is position 4 h + k
 template <int CPL>
 struct Quad<2, CPL> {
-  uint32_t w;                 // low half: slot 0, high half: slot 1 (four nibbles each, two when the group is 32)
+  uint32_t w;                 // low half: slot 0, high half: slot 1
   __device__ __forceinline__ void load(uint32_t row0, uint32_t row1, int q) {
     if (CPL == 4) w = pack_u16(lds8(row0), lds8(row1));
     else w = pack_u16(lds16(row0 + 2 * q), lds16(row1 + 2 * q));
@@ -153,35 +149,36 @@ struct Quad<2, CPL> {
   template <int NA>
   __device__ __forceinline__ void look(uint32_t z0, uint32_t z1, uint32_t base, uint32_t (&a)[NA]) const {
     const uint32_t z = pack_u16(z0, z1);
-    const uint32_t c[2] = {(w & 0x0F0F0F0Fu) | z, ((w >> 4) & 0x0F0F0F0Fu) | z};
 #pragma unroll
-    for (int m = 0; m < NA / 4; ++m)
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t c = ((w >> (2 * k)) & 0x03030303u) | z;
 #pragma unroll
-      for (int slot = 0; slot < 2; ++slot) {
-        const uint2 v = tab64(prmt(c[m & 1], base, 0x7604u | (uint32_t)((2 * slot + (m >> 1)) << 4)));
-        a[4 * m + 2 * slot] = v.x; a[4 * m + 2 * slot + 1] = v.y;
-      }
+      for (int h = 0; h < NA / 8; ++h)
+#pragma unroll
+        for (int slot = 0; slot < 2; ++slot)
+          a[4 * (2 * h + (k >> 1)) + 2 * slot + (k & 1)] = tab32(prmt(c, base, 0x7604u | (uint32_t)((2 * slot + h) << 4)));
+    }
   }
 };
-// 1-bit codes: two bits are the pair of M tile m
+// 1-bit codes: 8 positions = one byte, spread like the 2-bit ones
 template <int CPL>
 struct Quad<1, CPL> {
-  uint32_t w;                 // byte 0: slot 0, byte 2: slot 1
+  uint32_t w;                 // bytes: slot 0 positions 0.., 4.., slot 1 positions 0.., 4..
   __device__ __forceinline__ void load(uint32_t row0, uint32_t row1, int q, int g = 0) {
-    w = pack_u16(lds8(row0 + q), lds8(row1 + q));
-    if (CPL == 4) w = (w >> (4 * (g & 1))) & 0x000F000Fu;
+    const uint32_t sh = CPL == 4 ? 4 * (g & 1) : 0, b0 = lds8(row0 + q) >> sh, b1 = lds8(row1 + q) >> sh, b = pack_u16(b0, b1);
+    w = prmt(b, b >> 4, 0x6240u);
   }
   template <int NA>
   __device__ __forceinline__ void look(uint32_t z0, uint32_t z1, uint32_t base, uint32_t (&a)[NA]) const {
     const uint32_t z = pack_u16(z0, z1);
 #pragma unroll
-    for (int m = 0; m < NA / 4; ++m) {
-      const uint32_t c = ((w >> (2 * m)) & 0x03030303u) | z;
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t c = ((w >> k) & 0x01010101u) | z;
 #pragma unroll
-      for (int slot = 0; slot < 2; ++slot) {
-        const uint2 v = tab64(prmt(c, base, 0x7604u | (uint32_t)((2 * slot) << 4)));
-        a[4 * m + 2 * slot] = v.x; a[4 * m + 2 * slot + 1] = v.y;
-      }
+      for (int h = 0; h < NA / 8; ++h)
+#pragma unroll
+        for (int slot = 0; slot < 2; ++slot)
+          a[4 * (2 * h + (k >> 1)) + 2 * slot + (k & 1)] = tab32(prmt(c, base, 0x7604u | (uint32_t)((2 * slot + h) << 4)));
     }
   }
 };
@@ -194,36 +191,31 @@ __device__ __forceinline__ uint32_t lane_offset(int g) {
   return (uint32_t)(g * (CPL * BITS)) >> 3;
 }
 
-// ---- the lookup table, from the entries [2][NE * NE] = (keys' alpha, values' alpha) in global memory (nullptr: they
+// ---- the lookup table, from the entries [2][ENTRIES] = (keys' alpha, values' alpha) in global memory (nullptr: they
 // are computed here).  A thread takes whole entries: the loads of up to four are in flight together (one by one their
 // latency was most of a small call), then 16-byte stores of the copies, rotated so that eight neighbouring threads hit
 // eight different bank groups.
 template <class C, int BITS>
 __device__ __forceinline__ void fill_tables(uint32_t table, const uint32_t* __restrict__ lut, float alpha_key, float alpha_value) {
-  constexpr int NE2 = C::NE * C::NE, PER = C::PAIRED ? C::ENTRIES : NE2, COPIES = C::PAIRED ? 16 : 8;
+  constexpr int PER = C::ENTRIES, COPIES = 8;
   const int n = alpha_key == alpha_value ? PER : 2 * PER;
   auto entry = [&](int which, int idx) {
-    return lut != nullptr ? lut[which * NE2 + idx] : lookup_entry<BITS>(which ? alpha_value : alpha_key, idx);
+    return lut != nullptr ? lut[which * PER + idx] : lookup_entry<BITS, C::SUB>(which ? alpha_value : alpha_key, idx);
   };
   for (int i0 = threadIdx.x; i0 < n; i0 += 4 * blockDim.x) {
-    uint2 v[4];
+    uint32_t v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int i = min(i0 + k * (int)blockDim.x, n - 1), which = i / PER, idx = i % PER;
-      if (C::PAIRED) {
-        const int zc = (idx >> (2 * BITS)) << BITS;
-        v[k] = make_uint2(entry(which, zc | (idx & (C::NE - 1))), entry(which, zc | ((idx >> BITS) & (C::NE - 1))));
-      } else {
-        v[k].x = v[k].y = entry(which, idx);
-      }
+      v[k] = entry(which, idx);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int i = i0 + k * blockDim.x, which = i / PER, idx = i % PER;
       if (i < n) {
-        const uint32_t row = C::PAIRED ? table + (which * PER + idx) * 256 : table + idx * 256 + which * 128;
+        const uint32_t row = table + idx * 256 + which * 128;
 #pragma unroll
-        for (int c = 0; c < COPIES; ++c) sts128(row + (((c + threadIdx.x) & (COPIES - 1)) << 4), make_uint4(v[k].x, v[k].y, v[k].x, v[k].y));
+        for (int c = 0; c < COPIES; ++c) sts128(row + (((c + threadIdx.x) & (COPIES - 1)) << 4), make_uint4(v[k], v[k], v[k], v[k]));
       }
     }
   }
@@ -630,10 +622,9 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
   L.q = L.ri + C::RI_BYTES - C::Q_BYTES;
   L.a = L.ri + C::RI_BYTES;
   L.pbuf = L.a + C::A_BYTES;
-  const uint32_t lbK = window + TBL + lane * (C::PAIRED ? 8 : 4);
-  const uint32_t lbV = lbK + (s.alpha_key == s.alpha_value ? 0u : C::PAIRED ? C::ENTRIES * 256u : 128u);
-  // the values' table of pairs starts ENTRIES slots after the keys': an offset of the index byte
-  const uint32_t zaddV = C::PAIRED && s.alpha_key != s.alpha_value ? (uint32_t)C::ENTRIES * 0x01010101u : 0u;
+  const uint32_t lbK = window + TBL + lane * 4;
+  // equal alphas: the fill wrote one table, to the lower half of the slots
+  const uint32_t lbV = lbK + (s.alpha_key == s.alpha_value ? 0u : 128u);
   const int hq = g >> 1;                       // head (of each column set) this lane folds for (B operand column g)
   const uint32_t rem_mask = (g & 1) ? 0xFFFFFFFFu : 0u;   // odd columns carry the fp16 remainder of the folded query
   const bool bf = s.kv_dtype == MZ_BF16;
@@ -696,7 +687,8 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         span = mz_u16_to_float((uint16_t)lds16(buf + CODE_BYTES + D * 2 + r * 2), s.meta_dtype);
       }
     };
-    auto put_row = [&](int r, float span, float bup, float bdn, int zc) {
+    // frac: position of the anchor inside the bin of its zero code, [-0.5, 0.5]
+    auto put_row = [&](int r, float span, float bup, float bdn, int zc, float frac) {
       const int pos = values ? r / NG : r, grp = values ? r % NG : 0;
       if (C::WIDE) {
         const int blk = values ? (pos >> 4) * NG + grp : pos >> 4;
@@ -705,16 +697,21 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         sts128(at, make_uint4(__float_as_uint(8388608.0f + (float)zc), __float_as_uint(__fdividef(lg, (float)max(top - zc, 1))),
                               __float_as_uint(__fdividef(lg, (float)max(zc, 1))), __float_as_uint(bup * inv)));
         const float sp = fminf(span, 65504.f);
-        sts128(at + 64, make_uint4(__float_as_uint(-bdn * inv), h2_bits(__floats2half2_rn(sp, sp)), 0u, 0u));
+        const __half sh = __float2half_rn(sp);
+        sts128(at + 64, make_uint4(__float_as_uint(-bdn * inv), pack_u16(__half_as_ushort(sh), __half_as_ushort(__float2half_rn(sp - __half2float(sh)))), 0u, 0u));
       } else {
         // a row whose zero code is the first / last code has no codes on the other side: that side's constant only
         // ever multiplies the remainder half of the table entries
         if (zc == 0) bdn = bup;
         if (zc == top) bup = bdn;
         const int blk = values ? (pos >> 3) * NG + grp : pos >> 3;
-        const uint32_t z = ((uint32_t)zc << C::ZSHIFT) * 0x01010101u + (values ? zaddV : 0u);
-        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(L.ri + ((blk * 4 + (pos & 3)) * 2 + ((pos >> 2) & 1)) * 8),
-                     "r"(h2_bits(__floats2half2_rn(bup, bdn))), "r"(z) : "memory");
+        constexpr int SB = 1 << C::SUB;
+        const int zi = zc * SB + (SB > 1 ? min(max((int)((frac + 0.5f) * (float)SB), 0), SB - 1) : 0);
+        const __half2 hi = __floats2half2_rn(bup, bdn);
+        const float2 hf = __half22float2(hi);
+        const uint32_t lo = h2_bits(__floats2half2_rn(bup - hf.x, bdn - hf.y)), at = (blk * 4 + (pos & 3)) * 2 + ((pos >> 2) & 1);
+        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(L.ri + at * 8), "r"(h2_bits(hi)), "r"(lo) : "memory");
+        sts8(L.ri + D * 8 + at, (uint32_t)(zi << BITS));
       }
     };
     float A[D / 32];
@@ -724,10 +721,11 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
       const int r = lane + 32 * i;
       float lo, span, bup, bdn;
       int zc;
+      float frac;
       load_row(r, lo, span);
-      row_split(lo, span, (float)top, A[i], bup, bdn, zc, wild);
+      row_split(lo, span, (float)top, A[i], bup, bdn, zc, wild, &frac);
       any |= A[i] != 0.0f;
-      put_row(r, fmaxf(span, 1e-8f), bup, bdn, zc);
+      put_row(r, fmaxf(span, 1e-8f), bup, bdn, zc, frac);
     }
     if (__any_sync(0xffffffffu, wild)) {
 #pragma unroll 1
@@ -737,7 +735,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         int zc;
         load_row(r, lo, span);
         row_split(lo, span, (float)top, a, bup, bdn, zc, wild);
-        put_row(r, fmaxf(span, 1e-8f), bup, bdn, exact_zero_code(lo, span, (float)top));
+        put_row(r, fmaxf(span, 1e-8f), bup, bdn, exact_zero_code(lo, span, (float)top), 0.0f);
       }
     }
     any = __any_sync(0xffffffffu, any);
@@ -921,7 +919,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         constexpr int NS = NB * NQ, SPI = 2 * NQ;
         Quad<BITS, CPL> cw[2];
         uint4 rc[2];
-        uint32_t qq[2][NT], av[2][NA], bfr[2][NT][2];
+        uint32_t zz[2], qq[2][NT], av[2][NA], bfr[2][NT][2];
         auto load_step = [&](int blk, int u) {            // u: static step number, blk: its block
           const int q = u % NQ;
           const uint32_t r0 = L.kbuf + (8 * blk + t) * QB + lane_offset<BITS, CPL>(g);
@@ -929,18 +927,20 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
           else cw[u & 1].load(r0, r0 + 4 * QB, q);
           if (q == 0) {
             rc[(u / NQ) & 1] = lds128(L.ri + (blk * 4 + t) * 16);
+            zz[(u / NQ) & 1] = lds16(L.ri + D * 8 + (blk * 4 + t) * 2);
 #pragma unroll
             for (int n = 0; n < NT; ++n) qq[(u / NQ) & 1][n] = lds32(L.q + (n * NB + blk) * 64 + (hq * 4 + t) * 4);
           }
         };
         auto open_step = [&](int u) {
           const uint4& c = rc[(u / NQ) & 1];
-          cw[u & 1].look(c.y, c.w, lbK, av[u & 1]);
+          cw[u & 1].look(prmt(zz[(u / NQ) & 1], 0u, 0x0000u), prmt(zz[(u / NQ) & 1], 0u, 0x1111u), lbK, av[u & 1]);
           // fold q * B: even columns the product rounded to fp16, odd columns what that rounding dropped
 #pragma unroll
           for (int n = 0; n < NT; ++n) {
-            bfr[u & 1][n][0] = fold_pair(dup_lo(qq[(u / NQ) & 1][n]), c.x, rem_mask);
-            bfr[u & 1][n][1] = fold_pair(dup_hi(qq[(u / NQ) & 1][n]), c.z, rem_mask);
+            const uint32_t x = qq[(u / NQ) & 1][n], xm = x & rem_mask;
+            bfr[u & 1][n][0] = fold_pair(dup_lo(x), dup_lo(xm), c.x, c.y, rem_mask);
+            bfr[u & 1][n][1] = fold_pair(dup_hi(x), dup_hi(xm), c.z, c.w, rem_mask);
           }
         };
         load_step(0, 0);
@@ -968,7 +968,10 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
           for (int n = 0; n < NT; ++n)
 #pragma unroll
             for (int k = 0; k < 2; ++k)
-              bb[n][k] = fold_pair(bits_h2(lds32(L.q + (n * NB + 2 * blk + k) * 64 + (hq * 4 + t) * 4)), pack_u16(sp[2 * k], sp[2 * k + 1]), rem_mask);
+            {
+              const uint32_t x = lds32(L.q + (n * NB + 2 * blk + k) * 64 + (hq * 4 + t) * 4);
+              bb[n][k] = fold_pair(bits_h2(x), bits_h2(x & rem_mask), pack_u16(sp[2 * k], sp[2 * k + 1]), prmt(sp[2 * k], sp[2 * k + 1], 0x7632u), rem_mask);
+            }
         }, [&](int, int m, const uint32_t (&a)[4], const uint32_t (&bb)[NT][2]) {
 #pragma unroll
           for (int n = 0; n < NT; ++n) mma_f16(acc[n][m], a[0], a[1], a[2], a[3], bb[n][0], bb[n][1]);
@@ -1063,7 +1066,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         constexpr int NS = NB * NQ, BPI = NG > 2 ? NG : 2, SPI = BPI * NQ;       // blocks and steps of an iteration
         Quad<BITS, CPL> cw[2];
         uint4 rc[2];
-        uint32_t av[2][NA], bfr[2][NT][2], ph[2][NT], pl[2][NT];
+        uint32_t zz[2], av[2][NA], bfr[2][NT][2], ph[2][NT], pl[2][NT];
         auto load_step = [&](int blk, int u) {
           const int q = u % NQ, grp = (u / NQ) % NG, j = blk / NG;
           const uint32_t r0 = L.vbuf + (8 * j + t) * v_row + grp * v_grp + lane_offset<BITS, CPL>(g);
@@ -1071,6 +1074,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
           else cw[u & 1].load(r0, r0 + 4 * v_row, q);
           if (q == 0) {
             rc[(u / NQ) & 1] = lds128(L.ri + (blk * 4 + t) * 16);
+            zz[(u / NQ) & 1] = lds16(L.ri + D * 8 + (blk * 4 + t) * 2);
             if (grp == 0) {
 #pragma unroll
               for (int n = 0; n < NT; ++n) probs(n, j, ph[(u / NQ / NG) & 1][n], pl[(u / NQ / NG) & 1][n]);
@@ -1079,13 +1083,14 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         };
         auto open_step = [&](int u) {
           const uint4& c = rc[(u / NQ) & 1];
-          cw[u & 1].look(c.y, c.w, lbV, av[u & 1]);
+          cw[u & 1].look(prmt(zz[(u / NQ) & 1], 0u, 0x0000u), prmt(zz[(u / NQ) & 1], 0u, 0x1111u), lbV, av[u & 1]);
           // fold (ph + pl) * B: even columns fp16(ph * B), odd columns its remainder + pl * B
 #pragma unroll
           for (int n = 0; n < NT; ++n) {
             const uint32_t hi = ph[(u / NQ / NG) & 1][n], lo = pl[(u / NQ / NG) & 1][n];
-            bfr[u & 1][n][0] = h2_bits(__hfma2(dup_lo(lo), bits_h2(c.x), bits_h2(fold_pair(dup_lo(hi), c.x, rem_mask))));
-            bfr[u & 1][n][1] = h2_bits(__hfma2(dup_hi(lo), bits_h2(c.z), bits_h2(fold_pair(dup_hi(hi), c.z, rem_mask))));
+            const uint32_t hm = hi & rem_mask;
+            bfr[u & 1][n][0] = h2_bits(__hfma2(dup_lo(lo), bits_h2(c.x), bits_h2(fold_pair(dup_lo(hi), dup_lo(hm), c.x, c.y, rem_mask))));
+            bfr[u & 1][n][1] = h2_bits(__hfma2(dup_hi(lo), bits_h2(c.z), bits_h2(fold_pair(dup_hi(hi), dup_hi(hm), c.z, c.w, rem_mask))));
           }
         };
         // two iterations are unrolled where a token block's probabilities alternate between two registers across them
@@ -1120,7 +1125,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
               uint32_t hi, lo;
               probs(n, 2 * j + k, hi, lo);
               const uint32_t S = pack_u16(sp[2 * k], sp[2 * k + 1]);
-              bb[n][k] = h2_bits(__hfma2(bits_h2(lo), bits_h2(S), bits_h2(fold_pair(bits_h2(hi), S, rem_mask))));
+              bb[n][k] = h2_bits(__hfma2(bits_h2(lo), bits_h2(S), bits_h2(fold_pair(bits_h2(hi), bits_h2(hi & rem_mask), S, prmt(sp[2 * k], sp[2 * k + 1], 0x7632u), rem_mask))));
             }
         }, [&](int k, int m, const uint32_t (&a)[4], const uint32_t (&bb)[NT][2]) {
 #pragma unroll

@@ -83,13 +83,15 @@ __device__ __forceinline__ __half2 dup_hi(uint32_t v) { return __half2half2(__hi
 // of an entry carries the fp16 remainder of the active half, pre-scaled by the nominal ratio Bdn / Bup of a row
 // in that zero-code bin (anchor at the bin centre); the end bins have codes on one side only and row_constants
 // makes their two constants equal.  Called by every thread of the CTA; the caller synchronises afterwards.
-// entry idx = (zc << BITS | e) of the table for `alpha`, as the bits of half2(u+, u-)
-template <int BITS>
+// sub-bins of a zero code's anchor range in the general kernel's table, by code width (log2)
+constexpr int kSubBits[5] = {0, 0, 3, 2, 0};
+// entry idx = (zc, sub-bin, e) of the table for `alpha`, as the bits of half2(u+, u-)
+template <int BITS, int SUB = 0>
 __device__ __forceinline__ uint32_t lookup_entry(float alpha, int idx) {
-  constexpr int NE = 1 << BITS, TOP = NE - 1;
-  const int zc = idx >> BITS, e = idx & TOP;
+  constexpr int NE = 1 << BITS, TOP = NE - 1, SB = 1 << SUB;
+  const int zc = idx >> (BITS + SUB), e = idx & TOP;
   const float lb = log1pf(alpha);
-  const float zac = (float)zc / (float)TOP;
+  const float zac = ((float)zc + (((float)((idx >> BITS) & (SB - 1)) + 0.5f) / (float)SB - 0.5f)) / (float)TOP;    // middle of the bin
   const float ratio = (zc == 0 || zc == TOP) ? 1.0f : zac / (1.0f - zac);
   __half2 ent;
   if (e >= zc) {
@@ -161,7 +163,8 @@ __device__ __forceinline__ void row_constants(float lo, float span, int& zc, flo
 // an ulp of b/s, q + (b - q s) y rounds to RN(b/s)); that is branch-free, where the IEEE division costs a range test and a
 // slow path per row.  Ties matter: 16-bit extremes often give a quotient that lies exactly on a code boundary.
 // Spans from 2^125 on would flush the reciprocal: `wild` asks for the division.
-__device__ __forceinline__ void row_split(float lo, float span, float top, float& A, float& bup, float& bdn, int& zc, bool& wild) {
+__device__ __forceinline__ void row_split(float lo, float span, float top, float& A, float& bup, float& bdn, int& zc, bool& wild,
+                                          float* frac = nullptr) {
   span = fmaxf(span, 1e-8f);
   bdn = fminf(fmaxf(-lo, 0.0f), span);
   bup = span - bdn;
@@ -171,7 +174,9 @@ __device__ __forceinline__ void row_split(float lo, float span, float top, float
   y = fmaf(fmaf(-span, y, 1.0f), y, y);
   const float q0 = bdn * y;
   const float q = fmaf(fmaf(-q0, span, bdn), y, q0);
-  zc = __float_as_int(__fmul_rn(q, top) + 12582912.0f) & 0xff;
+  const float pos = __fmul_rn(q, top), r = pos + 12582912.0f;
+  zc = __float_as_int(r) & 0xff;
+  if (frac != nullptr) *frac = pos - (r - 12582912.0f);
   wild |= !(span < 4e37f);
   bup = fminf(bup, 65504.f);
   bdn = fminf(bdn, 65504.f);
