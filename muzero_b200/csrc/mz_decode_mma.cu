@@ -28,6 +28,13 @@ __global__ void build_lut_kernel(int slot, float alpha_key, float alpha_value) {
   constexpr int N = 1 << (2 * BITS + SUB);
   for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) g_lut[slot][i] = lookup_entry<BITS, SUB>(i / N ? alpha_value : alpha_key, i % N);
 }
+// 4 bits, equal alphas: [sub-bin][zero code, code]
+__global__ void build_twin_lut_kernel(int slot, float alpha) {
+  for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+    const int idx = i & 255;
+    g_lut[slot][i] = lookup_entry<4, 1>(alpha, (((idx >> 4) * 2 + (i >> 8)) << 4) | (idx & 15));
+  }
+}
 struct LutKey { int bits, sub; float ak, av; };
 struct LutDevice { uint32_t* base; int used; LutKey keys[kLutSlots]; };
 LutDevice g_lut_dev[kMaxDevices];
@@ -60,7 +67,8 @@ const unsigned* mz_mma_lookup_entries(int bits, int sub, float alpha_key, float 
   else if (bits == 2 && sub == 0) mzm::build_lut_kernel<2, 0><<<1, 32>>>(slot, alpha_key, alpha_value);
   else if (bits == 2) mzm::build_lut_kernel<2, mzm::kSubBits[2]><<<1, 256>>>(slot, alpha_key, alpha_value);
   else if (bits == 3) mzm::build_lut_kernel<3, mzm::kSubBits[3]><<<1, 256>>>(slot, alpha_key, alpha_value);
-  else mzm::build_lut_kernel<4, 0><<<1, 256>>>(slot, alpha_key, alpha_value);
+  else if (sub == 0) mzm::build_lut_kernel<4, 0><<<1, 256>>>(slot, alpha_key, alpha_value);
+  else mzm::build_twin_lut_kernel<<<1, 256>>>(slot, alpha_key);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
     (void)cudaGetLastError();
     return nullptr;
@@ -284,7 +292,7 @@ int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slo
   p.cluster = 0;
   MzMmaKernel k;
   if (!find_kernel(p, &k)) return mz_fail(MZ_ERR_UNSUPPORTED, "no tensor-core kernel for this shape");
-  p.lut = s.k_groups > 0 && s.bits <= 4 ? mz_mma_lookup_entries(s.bits, mzm::kSubBits[s.bits], s.alpha_key, s.alpha_value) : nullptr;
+  p.lut = s.k_groups > 0 && s.bits <= 4 ? mz_mma_lookup_entries(s.bits, s.bits == 4 && s.alpha_key == s.alpha_value ? 1 : mzm::kSubBits[s.bits], s.alpha_key, s.alpha_value) : nullptr;
   if (splits_request == 0 && plan_cluster(p, k, sm_count)) {
     *slots = 4;                                   // no records; a workspace is still asked for, so that its size is never 0
     return MZ_OK;

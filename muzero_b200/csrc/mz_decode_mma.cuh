@@ -22,8 +22,9 @@
 //     5 to 8 heads per kv head use a second set of 8 columns on the same A fragments
 //   * the idle half of a table entry (u- of a code above the zero code, u+ of one below) carries the fp16
 //     remainder of the active half, pre-scaled by the nominal ratio of the two side constants, which recovers most
-//     of the table's own fp16 rounding.  The ratio is nominal for the zero anchor's bin: one zero code at 4 bits,
-//     a fourth / an eighth of one at 3 / 2 bits (1 bit has end bins only, where it is exact).  With the constants as
+//     of the table's own fp16 rounding.  The ratio is nominal for the zero anchor's bin: half of a zero code's range at
+//     4 bits (all of it when the alphas of keys and values differ), a fourth / an eighth at 3 / 2 bits (1 bit has end bins
+//     only, where it is exact).  With the constants as
 //     value + remainder the result is within about 1e-5 of the fp32 evaluation (norms)
 //   * M rows are tokens (keys) or channels (values), permuted so that one load of packed codes
 //     feeds a thread's rows of all M tiles.
@@ -56,6 +57,7 @@ struct Cfg {
   static constexpr int NE = 1 << (WIDE ? 1 : BITS);
   // table: entries (zero code, sub-bin, code) in 256-byte slots, keys' copies in the lower, values' in the upper half
   static constexpr int SUB = WIDE ? 0 : kSubBits[BITS];
+  static constexpr bool TWIN = BITS == 4;      // no room in the index byte: the other half of a slot is the second sub-bin
   static constexpr int ENTRIES = WIDE ? 0 : NE * NE << SUB;
   static constexpr uint32_t TABLE_BYTES = ENTRIES * 256u;
   // row constants, and the folded-query source (the block loops are not unrolled over it)
@@ -97,12 +99,12 @@ struct Quad<4, CPL> {
     else { w0 = lds32(row0 + 4 * q); w1 = lds32(row1 + 4 * q); }
   }
   template <int NA>
-  __device__ __forceinline__ void look(uint32_t z0, uint32_t z1, uint32_t base, uint32_t (&a)[NA]) const {
+  __device__ __forceinline__ void look(uint32_t z0, uint32_t z1, uint32_t base0, uint32_t base1, uint32_t (&a)[NA]) const {
     const uint32_t c[4] = {(w0 & 0x0F0F0F0Fu) | z0, ((w0 >> 4) & 0x0F0F0F0Fu) | z0, (w1 & 0x0F0F0F0Fu) | z1, ((w1 >> 4) & 0x0F0F0F0Fu) | z1};
 #pragma unroll
     for (int m = 0; m < NA / 4; ++m)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) a[4 * m + k] = tab32(prmt(c[k], base, 0x7604u | (uint32_t)(m << 4)));
+      for (int k = 0; k < 4; ++k) a[4 * m + k] = tab32(prmt(c[k], k < 2 ? base0 : base1, 0x7604u | (uint32_t)(m << 4)));
   }
 };
 // 3-bit codes: 8 positions = 24 bits at any bit address
@@ -191,6 +193,17 @@ __device__ __forceinline__ uint32_t lane_offset(int g) {
   return (uint32_t)(g * (CPL * BITS)) >> 3;
 }
 
+// the table values of a step; zz: zero-code bytes of slot 0 and 1 (4 bits: bit 0 of a byte is the sub-bin = bit 7 of the address)
+template <class C, class Q, int NA>
+__device__ __forceinline__ void look_step(const Q& w, uint32_t zz, uint32_t base, uint32_t (&a)[NA]) {
+  if constexpr (C::TWIN) {
+    const uint32_t z = zz & 0xF0F0u;
+    w.look(prmt(z, 0u, 0x0000u), prmt(z, 0u, 0x1111u), base | ((zz & 1u) << 7), base | ((zz >> 1) & 128u), a);
+  } else {
+    w.look(prmt(zz, 0u, 0x0000u), prmt(zz, 0u, 0x1111u), base, a);
+  }
+}
+
 // ---- the lookup table, from the entries [2][ENTRIES] = (keys' alpha, values' alpha) in global memory (nullptr: they
 // are computed here).  A thread takes whole entries: the loads of up to four are in flight together (one by one their
 // latency was most of a small call), then 16-byte stores of the copies, rotated so that eight neighbouring threads hit
@@ -198,9 +211,13 @@ __device__ __forceinline__ uint32_t lane_offset(int g) {
 template <class C, int BITS>
 __device__ __forceinline__ void fill_tables(uint32_t table, const uint32_t* __restrict__ lut, float alpha_key, float alpha_value) {
   constexpr int PER = C::ENTRIES, COPIES = 8;
-  const int n = alpha_key == alpha_value ? PER : 2 * PER;
+  // equal alphas: one table, in the lower halves; at 4 bits the upper halves then hold its second sub-bin
+  const bool one = alpha_key == alpha_value, twin = one && C::TWIN;
+  const int n = one && !twin ? PER : 2 * PER;
   auto entry = [&](int which, int idx) {
-    return lut != nullptr ? lut[which * PER + idx] : lookup_entry<BITS, C::SUB>(which ? alpha_value : alpha_key, idx);
+    if (lut != nullptr) return lut[which * PER + idx];
+    if (twin) return lookup_entry<BITS, 1>(alpha_key, (((idx >> BITS) * 2 + which) << BITS) | (idx & (C::NE - 1)));
+    return lookup_entry<BITS, C::SUB>(which ? alpha_value : alpha_key, idx);
   };
   for (int i0 = threadIdx.x; i0 < n; i0 += 4 * blockDim.x) {
     uint32_t v[4];
@@ -624,7 +641,8 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
   L.pbuf = L.a + C::A_BYTES;
   const uint32_t lbK = window + TBL + lane * 4;
   // equal alphas: the fill wrote one table, to the lower half of the slots
-  const uint32_t lbV = lbK + (s.alpha_key == s.alpha_value ? 0u : 128u);
+  const bool one_alpha = s.alpha_key == s.alpha_value;
+  const uint32_t lbV = lbK + (one_alpha ? 0u : 128u);
   const int hq = g >> 1;                       // head (of each column set) this lane folds for (B operand column g)
   const uint32_t rem_mask = (g & 1) ? 0xFFFFFFFFu : 0u;   // odd columns carry the fp16 remainder of the folded query
   const bool bf = s.kv_dtype == MZ_BF16;
@@ -711,7 +729,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         const float2 hf = __half22float2(hi);
         const uint32_t lo = h2_bits(__floats2half2_rn(bup - hf.x, bdn - hf.y)), at = (blk * 4 + (pos & 3)) * 2 + ((pos >> 2) & 1);
         asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(L.ri + at * 8), "r"(h2_bits(hi)), "r"(lo) : "memory");
-        sts8(L.ri + D * 8 + at, (uint32_t)(zi << BITS));
+        sts8(L.ri + D * 8 + at, (uint32_t)(zi << BITS) | (C::TWIN && one_alpha && frac >= 0.0f ? 1u : 0u));
       }
     };
     float A[D / 32];
@@ -934,7 +952,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         };
         auto open_step = [&](int u) {
           const uint4& c = rc[(u / NQ) & 1];
-          cw[u & 1].look(prmt(zz[(u / NQ) & 1], 0u, 0x0000u), prmt(zz[(u / NQ) & 1], 0u, 0x1111u), lbK, av[u & 1]);
+          look_step<C>(cw[u & 1], zz[(u / NQ) & 1], lbK, av[u & 1]);
           // fold q * B: even columns the product rounded to fp16, odd columns what that rounding dropped
 #pragma unroll
           for (int n = 0; n < NT; ++n) {
@@ -1083,7 +1101,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         };
         auto open_step = [&](int u) {
           const uint4& c = rc[(u / NQ) & 1];
-          cw[u & 1].look(prmt(zz[(u / NQ) & 1], 0u, 0x0000u), prmt(zz[(u / NQ) & 1], 0u, 0x1111u), lbV, av[u & 1]);
+          look_step<C>(cw[u & 1], zz[(u / NQ) & 1], lbV, av[u & 1]);
           // fold (ph + pl) * B: even columns fp16(ph * B), odd columns its remainder + pl * B
 #pragma unroll
           for (int n = 0; n < NT; ++n) {
