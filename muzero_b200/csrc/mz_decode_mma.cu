@@ -177,7 +177,9 @@ void describe_tiles(MzTilesPlan& t, const MzDecodeParams& p) {
   t.dense_tokens = mzm::DT;
   const int dense_tiles = (s.res_len + mzm::DT - 1) / mzm::DT;
   t.tiles_per_pair = t.packed_tiles + dense_tiles;
-  t.cost_q = kCostPacked * s.group / 64 * s.head_dim / 128;
+  // a tile of 32 tokens still prepares as many rows: measured ratios (64 x 8 pairs x 4224 tokens, 4 bits)
+  t.cost_q = s.group == 32 ? 54 : s.group == 64 ? kCostPacked : 140;
+  if (s.head_dim == 64) t.cost_q = t.cost_q * 6 / 10;
   t.cost_d = kCostDense;
   t.pair_cost = (long long)t.packed_tiles * t.cost_q + (long long)dense_tiles * t.cost_d;
   if (t.pair_cost < 1) t.pair_cost = 1;
@@ -249,10 +251,23 @@ int clusters_at_once(const MzMmaKernel& k, int cs, int threads, unsigned smem) {
   return n;
 }
 
-// Cluster mode: one cluster per pair, no partial records in memory and no merge kernel (about 4 us and a launch).  It
-// pays when a single wave of clusters carries the work and its heaviest SM is not much busier than in an even cut over
-// all SMs: the difference must stay below what the merge costs, about 11 packed tiles on one SM (4 of wide codes, which take
-// three times as long).
+// Machine-filling plans of these shapes are faster on the SIMT kernel (measured at 16 x 8 x 4000 and 40 x 8 x 2500):
+//   * codes of 5 to 8 bits, which are computed one by one, with up to 4 heads per kv head (123 against 148 us); with 8
+//     heads the SIMT kernel pays for each
+//   * groups of 32, whose tiles prepare twice the rows per token here, with few heads (1 bit: 74 against 94 us) - from
+//     4 heads on the 4-bit ones are faster here (96 against 103)
+//   * 4 bits in groups of 128 with two heads (59 against 68)
+bool simt_is_faster(const MzDecodeParams& p) {
+  if (p.gqa > 4 || !mz_decode_tiles_supported(p)) return false;
+  if (p.s.bits > 4) return true;
+  if (p.s.group == 32) return p.gqa < 4 || p.s.bits < 4;
+  return p.s.group == 128 && p.s.bits == 4 && p.gqa == 2;
+}
+
+// Cluster mode: one cluster per pair, no partial records in memory and no merge kernel.  In units of a packed tile on a
+// busy SM (0.5 us, 1.5 us of wide codes): it takes what its heaviest SM has to do, times what a tile costs here over the
+// kernel that would run otherwise; an even cut over all SMs takes its share, but at least one tile's latency (about 4 us),
+// and the merge kernel (about 4 us).
 bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count) {
   const long long pairs = (long long)p.s.batch * p.s.kv_heads;
   if (pairs > sm_count) return false;
@@ -268,8 +283,9 @@ bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count) {
     if (want < 4) want = 4;
     const int nw = layout(t, p, k, want, rec);
     if (nw < 1) return false;
-    const long long even = pairs * t.pair_cost / sm_count, heaviest = t.pair_cost / cs;
-    if (heaviest - even > (p.s.bits > 4 ? 4 : 11) * kCostPacked) return false;        // smaller clusters are heavier still
+    const long long even = pairs * t.pair_cost / sm_count, heaviest = t.pair_cost / cs, wait = (p.s.bits > 4 ? 3 : 8) * kCostPacked;
+    const int here = p.s.bits > 4 ? 100 : simt_is_faster(p) ? 128 : mz_decode_flat_supported(p) ? 116 : 100;
+    if (heaviest * here / 100 > (even > wait ? even : wait) + wait) return false;      // smaller clusters are heavier still
     if (cs > 1 && clusters_at_once(k, cs, nw * 32, t.smem_bytes) < pairs) continue;
     // tiles are dealt to the cluster's warps by cost; every warp gets at most about one residual tile's cost more than its share
     if (cut(t, 1, (long long)cs * nw) != MZ_OK) return false;
@@ -298,9 +314,7 @@ int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slo
     return MZ_OK;
   }
   p.cluster = 0;
-  // Codes of 5 to 8 bits are computed one by one, and with up to 4 heads per kv head the SIMT kernel does that with fewer
-  // instructions (16 x 8 pairs x 4000 tokens at 8 bits: 123 against 148 us); with 8 heads it pays twice for the heads.
-  if (s.bits > 4 && p.gqa <= 4 && mz_decode_tiles_supported(p)) return mz_plan_tiles(p, splits_request, sm_count, slots);
+  if (simt_is_faster(p)) return mz_plan_tiles(p, splits_request, sm_count, slots);
   if (mz_decode_flat_supported(p)) return mz_plan_flat(p, splits_request, sm_count, slots);
   const long long pairs = (long long)s.batch * s.kv_heads;
   const int dense_tiles = (s.res_len + mzm::DT - 1) / mzm::DT;
