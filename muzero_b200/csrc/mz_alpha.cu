@@ -20,6 +20,7 @@ struct AlphaParams {
   unsigned* hist; unsigned* ticket; double* partial;
   float* out;                    // {p50, p95, p99, anchor offset}
   int k50, k95, k99;             // 1-based ranks
+  int vec;                       // channel groups of whole, aligned 16-byte vectors: G / 8 lanes per group
 };
 
 __device__ __forceinline__ bool last_cta(unsigned* ticket) {
@@ -111,6 +112,30 @@ __global__ void __launch_bounds__(256) alpha_anchor_kernel(const AlphaParams p) 
       if (t1 - t0 < p.G) { lo = fminf(lo, 0.f); hi = fmaxf(hi, 0.f); }
       sum += anchor_offset(lo, hi);
     }
+  } else if (p.vec) {
+    // G / 8 lanes per group, one 16-byte load each
+    const int lpg = p.G >> 3, sub = threadIdx.x % lpg;
+    const long long per_pass = (long long)gridDim.x * (blockDim.x / lpg), passes = (groups + per_pass - 1) / per_pass;
+    long long i = (long long)blockIdx.x * (blockDim.x / lpg) + threadIdx.x / lpg;
+    for (long long k = 0; k < passes; ++k, i += per_pass) {
+      const bool live = i < groups;
+      const long long at = live ? i : 0;
+      const long long row = at / ng, pair = row / p.S;
+      const uint16_t* src = p.x + (pair / p.H) * p.sb + (pair % p.H) * p.sh + (row % p.S) * p.st + (at % ng) * p.G + sub * 8;
+      const uint4 v = *(const uint4*)src;
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float a = mz_u16_to_float((uint16_t)(w[j] & 0xffffu), p.dt), b = mz_u16_to_float((uint16_t)(w[j] >> 16), p.dt);
+        lo = fminf(lo, fminf(a, b)); hi = fmaxf(hi, fmaxf(a, b));
+      }
+      for (int off = lpg >> 1; off > 0; off >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+      }
+      if (live && sub == 0) sum += anchor_offset(lo, hi);
+    }
   } else {
     // warp = one group of one token at a time
     const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
@@ -197,6 +222,8 @@ extern "C" int mz_alpha_stats(const void* block, int dtype, const int* shape, co
     const long long groups = (long long)p.B * p.H * ng * (keys ? p.D : p.S);
     long long ctas = keys ? (groups + 255) / 256 : (groups + 63) / 64;
     if (ctas > 148 * 8) ctas = 148 * 8;
+    p.vec = !keys && p.D % group == 0 && (group & (group - 1)) == 0 && group >= 8 && group <= 256 && ((uintptr_t)block & 15) == 0 &&
+            !((p.sb | p.sh | p.st) & 7);
     if (keys) alpha_anchor_kernel<true><<<(unsigned)ctas, 256, 0, st>>>(p);
     else alpha_anchor_kernel<false><<<(unsigned)ctas, 256, 0, st>>>(p);
     MZ_LAUNCH_CHECK("alpha_anchor");
