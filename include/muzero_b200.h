@@ -176,14 +176,15 @@ int mz_dequantize_kv(const mz_kv_store* store, int g0, int g1, void* out_k,
 int mz_materialize_kv(const mz_kv_store* store, void* out_k, void* out_v, int out_dtype, float eps, void* stream);
 
 /*
- * Quantize and dequantize a 16-bit block x[B,H,S,D] (shape[4], element strides[3], innermost contiguous) in fp32
- * without keeping the codes: out[B,H,S,D] contiguous in x's type, every value through the codes of mz_quantize_rows
- * on fp32 rows, metadata rounded to meta_dtype, and the fp32 dequantizer.  keys = 1: groups of tokens (S a multiple
- * of group), 0: groups of channels (zero-padded).
+ * Quantize and dequantize a 16-bit key block and a 16-bit value block ([B,H,S,D]: shape[4], element strides[3], innermost
+ * contiguous; either may be NULL) in fp32 without keeping the codes, in one launch: out[B,H,S,D] contiguous in the blocks'
+ * type, every value through the codes of mz_quantize_rows on fp32 rows, metadata rounded to meta_dtype, and the fp32
+ * dequantizer.  Keys: groups of tokens (S a multiple of group); values: groups of channels (D a multiple of group).
  * Replaces: roundtrip, muzero/quantizer.py:273-323.
  */
-int mz_roundtrip_kv(const void* x, int dtype, const int* shape, const long long* strides, int group, int bits, float alpha,
-                    float eps, int meta_dtype, int keys, void* out, void* stream);
+int mz_roundtrip_kv(const void* k, const int* k_shape, const long long* k_strides, float alpha_key, void* k_out, const void* v,
+                    const int* v_shape, const long long* v_strides, float alpha_value, void* v_out, int dtype, int group,
+                    int bits, float eps, int meta_dtype, void* stream);
 
 /*
  * Re-indexes a whole layer cache along the batch in one launch: entry i of dst takes entry index[i] of

@@ -1,6 +1,7 @@
 // Quantize -> dequantize of a 16-bit K or V block in fp32 (the quality tool's path), without materialising fp32 rows,
 // a transposed copy, codes or metadata.  Bound by instruction issue (about 40 per value, most of them the exact
 // dequantizer); HBM traffic is the block once in and once out.
+// One launch for a K and a V block (either may be absent): the two halves fill each other's last waves.
 // Keys: thread = two neighbouring channels of 16 tokens, the parts of a channel meet in shared memory; values: thread =
 // 16 channels of one row, shuffles over the row's lanes (the layouts of the flush).
 #include "mz_quant16.cuh"
@@ -60,12 +61,9 @@ __device__ __forceinline__ const float* stage_table(const RoundtripParams& p, fl
 }
 
 template <int DT>
-__global__ void __launch_bounds__(256) roundtrip_keys_kernel(const RoundtripParams p) {
+__device__ __forceinline__ void roundtrip_keys(const RoundtripParams& p, uint32_t* s_red, float* s_row, float* s_table) {
   using P = mzq::P2<DT>;
   constexpr int TPT = 16;
-  __shared__ uint32_t s_red[1024];
-  __shared__ float s_row[(kRowFloats - 1) * 256];
-  __shared__ float s_table[256];
   const int G = p.G, D = p.D, pairs = D >> 1, parts = G / TPT, tt = pairs * parts, per_cta = tt >= 256 ? 1 : 256 / tt, rows = per_cta * D;
   const int nsg = p.S / G, tid = threadIdx.x;
   const float* table = stage_table(p, s_table);
@@ -118,13 +116,12 @@ __global__ void __launch_bounds__(256) roundtrip_keys_kernel(const RoundtripPara
 }
 
 template <int DT>
-__global__ void __launch_bounds__(256) roundtrip_values_kernel(const RoundtripParams p) {
+__device__ __forceinline__ void roundtrip_values(const RoundtripParams& p, unsigned block, float* s_table) {
   using P = mzq::P2<DT>;
-  __shared__ float s_table[256];
   const float* table = stage_table(p, s_table);
   __syncthreads();
   const int G = p.G, D = p.D, NG = D / G, lpr = G >> 4;
-  const unsigned pair = blockIdx.x / p.per_pair, chunk = blockIdx.x % p.per_pair;
+  const unsigned pair = block / p.per_pair, chunk = block % p.per_pair;
   const int row = chunk * (256 / lpr) + threadIdx.x / lpr, sub = threadIdx.x % lpr;
   const bool live = row < p.S * NG;
   uint32_t x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -152,50 +149,65 @@ __global__ void __launch_bounds__(256) roundtrip_values_kernel(const RoundtripPa
     *(uint4*)(dst + c * lpr * 8) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
-}  // namespace
 
-extern "C" int mz_roundtrip_kv(const void* x, int dtype, const int* shape, const long long* strides, int group, int bits, float alpha,
-                               float eps, int meta_dtype, int keys, void* out, void* stream) {
-  MZ_RANGE("mz_roundtrip_kv");
+template <int DT>
+__global__ void __launch_bounds__(256, 4) roundtrip_kernel(const RoundtripParams k, const RoundtripParams v, unsigned key_blocks) {
+  __shared__ uint32_t s_red[1024];
+  __shared__ float s_row[(kRowFloats - 1) * 256];
+  __shared__ float s_table[256];
+  if (blockIdx.x < key_blocks) roundtrip_keys<DT>(k, s_red, s_row, s_table);
+  else roundtrip_values<DT>(v, blockIdx.x - key_blocks, s_table);
+}
+
+// fills the parameters of one block and the CTAs it takes
+int prepare(const void* x, const int* shape, const long long* strides, int group, int bits, float alpha, float eps, int meta_dtype, int keys,
+            void* out, RoundtripParams* q, long long* blocks) {
   MZ_REQUIRE(x && shape && strides && out, "NULL pointer");
-  MZ_REQUIRE((dtype == MZ_BF16 || dtype == MZ_F16) && mz_dtype_ok(meta_dtype), "bad dtype code");
-  MZ_REQUIRE(bits >= 1 && bits <= 8, "bits must be 1..8, got %d", bits);
-  MZ_REQUIRE(alpha > 0.f && eps > 0.f, "alpha and eps must be > 0");
   MZ_REQUIRE(shape[0] > 0 && shape[1] > 0 && shape[2] > 0, "bad shape");
+  MZ_REQUIRE(alpha > 0.f && eps > 0.f, "alpha and eps must be > 0");
   const int D = shape[3], S = shape[2];
   const int unit = keys ? 1 : 7;             // element granularity of the loads
   if ((D != 64 && D != 128) || (group != 32 && group != 64 && group != 128) || D % group != 0 || (keys && S % group != 0) ||
       ((strides[0] | strides[1] | strides[2]) & unit) || ((uintptr_t)x & (keys ? 3 : 15)) || ((uintptr_t)out & 15) || S >= (1 << 27))
     return mz_fail(MZ_ERR_UNSUPPORTED, "shape served by mz_quantize_rows / mz_dequantize_rows: head_dim %d, group %d, %d tokens", D, group, S);
-  RoundtripParams p;
+  RoundtripParams& p = *q;
   p.x = (const uint16_t*)x; p.sb = strides[0]; p.sh = strides[1]; p.st = strides[2];
   p.B = shape[0]; p.H = shape[1]; p.S = S; p.D = D; p.G = group; p.bits = bits; p.meta_dtype = meta_dtype;
   p.alpha = alpha; p.eps = eps; p.out = (uint16_t*)out;
   int rc = mz_get_expand_table(bits, alpha, &p.table);
   if (rc) return rc;
   const long long pairs = (long long)p.B * p.H;
-  cudaStream_t st = (cudaStream_t)stream;
-  long long blocks;
   if (keys) {
     const int tt = (D / 2) * (group / 16), per_cta = tt >= 256 ? 1 : 256 / tt;
     const long long tiles = pairs * (S / group);
     MZ_REQUIRE(tiles < (1LL << 31), "problem too large");
     p.tiles = (unsigned)tiles; p.per_pair = 0;
-    blocks = (tiles + per_cta - 1) / per_cta;
+    *blocks = (tiles + per_cta - 1) / per_cta;
   } else {
     const int rows_per_cta = 256 / (group / 16);
     p.tiles = 0;
     p.per_pair = (unsigned)(((long long)S * (D / group) + rows_per_cta - 1) / rows_per_cta);
-    blocks = pairs * p.per_pair;
-    MZ_REQUIRE(blocks < (1LL << 31), "problem too large");
+    *blocks = pairs * p.per_pair;
   }
-  if (keys) {
-    if (dtype == MZ_BF16) roundtrip_keys_kernel<MZ_BF16><<<(unsigned)blocks, 256, 0, st>>>(p);
-    else roundtrip_keys_kernel<MZ_F16><<<(unsigned)blocks, 256, 0, st>>>(p);
-  } else {
-    if (dtype == MZ_BF16) roundtrip_values_kernel<MZ_BF16><<<(unsigned)blocks, 256, 0, st>>>(p);
-    else roundtrip_values_kernel<MZ_F16><<<(unsigned)blocks, 256, 0, st>>>(p);
-  }
+  return MZ_OK;
+}
+}  // namespace
+
+extern "C" int mz_roundtrip_kv(const void* k, const int* k_shape, const long long* k_strides, float alpha_key, void* k_out, const void* v,
+                               const int* v_shape, const long long* v_strides, float alpha_value, void* v_out, int dtype, int group, int bits,
+                               float eps, int meta_dtype, void* stream) {
+  MZ_RANGE("mz_roundtrip_kv");
+  MZ_REQUIRE((dtype == MZ_BF16 || dtype == MZ_F16) && mz_dtype_ok(meta_dtype), "bad dtype code");
+  MZ_REQUIRE(bits >= 1 && bits <= 8, "bits must be 1..8, got %d", bits);
+  MZ_REQUIRE(k != nullptr || v != nullptr, "neither keys nor values");
+  RoundtripParams pk = {}, pv = {};
+  long long kb = 0, vb = 0;
+  int rc;
+  if (k && (rc = prepare(k, k_shape, k_strides, group, bits, alpha_key, eps, meta_dtype, 1, k_out, &pk, &kb))) return rc;
+  if (v && (rc = prepare(v, v_shape, v_strides, group, bits, alpha_value, eps, meta_dtype, 0, v_out, &pv, &vb))) return rc;
+  MZ_REQUIRE(kb + vb < (1LL << 31), "problem too large");
+  if (dtype == MZ_BF16) roundtrip_kernel<MZ_BF16><<<(unsigned)(kb + vb), 256, 0, (cudaStream_t)stream>>>(pk, pv, (unsigned)kb);
+  else roundtrip_kernel<MZ_F16><<<(unsigned)(kb + vb), 256, 0, (cudaStream_t)stream>>>(pk, pv, (unsigned)kb);
   MZ_LAUNCH_CHECK("roundtrip");
   return MZ_OK;
 }

@@ -114,8 +114,8 @@ def load_library() -> ctypes.CDLL:
     lib.mz_bounds_violations.argtypes = [ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(c_int), c_int]
     lib.mz_bounds_violations.restype = ctypes.c_longlong
     lib.mz_materialize_kv.argtypes = [POINTER(KVStore), c_void_p, c_void_p, c_int, c_float, c_void_p]
-    lib.mz_roundtrip_kv.argtypes = [c_void_p, c_int, POINTER(c_int), POINTER(c_longlong), c_int, c_int, c_float, c_float, c_int, c_int,
-                                    c_void_p, c_void_p]
+    lib.mz_roundtrip_kv.argtypes = [c_void_p, POINTER(c_int), POINTER(c_longlong), c_float, c_void_p] * 2 + [
+        c_int, c_int, c_int, c_float, c_int, c_void_p]
     lib.mz_alpha_stats.argtypes = [c_void_p, c_int, POINTER(c_int), POINTER(c_longlong), c_int, c_int, c_int, c_int, c_int, c_void_p,
                                    c_void_p, c_void_p]
     lib.mz_alpha_stats_workspace_bytes.argtypes = []

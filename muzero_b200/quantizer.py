@@ -14,7 +14,7 @@ from typing import Optional
 import torch
 import torch.nn.functional as F
 
-from .kernels._cabi import check, dtype_code, stream_ptr
+from .kernels._cabi import check, dtype_code, on_device, stream_ptr
 from .kernels.loader import (MuZeroKernelError, ensure_expand_table, load_mu_zero_cuda_extension, mu_zero_dequantize_cuda,
                              mu_zero_quantize_cuda)
 
@@ -240,15 +240,16 @@ def _fused_roundtrip_serves(t: torch.Tensor, g: int, kind: str) -> bool:
             and t.data_ptr() % (4 if kind == "key" else 16) == 0)
 
 
-def _fused_roundtrip(t: torch.Tensor, bits: int, g: int, alpha: float, amax_dtype: torch.dtype, amax_eps: float, kind: str):
-    out = torch.empty(t.shape, dtype=t.dtype, device=t.device)
-    ensure_expand_table(bits, alpha, t.device)
-    with torch.cuda.device(t.device):
-        check(load_mu_zero_cuda_extension().mz_roundtrip_kv(
-            t.data_ptr(), dtype_code(t.dtype), (ctypes.c_int * 4)(*t.shape), (ctypes.c_longlong * 3)(*t.stride()[:3]), g, bits,
-            float(alpha), float(amax_eps), dtype_code(amax_dtype), int(kind == "key"), out.data_ptr(), stream_ptr(t.device)),
-            "mz_roundtrip_kv")
-    return out
+def _fused_roundtrip(key: torch.Tensor, value: torch.Tensor, bits: int, g: int, alpha_key: float, alpha_value: float,
+                     amax_dtype: torch.dtype, amax_eps: float):
+    outs, args = [], []
+    for t, alpha in ((key, alpha_key), (value, alpha_value)):
+        ensure_expand_table(bits, alpha, t.device)
+        outs.append(t.new_empty(t.shape))
+        args += [t.data_ptr(), (ctypes.c_int * 4)(*t.shape), (ctypes.c_longlong * 3)(*t.stride()[:3]), float(alpha), outs[-1].data_ptr()]
+    check(on_device(key.device, load_mu_zero_cuda_extension().mz_roundtrip_kv, *args, dtype_code(key.dtype), g, bits, float(amax_eps),
+                    dtype_code(amax_dtype), stream_ptr(key.device)), "mz_roundtrip_kv")
+    return tuple(outs)
 
 
 def roundtrip(key: torch.Tensor, value: torch.Tensor, *, bits: int = 4, q_group_size: int = 64,
@@ -261,9 +262,9 @@ def roundtrip(key: torch.Tensor, value: torch.Tensor, *, bits: int = 4, q_group_
     if alpha_value is None:
         alpha_value = select_alpha(value, bits=bits, q_group_size=g, kind="value")
 
-    if all(_fused_roundtrip_serves(t, g, kind) for t, kind in ((key, "key"), (value, "value"))):
-        return tuple(_fused_roundtrip(t, bits, g, alpha, amax_dtype, amax_eps, kind)
-                     for t, alpha, kind in ((key, alpha_key, "key"), (value, alpha_value, "value")))
+    if (key.dtype == value.dtype and key.device == value.device and _fused_roundtrip_serves(key, g, "key")
+            and _fused_roundtrip_serves(value, g, "value")):
+        return _fused_roundtrip(key, value, bits, g, alpha_key, alpha_value, amax_dtype, amax_eps)
     b, h, s, d = key.shape
     nsg = s // g
     rows = key.reshape(b, h, nsg, g, d).transpose(3, 4).contiguous().reshape(-1, g).float()
