@@ -52,13 +52,15 @@ __device__ __forceinline__ void dense_keys(const DenseParams& p, uint8_t* smem) 
     j = tile % p.n_groups; tile /= p.n_groups;
     h = tile % s.kv_heads; b = tile / s.kv_heads;
   };
+  // i / wpr by multiplication: exact for i < 4096 and wpr <= 32
   const int words = D * QB / 4, wpr = QB / 4;
+  const unsigned wpr_inv = ((1u << 20) + wpr - 1) / wpr;
   for (int l = 0; l < per_cta && tile0 + l < p.key_tiles; ++l) {
     int j, h, b;
     locate(tile0 + l, j, h, b);
     const uint32_t* src = (const uint32_t*)(s.packed_k + b * s.pk_stride_b + h * s.pk_stride_h + (long long)(p.g0 + j) * D * QB);
     for (int i = tid; i < words; i += 256) {
-      const int d = i / wpr, w = i % wpr;
+      const int d = (int)(((unsigned)i * wpr_inv) >> 20), w = i - d * wpr;
       *(uint32_t*)(s_code + (size_t)((d & 1) * per_cta * pairs + l * pairs + (d >> 1)) * stride + 4 * w) = __ldg(src + i);
     }
   }
@@ -137,11 +139,30 @@ __device__ __forceinline__ void dense_keys(const DenseParams& p, uint8_t* smem) 
   }
 }
 
+// A CTA takes kValChunks x 256 / lanes-per-row rows; the codes and metadata of all of a thread's rows are in flight before the
+// table is staged (one chunk per CTA spent most of its life in those two latencies).
+constexpr int kValChunks = 4;
 template <int DT, int BITS>
 __device__ __forceinline__ void dense_values(const DenseParams& p, unsigned blk, uint8_t* smem) {
   constexpr int NE = 1 << BITS, top = NE - 1;
   const mz_kv_store& s = p.s;
-  const int G = s.group, D = s.head_dim, NG = p.NG, lpr = G >> 4;
+  const int G = s.group, D = s.head_dim, NG = p.NG, lpr = G >> 4, rows = 256 / lpr;
+  const unsigned pair = blk / p.val_per_pair, chunk = blk % p.val_per_pair;
+  const int b = pair / s.kv_heads, h = pair % s.kv_heads;
+  const int row0 = chunk * (rows * kValChunks) + threadIdx.x / lpr, sub = threadIdx.x % lpr, n_rows = p.n_tok * NG;
+  const uint8_t* pv = s.packed_v + b * s.pv_stride_b + h * s.pv_stride_h;
+  const long long m0 = b * s.vm_stride_b + h * s.vm_stride_h, at0 = (long long)p.t0 * NG;
+  unsigned long long w[kValChunks][2];
+  float lo[kValChunks], span[kValChunks];
+#pragma unroll
+  for (int k = 0; k < kValChunks; ++k) {
+    const int row = min(row0 + k * rows, n_rows - 1);
+    const uint8_t* src = pv + (at0 + row) * p.QB;
+    w[k][0] = mz_load_octet(src + sub * BITS, BITS);
+    w[k][1] = mz_load_octet(src + (sub + lpr) * BITS, BITS);
+    lo[k] = meta16(s.v_mn, m0 + at0 + row, s.meta_dtype);
+    span[k] = meta16(s.v_scale, m0 + at0 + row, s.meta_dtype);
+  }
   const float* table = p.tab_v;
   if (BITS <= 4) {
     float* t = (float*)smem;
@@ -149,25 +170,21 @@ __device__ __forceinline__ void dense_values(const DenseParams& p, unsigned blk,
     __syncthreads();
     table = t;
   }
-  const unsigned pair = blk / p.val_per_pair, chunk = blk % p.val_per_pair;
-  const int b = pair / s.kv_heads, h = pair % s.kv_heads;
-  const int row = chunk * (256 / lpr) + threadIdx.x / lpr, sub = threadIdx.x % lpr;
-  if (row >= p.n_tok * NG) return;
-  const long long at = (long long)p.t0 * NG + row;
-  const long long m = b * s.vm_stride_b + h * s.vm_stride_h + at;
-  const MzRowParams r = mz_row_params(meta16(s.v_mn, m, s.meta_dtype), meta16(s.v_scale, m, s.meta_dtype), top, p.eps);
-  const uint8_t* src = s.packed_v + b * s.pv_stride_b + h * s.pv_stride_h + at * p.QB;
-  uint16_t* dst = (uint16_t*)p.out_v + ((long long)pair * p.sv) * D + (long long)row * G;
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    const int o = sub + c * lpr;
-    const unsigned long long w = mz_load_octet(src + o * BITS, BITS);
-    uint32_t v[4];
+  for (int k = 0; k < kValChunks; ++k) {
+    const int row = row0 + k * rows;
+    if (row >= n_rows) return;
+    const MzRowParams r = mz_row_params(lo[k], span[k], top, p.eps);
+    uint16_t* dst = (uint16_t*)p.out_v + ((long long)pair * p.sv) * D + (long long)row * G;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      v[i] = pack16<DT>(mz_dequant_exact(r, (int)(w >> (2 * i * BITS)) & top, table, NE),
-                        mz_dequant_exact(r, (int)(w >> ((2 * i + 1) * BITS)) & top, table, NE));
-    *(uint4*)(dst + o * 8) = make_uint4(v[0], v[1], v[2], v[3]);
+    for (int c = 0; c < 2; ++c) {
+      uint32_t v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        v[i] = pack16<DT>(mz_dequant_exact(r, (int)(w[k][c] >> (2 * i * BITS)) & top, table, NE),
+                          mz_dequant_exact(r, (int)(w[k][c] >> ((2 * i + 1) * BITS)) & top, table, NE));
+      *(uint4*)(dst + (sub + c * lpr) * 8) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
   }
 }
 
@@ -291,7 +308,7 @@ int run_dense(DenseParams& p, int out_dtype, float eps, cudaStream_t st) {
                     (!p.n_tok || (al(s.packed_v, 8) && !((s.pv_stride_b | s.pv_stride_h) & 7))) &&
                     al(p.out_k, 16) && al(p.out_v, 16) && p.n_tok < (1 << 28);
   if (fast) {
-    const int tt = (g.D / 2) * (g.G / 16), per_cta = tt >= 256 ? 1 : 256 / tt, rows_per_cta = 256 / (g.G / 16), vpr = g.D / 8;
+    const int tt = (g.D / 2) * (g.G / 16), per_cta = tt >= 256 ? 1 : 256 / tt, rows_per_cta = 256 / (g.G / 16) * kValChunks, vpr = g.D / 8;
     const long long tiles = pairs * p.n_groups;
     p.val_per_pair = (unsigned)(((long long)p.n_tok * g.NG + rows_per_cta - 1) / rows_per_cta);
     p.kres_per_pair = (unsigned)((p.res_k * vpr + 255) / 256);

@@ -412,7 +412,9 @@ __device__ __forceinline__ void flush16_keys(const Flush16Params& p, uint8_t* sm
   }
   __syncthreads();
   // code tile -> store: the D rows of a tile are contiguous there
+  // i / wpr by multiplication: exact for i < 4096 and wpr <= 32
   const int words = D * QB / 4, wpr = QB / 4;
+  const unsigned wpr_inv = ((1u << 20) + wpr - 1) / wpr;
   for (int l = 0; l < per_cta && tile0 + l < p.tiles; ++l) {
     int j, h, b;
     locate(tile0 + l, j, h, b);
@@ -420,7 +422,7 @@ __device__ __forceinline__ void flush16_keys(const Flush16Params& p, uint8_t* sm
     if (!MZ_IN_BOUNDS((grp + 1) * D * QB - 1, s.pk_stride_h, 1)) continue;
     uint32_t* out = (uint32_t*)(s.packed_k + b * s.pk_stride_b + h * s.pk_stride_h + grp * D * QB);
     for (int i = tid; i < words; i += 256) {
-      const int d = i / wpr, w = i % wpr;
+      const int d = (int)(((unsigned)i * wpr_inv) >> 20), w = i - d * wpr;
       out[i] = *(const uint32_t*)(s_code + (size_t)((d & 1) * per_cta * pairs + l * pairs + (d >> 1)) * stride + 4 * w);
     }
   }
