@@ -117,9 +117,12 @@ class MuZeroCacheLayer:
 
     # ------------------------------------------------------------------ init
     def lazy_initialization(self, key_states: torch.Tensor, value_states: torch.Tensor) -> None:
-        self.dtype, self.device = key_states.dtype, key_states.device
+        self._take_shape(key_states, value_states)
         self.keys = torch.empty(0, dtype=self.dtype, device=self.device)
         self.values = torch.empty(0, dtype=self.dtype, device=self.device)
+
+    def _take_shape(self, key_states: torch.Tensor, value_states: torch.Tensor) -> None:
+        self.dtype, self.device = key_states.dtype, key_states.device
         self.k_head_dim = key_states.shape[-1]
         self.v_head_dim = value_states.shape[-1]
         g = self.q_group_size
@@ -152,12 +155,13 @@ class MuZeroCacheLayer:
         s.alpha_key = float(self._selected_alpha_key if self._selected_alpha_key is not None else 2.0)
         s.alpha_value = float(self._selected_alpha_value if self._selected_alpha_value is not None else 2.0)
         if b:
-            s.packed_k, s.k_mn, s.k_scale = b["pk"].data_ptr(), b["kmn"].data_ptr(), b["ksc"].data_ptr()
-            s.pk_stride_b, s.pk_stride_h = b["pk"].stride(0), b["pk"].stride(1)
-            s.km_stride_b, s.km_stride_h = b["kmn"].stride(0), b["kmn"].stride(1)
-            s.packed_v, s.v_mn, s.v_scale = b["pv"].data_ptr(), b["vmn"].data_ptr(), b["vsc"].data_ptr()
-            s.pv_stride_b, s.pv_stride_h = b["pv"].stride(0), b["pv"].stride(1)
-            s.vm_stride_b, s.vm_stride_h = b["vmn"].stride(0), b["vmn"].stride(1)
+            pk, kmn, pv, vmn = b["pk"], b["kmn"], b["pv"], b["vmn"]
+            s.packed_k, s.k_mn, s.k_scale = pk.data_ptr(), kmn.data_ptr(), b["ksc"].data_ptr()
+            s.pk_stride_b, s.pk_stride_h = pk.stride()[:2]
+            s.km_stride_b, s.km_stride_h = kmn.stride()[:2]
+            s.packed_v, s.v_mn, s.v_scale = pv.data_ptr(), vmn.data_ptr(), b["vsc"].data_ptr()
+            s.pv_stride_b, s.pv_stride_h = pv.stride()[:2]
+            s.vm_stride_b, s.vm_stride_h = vmn.stride()[:2]
         s.k_groups, s.v_tokens = self._key_group_count, self._value_storage_len
         v = self.values
         if self._key_buffer is not None:
@@ -224,7 +228,7 @@ class MuZeroCacheLayer:
 
     def _append_dense(self, key_states: torch.Tensor, value_states: torch.Tensor) -> None:
         n_new = int(key_states.shape[2])
-        if self.keys.numel() == 0 and self._key_buffer is None:
+        if self._key_buffer is None and (self._keys is None or self._keys.numel() == 0):
             self.keys, self.values = key_states, value_states      # alias the caller's block
             self._res_start = 0
             if key_states.stride(-1) != 1 or value_states.stride(-1) != 1 or key_states.stride() != value_states.stride():
@@ -289,11 +293,10 @@ class MuZeroCacheLayer:
         new = {
             "pk": torch.empty((b, kvh, cap_g, d, qb), dtype=torch.uint8, device=dev),
             "kmn": torch.empty((b, kvh, cap_g, d, 1), dtype=md, device=dev),
-            "ksc": torch.empty((b, kvh, cap_g, d, 1), dtype=md, device=dev),
             "pv": torch.empty((b, kvh, cap_t, ng, qb), dtype=torch.uint8, device=dev),
             "vmn": torch.empty((b, kvh, cap_t, ng, 1), dtype=md, device=dev),
-            "vsc": torch.empty((b, kvh, cap_t, ng, 1), dtype=md, device=dev),
         }
+        new["ksc"], new["vsc"] = torch.empty_like(new["kmn"]), torch.empty_like(new["vmn"])
         if self._bufs:
             kg, vt = self._key_group_count, self._value_storage_len
             for name in ("pk", "kmn", "ksc"):
@@ -311,8 +314,11 @@ class MuZeroCacheLayer:
                 setattr(self, name, None)
             return
         b = self._bufs
-        self._packed_key_q, self._key_mn, self._key_scale = b["pk"][:, :, :kg], b["kmn"][:, :, :kg], b["ksc"][:, :, :kg]
-        self._packed_value_q, self._value_mn, self._value_scale = b["pv"][:, :, :vt], b["vmn"][:, :, :vt], b["vsc"][:, :, :vt]
+        def first(t, n):
+            sh = t.shape
+            return t.as_strided((sh[0], sh[1], n, sh[3], sh[4]), t.stride(), t.storage_offset())     # t[:, :, :n]
+        self._packed_key_q, self._key_mn, self._key_scale = first(b["pk"], kg), first(b["kmn"], kg), first(b["ksc"], kg)
+        self._packed_value_q, self._value_mn, self._value_scale = first(b["pv"], vt), first(b["vmn"], vt), first(b["vsc"], vt)
 
     def _adopt_store(self, tensors: dict[str, torch.Tensor]) -> None:
         """Replaces the store by exact-size tensors (after batch reindexing / device moves)."""
@@ -367,7 +373,7 @@ class MuZeroCacheLayer:
             # a prompt block: what stays dense moves into a window of the layer's own, in the same launch
             cur, lead = s.res_len - n, self._value_lead + nv - n
             cap = residual_capacity(cur + 1, self.residual_length, g)
-            kb = torch.empty((s.batch, s.kv_heads, cap, self.k_head_dim), dtype=self.dtype, device=self.device)
+            kb = self._keys.new_empty((s.batch, s.kv_heads, cap, self.k_head_dim))
             vb = torch.empty_like(kb)
             sb, sh, srow, _ = kb.stride()
             check(on_device(self.device, lib.mz_flush_kv_move, ctypes.byref(s), n, self._value_lead, nv, kb.data_ptr(), vb.data_ptr(),
@@ -426,7 +432,7 @@ class MuZeroCacheLayer:
         defer = kw.get("defer_quantize", False)
         first = not self.is_initialized
         if first:
-            self.lazy_initialization(key_states, value_states)
+            self._take_shape(key_states, value_states)
         self._append_dense(key_states, value_states)
         self.cumulative_length += key_states.shape[-2]
         raw_k, raw_v = self.keys, self.values
@@ -446,7 +452,7 @@ class MuZeroCacheLayer:
         attention (reference: muzero/cache/layer.py:407-459 and muzero/cache/attention.py:48-295), but in the
         steady state (window inside its buffer, store with room, alphas chosen) it is a single C call,
         ``mz_decode_step``.  Anything else takes the two-call route.  Returns ``[B,1,H,D]``."""
-        from .attention import build_decode_args, decode_attention, _workspace
+        A = _attention()
         g = self.q_group_size
         fast = (self.is_initialized and self._key_buffer is not None and key_states.shape[2] == 1 and key_states.is_cuda
                 and key_states.dtype == self.dtype and not self.cfg.logq_compatible_layout
@@ -467,7 +473,7 @@ class MuZeroCacheLayer:
                     self._ensure_store(self._key_group_count + n // g, self._value_storage_len + n)
         if not fast:
             self.update(key_states, value_states, {"materialize_full_kv": False})
-            return decode_attention(self, query, scaling, attention_mask)
+            return A.decode_attention(self, query, scaling, attention_mask)
         b, h, _, d = query.shape
         out = query.new_empty((b, 1, h, d))
         lib = load_mu_zero_cuda_extension()
@@ -475,7 +481,7 @@ class MuZeroCacheLayer:
         if attention_mask is not None or args is None or query.stride(-1) != 1 or query.dtype != self.dtype:
             # (re)build the argument block: pointers, strides and counters of the current state.  With a mask
             # the block is built per call (the mask tensor may be converted and has to stay alive).
-            args = build_decode_args(self, query, scaling, attention_mask, out, step=(self.residual_length, unit), bound=True)
+            args = A.build_decode_args(self, query, scaling, attention_mask, out, step=(self.residual_length, unit), bound=True)
             self._step_ws_bound = args.workspace_bytes
             self._step_args = args if attention_mask is None else None
         else:
@@ -483,7 +489,7 @@ class MuZeroCacheLayer:
             args.query, args.q_stride_b, args.q_stride_h = query.data_ptr(), query.stride(0), query.stride(1)
             args.q_heads, args.scaling = h, float(scaling)
             args.out, args.out_dtype = out.data_ptr(), dtype_code(out.dtype)
-            ws = _workspace(query.device, self._step_ws_bound)
+            ws = A._workspace(query.device, self._step_ws_bound)
             args.workspace, args.workspace_bytes = ws.data_ptr(), ws.numel()
         rc = on_device(
             self.device, lib.mz_decode_step, ctypes.byref(args), key_states.data_ptr(), value_states.data_ptr(), key_states.stride(0),
@@ -659,6 +665,18 @@ class MuZeroCacheLayer:
 
     def reset(self) -> None:
         self._clear_state()
+
+
+_attention_module = None
+
+
+def _attention():
+    """``cache.attention`` (imports this module): looked up once, not with an import statement per decode step."""
+    global _attention_module
+    if _attention_module is None:
+        from . import attention
+        _attention_module = attention
+    return _attention_module
 
 
 _side_streams: dict = {}
