@@ -252,22 +252,30 @@ int clusters_at_once(const MzMmaKernel& k, int cs, int threads, unsigned smem) {
 }
 
 // Machine-filling plans of these shapes are faster on the SIMT kernel (measured at 16 x 8 x 4000 and 40 x 8 x 2500):
-//   * codes of 5 to 8 bits, which are computed one by one, with up to 4 heads per kv head (123 against 148 us); with 8
-//     heads the SIMT kernel pays for each
+//   * codes of 7 and 8 bits, which are computed one by one, with up to 4 heads per kv head (123 against 148 us); with 8
+//     heads, for which the SIMT kernel pays one by one, groups of 32 (8 bits, 16 x 8 x 4224: 162 against 186 us), 8 bits
+//     in groups of 128 (161 against 202) and 7 bits in groups of 64 (161 against 170)
 //   * groups of 32, whose tiles prepare twice the rows per token here, with few heads (1 bit: 74 against 94 us) - from
 //     4 heads on the 4-bit ones are faster here (96 against 103)
 //   * 4 bits in groups of 128 with two heads (59 against 68)
+//   * 3 bits with one or two heads (8 x 8 x 33364, one head: 183 against 201; 3 x 8 x 47136 in groups of 128: 105 against
+//     118) and 1 bit in groups of 64 (28 x 4 x 15385: 143 against 151)
 bool simt_is_faster(const MzDecodeParams& p) {
-  if (p.gqa > 4 || !mz_decode_tiles_supported(p)) return false;
-  if (p.s.bits > 4) return true;
-  if (p.s.group == 32) return p.gqa < 4 || p.s.bits < 4;
-  return p.s.group == 128 && p.s.bits == 4 && p.gqa == 2;
+  if (!mz_decode_tiles_supported(p)) return false;
+  const int bits = p.s.bits, group = p.s.group;
+  if (bits > 4) return p.gqa <= 4 || group == 32 || group == (bits == 8 ? 128 : 64);
+  if (p.gqa > 4) return false;
+  if (group == 32) return p.gqa < 4 || bits < 4;
+  if (p.gqa <= 2 && (bits == 3 || (bits == 1 && group == 64))) return true;
+  return group == 128 && bits == 4 && p.gqa == 2;
 }
 
 // Cluster mode: one cluster per pair, no partial records in memory and no merge kernel.  In units of a packed tile on a
 // busy SM (0.5 us, 1.5 us of wide codes): it takes what its heaviest SM has to do, times what a tile costs here over the
 // kernel that would run otherwise; an even cut over all SMs takes its share, but at least one tile's latency (about 4 us),
-// and the merge kernel (about 4 us).
+// and the merge kernel (about 4 us).  Where the even cut would run on the unrolled kernel and every pair could have two SMs,
+// a cluster whose warps need one more turn over their tiles than the even cut's loses what the merge costs and more
+// (8 x 8 x 3420, 4 bits: 36 against 31 us; 18 x 2 x 1500: 23 against 18.5).
 bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count) {
   const long long pairs = (long long)p.s.batch * p.s.kv_heads;
   if (pairs > sm_count) return false;
@@ -284,8 +292,13 @@ bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count) {
     const int nw = layout(t, p, k, want, rec);
     if (nw < 1) return false;
     const long long even = pairs * t.pair_cost / sm_count, heaviest = t.pair_cost / cs, wait = (p.s.bits > 4 ? 3 : 8) * kCostPacked;
-    const int here = p.s.bits > 4 ? 100 : simt_is_faster(p) ? 128 : mz_decode_flat_supported(p) ? 116 : 100;
+    const bool simt = simt_is_faster(p), flat = !simt && mz_decode_flat_supported(p);
+    // 1 and 3 bits with few heads cost about the same on both kernels
+    const int here = p.s.bits > 4 || (p.s.group > 32 && (p.s.bits & 1)) ? 100 : simt ? 128 : flat ? 116 : 100;
     if (heaviest * here / 100 > (even > wait ? even : wait) + wait) return false;      // smaller clusters are heavier still
+    // a turn: every warp of the SM over one packed tile; even shares of the cost leave some warp up to a tile more
+    const long long turn = (long long)k.max_warps * kCostPacked;
+    if (flat && 2 * pairs <= sm_count && (t.pair_cost + kCostPacked * 3 / 2 + cs * turn - 1) / (cs * turn) > (even + turn - 1) / turn) return false;
     if (cs > 1 && clusters_at_once(k, cs, nw * 32, t.smem_bytes) < pairs) continue;
     // tiles are dealt to the cluster's warps by cost; every warp gets at most about one residual tile's cost more than its share
     if (cut(t, 1, (long long)cs * nw) != MZ_OK) return false;
