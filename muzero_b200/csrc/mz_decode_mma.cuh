@@ -35,6 +35,9 @@
 // Work: tiles of G packed tokens or 16 residual tokens of one (batch, kv head) pair.  Either the flat list of all
 // tiles is cut by cost into one contiguous range per warp of a machine-filling grid and a merge kernel combines the
 // partial records, or (few pairs) a cluster of CTAs owns a pair and merges through distributed shared memory.
+// Measured (8 kv heads, call included): one sequence of 500 tokens, 4 bits 27.8 -> 13.7 us (cluster against cut + merge); 6 x 1777
+// with 8 heads per kv head under a mask 43.0 -> 32.5 us; head_dim 64, 16 x 2050 333 -> 19.8 us (was the generic kernel).
+// Bound by the latency of a tile's chain there, and by issue and lookups (one wavefront per code) on a full machine.
 #pragma once
 #include <type_traits>
 

@@ -1,5 +1,7 @@
 // Store -> dense keys and values: a range of the packed prefix, optionally followed by the residual window, in one
 // launch.  Bit-exact with the reference's fp32 dequantizer (muzero/quantizer.py:229-266).
+// Measured (8 x 8 x 4224 tokens, head_dim 128, 4 bits, call included): 721 us as two dequantizers, conversions and
+// concatenations, 65.6 us now (0.42 of the copy rate).
 //
 // head_dim 64 / 128, groups of 32 / 64 / 128 that divide it, 16-bit output: bound by HBM (the output is 4 to 16 times
 // the packed input).  Keys are packed along tokens and written along channels, so a key tile is staged in shared

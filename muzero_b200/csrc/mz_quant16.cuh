@@ -9,6 +9,7 @@
 //     thresholds of every anchor in [0, 1] are a table (15 x 2 bytes per anchor at 4 bits, 0.5 MB, L2 resident)
 //     built once per device by evaluating the chain itself; a binary search over it takes BITS packed compares.
 // Wider codes (5..8 bits) would need hundreds of thresholds per row and evaluate the chain on the unit instead.
+// Bound by instruction issue; the chain itself takes about 100 instructions per value and most of a prompt's time.
 #pragma once
 #include "mz_quant_math.cuh"
 

@@ -4,6 +4,8 @@
 // One launch for a K and a V block (either may be absent): the two halves fill each other's last waves.
 // Keys: thread = two neighbouring channels of 16 tokens, the parts of a channel meet in shared memory; values: thread =
 // 16 channels of one row, shuffles over the row's lanes (the layouts of the flush).
+// Measured (2 x 8 x 2048 tokens, head_dim 128, 4 bits, K and V, call included): 185 us as quantizer, dequantizer and copies,
+// 28.7 us now.
 #include "mz_quant16.cuh"
 #include "mz_quant_f32.cuh"
 
