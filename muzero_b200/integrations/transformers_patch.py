@@ -62,6 +62,20 @@ class MuZeroCache(_HFCache):
         else:
             super().__init__(layer_class_to_replicate=self._new_layer)
 
+    # The base class keeps the factory as an attribute; a bound method stored there would tie the cache to itself, and its
+    # device memory would stay until the garbage collector comes by (a new cache per prompt then pays cudaMalloc: 1.6 ms
+    # against 0.14 for a 16 x 4096-token block)
+    @property
+    def layer_class_to_replicate(self):
+        return self.__dict__.get("_layer_factory", self._new_layer)
+
+    @layer_class_to_replicate.setter
+    def layer_class_to_replicate(self, factory):
+        if factory == self._new_layer:
+            self.__dict__.pop("_layer_factory", None)
+        else:
+            self.__dict__["_layer_factory"] = factory
+
     def _new_layer(self) -> MuZeroCacheLayer:
         layer = MuZeroCacheLayer(self.cfg)
         layer.max_cache_length = self.max_cache_length
