@@ -131,7 +131,7 @@ bool mz_decode_flat_supported(const MzDecodeParams& p);
 int mz_plan_flat(MzDecodeParams& p, int splits_request, int sm_count, size_t* slots);
 int mz_launch_decode_flat(const MzDecodeParams& p, cudaStream_t st);
 int mz_smem_window_base();
-const unsigned* mz_mma_lookup_entries(int bits, int sub, float alpha_key, float alpha_value);
+const unsigned* mz_mma_lookup_entries(int bits, bool split, float alpha_key, float alpha_value);
 // one instance of the tensor-core kernel: its function and the shared-memory sizes its configuration needs
 struct MzMmaKernel { const void* fn; unsigned ri_bytes, a_bytes, p_bytes, table_bytes; int max_warps; };
 bool mz_mma_kernel_b1(int D, int G, int nt, MzMmaKernel* k);

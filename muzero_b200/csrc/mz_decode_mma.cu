@@ -19,38 +19,35 @@ constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 int g_window_base[kMaxDevices];      // 0 = not probed yet, -1 = probe failed, else the address
 
-// Lookup-table entries kept in a static device array (no allocation): one slot per (bits, alpha of keys, alpha
-// of values) seen on a device.
-constexpr int kLutSlots = 16;
-__device__ uint32_t g_lut[kLutSlots][512];
-template <int BITS, int SUB>
+// Lookup-table entries kept in a static device array (no allocation): one slot per (bits, form, alpha of keys, alpha
+// of values) seen on a device.  Form: 32-bit entries of the unrolled kernel, or 64-bit entries of the general one.
+constexpr int kLutSlots = 16, kLutWords = 1024;
+__device__ __align__(16) uint32_t g_lut[kLutSlots][kLutWords];
+template <int BITS, bool SPLIT>
 __global__ void build_lut_kernel(int slot, float alpha_key, float alpha_value) {
-  constexpr int N = 1 << (2 * BITS + SUB);
-  for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) g_lut[slot][i] = lookup_entry<BITS, SUB>(i / N ? alpha_value : alpha_key, i % N);
-}
-// 4 bits, equal alphas: [sub-bin][zero code, code]
-__global__ void build_twin_lut_kernel(int slot, float alpha) {
-  for (int i = threadIdx.x; i < 512; i += blockDim.x) {
-    const int idx = i & 255;
-    g_lut[slot][i] = lookup_entry<4, 1>(alpha, (((idx >> 4) * 2 + (i >> 8)) << 4) | (idx & 15));
+  constexpr int N = 1 << (2 * BITS);
+  for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) {
+    const float alpha = i / N ? alpha_value : alpha_key;
+    if (SPLIT) ((uint2*)g_lut[slot])[i] = split_entry<BITS>(alpha, i % N);
+    else g_lut[slot][i] = lookup_entry<BITS>(alpha, i % N);
   }
 }
-struct LutKey { int bits, sub; float ak, av; };
+struct LutKey { int bits; bool split; float ak, av; };
 struct LutDevice { uint32_t* base; int used; LutKey keys[kLutSlots]; };
 LutDevice g_lut_dev[kMaxDevices];
 }  // namespace mzm
 
-// Device pointer to the table entries for (bits, sub-bins, alphas) on the current device, or nullptr when they cannot be
+// Device pointer to the table entries for (bits, form, alphas) on the current device, or nullptr when they cannot be
 // provided (all slots taken, or the one-time build is not possible right now, e.g. during stream capture): the
 // kernel then computes the entries in every CTA.  The first request for a combination launches a one-block
 // kernel on the default stream and waits for it, so that any stream may use the entries afterwards.
-const unsigned* mz_mma_lookup_entries(int bits, int sub, float alpha_key, float alpha_value) {
+const unsigned* mz_mma_lookup_entries(int bits, bool split, float alpha_key, float alpha_value) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= mzm::kMaxDevices) return nullptr;
   std::lock_guard<std::mutex> lk(mzm::g_mu);
   mzm::LutDevice& d = mzm::g_lut_dev[dev];
   for (int i = 0; i < d.used; ++i)
-    if (d.keys[i].bits == bits && d.keys[i].sub == sub && d.keys[i].ak == alpha_key && d.keys[i].av == alpha_value) return d.base + i * 512;
+    if (d.keys[i].bits == bits && d.keys[i].split == split && d.keys[i].ak == alpha_key && d.keys[i].av == alpha_value) return d.base + i * mzm::kLutWords;
   if (d.used >= mzm::kLutSlots) return nullptr;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
@@ -63,19 +60,19 @@ const unsigned* mz_mma_lookup_entries(int bits, int sub, float alpha_key, float 
     return nullptr;
   }
   const int slot = d.used;
-  if (bits == 1) mzm::build_lut_kernel<1, mzm::kSubBits[1]><<<1, 32>>>(slot, alpha_key, alpha_value);
-  else if (bits == 2 && sub == 0) mzm::build_lut_kernel<2, 0><<<1, 32>>>(slot, alpha_key, alpha_value);
-  else if (bits == 2) mzm::build_lut_kernel<2, mzm::kSubBits[2]><<<1, 256>>>(slot, alpha_key, alpha_value);
-  else if (bits == 3) mzm::build_lut_kernel<3, mzm::kSubBits[3]><<<1, 256>>>(slot, alpha_key, alpha_value);
-  else if (sub == 0) mzm::build_lut_kernel<4, 0><<<1, 256>>>(slot, alpha_key, alpha_value);
-  else mzm::build_twin_lut_kernel<<<1, 256>>>(slot, alpha_key);
+  if (!split && bits == 2) mzm::build_lut_kernel<2, false><<<1, 32>>>(slot, alpha_key, alpha_value);
+  else if (!split) mzm::build_lut_kernel<4, false><<<1, 256>>>(slot, alpha_key, alpha_value);
+  else if (bits == 1) mzm::build_lut_kernel<1, true><<<1, 32>>>(slot, alpha_key, alpha_value);
+  else if (bits == 2) mzm::build_lut_kernel<2, true><<<1, 32>>>(slot, alpha_key, alpha_value);
+  else if (bits == 3) mzm::build_lut_kernel<3, true><<<1, 128>>>(slot, alpha_key, alpha_value);
+  else mzm::build_lut_kernel<4, true><<<1, 256>>>(slot, alpha_key, alpha_value);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
     (void)cudaGetLastError();
     return nullptr;
   }
-  d.keys[slot] = {bits, sub, alpha_key, alpha_value};
+  d.keys[slot] = {bits, split, alpha_key, alpha_value};
   d.used = slot + 1;
-  return d.base + slot * 512;
+  return d.base + slot * mzm::kLutWords;
 }
 
 // Shared-window address at which this device places dynamic shared memory (a kernel without static shared
@@ -321,7 +318,7 @@ int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slo
   p.cluster = 0;
   MzMmaKernel k;
   if (!find_kernel(p, &k)) return mz_fail(MZ_ERR_UNSUPPORTED, "no tensor-core kernel for this shape");
-  p.lut = s.k_groups > 0 && s.bits <= 4 ? mz_mma_lookup_entries(s.bits, s.bits == 4 && s.alpha_key == s.alpha_value ? 1 : mzm::kSubBits[s.bits], s.alpha_key, s.alpha_value) : nullptr;
+  p.lut = s.k_groups > 0 && s.bits <= 4 ? mz_mma_lookup_entries(s.bits, true, s.alpha_key, s.alpha_value) : nullptr;
   if (splits_request == 0 && plan_cluster(p, k, sm_count)) {
     *slots = 4;                                   // no records; a workspace is still asked for, so that its size is never 0
     return MZ_OK;

@@ -10,22 +10,19 @@
 //     logit[h,t]  = sum_d  (q[h,d]*Bup_d) u+  +  (q[h,d]*Bdn_d) u-   + sum_d q[h,d] A_d
 //     out[h,c]    = sum_t  (p[h,t]*Bup_tg) u+ +  (p[h,t]*Bdn_tg) u-  + sum_t p[h,t] A_tg
 // Both contractions run on the tensor cores (mma.sync m16n8k16, fp16 operands, fp32 accumulate):
-//   * the A operand holds table values; one code = 32 bits of a shared-memory lookup that returns the
-//     fp16 pair (u+, u-), which is one A-fragment register (the reduction index is doubled: one slot for
-//     the part above the zero code, one for the part below it)
-//   * the table is replicated once per lane, so no lookup pattern can cause a bank conflict, and it sits
+//   * the A operand holds table values; one code = a 64-bit shared-memory lookup that returns the fp16 pair (u+, u-),
+//     which is one A-fragment register (the reduction index is doubled: one slot for the part above the zero code, one
+//     for the part below it), and the pair of what rounding to fp16 dropped
+//   * the table is replicated once per lane of a half warp, so no lookup pattern can cause a bank conflict, and it sits
 //     at shared-window address 65536 with a stride of 256 bytes, so that the address of a lookup is one byte
-//     permute: byte 1 of the address <- (zc, sub-bin, code)
+//     permute: byte 1 of the address <- (zc, code)
 //   * the B operand holds the folded query (keys) or folded probabilities (values); its 8 columns are
 //     4 heads x {product rounded to fp16, its exact fp16 remainder (+ the remainders of the constant and of the
 //     probability)};
 //     5 to 8 heads per kv head use a second set of 8 columns on the same A fragments
-//   * the idle half of a table entry (u- of a code above the zero code, u+ of one below) carries the fp16
-//     remainder of the active half, pre-scaled by the nominal ratio of the two side constants, which recovers most
-//     of the table's own fp16 rounding.  The ratio is nominal for the zero anchor's bin: half of a zero code's range at
-//     4 bits (all of it when the alphas of keys and values differ), a fourth / an eighth at 3 / 2 bits (1 bit has end bins
-//     only, where it is exact).  With the constants as
-//     value + remainder the result is within about 1e-5 of the fp32 evaluation (norms)
+//   * a second product takes the fp16 remainders of the table values (the upper half of the 64-bit entry).  With constants,
+//     query products and probabilities as value + remainder too, and the running sums kept outside the tensor cores, the
+//     result has the error of the fp32 kernels (a few 1e-7)
 //   * M rows are tokens (keys) or channels (values), permuted so that one load of packed codes
 //     feeds a thread's rows of all M tiles.
 // Codes of 5 to 8 bits have no table (2^16 entries): their value (v - A) / span is computed per code (one ex2) and
@@ -58,10 +55,8 @@ struct Cfg {
   static constexpr int NB = D / 8;            // reduction blocks of 8 rows per tile side (both sides have D rows)
   static constexpr int MAXW = NT == 1 ? 12 : 8;
   static constexpr int NE = 1 << (WIDE ? 1 : BITS);
-  // table: entries (zero code, sub-bin, code) in 256-byte slots, keys' copies in the lower, values' in the upper half
-  static constexpr int SUB = WIDE ? 0 : kSubBits[BITS];
-  static constexpr bool TWIN = BITS == 4;      // no room in the index byte: the other half of a slot is the second sub-bin
-  static constexpr int ENTRIES = WIDE ? 0 : NE * NE << SUB;
+  // table: entries (zero code, code) in 256-byte slots, keys' copies in the lower, values' in the upper half
+  static constexpr int ENTRIES = WIDE ? 0 : NE * NE;
   static constexpr uint32_t TABLE_BYTES = ENTRIES * 256u;
   // row constants, and the folded-query source (the block loops are not unrolled over it)
   static constexpr uint32_t Q_BYTES = NT * NB * 64;
@@ -80,17 +75,18 @@ __device__ __forceinline__ uint32_t fold_pair(__half2 x, __half2 xm, uint32_t B,
 }
 
 // table lookups: the table never changes after the fill, so the compiler may move them freely
-__device__ __forceinline__ uint32_t tab32(uint32_t a) {
-  uint32_t v;
-  asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
+__device__ __forceinline__ uint2 tab64(uint32_t a) {
+  uint2 v;
+  asm("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
   return v;
 }
 __device__ __forceinline__ uint32_t pack_u16(uint32_t lo, uint32_t hi) { return prmt(lo, hi, 0x5410u); }
 
 // ---- lookups.  A thread (g = lane / 4, t = lane % 4) holds, per reduction block, the codes of two rows (slot 0 and 1)
 // for the CPL consecutive positions CPL*g + i along the row; position i belongs to M tile i / 2, fragment row
-// g + 8 * (i & 1).  `row0` / `row1` are the shared addresses of the lane's first code byte in the two rows; a quad of
-// M tiles (8 positions; 4 when the group is 32) is looked up at a time: a[4m + 2*slot + r].
+// g + 8 * (i & 1).  `row0` / `row1` are the shared addresses of the lane's first code byte in the two rows.  Codes are
+// loaded a quad of M tiles at a time (8 positions; 4 when the group is 32) and looked up half a quad at a time: half h
+// has the positions 4 h + i, a[4 (i / 2) + 2 slot + (i & 1)].
 template <int BITS, int CPL>
 struct Quad;
 // 4-bit codes: 8 positions = one word
@@ -101,13 +97,12 @@ struct Quad<4, CPL> {
     if (CPL == 4) { w0 = lds16(row0); w1 = lds16(row1); }
     else { w0 = lds32(row0 + 4 * q); w1 = lds32(row1 + 4 * q); }
   }
-  template <int NA>
-  __device__ __forceinline__ void look(uint32_t z0, uint32_t z1, uint32_t base0, uint32_t base1, uint32_t (&a)[NA]) const {
+  __device__ __forceinline__ void look(int h, uint32_t z0, uint32_t z1, uint32_t base, uint2 (&a)[8]) const {
     const uint32_t c[4] = {(w0 & 0x0F0F0F0Fu) | z0, ((w0 >> 4) & 0x0F0F0F0Fu) | z0, (w1 & 0x0F0F0F0Fu) | z1, ((w1 >> 4) & 0x0F0F0F0Fu) | z1};
 #pragma unroll
-    for (int m = 0; m < NA / 4; ++m)
+    for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) a[4 * m + k] = tab32(prmt(c[k], k < 2 ? base0 : base1, 0x7604u | (uint32_t)(m << 4)));
+      for (int k = 0; k < 4; ++k) a[4 * m + k] = tab64(prmt(c[k], base, 0x7604u | (uint32_t)((2 * h + m) << 4)));
   }
 };
 // 3-bit codes: 8 positions = 24 bits at any bit address
@@ -128,22 +123,18 @@ struct Quad<3, CPL> {
     x = (x | (x << 10)) & 0x003F003Fu;
     return (x | (x << 5)) & 0x07070707u;
   }
-  template <int NA>
-  __device__ __forceinline__ void look(uint32_t z0, uint32_t z1, uint32_t base, uint32_t (&a)[NA]) const {
+  __device__ __forceinline__ void look(int h, uint32_t z0, uint32_t z1, uint32_t base, uint2 (&a)[8]) const {
+    const uint32_t c0 = spread((w0 >> (12 * h)) & 0xfffu) | z0, c1 = spread((w1 >> (12 * h)) & 0xfffu) | z1;
 #pragma unroll
-    for (int h = 0; h < NA / 8; ++h) {       // four positions (two M tiles) at a time
-      const uint32_t c0 = spread((w0 >> (12 * h)) & 0xfffu) | z0, c1 = spread((w1 >> (12 * h)) & 0xfffu) | z1;
+    for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          a[4 * (2 * h + m) + r] = tab32(prmt(c0, base, 0x7604u | (uint32_t)((2 * m + r) << 4)));
-          a[4 * (2 * h + m) + 2 + r] = tab32(prmt(c1, base, 0x7604u | (uint32_t)((2 * m + r) << 4)));
-        }
-    }
+      for (int r = 0; r < 2; ++r) {
+        a[4 * m + r] = tab64(prmt(c0, base, 0x7604u | (uint32_t)((2 * m + r) << 4)));
+        a[4 * m + 2 + r] = tab64(prmt(c1, base, 0x7604u | (uint32_t)((2 * m + r) << 4)));
+      }
   }
 };
-// 2-bit codes: 8 positions = 16 bits; byte 2 slot + h of c[k] is position 4 h + k
+// 2-bit codes: 8 positions = 16 bits; byte 2 slot + h of c is position 4 h + k
 template <int CPL>
 struct Quad<2, CPL> {
   uint32_t w;                 // low half: slot 0, high half: slot 1
@@ -151,17 +142,13 @@ struct Quad<2, CPL> {
     if (CPL == 4) w = pack_u16(lds8(row0), lds8(row1));
     else w = pack_u16(lds16(row0 + 2 * q), lds16(row1 + 2 * q));
   }
-  template <int NA>
-  __device__ __forceinline__ void look(uint32_t z0, uint32_t z1, uint32_t base, uint32_t (&a)[NA]) const {
+  __device__ __forceinline__ void look(int h, uint32_t z0, uint32_t z1, uint32_t base, uint2 (&a)[8]) const {
     const uint32_t z = pack_u16(z0, z1);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const uint32_t c = ((w >> (2 * k)) & 0x03030303u) | z;
 #pragma unroll
-      for (int h = 0; h < NA / 8; ++h)
-#pragma unroll
-        for (int slot = 0; slot < 2; ++slot)
-          a[4 * (2 * h + (k >> 1)) + 2 * slot + (k & 1)] = tab32(prmt(c, base, 0x7604u | (uint32_t)((2 * slot + h) << 4)));
+      for (int slot = 0; slot < 2; ++slot) a[4 * (k >> 1) + 2 * slot + (k & 1)] = tab64(prmt(c, base, 0x7604u | (uint32_t)((2 * slot + h) << 4)));
     }
   }
 };
@@ -173,17 +160,13 @@ struct Quad<1, CPL> {
     const uint32_t sh = CPL == 4 ? 4 * (g & 1) : 0, b0 = lds8(row0 + q) >> sh, b1 = lds8(row1 + q) >> sh, b = pack_u16(b0, b1);
     w = prmt(b, b >> 4, 0x6240u);
   }
-  template <int NA>
-  __device__ __forceinline__ void look(uint32_t z0, uint32_t z1, uint32_t base, uint32_t (&a)[NA]) const {
+  __device__ __forceinline__ void look(int h, uint32_t z0, uint32_t z1, uint32_t base, uint2 (&a)[8]) const {
     const uint32_t z = pack_u16(z0, z1);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const uint32_t c = ((w >> k) & 0x01010101u) | z;
 #pragma unroll
-      for (int h = 0; h < NA / 8; ++h)
-#pragma unroll
-        for (int slot = 0; slot < 2; ++slot)
-          a[4 * (2 * h + (k >> 1)) + 2 * slot + (k & 1)] = tab32(prmt(c, base, 0x7604u | (uint32_t)((2 * slot + h) << 4)));
+      for (int slot = 0; slot < 2; ++slot) a[4 * (k >> 1) + 2 * slot + (k & 1)] = tab64(prmt(c, base, 0x7604u | (uint32_t)((2 * slot + h) << 4)));
     }
   }
 };
@@ -196,15 +179,20 @@ __device__ __forceinline__ uint32_t lane_offset(int g) {
   return (uint32_t)(g * (CPL * BITS)) >> 3;
 }
 
-// the table values of a step; zz: zero-code bytes of slot 0 and 1 (4 bits: bit 0 of a byte is the sub-bin = bit 7 of the address)
-template <class C, class Q, int NA>
-__device__ __forceinline__ void look_step(const Q& w, uint32_t zz, uint32_t base, uint32_t (&a)[NA]) {
-  if constexpr (C::TWIN) {
-    const uint32_t z = zz & 0xF0F0u;
-    w.look(prmt(z, 0u, 0x0000u), prmt(z, 0u, 0x1111u), base | ((zz & 1u) << 7), base | ((zz >> 1) & 128u), a);
-  } else {
-    w.look(prmt(zz, 0u, 0x0000u), prmt(zz, 0u, 0x1111u), base, a);
-  }
+// the table values of half a quad; zz: zero-code bytes of slot 0 and 1
+template <class Q>
+__device__ __forceinline__ void look_step(const Q& w, int h, uint32_t zz, uint32_t base, uint2 (&a)[8]) {
+  w.look(h, prmt(zz, 0u, 0x0000u), prmt(zz, 0u, 0x1111u), base, a);
+}
+
+// One step's product with M tile `m` of half a quad, added to c: the remainders first, then the rounded values, on a
+// fresh accumulator, so that the running sum is rounded to nearest (the tensor cores truncate theirs: over the 256 steps
+// of eight tiles that alone would be 1e-5).
+__device__ __forceinline__ void mma_step(float (&c)[4], const uint2 (&a)[8], int m, uint32_t b0, uint32_t b1) {
+  float x[4];
+  mma_f16_first(x, a[4 * m].y, a[4 * m + 1].y, a[4 * m + 2].y, a[4 * m + 3].y, b0, b1);
+  mma_f16(x, a[4 * m].x, a[4 * m + 1].x, a[4 * m + 2].x, a[4 * m + 3].x, b0, b1);
+  add4(c, x);
 }
 
 // ---- the lookup table, from the entries [2][ENTRIES] = (keys' alpha, values' alpha) in global memory (nullptr: they
@@ -212,22 +200,15 @@ __device__ __forceinline__ void look_step(const Q& w, uint32_t zz, uint32_t base
 // latency was most of a small call), then 16-byte stores of the copies, rotated so that eight neighbouring threads hit
 // eight different bank groups.
 template <class C, int BITS>
-__device__ __forceinline__ void fill_tables(uint32_t table, const uint32_t* __restrict__ lut, float alpha_key, float alpha_value) {
-  constexpr int PER = C::ENTRIES, COPIES = 8;
-  // equal alphas: one table, in the lower halves; at 4 bits the upper halves then hold its second sub-bin
-  const bool one = alpha_key == alpha_value, twin = one && C::TWIN;
-  const int n = one && !twin ? PER : 2 * PER;
-  auto entry = [&](int which, int idx) {
-    if (lut != nullptr) return lut[which * PER + idx];
-    if (twin) return lookup_entry<BITS, 1>(alpha_key, (((idx >> BITS) * 2 + which) << BITS) | (idx & (C::NE - 1)));
-    return lookup_entry<BITS, C::SUB>(which ? alpha_value : alpha_key, idx);
-  };
+__device__ __forceinline__ void fill_tables(uint32_t table, const uint2* __restrict__ lut, float alpha_key, float alpha_value) {
+  constexpr int PER = C::ENTRIES, CHUNKS = 8;
+  const int n = alpha_key == alpha_value ? PER : 2 * PER;        // equal alphas: one table, in the lower halves
   for (int i0 = threadIdx.x; i0 < n; i0 += 4 * blockDim.x) {
-    uint32_t v[4];
+    uint2 v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int i = min(i0 + k * (int)blockDim.x, n - 1), which = i / PER, idx = i % PER;
-      v[k] = entry(which, idx);
+      const int i = min(i0 + k * (int)blockDim.x, n - 1);
+      v[k] = lut != nullptr ? lut[i] : split_entry<BITS>(i / PER ? alpha_value : alpha_key, i % PER);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -235,7 +216,7 @@ __device__ __forceinline__ void fill_tables(uint32_t table, const uint32_t* __re
       if (i < n) {
         const uint32_t row = table + idx * 256 + which * 128;
 #pragma unroll
-        for (int c = 0; c < COPIES; ++c) sts128(row + (((c + threadIdx.x) & (COPIES - 1)) << 4), make_uint4(v[k], v[k], v[k], v[k]));
+        for (int c = 0; c < CHUNKS; ++c) sts128(row + (((c + threadIdx.x) & (CHUNKS - 1)) << 4), make_uint4(v[k].x, v[k].y, v[k].x, v[k].y));
       }
     }
   }
@@ -260,7 +241,7 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
 }
 // One tile side of wide codes: blocks of 16 rows, a lane holds rows 4 s + t (s = 0..3).  INNER consecutive blocks are
 // unrolled (the value groups of a token block).  row(blk, s): byte offset of the row; fold(blk, spans, b): the B operand;
-// mma(k, m, a, b): multiply M tile m of inner block k.
+// mma(k, m, hi, lo, b): multiply M tile m of inner block k.
 template <class C, int BITS, int INNER, class RowF, class FoldF, class MmaF>
 __device__ __forceinline__ void wide_side(uint32_t buf, uint32_t ri, int g, int t, int bits, RowF row, FoldF fold, MmaF mma) {
   constexpr int PER = C::CPL < 8 ? C::CPL : 8;          // codes of a row taken at once
@@ -311,8 +292,7 @@ __device__ __forceinline__ void wide_side(uint32_t buf, uint32_t ri, int g, int 
             split_pair(v[0], v[1], hi[rr], lo[rr]);
             split_pair(v[2], v[3], hi[2 + rr], lo[2 + rr]);
           }
-          mma(k, q * (PER / 2) + m, hi, bb);
-          mma(k, q * (PER / 2) + m, lo, bb);
+          mma(k, q * (PER / 2) + m, hi, lo, bb);
         }
       }
     }
@@ -432,20 +412,23 @@ __device__ __forceinline__ void dense_tile(const MzDecodeParams& p, uint32_t kbu
   }
 #pragma unroll
   for (int n = 0; n < NT; ++n) {
-    // B operand: probabilities of head 4 n + hq, split into the 16-bit value (even columns) and its remainder
-    uint32_t bb[2];
+    // B operand: probabilities of head 4 n + hq, split into the 16-bit value (even columns) and its remainder; bf16 pairs
+    // leave a third part of 8 bits, which goes through a product of its own
+    uint32_t bb[2], b3[2];
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-      float pv[2];
+      float pv[2], rest[2];
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const float pf = __shfl_sync(0xffffffffu, sv[n][half], 4 * (2 * t + k) + hq);
         const float hi = bf ? __bfloat162float(__float2bfloat16_rn(pf)) : __half2float(__float2half_rn(pf));
         pv[k] = (g & 1) ? pf - hi : hi;
+        rest[k] = (g & 1) ? pv[k] - __bfloat162float(__float2bfloat16_rn(pv[k])) : 0.f;
       }
       if (bf) {
-        const __nv_bfloat162 v = __floats2bfloat162_rn(pv[0], pv[1]);
+        const __nv_bfloat162 v = __floats2bfloat162_rn(pv[0], pv[1]), r = __floats2bfloat162_rn(rest[0], rest[1]);
         bb[half] = *reinterpret_cast<const uint32_t*>(&v);
+        b3[half] = *reinterpret_cast<const uint32_t*>(&r);
       } else {
         bb[half] = h2_bits(__floats2half2_rn(pv[0], pv[1]));
       }
@@ -455,8 +438,14 @@ __device__ __forceinline__ void dense_tile(const MzDecodeParams& p, uint32_t kbu
       // rows g / g+8 = channels 2m / 2m+1 of the lane's; columns = tokens (2t, 2t+1) and (2t+8, 2t+9)
       const uint32_t a0 = prmt(vx[0][m], vx[1][m], 0x5410u), a1 = prmt(vx[0][m], vx[1][m], 0x7632u);
       const uint32_t a2 = prmt(vx[2][m], vx[3][m], 0x5410u), a3 = prmt(vx[2][m], vx[3][m], 0x7632u);
-      if (bf) mma_bf16(out[n][m], a0, a1, a2, a3, bb[0], bb[1]);
-      else mma_f16(out[n][m], a0, a1, a2, a3, bb[0], bb[1]);
+      float x[4];
+      if (bf) {
+        mma_bf16_first(x, a0, a1, a2, a3, b3[0], b3[1]);
+        mma_bf16(x, a0, a1, a2, a3, bb[0], bb[1]);
+      } else {
+        mma_f16_first(x, a0, a1, a2, a3, bb[0], bb[1]);
+      }
+      add4(out[n][m], x);
     }
   }
 }
@@ -600,9 +589,9 @@ template <int BITS, int D_, int G_, int NT>
 __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mma_kernel(const __grid_constant__ MzDecodeParams p) {
   using C = Cfg<BITS, D_, G_, NT>;
   constexpr int D = D_, G = G_, NG = C::NG, CPL = C::CPL, MT = C::MT, NB = C::NB;
-  constexpr int QT = MT < 4 ? MT : 4;         // M tiles of one quad of lookups
-  constexpr int NQ = MT / QT;                 // quads along a row (2 when the group is 128)
-  constexpr int NA = 4 * QT;
+  constexpr int QT = 2;                       // M tiles of a step: half a quad of lookups
+  constexpr int NQ = MT / QT;                 // steps along a row
+  constexpr int SPQ = MT < 4 ? 1 : 2;         // steps of a quad
   const mz_kv_store& s = p.s;
   const int bits = BITS == 0 ? s.bits : BITS;
   const int QB = G * bits / 8;                // bytes of one packed row
@@ -642,10 +631,9 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
   L.q = L.ri + C::RI_BYTES - C::Q_BYTES;
   L.a = L.ri + C::RI_BYTES;
   L.pbuf = L.a + C::A_BYTES;
-  const uint32_t lbK = window + TBL + lane * 4;
-  // equal alphas: the fill wrote one table, to the lower half of the slots
-  const bool one_alpha = s.alpha_key == s.alpha_value;
-  const uint32_t lbV = lbK + (one_alpha ? 0u : 128u);
+  // a 64-bit load is served one half of the warp at a time: 16 copies are enough to keep the lookups free of conflicts
+  const uint32_t lbK = window + TBL + (lane & 15) * 8;
+  const uint32_t lbV = lbK + (s.alpha_key == s.alpha_value ? 0u : 128u);      // equal alphas: one table, in the lower halves
   const int hq = g >> 1;                       // head (of each column set) this lane folds for (B operand column g)
   const uint32_t rem_mask = (g & 1) ? 0xFFFFFFFFu : 0u;   // odd columns carry the fp16 remainder of the folded query
   const bool bf = s.kv_dtype == MZ_BF16;
@@ -698,7 +686,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
   // group.  Returns whether any row has a real A (then they are in L.a: keys by channel, values [group][token]).
   auto prep_rows = [&](uint32_t buf, bool values, float alpha) -> bool {
     const int top = (1 << bits) - 1;
-    const float lg = C::WIDE ? __log2f(1.0f + alpha) : 0.f, inv_alpha = C::WIDE ? 1.0f / alpha : 0.f;
+    const float lg = C::WIDE ? log2f(1.0f + alpha) : 0.f, inv_alpha = C::WIDE ? 1.0f / alpha : 0.f;
     auto load_row = [&](int r, float& lo, float& span) {
       if (msz == 4) {
         lo = ldsf(buf + CODE_BYTES + r * 4);
@@ -708,31 +696,24 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         span = mz_u16_to_float((uint16_t)lds16(buf + CODE_BYTES + D * 2 + r * 2), s.meta_dtype);
       }
     };
-    // frac: position of the anchor inside the bin of its zero code, [-0.5, 0.5]
-    auto put_row = [&](int r, float span, float bup, float bdn, int zc, float frac) {
+    auto put_row = [&](int r, float span, float bup, float bdn, int zc) {
       const int pos = values ? r / NG : r, grp = values ? r % NG : 0;
       if (C::WIDE) {
         const int blk = values ? (pos >> 4) * NG + grp : pos >> 4;
         const uint32_t at = L.ri + (blk * 4 + ((pos >> 2) & 3)) * 128 + (pos & 3) * 16;
-        const float inv = __fdividef(inv_alpha, span);
-        sts128(at, make_uint4(__float_as_uint(8388608.0f + (float)zc), __float_as_uint(__fdividef(lg, (float)max(top - zc, 1))),
-                              __float_as_uint(__fdividef(lg, (float)max(zc, 1))), __float_as_uint(bup * inv)));
+        const float inv = __fdiv_rn(inv_alpha, span);
+        sts128(at, make_uint4(__float_as_uint(8388608.0f + (float)zc), __float_as_uint(__fdiv_rn(lg, (float)max(top - zc, 1))),
+                              __float_as_uint(__fdiv_rn(lg, (float)max(zc, 1))), __float_as_uint(bup * inv)));
         const float sp = fminf(span, 65504.f);
         const __half sh = __float2half_rn(sp);
         sts128(at + 64, make_uint4(__float_as_uint(-bdn * inv), pack_u16(__half_as_ushort(sh), __half_as_ushort(__float2half_rn(sp - __half2float(sh)))), 0u, 0u));
       } else {
-        // a row whose zero code is the first / last code has no codes on the other side: that side's constant only
-        // ever multiplies the remainder half of the table entries
-        if (zc == 0) bdn = bup;
-        if (zc == top) bup = bdn;
         const int blk = values ? (pos >> 3) * NG + grp : pos >> 3;
-        constexpr int SB = 1 << C::SUB;
-        const int zi = zc * SB + (SB > 1 ? min(max((int)((frac + 0.5f) * (float)SB), 0), SB - 1) : 0);
         const __half2 hi = __floats2half2_rn(bup, bdn);
         const float2 hf = __half22float2(hi);
         const uint32_t lo = h2_bits(__floats2half2_rn(bup - hf.x, bdn - hf.y)), at = (blk * 4 + (pos & 3)) * 2 + ((pos >> 2) & 1);
         asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(L.ri + at * 8), "r"(h2_bits(hi)), "r"(lo) : "memory");
-        sts8(L.ri + D * 8 + at, (uint32_t)(zi << BITS) | (C::TWIN && one_alpha && frac >= 0.0f ? 1u : 0u));
+        sts8(L.ri + D * 8 + at, (uint32_t)(zc << BITS));
       }
     };
     float A[D / 32];
@@ -742,11 +723,10 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
       const int r = lane + 32 * i;
       float lo, span, bup, bdn;
       int zc;
-      float frac;
       load_row(r, lo, span);
-      row_split(lo, span, (float)top, A[i], bup, bdn, zc, wild, &frac);
+      row_split(lo, span, (float)top, A[i], bup, bdn, zc, wild);
       any |= A[i] != 0.0f;
-      put_row(r, fmaxf(span, 1e-8f), bup, bdn, zc, frac);
+      put_row(r, fmaxf(span, 1e-8f), bup, bdn, zc);
     }
     if (__any_sync(0xffffffffu, wild)) {
 #pragma unroll 1
@@ -756,7 +736,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         int zc;
         load_row(r, lo, span);
         row_split(lo, span, (float)top, a, bup, bdn, zc, wild);
-        put_row(r, fmaxf(span, 1e-8f), bup, bdn, exact_zero_code(lo, span, (float)top), 0.0f);
+        put_row(r, fmaxf(span, 1e-8f), bup, bdn, exact_zero_code(lo, span, (float)top));
       }
     }
     any = __any_sync(0xffffffffu, any);
@@ -868,7 +848,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
   // kernel was launched as a programmatic dependent of the previous kernel in the stream (the merge kernel of the
   // previous call, the flush of this step) this prologue runs while that kernel drains.  Global memory is first
   // touched after the wait (the table entries were written long before).
-  if (!C::WIDE && kt > 0) fill_tables<C, C::WIDE ? 1 : BITS>(window + TBL, p.lut, s.alpha_key, s.alpha_value);
+  if (!C::WIDE && kt > 0) fill_tables<C, C::WIDE ? 1 : BITS>(window + TBL, (const uint2*)p.lut, s.alpha_key, s.alpha_value);
   for (int i = lane; i < (int)C::P_BYTES / 4; i += 32) sts32(L.pbuf + i * 4, 0u);   // columns of absent heads stay zero for good
   asm volatile("griddepcontrol.wait;" ::: "memory");
   stage_k(cur, active);
@@ -934,18 +914,21 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
 #pragma unroll
           for (int k = 0; k < 4; ++k) acc[n][m][k] = 0.f;
       if constexpr (!C::WIDE) {
-        // steps (block, quad), a loop of two blocks: the code words and constants of step i+2 and the table values of step
-        // i+1 are in flight while the tensor cores work on step i.  (Unrolled over all blocks the kernel was 48 KB of
+        // steps (block, half a quad), a loop of two blocks: the code words and constants of step i+2 and the table values of
+        // step i+1 are in flight while the tensor cores work on step i.  (Unrolled over all blocks the kernel was 48 KB of
         // code and 168 registers; instruction fetch and three warps per scheduler were what it waited for.)
         constexpr int NS = NB * NQ, SPI = 2 * NQ;
         Quad<BITS, CPL> cw[2];
         uint4 rc[2];
-        uint32_t zz[2], qq[2][NT], av[2][NA], bfr[2][NT][2];
+        uint2 av[2][8];
+        uint32_t zz[2], qq[2][NT], bfr[2][NT][2];
         auto load_step = [&](int blk, int u) {            // u: static step number, blk: its block
           const int q = u % NQ;
-          const uint32_t r0 = L.kbuf + (8 * blk + t) * QB + lane_offset<BITS, CPL>(g);
-          if constexpr (BITS == 3 || BITS == 1) cw[u & 1].load(r0, r0 + 4 * QB, q, g);
-          else cw[u & 1].load(r0, r0 + 4 * QB, q);
+          if (q % SPQ == 0) {
+            const uint32_t r0 = L.kbuf + (8 * blk + t) * QB + lane_offset<BITS, CPL>(g);
+            if constexpr (BITS == 3 || BITS == 1) cw[(u / SPQ) & 1].load(r0, r0 + 4 * QB, q / SPQ, g);
+            else cw[(u / SPQ) & 1].load(r0, r0 + 4 * QB, q / SPQ);
+          }
           if (q == 0) {
             rc[(u / NQ) & 1] = lds128(L.ri + (blk * 4 + t) * 16);
             zz[(u / NQ) & 1] = lds16(L.ri + D * 8 + (blk * 4 + t) * 2);
@@ -954,14 +937,16 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
           }
         };
         auto open_step = [&](int u) {
-          const uint4& c = rc[(u / NQ) & 1];
-          look_step<C>(cw[u & 1], zz[(u / NQ) & 1], lbK, av[u & 1]);
+          const int o = (u / NQ) & 1;
+          look_step(cw[(u / SPQ) & 1], u % SPQ, zz[o], lbK, av[u & 1]);
           // fold q * B: even columns the product rounded to fp16, odd columns what that rounding dropped
+          if (u % NQ == 0) {
 #pragma unroll
-          for (int n = 0; n < NT; ++n) {
-            const uint32_t x = qq[(u / NQ) & 1][n], xm = x & rem_mask;
-            bfr[u & 1][n][0] = fold_pair(dup_lo(x), dup_lo(xm), c.x, c.y, rem_mask);
-            bfr[u & 1][n][1] = fold_pair(dup_hi(x), dup_hi(xm), c.z, c.w, rem_mask);
+            for (int n = 0; n < NT; ++n) {
+              const uint32_t x = qq[o][n], xm = x & rem_mask;
+              bfr[o][n][0] = fold_pair(dup_lo(x), dup_lo(xm), rc[o].x, rc[o].y, rem_mask);
+              bfr[o][n][1] = fold_pair(dup_hi(x), dup_hi(xm), rc[o].z, rc[o].w, rem_mask);
+            }
           }
         };
         load_step(0, 0);
@@ -977,9 +962,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
 #pragma unroll
             for (int n = 0; n < NT; ++n)
 #pragma unroll
-              for (int m = 0; m < QT; ++m)
-                mma_f16(acc[n][(u % NQ) * QT + m], av[u & 1][4 * m], av[u & 1][4 * m + 1], av[u & 1][4 * m + 2], av[u & 1][4 * m + 3],
-                        bfr[u & 1][n][0], bfr[u & 1][n][1]);
+              for (int m = 0; m < QT; ++m) mma_step(acc[n][(u % NQ) * QT + m], av[u & 1], m, bfr[(u / NQ) & 1][n][0], bfr[(u / NQ) & 1][n][1]);
           }
         }
       } else {
@@ -993,9 +976,14 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
               const uint32_t x = lds32(L.q + (n * NB + 2 * blk + k) * 64 + (hq * 4 + t) * 4);
               bb[n][k] = fold_pair(bits_h2(x), bits_h2(x & rem_mask), pack_u16(sp[2 * k], sp[2 * k + 1]), prmt(sp[2 * k], sp[2 * k + 1], 0x7632u), rem_mask);
             }
-        }, [&](int, int m, const uint32_t (&a)[4], const uint32_t (&bb)[NT][2]) {
+        }, [&](int, int m, const uint32_t (&hi)[4], const uint32_t (&lo)[4], const uint32_t (&bb)[NT][2]) {
 #pragma unroll
-          for (int n = 0; n < NT; ++n) mma_f16(acc[n][m], a[0], a[1], a[2], a[3], bb[n][0], bb[n][1]);
+          for (int n = 0; n < NT; ++n) {
+            float x[4];
+            mma_f16_first(x, lo[0], lo[1], lo[2], lo[3], bb[n][0], bb[n][1]);
+            mma_f16(x, hi[0], hi[1], hi[2], hi[3], bb[n][0], bb[n][1]);
+            add4(acc[n][m], x);
+          }
         });
       }
       // constant term sum_d q[t][d] * A_d (rows whose range does not straddle zero)
@@ -1082,17 +1070,20 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
       };
       const uint32_t v_row = regroup ? QB : NG * QB, v_grp = regroup ? G * QB : QB;     // token and group strides in the staged tile
       if constexpr (!C::WIDE) {
-        // steps (token block j, group, quad), a loop of one or two token blocks; the probabilities of a token block are
-        // read once
+        // steps (token block j, group, half a quad), a loop of one or two token blocks; the probabilities of a token block
+        // are read once
         constexpr int NS = NB * NQ, BPI = NG > 2 ? NG : 2, SPI = BPI * NQ;       // blocks and steps of an iteration
         Quad<BITS, CPL> cw[2];
         uint4 rc[2];
-        uint32_t zz[2], av[2][NA], bfr[2][NT][2], ph[2][NT], pl[2][NT];
+        uint2 av[2][8];
+        uint32_t zz[2], bfr[2][NT][2], ph[2][NT], pl[2][NT];
         auto load_step = [&](int blk, int u) {
           const int q = u % NQ, grp = (u / NQ) % NG, j = blk / NG;
-          const uint32_t r0 = L.vbuf + (8 * j + t) * v_row + grp * v_grp + lane_offset<BITS, CPL>(g);
-          if constexpr (BITS == 3 || BITS == 1) cw[u & 1].load(r0, r0 + 4 * v_row, q, g);
-          else cw[u & 1].load(r0, r0 + 4 * v_row, q);
+          if (q % SPQ == 0) {
+            const uint32_t r0 = L.vbuf + (8 * j + t) * v_row + grp * v_grp + lane_offset<BITS, CPL>(g);
+            if constexpr (BITS == 3 || BITS == 1) cw[(u / SPQ) & 1].load(r0, r0 + 4 * v_row, q / SPQ, g);
+            else cw[(u / SPQ) & 1].load(r0, r0 + 4 * v_row, q / SPQ);
+          }
           if (q == 0) {
             rc[(u / NQ) & 1] = lds128(L.ri + (blk * 4 + t) * 16);
             zz[(u / NQ) & 1] = lds16(L.ri + D * 8 + (blk * 4 + t) * 2);
@@ -1103,15 +1094,17 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
           }
         };
         auto open_step = [&](int u) {
-          const uint4& c = rc[(u / NQ) & 1];
-          look_step<C>(cw[u & 1], zz[(u / NQ) & 1], lbV, av[u & 1]);
+          const int o = (u / NQ) & 1;
+          look_step(cw[(u / SPQ) & 1], u % SPQ, zz[o], lbV, av[u & 1]);
           // fold (ph + pl) * B: even columns fp16(ph * B), odd columns its remainder + pl * B
+          if (u % NQ == 0) {
 #pragma unroll
-          for (int n = 0; n < NT; ++n) {
-            const uint32_t hi = ph[(u / NQ / NG) & 1][n], lo = pl[(u / NQ / NG) & 1][n];
-            const uint32_t hm = hi & rem_mask;
-            bfr[u & 1][n][0] = h2_bits(__hfma2(dup_lo(lo), bits_h2(c.x), bits_h2(fold_pair(dup_lo(hi), dup_lo(hm), c.x, c.y, rem_mask))));
-            bfr[u & 1][n][1] = h2_bits(__hfma2(dup_hi(lo), bits_h2(c.z), bits_h2(fold_pair(dup_hi(hi), dup_hi(hm), c.z, c.w, rem_mask))));
+            for (int n = 0; n < NT; ++n) {
+              const uint32_t hi = ph[(u / NQ / NG) & 1][n], lo = pl[(u / NQ / NG) & 1][n];
+              const uint32_t hm = hi & rem_mask;
+              bfr[o][n][0] = h2_bits(__hfma2(dup_lo(lo), bits_h2(rc[o].x), bits_h2(fold_pair(dup_lo(hi), dup_lo(hm), rc[o].x, rc[o].y, rem_mask))));
+              bfr[o][n][1] = h2_bits(__hfma2(dup_hi(lo), bits_h2(rc[o].z), bits_h2(fold_pair(dup_hi(hi), dup_hi(hm), rc[o].z, rc[o].w, rem_mask))));
+            }
           }
         };
         // two iterations are unrolled where a token block's probabilities alternate between two registers across them
@@ -1130,8 +1123,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
             for (int n = 0; n < NT; ++n)
 #pragma unroll
               for (int m = 0; m < QT; ++m)
-                mma_f16(out[n][((u / NQ) % NG) * MT + (u % NQ) * QT + m], av[u & 1][4 * m], av[u & 1][4 * m + 1], av[u & 1][4 * m + 2],
-                        av[u & 1][4 * m + 3], bfr[u & 1][n][0], bfr[u & 1][n][1]);
+                mma_step(out[n][((u / NQ) % NG) * MT + (u % NQ) * QT + m], av[u & 1], m, bfr[(u / NQ) & 1][n][0], bfr[(u / NQ) & 1][n][1]);
           }
         }
       } else {
@@ -1148,9 +1140,14 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
               const uint32_t S = pack_u16(sp[2 * k], sp[2 * k + 1]);
               bb[n][k] = h2_bits(__hfma2(bits_h2(lo), bits_h2(S), bits_h2(fold_pair(bits_h2(hi), bits_h2(hi & rem_mask), S, prmt(sp[2 * k], sp[2 * k + 1], 0x7632u), rem_mask))));
             }
-        }, [&](int k, int m, const uint32_t (&a)[4], const uint32_t (&bb)[NT][2]) {
+        }, [&](int k, int m, const uint32_t (&hi)[4], const uint32_t (&lo)[4], const uint32_t (&bb)[NT][2]) {
 #pragma unroll
-          for (int n = 0; n < NT; ++n) mma_f16(out[n][k * MT + m], a[0], a[1], a[2], a[3], bb[n][0], bb[n][1]);
+          for (int n = 0; n < NT; ++n) {
+            float x[4];
+            mma_f16_first(x, lo[0], lo[1], lo[2], lo[3], bb[n][0], bb[n][1]);
+            mma_f16(x, hi[0], hi[1], hi[2], hi[3], bb[n][0], bb[n][1]);
+            add4(out[n][k * MT + m], x);
+          }
         });
       }
       warp_sync();                  // every lane is done with vbuf, the row constants and the probabilities

@@ -712,7 +712,7 @@ int plan_single(MzDecodeParams& p, int splits_request, int sm_count, size_t* slo
   if ((unsigned)warps > (window_end - high_base) / per_high) warps = (int)((window_end - high_base) / per_high);
   if (warps < 1) return mz_fail(MZ_ERR_UNSUPPORTED, "tile does not fit shared memory");
   t.kind = 3;
-  p.lut = s.k_groups > 0 ? mz_mma_lookup_entries(s.bits, 0, s.alpha_key, s.alpha_value) : nullptr;
+  p.lut = s.k_groups > 0 ? mz_mma_lookup_entries(s.bits, false, s.alpha_key, s.alpha_value) : nullptr;
   t.stage_bytes = sb;
   t.low_base = low_base;
   t.high_base = high_base;

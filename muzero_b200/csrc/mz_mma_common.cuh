@@ -61,7 +61,25 @@ __device__ __forceinline__ void cp16(uint32_t sa, const void* g) {
 }
 __device__ __forceinline__ void warp_sync() { __syncwarp(); }
 
-// D(16x8, fp32) += A(16x16) * B(16x8), 16-bit operands of the named type
+// D(16x8, fp32) += A(16x16) * B(16x8), 16-bit operands of the named type; the _first forms start from zero
+__device__ __forceinline__ void mma_f16_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void mma_bf16_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+// c += t, rounded to nearest (the tensor cores' own accumulation truncates)
+__device__ __forceinline__ void add4(float (&c)[4], const float (&t)[4]) {
+  asm("{\n\t.reg .b64 x, y;\n\t"
+      "mov.b64 x, {%0, %1};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%6, %7};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%2, %3}, x;\n\t}"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "f"(t[0]), "f"(t[1]), "f"(t[2]), "f"(t[3]));
+}
 __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -83,15 +101,13 @@ __device__ __forceinline__ __half2 dup_hi(uint32_t v) { return __half2half2(__hi
 // of an entry carries the fp16 remainder of the active half, pre-scaled by the nominal ratio Bdn / Bup of a row
 // in that zero-code bin (anchor at the bin centre); the end bins have codes on one side only and row_constants
 // makes their two constants equal.  Called by every thread of the CTA; the caller synchronises afterwards.
-// sub-bins of a zero code's anchor range in the general kernel's table, by code width (log2)
-constexpr int kSubBits[5] = {0, 0, 3, 2, 0};
-// entry idx = (zc, sub-bin, e) of the table for `alpha`, as the bits of half2(u+, u-)
-template <int BITS, int SUB = 0>
+// entry idx = (zc, e) of the table for `alpha`, as the bits of half2(u+, u-)
+template <int BITS>
 __device__ __forceinline__ uint32_t lookup_entry(float alpha, int idx) {
-  constexpr int NE = 1 << BITS, TOP = NE - 1, SB = 1 << SUB;
-  const int zc = idx >> (BITS + SUB), e = idx & TOP;
+  constexpr int NE = 1 << BITS, TOP = NE - 1;
+  const int zc = idx >> BITS, e = idx & TOP;
   const float lb = log1pf(alpha);
-  const float zac = ((float)zc + (((float)((idx >> BITS) & (SB - 1)) + 0.5f) / (float)SB - 0.5f)) / (float)TOP;    // middle of the bin
+  const float zac = (float)zc / (float)TOP;    // middle of the bin
   const float ratio = (zc == 0 || zc == TOP) ? 1.0f : zac / (1.0f - zac);
   __half2 ent;
   if (e >= zc) {
@@ -106,6 +122,17 @@ __device__ __forceinline__ uint32_t lookup_entry(float alpha, int idx) {
     ent = __floats2half2_rn((u - uh) * ratio, uh);
   }
   return h2_bits(ent);
+}
+// entry idx = (zc, e) of the general kernel's table: half2(u+, u-) rounded, and what the rounding dropped
+template <int BITS>
+__device__ __forceinline__ uint2 split_entry(float alpha, int idx) {
+  constexpr int NE = 1 << BITS, TOP = NE - 1;
+  const int zc = idx >> BITS, e = idx & TOP;
+  const int room = max(e >= zc ? TOP - zc : zc, 1), n = min(abs(e - zc), room);
+  const float grow = expm1f((float)n / (float)room * log1pf(alpha)) / alpha, u = e >= zc ? grow : -grow;
+  const __half h = __float2half_rn(u), l = __float2half_rn(u - __half2float(h)), z = __ushort_as_half(0);
+  return e >= zc ? make_uint2(h2_bits(__halves2half2(h, z)), h2_bits(__halves2half2(l, z)))
+                 : make_uint2(h2_bits(__halves2half2(z, h)), h2_bits(__halves2half2(z, l)));
 }
 // stores one entry to the 32 lane copies of its slot half (rotated so that the lanes of a warp, which hold
 // consecutive entries, hit different banks)
@@ -163,8 +190,7 @@ __device__ __forceinline__ void row_constants(float lo, float span, int& zc, flo
 // an ulp of b/s, q + (b - q s) y rounds to RN(b/s)); that is branch-free, where the IEEE division costs a range test and a
 // slow path per row.  Ties matter: 16-bit extremes often give a quotient that lies exactly on a code boundary.
 // Spans from 2^125 on would flush the reciprocal: `wild` asks for the division.
-__device__ __forceinline__ void row_split(float lo, float span, float top, float& A, float& bup, float& bdn, int& zc, bool& wild,
-                                          float* frac = nullptr) {
+__device__ __forceinline__ void row_split(float lo, float span, float top, float& A, float& bup, float& bdn, int& zc, bool& wild) {
   span = fmaxf(span, 1e-8f);
   bdn = fminf(fmaxf(-lo, 0.0f), span);
   bup = span - bdn;
@@ -176,7 +202,6 @@ __device__ __forceinline__ void row_split(float lo, float span, float top, float
   const float q = fmaf(fmaf(-q0, span, bdn), y, q0);
   const float pos = __fmul_rn(q, top), r = pos + 12582912.0f;
   zc = __float_as_int(r) & 0xff;
-  if (frac != nullptr) *frac = pos - (r - 12582912.0f);
   wild |= !(span < 4e37f);
   bup = fminf(bup, 65504.f);
   bdn = fminf(bdn, 65504.f);

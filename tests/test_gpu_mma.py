@@ -37,3 +37,62 @@ def test_widths_groups_heads(oracle, bits, D, group, gqa, S, residual):
     want = oracle.decode_attention_oracle(q, ref, D ** -0.5, gqa, mask=mask, compute_dtype=torch.float32)
     check_output(decode_attention(layer, q.cuda(), D ** -0.5, mask.cuda(), out_dtype=torch.float32),
                  decode_attention(layer, q.cuda(), D ** -0.5, mask.cuda()), want)
+
+
+def attention64(oracle, ref, q, scaling, mask=None):
+    """Attention over the oracle's dequantized store and window, evaluated in 64 bits: [B,1,H,D]."""
+    k = torch.cat(([ref.key_prefix(torch.float32)] if ref.packed_k is not None else []) + [ref.keys.float()], dim=2).double()
+    v = torch.cat(([ref.value_prefix(torch.float32)] if ref.packed_v is not None else []) + [ref.values.float()], dim=2).double()
+    b, h, _, d = q.shape
+    logits = torch.matmul(q.double().reshape(b, k.shape[1], -1, d), k.transpose(2, 3)) * scaling
+    if mask is not None:
+        logits = logits + mask.double()
+    return torch.matmul(torch.softmax(logits, dim=-1), v).reshape(b, 1, h, d)
+
+
+def relative_error(got, want):
+    return ((got.double().cpu() - want).norm() / want.norm()).item()
+
+
+# About twenty fp32 roundings (2^-24 each) lie between the inputs and an output: the dequantizer's, the product and sum of
+# the logits (relative to a logit of up to about 8), exponential, products and sums of the values.  Sums over tokens
+# average them.  2e-6 is the plain sum of the twenty, times 1.6.
+FP32_ERROR = 2e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bits,D,group,gqa", [(1, 128, 64, 8), (2, 128, 128, 4), (2, 64, 64, 3), (3, 128, 64, 4), (3, 64, 32, 8), (4, 128, 64, 8),
+                                              (4, 128, 32, 4), (4, 64, 64, 1), (5, 64, 64, 4), (8, 128, 64, 8), (8, 64, 32, 2)])
+def test_error_against_64_bits(oracle, bits, D, group, gqa, dtype):
+    """The general tensor-core kernel (cluster mode and flat cut) has the error of an fp32 evaluation; the residual window
+    alone as well."""
+    import muzero_b200 as mz
+    from muzero_b200.cache.attention import decode_attention
+    for S in (100, 900):
+        k, v, q = oracle.synth_kv(2, 2, S, D, 2 * gqa, seed=bits + D, dtype=dtype)
+        ref = oracle.OracleCacheLayer(bits=bits, group=group, residual=128, alpha_key=2.0, alpha_value=4.0)
+        ref.append(k, v)
+        cfg = mz.MuZeroConfig(bits=4, q_group_size=group, residual_length=128, alpha_key=2.0, alpha_value=4.0)
+        cfg.bits = bits
+        layer = mz.MuZeroCacheLayer(cfg)
+        layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+        want = attention64(oracle, ref, q, D ** -0.5)
+        for splits in (0, 5):
+            got = decode_attention(layer, q.cuda(), D ** -0.5, out_dtype=torch.float32, splits=splits)
+            assert relative_error(got, want) <= FP32_ERROR, (S, splits)
+
+
+@pytest.mark.parametrize("bits,bound", [(2, 1.2e-4), (4, 5e-5)])
+def test_error_of_the_unrolled_kernel(oracle, bits, bound):
+    """Head_dim 128, group 64, up to four heads, more pairs than SMs: the unrolled kernel's table keeps 11 bits and a nominal
+    remainder.  The remainder's ratio is off by up to the width of a zero code's bin, so an entry is wrong by up to
+    2^-12 (half an fp16 ulp) at 2 bits, a fourth of that at 4 bits; sums over channels and tokens average it down by half."""
+    import muzero_b200 as mz
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = oracle.synth_kv(20, 8, 400, 128, 32, seed=bits)
+    ref = oracle.OracleCacheLayer(bits=bits, group=64, residual=128, alpha_key=2.0, alpha_value=2.0)
+    ref.append(k, v)
+    layer = mz.MuZeroCacheLayer(mz.MuZeroConfig(bits=bits, alpha_key=2.0, alpha_value=2.0))
+    layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+    got = decode_attention(layer, q.cuda(), 128 ** -0.5, out_dtype=torch.float32)
+    assert relative_error(got, attention64(oracle, ref, q, 128 ** -0.5)) <= bound
