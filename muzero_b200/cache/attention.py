@@ -21,6 +21,7 @@ from ..kernels.loader import load_mu_zero_cuda_extension
 
 _MU_ZERO_DECODE_STATS = defaultdict(int)
 _workspaces: dict = {}
+_outgrown: list = []
 
 
 def reset_mu_zero_decode_stats() -> None:
@@ -32,13 +33,17 @@ def get_mu_zero_decode_stats() -> dict[str, int]:
 
 
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """One reusable scratch buffer per (device, stream); grows, never shrinks."""
+    """One reusable scratch buffer per (device, stream); grows, never shrinks.
+
+    A captured CUDA graph keeps the address of the buffer that it was captured with, so none is ever given up: there are
+    as many as streams (torch hands out 32 per device and priority), and one that has to grow at least doubles and its
+    predecessors, together smaller than it, are kept."""
     key = (device.index, stream_ptr(device))
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
-        if len(_workspaces) >= 64:      # streams come and go
-            _workspaces.clear()
-        buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+        if buf is not None:
+            _outgrown.append(buf)
+        buf = torch.empty(max(nbytes, 1 << 20, 0 if buf is None else 2 * buf.numel()), dtype=torch.uint8, device=device)
         _workspaces[key] = buf
     return buf
 

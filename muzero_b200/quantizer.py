@@ -67,8 +67,8 @@ def _stat_workspace(device: torch.device) -> torch.Tensor:
     key = (device.index, torch.cuda.current_stream(device).cuda_stream)
     ws = _stat_workspaces.get(key)
     if ws is None:
-        if len(_stat_workspaces) >= 64:      # streams come and go
-            _stat_workspaces.clear()
+        if len(_stat_workspaces) >= 64:      # streams come and go; the oldest buffer's stream orders what is still in flight
+            _stat_workspaces.pop(next(iter(_stat_workspaces)), None)
         ws = torch.zeros(load_mu_zero_cuda_extension().mz_alpha_stats_workspace_bytes(), dtype=torch.uint8, device=device)
         _stat_workspaces[key] = ws
     return ws

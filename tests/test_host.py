@@ -178,3 +178,23 @@ def test_prefill_deferral_rules(monkeypatch):
     chunked.defer_prefill_quantization = True
     chunked.single_shot_prefill = False
     assert chunked.prefill_block_defers(0) is False          # ... unless chunks are to be quantized as they arrive
+
+
+def test_scratch_buffers_stay_where_a_captured_graph_saw_them(monkeypatch):
+    """Addresses handed out once stay allocated: through any number of other streams, and when the buffer has to grow."""
+    from muzero_b200.cache import attention as A
+    stream = [1]
+    monkeypatch.setattr(A, "_workspaces", {})
+    monkeypatch.setattr(A, "_outgrown", [], raising=False)
+    monkeypatch.setattr(A, "stream_ptr", lambda device: stream[0])
+    cpu = torch.device("cpu")
+    first = A._workspace(cpu, 100).data_ptr()
+    alive = lambda: {t.data_ptr() for t in [*A._workspaces.values(), *A._outgrown]}
+    for stream[0] in range(2, 200):
+        A._workspace(cpu, 100)
+    assert first in alive()
+    stream[0] = 1
+    assert A._workspace(cpu, 100).data_ptr() == first
+    grown = A._workspace(cpu, (1 << 20) + 1)
+    assert grown.numel() >= 2 << 20 and first in alive()
+    assert sum(t.numel() for t in A._outgrown) < grown.numel()
