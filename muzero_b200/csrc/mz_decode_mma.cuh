@@ -43,6 +43,11 @@
 namespace mzm {
 constexpr int DT = 16;                      // tokens per residual tile
 constexpr uint32_t WIDE_ROW = 32;           // row constants of a wide code: 8 words
+// Operands are kept away from fp16's subnormals (2^-24) and its largest value (65504): the query's largest element is
+// scaled by a power of two into [64, 128), the largest range among the rows of a tile (of each value group) into
+// [128, 256), probabilities by 128.  Products stay below 2^15, and what a remainder can lose is 2^-40 of the largest
+// product.  The powers of two are taken back in the fp32 sums.
+constexpr float P_SCALE = 128.0f;
 
 // BITS: 1..4 and 8, or 0 for 5..7 (code width at run time)
 template <int BITS, int D_, int G_, int NT_>
@@ -188,11 +193,13 @@ __device__ __forceinline__ void look_step(const Q& w, int h, uint32_t zz, uint32
 // One step's product with M tile `m` of half a quad, added to c: the remainders first, then the rounded values, on a
 // fresh accumulator, so that the running sum is rounded to nearest (the tensor cores truncate theirs: over the 256 steps
 // of eight tiles that alone would be 1e-5).
-__device__ __forceinline__ void mma_step(float (&c)[4], const uint2 (&a)[8], int m, uint32_t b0, uint32_t b1) {
+template <bool SCALED = false>
+__device__ __forceinline__ void mma_step(float (&c)[4], const uint2 (&a)[8], int m, uint32_t b0, uint32_t b1, float unit = 1.0f) {
   float x[4];
   mma_f16_first(x, a[4 * m].y, a[4 * m + 1].y, a[4 * m + 2].y, a[4 * m + 3].y, b0, b1);
   mma_f16(x, a[4 * m].x, a[4 * m + 1].x, a[4 * m + 2].x, a[4 * m + 3].x, b0, b1);
-  add4(c, x);
+  if (SCALED) fma4(c, x, unit);
+  else add4(c, x);
 }
 
 // ---- the lookup table, from the entries [2][ENTRIES] = (keys' alpha, values' alpha) in global memory (nullptr: they
@@ -420,7 +427,7 @@ __device__ __forceinline__ void dense_tile(const MzDecodeParams& p, uint32_t kbu
       float pv[2], rest[2];
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const float pf = __shfl_sync(0xffffffffu, sv[n][half], 4 * (2 * t + k) + hq);
+        const float pf = P_SCALE * __shfl_sync(0xffffffffu, sv[n][half], 4 * (2 * t + k) + hq);
         const float hi = bf ? __bfloat162float(__float2bfloat16_rn(pf)) : __half2float(__float2half_rn(pf));
         pv[k] = (g & 1) ? pf - hi : hi;
         rest[k] = (g & 1) ? pv[k] - __bfloat162float(__float2bfloat16_rn(pv[k])) : 0.f;
@@ -445,7 +452,7 @@ __device__ __forceinline__ void dense_tile(const MzDecodeParams& p, uint32_t kbu
       } else {
         mma_f16_first(x, a0, a1, a2, a3, bb[0], bb[1]);
       }
-      add4(out[n][m], x);
+      fma4(out[n][m], x, 1.0f / P_SCALE);
     }
   }
 }
@@ -684,7 +691,8 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
 
   // ---- per-row constants of one staged tile side -> L.ri; row r of the side: keys r = channel, values r = token * NG +
   // group.  Returns whether any row has a real A (then they are in L.a: keys by channel, values [group][token]).
-  auto prep_rows = [&](uint32_t buf, bool values, float alpha) -> bool {
+  // unit: what one unit of the scaled constants stands for, in the rows of this lane's value group (lane % NG).
+  auto prep_rows = [&](uint32_t buf, bool values, float alpha, float& unit) -> bool {
     const int top = (1 << bits) - 1;
     const float lg = C::WIDE ? log2f(1.0f + alpha) : 0.f, inv_alpha = C::WIDE ? 1.0f / alpha : 0.f;
     auto load_row = [&](int r, float& lo, float& span) {
@@ -704,9 +712,8 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         const float inv = __fdiv_rn(inv_alpha, span);
         sts128(at, make_uint4(__float_as_uint(8388608.0f + (float)zc), __float_as_uint(__fdiv_rn(lg, (float)max(top - zc, 1))),
                               __float_as_uint(__fdiv_rn(lg, (float)max(zc, 1))), __float_as_uint(bup * inv)));
-        const float sp = fminf(span, 65504.f);
-        const __half sh = __float2half_rn(sp);
-        sts128(at + 64, make_uint4(__float_as_uint(-bdn * inv), pack_u16(__half_as_ushort(sh), __half_as_ushort(__float2half_rn(sp - __half2float(sh)))), 0u, 0u));
+        const __half sh = __float2half_rn(span);
+        sts128(at + 64, make_uint4(__float_as_uint(-bdn * inv), pack_u16(__half_as_ushort(sh), __half_as_ushort(__float2half_rn(span - __half2float(sh)))), 0u, 0u));
       } else {
         const int blk = values ? (pos >> 3) * NG + grp : pos >> 3;
         const __half2 hi = __floats2half2_rn(bup, bdn);
@@ -716,29 +723,35 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         sts8(L.ri + D * 8 + at, (uint32_t)(zc << BITS));
       }
     };
-    float A[D / 32];
+    float A[D / 32], sp[D / 32], bup[D / 32], bdn[D / 32];
+    int zc[D / 32];
     bool any = false, wild = false;
+    float most = 0.f;
 #pragma unroll
     for (int i = 0; i < D / 32; ++i) {
-      const int r = lane + 32 * i;
-      float lo, span, bup, bdn;
-      int zc;
-      load_row(r, lo, span);
-      row_split(lo, span, (float)top, A[i], bup, bdn, zc, wild);
+      float lo;
+      load_row(lane + 32 * i, lo, sp[i]);
+      row_split(lo, sp[i], (float)top, A[i], bup[i], bdn[i], zc[i], wild);
       any |= A[i] != 0.0f;
-      put_row(r, fmaxf(span, 1e-8f), bup, bdn, zc);
+      sp[i] = fmaxf(sp[i], 1e-8f);
+      most = fmaxf(most, sp[i] < INFINITY ? sp[i] : 0.f);
     }
     if (__any_sync(0xffffffffu, wild)) {
-#pragma unroll 1
+#pragma unroll
       for (int i = 0; i < D / 32; ++i) {
-        const int r = lane + 32 * i;
-        float lo, span, a, bup, bdn;
-        int zc;
-        load_row(r, lo, span);
-        row_split(lo, span, (float)top, a, bup, bdn, zc, wild);
-        put_row(r, fmaxf(span, 1e-8f), bup, bdn, exact_zero_code(lo, span, (float)top));
+        float lo, span;
+        load_row(lane + 32 * i, lo, span);
+        zc[i] = exact_zero_code(lo, span, (float)top);
       }
     }
+    // the largest range of the tile side (keys) or of the value group
+#pragma unroll
+    for (int off = values ? NG : 1; off < 32; off <<= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, off));
+    const int ex = max(__float_as_int(most) >> 23, 64);              // most in [2^(ex-127), 2^(ex-126)), at least 1e-8 unless no range is finite
+    const float scale = __int_as_float((261 - ex) << 23);           // most * scale in [128, 256)
+    unit = __int_as_float((ex - 7) << 23);
+#pragma unroll
+    for (int i = 0; i < D / 32; ++i) put_row(lane + 32 * i, sp[i] * scale, bup[i] * scale, bdn[i] * scale, zc[i]);
     any = __any_sync(0xffffffffu, any);
     if (any) {
 #pragma unroll
@@ -863,7 +876,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
       if (cur_pair >= 0) { write_partial(); ++seg; }
       cur_pair = pair;
       reset_state();
-      // folded-query source: half2(q[8j+t], q[8j+4+t]) of head 4 n + hq, scaled by a power of two into [0.5, 1)
+      // folded-query source: half2(q[8j+t], q[8j+4+t]) of head 4 n + hq, scaled by a power of two into [64, 128)
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
         const int h = 4 * n + hq;
@@ -879,9 +892,9 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         int ex = (__float_as_int(amax) >> 23) & 0xff;            // amax in [2^(ex-127), 2^(ex-126))
-        ex = min(max(ex, 1), 253);
-        const float down = __int_as_float((253 - ex) << 23);     // 2^(126-ex): amax*down in [0.5, 1)
-        const float up = __int_as_float((ex + 1) << 23);         // 2^(ex-126)
+        ex = min(max(ex, 7), 254);
+        const float down = __int_as_float((260 - ex) << 23);     // 2^(133-ex): amax*down in [64, 128)
+        const float up = __int_as_float((ex - 6) << 23);         // 2^(ex-133)
 #pragma unroll
         for (int j = 0; j < NB; ++j)
           if ((g & 1) == 0) sts32(L.q + (n * NB + j) * 64 + (hq * 4 + t) * 4, h2_bits(__floats2half2_rn(qv[2 * j] * down, qv[2 * j + 1] * down)));
@@ -904,7 +917,8 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         for (int i = 0; i < CPL; ++i) mv[i] = mz_load_as_float(p.mask, mask0 + CPL * g + i, p.mask_dtype);
       }
       // ================= keys =================
-      const bool hasA = prep_rows(L.kbuf, false, s.alpha_key);
+      float un_k;
+      const bool hasA = prep_rows(L.kbuf, false, s.alpha_key, un_k);
       warp_sync();
       float acc[NT][MT][4];
 #pragma unroll
@@ -1010,8 +1024,8 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
       for (int n = 0; n < NT; ++n) {
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-          sv[n][2 * m] = fmaf(acc[n][m][0] + acc[n][m][1], qs[n], cA[n]);
-          sv[n][2 * m + 1] = fmaf(acc[n][m][2] + acc[n][m][3], qs[n], cA[n]);
+          sv[n][2 * m] = fmaf(acc[n][m][0] + acc[n][m][1], qs[n] * un_k, cA[n]);
+          sv[n][2 * m + 1] = fmaf(acc[n][m][2] + acc[n][m][3], qs[n] * un_k, cA[n]);
         }
         if (p.mask) {
 #pragma unroll
@@ -1019,9 +1033,10 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
         }
         softmax_update(n, sv[n]);
         if (4 * n + t < gqa) {
-          // probabilities as fp16 pairs (p[8j+i], p[8j+4+i]): column 2t the rounded values, column 2t+1 their
+          // scaled probabilities as fp16 pairs (p[8j+i], p[8j+4+i]): column 2t the rounded values, column 2t+1 their
           // remainders; word (j, i, column) is swizzled over the banks by j
           auto put = [&](int j, int i, float a, float b2) {
+            a *= P_SCALE; b2 *= P_SCALE;
             const __half2 ph = __floats2half2_rn(a, b2);
             const float2 phf = __half22float2(ph);
             const uint32_t wa = L.pbuf + j * (128 * NT), wi = (8 * NT) * i + 8 * n + 2 * t;
@@ -1040,9 +1055,10 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const uint32_t wi = (8 * NT) * i + 8 * n + 2 * t;
-              const __half ph = __float2half_rn(sv[n][i % CPL]);
+              const float a = sv[n][i % CPL] * P_SCALE;
+              const __half ph = __float2half_rn(a);
               sts16(wa + ((wi ^ pswz(j)) << 2), __half_as_ushort(ph));
-              sts16(wa + (((wi + 1) ^ pswz(j)) << 2), __half_as_ushort(__float2half_rn(sv[n][i % CPL] - __half2float(ph))));
+              sts16(wa + (((wi + 1) ^ pswz(j)) << 2), __half_as_ushort(__float2half_rn(a - __half2float(ph))));
             }
           }
         }
@@ -1050,8 +1066,11 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
       cp_async_wait<1>();
       warp_sync();                  // value tile landed; probabilities visible
       // ================= values =================
-      const bool hasAV = prep_rows(L.vbuf, true, s.alpha_value);
+      float un_mine, un_v[NG];
+      const bool hasAV = prep_rows(L.vbuf, true, s.alpha_value, un_mine);
       warp_sync();
+#pragma unroll
+      for (int k = 0; k < NG; ++k) un_v[k] = __shfl_sync(0xffffffffu, un_mine, k) * (1.0f / P_SCALE);
       if (hasAV) {
 #pragma unroll
         for (int n = 0; n < NT; ++n)
@@ -1123,7 +1142,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
             for (int n = 0; n < NT; ++n)
 #pragma unroll
               for (int m = 0; m < QT; ++m)
-                mma_step(out[n][((u / NQ) % NG) * MT + (u % NQ) * QT + m], av[u & 1], m, bfr[(u / NQ) & 1][n][0], bfr[(u / NQ) & 1][n][1]);
+                mma_step<true>(out[n][((u / NQ) % NG) * MT + (u % NQ) * QT + m], av[u & 1], m, bfr[(u / NQ) & 1][n][0], bfr[(u / NQ) & 1][n][1], un_v[(u / NQ) % NG]);
           }
         }
       } else {
@@ -1146,7 +1165,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
             float x[4];
             mma_f16_first(x, lo[0], lo[1], lo[2], lo[3], bb[n][0], bb[n][1]);
             mma_f16(x, hi[0], hi[1], hi[2], hi[3], bb[n][0], bb[n][1]);
-            add4(out[n][k * MT + m], x);
+            fma4(out[n][k * MT + m], x, un_v[k]);
           }
         });
       }

@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) decode_mma_kernel(const MzD
       int zc;
       load_row(r, lo, span);
       row_split(lo, span, (float)TOP, A[i], bup, bdn, zc, wild);
+      bup = fminf(bup, 65504.f); bdn = fminf(bdn, 65504.f);
       any |= A[i] != 0.0f;
       put_row(r, bup, bdn, zc);
     }
@@ -248,6 +249,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) decode_mma_kernel(const MzD
         int zc;
         load_row(r, lo, span);
         row_split(lo, span, (float)TOP, a, bup, bdn, zc, wild);
+        bup = fminf(bup, 65504.f); bdn = fminf(bdn, 65504.f);
         put_row(r, bup, bdn, exact_zero_code(lo, span, (float)TOP));
       }
     }

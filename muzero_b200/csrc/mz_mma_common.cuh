@@ -72,6 +72,14 @@ __device__ __forceinline__ void mma_bf16_first(float (&c)[4], uint32_t a0, uint3
       : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
+// c += t * f, rounded to nearest
+__device__ __forceinline__ void fma4(float (&c)[4], const float (&t)[4], float f) {
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 z, {%8, %8};\n\t"
+      "mov.b64 x, {%0, %1};\n\tmov.b64 y, {%4, %5};\n\tfma.rn.f32x2 x, y, z, x;\n\tmov.b64 {%0, %1}, x;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%6, %7};\n\tfma.rn.f32x2 x, y, z, x;\n\tmov.b64 {%2, %3}, x;\n\t}"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "f"(t[0]), "f"(t[1]), "f"(t[2]), "f"(t[3]), "f"(f));
+}
 // c += t, rounded to nearest (the tensor cores' own accumulation truncates)
 __device__ __forceinline__ void add4(float (&c)[4], const float (&t)[4]) {
   asm("{\n\t.reg .b64 x, y;\n\t"
@@ -203,8 +211,6 @@ __device__ __forceinline__ void row_split(float lo, float span, float top, float
   const float pos = __fmul_rn(q, top), r = pos + 12582912.0f;
   zc = __float_as_int(r) & 0xff;
   wild |= !(span < 4e37f);
-  bup = fminf(bup, 65504.f);
-  bdn = fminf(bdn, 65504.f);
 }
 __device__ __forceinline__ int exact_zero_code(float lo, float span, float top) {
   const float anchor = fminf(fmaxf(__fdiv_rn(__fsub_rn(0.0f, lo), fmaxf(span, 1e-8f)), 0.0f), 1.0f);

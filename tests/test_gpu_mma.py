@@ -58,6 +58,8 @@ def relative_error(got, want):
 # the logits (relative to a logit of up to about 8), exponential, products and sums of the values.  Sums over tokens
 # average them.  2e-6 is the plain sum of the twenty, times 1.6.
 FP32_ERROR = 2e-6
+# channels a thousandth of their group's range: the group's dequantized values round relative to the range
+SHARED_GROUP_ERROR = 1e3 * FP32_ERROR
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -80,6 +82,30 @@ def test_error_against_64_bits(oracle, bits, D, group, gqa, dtype):
         for splits in (0, 5):
             got = decode_attention(layer, q.cuda(), D ** -0.5, out_dtype=torch.float32, splits=splits)
             assert relative_error(got, want) <= FP32_ERROR, (S, splits)
+
+
+@pytest.mark.parametrize("vs,ks,qs,meta", [(1e-4, 1.0, 1.0, torch.float16), (1e-6, 1.0, 1.0, torch.float32), (1e5, 1.0, 1.0, torch.float32),
+                                           (1e5, 1.0, 1.0, torch.bfloat16), (1.0, 1e-4, 1e4, torch.float16), (1.0, 1e5, 1e-5, torch.float32)])
+@pytest.mark.parametrize("bits,D,group,gqa", [(1, 128, 128, 2), (3, 128, 64, 4), (4, 128, 64, 8), (4, 64, 32, 4), (8, 64, 64, 4)])
+def test_error_at_any_scale(oracle, bits, D, group, gqa, vs, ks, qs, meta):
+    """Ranges far from 1: below fp16's smallest normal value times 2^11, above its largest; value groups of unlike scale."""
+    import muzero_b200 as mz
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = (t.float() for t in oracle.synth_kv(2, 2, 700, D, 2 * gqa, seed=bits))
+    v[..., :32] *= 1e-3
+    k, v, q = ((t * f).to(torch.bfloat16) for t, f in ((k, ks), (v, vs), (q, qs)))
+    ref = oracle.OracleCacheLayer(bits=bits, group=group, residual=128, meta_dtype=meta, alpha_key=2.0, alpha_value=2.0)
+    ref.append(k, v)
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=group, residual_length=128, amax_dtype=str(meta)[6:], alpha_key=2.0, alpha_value=2.0)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+    want = attention64(oracle, ref, q, D ** -0.5)
+    for splits in (0, 3):
+        got = decode_attention(layer, q.cuda(), D ** -0.5, out_dtype=torch.float32, splits=splits)
+        assert bool(torch.isfinite(got).all())
+        for part in (slice(0, 32), slice(32, D)):
+            assert relative_error(got[..., part], want[..., part]) <= (FP32_ERROR if part.start or group == 32 else SHARED_GROUP_ERROR)
 
 
 @pytest.mark.parametrize("bits,bound", [(2, 1.2e-4), (4, 5e-5)])
