@@ -113,6 +113,7 @@ int make_plan(const mz_decode_args* a, Plan* plan, bool need_tables) {
   p.o = MzDecodeOut{};
   p.new_k = p.new_v = nullptr;
   p.new_sb = p.new_sh = 0;
+  p.new_rows = 0;
   const int force = kernel_override();
   // 1 = tcgen05, 2 = tensor cores (mma.sync), 3 = SIMT tiles, 0 = shape-generic
   const int which = force == 1 ? 0 : force == 4 && mz_decode_umma_supported(p) ? 1 : force != 2 && mz_decode_mma_supported(p) ? 2
@@ -211,9 +212,9 @@ bool mz_decode_takes_new_token(const MzDecodePlan& plan, const void* k_new, cons
   return plan.tiles && plan.p.tp.kind == 1 && (((uintptr_t)k_new | (uintptr_t)v_new) & 15) == 0 && ((nsb | nsh) & 7) == 0;
 }
 int mz_decode_run_plan(const mz_decode_args* a, MzDecodePlan* plan, const void* k_new, const void* v_new, long long nsb, long long nsh,
-                       cudaStream_t st) {
+                       int rows, cudaStream_t st) {
   MzDecodeParams& p = plan->p;
-  p.new_k = k_new; p.new_v = v_new; p.new_sb = nsb; p.new_sh = nsh;
+  p.new_k = k_new; p.new_v = v_new; p.new_sb = nsb; p.new_sh = nsh; p.new_rows = rows;
   const MzDecodeOut o = {a->out, a->out_dtype, nullptr, nullptr, nullptr, 0, 0};
   int rc = launch_partials(a, plan, o, st);
   return rc ? rc : finish(*plan, o, st);

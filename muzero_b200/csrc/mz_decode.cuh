@@ -95,6 +95,7 @@ struct MzDecodeParams {
   // tensor-core kernel: the window's newest token, still in the caller's tensors [B,KVH,1,D] (nullptr: none); the kernel
   // uses it from there and stores it into the window
   const void* new_k; const void* new_v; long long new_sb, new_sh;
+  int new_rows;      // rows of the window's buffer (read by the checked build only)
 };
 
 // A validated call: which kernel runs, its parameters, the partial records and scratch bytes it needs.
@@ -106,9 +107,10 @@ struct MzDecodePlan {
 };
 // validation + planning of mz_decode_attention(a), and the launches of an existing plan
 int mz_decode_plan(const mz_decode_args* a, MzDecodePlan* plan);
-// k_new / v_new (with their strides): the newest token of the window, if the kernel shall take it from there
+// k_new / v_new (with their strides): the newest token of the window, if the kernel shall take it from there; the window's
+// buffer has `rows` rows
 int mz_decode_run_plan(const mz_decode_args* a, MzDecodePlan* plan, const void* k_new, const void* v_new, long long nsb, long long nsh,
-                       cudaStream_t st);
+                       int rows, cudaStream_t st);
 // whether the plan's kernel can take the newest token from the caller's tensors
 bool mz_decode_takes_new_token(const MzDecodePlan& plan, const void* k_new, const void* v_new, long long nsb, long long nsh);
 

@@ -348,7 +348,7 @@ __device__ __forceinline__ void dense_tile(const MzDecodeParams& p, uint32_t kbu
   if (fresh >= 0 && fresh < DT) {
 #pragma unroll
     for (int r = 0; r < 2; ++r)
-      if (g + 8 * r == fresh) {
+      if (g + 8 * r == fresh && MZ_IN_BOUNDS(s.res_start + tok0 + fresh, p.new_rows, 15)) {
 #pragma unroll
         for (int i = 0; i < D / 32; ++i) *(uint4*)(rk + (g + 8 * r) * s.res_stride_t + 32 * i + 8 * t) = kx[r][i];
       }
@@ -410,7 +410,7 @@ __device__ __forceinline__ void dense_tile(const MzDecodeParams& p, uint32_t kbu
         }
       }
     }
-    if (row == fresh) {
+    if (row == fresh && MZ_IN_BOUNDS(s.res_start + tok0 + fresh, p.new_rows, 16)) {
 #pragma unroll
       for (int n = 0; n < NG; ++n)
 #pragma unroll
@@ -548,6 +548,7 @@ __device__ __forceinline__ void finish_cluster(const MzDecodeParams& p, uint32_t
   auto write_out = [&](int h, int d, float mx, float lsum, float4 a) {
     const long long row = (long long)pair * gqa + h;
     const MzDecodeOut& o = p.o;
+    if (!MZ_IN_BOUNDS(row, (long long)p.s.batch * p.H, 17)) return;
     if (o.out) {
       const float den = fmaxf(lsum, 1e-20f);
       mz_store_from_float(o.out, row * D + d, a.x / den, o.out_dt);

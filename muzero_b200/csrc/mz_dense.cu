@@ -91,7 +91,9 @@ __device__ __forceinline__ void dense_keys(const DenseParams& p, uint8_t* smem) 
     const uint8_t* ca = s_code + (size_t)(local * pairs + cp) * stride + part * CB;
     const uint8_t* cb = ca + (size_t)per_cta * pairs * stride;
     const int row = local * D + 2 * cp;
-    uint32_t* dst = (uint32_t*)((uint16_t*)p.out_k + (((long long)b * s.kv_heads + h) * p.sk + (long long)j * G + part * TPT) * D + 2 * cp);
+    const long long at = (((long long)b * s.kv_heads + h) * p.sk + (long long)j * G + part * TPT) * D + 2 * cp;
+    if (!MZ_IN_BOUNDS(at + (TPT - 1) * D + 1, (long long)s.batch * s.kv_heads * p.sk * D, 18)) continue;
+    uint32_t* dst = (uint32_t*)((uint16_t*)p.out_k + at);
     if (BOOK) {
       // 16 codes of each channel, LSB first
       unsigned long long a, c;
@@ -177,7 +179,9 @@ __device__ __forceinline__ void dense_values(const DenseParams& p, unsigned blk,
     const int row = row0 + k * rows;
     if (row >= n_rows) return;
     const MzRowParams r = mz_row_params(lo[k], span[k], top, p.eps);
-    uint16_t* dst = (uint16_t*)p.out_v + ((long long)pair * p.sv) * D + (long long)row * G;
+    const long long at = (long long)pair * p.sv * D + (long long)row * G;
+    if (!MZ_IN_BOUNDS(at + G - 1, (long long)s.batch * s.kv_heads * p.sv * D, 19)) continue;
+    uint16_t* dst = (uint16_t*)p.out_v + at;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       uint32_t v[4];
@@ -198,7 +202,9 @@ __device__ __forceinline__ void dense_residual(const mz_kv_store& s, const void*
   if (i >= n * vpr) return;
   const int t = i / vpr, c = i % vpr;
   const int b = pair / s.kv_heads, h = pair % s.kv_heads;
-  *(uint4*)((uint16_t*)out + (pair * s_out + prefix + t) * s.head_dim + c * 8) =
+  const long long at = (pair * s_out + prefix + t) * s.head_dim + c * 8;
+  if (!MZ_IN_BOUNDS(at + 7, (long long)s.batch * s.kv_heads * s_out * s.head_dim, 20)) return;
+  *(uint4*)((uint16_t*)out + at) =
       *(const uint4*)((const uint16_t*)res + b * s.res_stride_b + h * s.res_stride_h + (long long)(s.res_start + first + t) * s.res_stride_t + c * 8);
 }
 
@@ -230,6 +236,7 @@ __global__ void __launch_bounds__(256) dequant_keys_kernel(const DenseParams p, 
   const uint8_t* row = s.packed_k + b * s.pk_stride_b + h * s.pk_stride_h + ((long long)g * D + d) * p.QB;
   const long long o0 = (((long long)b * s.kv_heads + h) * p.sk + (long long)(g - p.g0) * G + oct * 8) * D + d;
   const int n = min(8, G - oct * 8);
+  if (!MZ_IN_BOUNDS(o0 + (long long)(n - 1) * D, (long long)s.batch * s.kv_heads * p.sk * D, 18)) return;
   for (int k = 0; k < n; ++k) {
     const int q = mz_extract_code(row, oct * 8 + k, s.bits, p.QB);
     mz_store_from_float(p.out_k, o0 + (long long)k * D, mz_dequant_exact(r, q, p.tab_k, top + 1), out_dt);
@@ -253,7 +260,7 @@ __global__ void __launch_bounds__(256) dequant_values_kernel(const DenseParams p
   const long long o0 = (((long long)b * s.kv_heads + h) * p.sv + t) * D;
   for (int k = 0; k < 8; ++k) {
     const int idx = oct * 8 + k, c = grp * G + idx;
-    if (idx >= G || c >= D) break;
+    if (idx >= G || c >= D || !MZ_IN_BOUNDS(o0 + c, (long long)s.batch * s.kv_heads * p.sv * D, 19)) break;
     const int q = mz_extract_code(row, idx, s.bits, p.QB);
     mz_store_from_float(p.out_v, o0 + c, mz_dequant_exact(r, q, p.tab_v, top + 1), out_dt);
   }
@@ -268,7 +275,8 @@ __global__ void __launch_bounds__(256) copy_residual_kernel(const mz_kv_store s,
   const long long pair = i / D / n;
   const int b = (int)(pair / s.kv_heads), h = (int)(pair % s.kv_heads);
   const float v = mz_u16_to_float(res[b * s.res_stride_b + h * s.res_stride_h + (long long)(s.res_start + first + t) * s.res_stride_t + d], s.kv_dtype);
-  mz_store_from_float(out, (pair * s_out + (s_out - n) + t) * D + d, v, out_dt);
+  const long long at = (pair * s_out + (s_out - n) + t) * D + d;
+  if (MZ_IN_BOUNDS(at, (long long)s.batch * s.kv_heads * s_out * D, 20)) mz_store_from_float(out, at, v, out_dt);
 }
 
 template <int DT>

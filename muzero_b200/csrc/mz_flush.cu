@@ -16,6 +16,10 @@ struct MoveParams {
   uint16_t* dst_k; uint16_t* dst_v;
   long long sb, sh, st;      // element strides of the new window
   int k_first, v_first;      // first key / value row that stays; key row k_first becomes row 0 of the new window
+  // checked build: element `rel` of head h's rows lies inside the head's slab (heads outermost) or the batch entry's
+  __device__ __forceinline__ bool holds(int h, long long rel) const {
+    return sh >= st ? MZ_IN_BOUNDS(rel, sh, 23) : MZ_IN_BOUNDS(h * sh + rel, sb, 23);
+  }
 };
 
 struct FlushParams {
@@ -468,6 +472,7 @@ __device__ __forceinline__ void move_rows16(const mz_kv_store& s, const MovePara
   if (row >= s.res_len) return;
   const int b = pair / s.kv_heads, h = pair % s.kv_heads;
   const long long src = b * s.res_stride_b + h * s.res_stride_h + (long long)(s.res_start + row) * s.res_stride_t + c;
+  if (!m.holds(h, (long long)(row - m.k_first) * m.st + c + 7)) return;
   const long long dst = b * m.sb + h * m.sh + (long long)(row - m.k_first) * m.st + c;
   *(uint4*)(m.dst_k + dst) = *(const uint4*)((const uint16_t*)s.res_k + src);
   if (row >= m.v_first) *(uint4*)(m.dst_v + dst) = *(const uint4*)((const uint16_t*)s.res_v + src);
@@ -489,6 +494,7 @@ __global__ void __launch_bounds__(256) move_rows_kernel(const mz_kv_store s, con
   const long long pair = i / D / nk;
   const long long src = (pair / s.kv_heads) * s.res_stride_b + (pair % s.kv_heads) * s.res_stride_h + (long long)(s.res_start + row) * s.res_stride_t + d;
   const long long dst = (pair / s.kv_heads) * m.sb + (pair % s.kv_heads) * m.sh + (long long)(row - m.k_first) * m.st + d;
+  if (!m.holds((int)(pair % s.kv_heads), (long long)(row - m.k_first) * m.st + d)) return;
   m.dst_k[dst] = ((const uint16_t*)s.res_k)[src];
   if (row >= m.v_first) m.dst_v[dst] = ((const uint16_t*)s.res_v)[src];
 }

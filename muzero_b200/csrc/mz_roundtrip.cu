@@ -105,7 +105,9 @@ __device__ __forceinline__ void roundtrip_keys(const RoundtripParams& p, uint32_
     if (tile >= p.tiles) break;
     const int j = tile % nsg, pair = tile / nsg;
     const uint16_t* src = p.x + (pair / p.H) * p.sb + (pair % p.H) * p.sh + (long long)(j * G + part * TPT) * p.st + 2 * cp;
-    uint32_t* dst = (uint32_t*)(p.out + ((long long)pair * p.S + j * G + part * TPT) * D + 2 * cp);
+    const long long at = ((long long)pair * p.S + j * G + part * TPT) * D + 2 * cp;
+    if (!MZ_IN_BOUNDS(at + (TPT - 1) * D + 1, (long long)p.B * p.H * p.S * D, 21)) continue;
+    uint32_t* dst = (uint32_t*)(p.out + at);
     Row ra, rb;
     get_row(ra, s_row + local * D + 2 * cp, p.bits);
     get_row(rb, s_row + local * D + 2 * cp + 1, p.bits);
@@ -142,7 +144,9 @@ __device__ __forceinline__ void roundtrip_values(const RoundtripParams& p, unsig
   if (!live) return;
   Row r;
   make_row(r, fminf(P::lo(mn), P::hi(mn)), fmaxf(P::lo(mx), P::hi(mx)), p);
-  uint16_t* dst = p.out + ((long long)pair * p.S * NG + row) * G + sub * 8;
+  const long long at = ((long long)pair * p.S * NG + row) * G + sub * 8;
+  if (!MZ_IN_BOUNDS(at + lpr * 8 + 7, (long long)p.B * p.H * p.S * D, 22)) return;
+  uint16_t* dst = p.out + at;
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
     uint32_t o[4];

@@ -56,7 +56,7 @@ extern "C" int mz_decode_step(mz_decode_args* a, const void* k_new, const void* 
   // less), provided that a flush of this step does not need it.
   if (n <= s->res_len && post.store.res_len > 0 && mz_decode_takes_new_token(plan, k_new, v_new, new_stride_b, new_stride_h)) {
     if (n > 0 && (rc = mz_flush_kv(s, n, eps, stream))) return rc;
-    rc = mz_decode_run_plan(&post, &plan, k_new, v_new, new_stride_b, new_stride_h, (cudaStream_t)stream);
+    rc = mz_decode_run_plan(&post, &plan, k_new, v_new, new_stride_b, new_stride_h, window_capacity, (cudaStream_t)stream);
   } else {
     if ((rc = mz_append_kv(s, k_new, v_new, new_stride_b, new_stride_h, stream))) return rc;
     if (n > 0) {
@@ -64,7 +64,7 @@ extern "C" int mz_decode_step(mz_decode_args* a, const void* k_new, const void* 
       appended.res_len += 1;
       if ((rc = mz_flush_kv(&appended, n, eps, stream))) return rc;
     }
-    rc = mz_decode_run_plan(&post, &plan, nullptr, nullptr, 0, 0, (cudaStream_t)stream);
+    rc = mz_decode_run_plan(&post, &plan, nullptr, nullptr, 0, 0, 0, (cudaStream_t)stream);
   }
   if (rc) return rc;
   *s = post.store;

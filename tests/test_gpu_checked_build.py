@@ -54,7 +54,12 @@ for bits, gqa in ((4, 4), (2, 2), (3, 1)):
     # decode steps across a flush, then a batch gather
     for step in range(70):
         kn, vn, _ = orc.synth_kv(3, KVH, 1, 128, KVH * gqa, seed=5000 + step)
-        layer.update(kn.cuda(), vn.cuda(), {{"materialize_full_kv": False}})
+        if step % 2:
+            layer.update(kn.cuda(), vn.cuda(), {{"materialize_full_kv": False}})
+        else:                                       # the decode kernel stores the new token itself
+            layer.decode_step(kn.cuda(), vn.cuda(), q.cuda(), 0.088)
+    layer._full_kv()
+    mz.roundtrip(k[:, :, :448].cuda(), v[:, :, :448].cuda(), bits=bits, q_group_size=64)
     layer.batch_select_indices(torch.tensor([2, 0], device="cuda"))
     c = violations()
     assert c[0] == 0, (bits, c)
@@ -75,6 +80,21 @@ assert count > 0 and index >= extent and 1 <= site <= 6, (count, index, extent, 
 for n, t in bufs.items():                         # bit patterns: unused capacity is uninitialised and may hold NaN
     assert torch.equal(t.view(torch.uint8), before[n].view(torch.uint8)), n
 assert violations()[0] == 0                        # cleared
+
+# a flush that moves what stays dense into a window declared four rows too short (its memory is not): the rows outside are
+# skipped and counted, those inside arrive
+s = layer._store_struct()
+layer._ensure_store(s.k_groups + 1, s.v_tokens + 64)
+s = layer._store_struct()
+stay, cols = s.res_len - 64, 128
+win = [torch.zeros(2, 2, stay, cols, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+short = (stay - 4) * cols
+check(lib.mz_flush_kv_move(ctypes.byref(s), 64, 0, 64, win[0].data_ptr(), win[1].data_ptr(), 2 * stay * cols, short, cols, 1e-8,
+                           stream_ptr(torch.device("cuda"))), "mz_flush_kv_move")
+moved = violations(reset=1)
+assert moved[0] == 2 * 2 * 4 * cols // 8 and moved[3] == 23, moved
+got = win[0].reshape(2, -1)[:, : 2 * short].reshape(2, 2, stay - 4, cols)
+assert torch.equal(got, layer.keys[:, :, 64:64 + stay - 4])
 torch.cuda.synchronize()
 print("CHECKED-BUILD-OK", count, site)
 """
