@@ -312,20 +312,26 @@ bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count) {
 // warp is bound by memory latency.
 constexpr int kDenseCtaCost = 36;
 
+// the general kernel's table; asked for by the plans that run it only (a build costs a synchronisation and one of 16 slots)
+static void take_lookup_entries(MzDecodeParams& p) {
+  p.lut = p.s.k_groups > 0 && p.s.bits <= 4 ? mz_mma_lookup_entries(p.s.bits, true, p.s.alpha_key, p.s.alpha_value) : nullptr;
+}
+
 int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slots) {
   const mz_kv_store& s = p.s;
   p.hetero = 0;
   p.cluster = 0;
   MzMmaKernel k;
   if (!find_kernel(p, &k)) return mz_fail(MZ_ERR_UNSUPPORTED, "no tensor-core kernel for this shape");
-  p.lut = s.k_groups > 0 && s.bits <= 4 ? mz_mma_lookup_entries(s.bits, true, s.alpha_key, s.alpha_value) : nullptr;
   if (splits_request == 0 && plan_cluster(p, k, sm_count)) {
     *slots = 4;                                   // no records; a workspace is still asked for, so that its size is never 0
+    take_lookup_entries(p);
     return MZ_OK;
   }
   p.cluster = 0;
   if (simt_is_faster(p)) return mz_plan_tiles(p, splits_request, sm_count, slots);
   if (mz_decode_flat_supported(p)) return mz_plan_flat(p, splits_request, sm_count, slots);
+  take_lookup_entries(p);
   const long long pairs = (long long)s.batch * s.kv_heads;
   const int dense_tiles = (s.res_len + mzm::DT - 1) / mzm::DT;
   // enough packed work to fill every warp of the machine, and a residual window: split the CTAs
