@@ -248,37 +248,61 @@ int clusters_at_once(const MzMmaKernel& k, int cs, int threads, unsigned smem) {
   return n;
 }
 
-// Machine-filling plans of these shapes are faster on the SIMT kernel (measured at 16 x 8 x 4000 and 40 x 8 x 2500):
-//   * codes of 7 and 8 bits, which are computed one by one, with up to 4 heads per kv head (123 against 148 us); with 8
-//     heads, for which the SIMT kernel pays one by one, groups of 32 (8 bits, 16 x 8 x 4224: 162 against 186 us), 8 bits
-//     in groups of 128 (161 against 202) and 7 bits in groups of 64 (161 against 170)
-//   * groups of 32, whose tiles prepare twice the rows per token here, with few heads (1 bit: 74 against 94 us) - from
-//     4 heads on the 4-bit ones are faster here (96 against 103)
-//   * 4 bits in groups of 128 with two heads (59 against 68)
-//   * 3 bits with one or two heads (8 x 8 x 33364, one head: 183 against 201; 3 x 8 x 47136 in groups of 128: 105 against
-//     118) and 1 bit in groups of 64 (28 x 4 x 15385: 143 against 151)
-bool simt_is_faster(const MzDecodeParams& p) {
-  if (!mz_decode_tiles_supported(p)) return false;
-  const int bits = p.s.bits, group = p.s.group;
-  if (bits > 4) return p.gqa <= 4 || group == 32 || group == (bits == 8 ? 128 : 64);
-  if (p.gqa > 4) return false;
-  if (group == 32) return p.gqa < 4 || bits < 4;
-  if (p.gqa <= 2 && (bits == 3 || (bits == 1 && group == 64))) return true;
-  return group == 128 && bits == 4 && p.gqa == 2;
+// ---- choice between cluster mode and an even cut of the tiles over all SMs, and of the kernel for the cut, by measured
+// cost.  The constants are least-squares fits, in us, to device times of calls of 1..40 sequences x 2, 4 or 8 kv heads x
+// 260..40000 tokens (1060 shapes, each run in every form that serves it).  x = packed tiles per SM, a residual tile counted by
+// its cost.
+struct CutCost { float base, tile; };      // base + tile * x: launch, prologue, last turn and merge kernel; a tile's share of an SM
+// [group 32, 64, 128][codes up to 4 bits, wider][heads per kv head: 1 and 2, 4, 8]; the fits are within 10 to 19 % (rms)
+constexpr CutCost kSimtCost[3][2][3] = {{{{19.f, 0.59f}, {22.7f, 0.64f}, {24.8f, 1.05f}}, {{17.3f, 0.94f}, {19.4f, 1.03f}, {24.7f, 1.35f}}},
+                                        {{{23.2f, 0.87f}, {27.3f, 0.93f}, {35.3f, 1.62f}}, {{21.f, 1.54f}, {23.4f, 1.71f}, {32.7f, 2.40f}}},
+                                        {{{28.3f, 1.30f}, {33.3f, 1.61f}, {43.7f, 2.88f}}, {{25.3f, 2.97f}, {31.3f, 3.66f}, {43.2f, 4.75f}}}};
+constexpr CutCost kUnrolledCost = {18.f, 0.69f};
+// Cluster mode: base + tile * warps * turns, a turn being one packed tile for every warp of the cluster: [group][width][up to 4
+// heads, up to 8] (within 4 to 13 %, 22 % in groups of 128).  Tiles of head_dim 64 take 0.6 of it.
+constexpr float kClusterTile[3][2][2] = {{{0.57f, 1.03f}, {0.95f, 1.36f}}, {{0.83f, 1.47f}, {1.70f, 1.91f}}, {{1.40f, 2.10f}, {3.80f, 4.57f}}};
+constexpr float kClusterBase[2] = {10.5f, 13.5f};
+// The general kernel's own cut: a tile costs 1.25 of the cluster's (its turns are not aligned), its base is 24 / 35 us.
+constexpr float kGeneralBase[2] = {24.f, 35.f}, kGeneralTile = 1.25f;
+
+int group_index(int group) { return group == 32 ? 0 : group == 64 ? 1 : 2; }
+float cluster_tile_us(const MzDecodeParams& p) {
+  return kClusterTile[group_index(p.s.group)][p.s.bits > 4][p.gqa > 4] * (p.s.head_dim == 64 ? 0.6f : 1.0f);
 }
 
-// Cluster mode: one cluster per pair, no partial records in memory and no merge kernel.  In units of a packed tile on a
-// busy SM (0.5 us, 1.5 us of wide codes): it takes what its heaviest SM has to do, times what a tile costs here over the
-// kernel that would run otherwise; an even cut over all SMs takes its share, but at least one tile's latency (about 4 us),
-// and the merge kernel (about 4 us).  Where the even cut would run on the unrolled kernel and every pair could have two SMs,
-// a cluster whose warps need one more turn over their tiles than the even cut's loses what the merge costs and more
-// (8 x 8 x 3420, 4 bits: 36 against 31 us; 18 x 2 x 1500: 23 against 18.5).
+// The kernel of an even cut: the unrolled kernel where it serves; else the SIMT kernel where it serves.  The general
+// kernel has a larger base and needs as much or more per tile (groups of 32, 4 heads: 0.75 against 0.64 us; 64, 8 heads: 1.70 against
+// 1.62; 128, 8 heads: 2.86 against 2.88; wide codes, 64, 4 heads: 2.16 against 1.71), except for codes of up to 4 bits in groups of 64 with 4 heads, where its smaller base (24.4 against
+// 27.3 us) and its separate residual CTAs win up to about 40 tiles per SM (3 bits: 24 x 8 x 1537 51 against 63 us, 16 x 8 x 4000 81 against 80,
+// 2 x 8 x 60000 144 against 127).
+enum class Cut { kUnrolled, kSimt, kGeneral };
+Cut choose_cut(const MzDecodeParams& p, float x) {
+  if (mz_decode_flat_supported(p)) return Cut::kUnrolled;
+  if (!mz_decode_tiles_supported(p)) return Cut::kGeneral;
+  return p.s.bits <= 4 && p.s.group == 64 && p.gqa == 4 && x < 40.f ? Cut::kGeneral : Cut::kSimt;
+}
+float cut_us(const MzDecodeParams& p, float x) {
+  CutCost c = kUnrolledCost;
+  switch (choose_cut(p, x)) {
+    case Cut::kUnrolled: break;
+    case Cut::kSimt: c = kSimtCost[group_index(p.s.group)][p.s.bits > 4][p.gqa > 4 ? 2 : p.gqa == 4 ? 1 : 0]; break;
+    case Cut::kGeneral: c = {kGeneralBase[p.gqa > 4], kGeneralTile * cluster_tile_us(p)}; break;
+  }
+  return c.base + c.tile * x;
+}
+float tiles_per_sm(const MzDecodeParams& p, const MzTilesPlan& t, int sm_count) {
+  return (float)((double)p.s.batch * p.s.kv_heads * (double)t.pair_cost / t.cost_q / sm_count);
+}
+
+// Cluster mode: one cluster per pair, no partial records in memory and no merge kernel; taken where the estimates above say that it
+// is not slower than the cut.
 bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count) {
   const long long pairs = (long long)p.s.batch * p.s.kv_heads;
   if (pairs > sm_count) return false;
   MzTilesPlan& t = p.tp;
   describe_tiles(t, p);
   const int T = t.tiles_per_pair;
+  const float limit = cut_us(p, tiles_per_sm(p, t, sm_count));
   int cs = 1;
   while (cs < 8 && cs * 2 * pairs <= sm_count && cs * 4 < T) cs *= 2;
   const unsigned rec = (unsigned)(p.gqa * (p.s.head_dim + 4) * 4);
@@ -288,14 +312,8 @@ bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count) {
     if (want < 4) want = 4;
     const int nw = layout(t, p, k, want, rec);
     if (nw < 1) return false;
-    const long long even = pairs * t.pair_cost / sm_count, heaviest = t.pair_cost / cs, wait = (p.s.bits > 4 ? 3 : 8) * kCostPacked;
-    const bool simt = simt_is_faster(p), flat = !simt && mz_decode_flat_supported(p);
-    // 1 and 3 bits with few heads cost about the same on both kernels
-    const int here = p.s.bits > 4 || (p.s.group > 32 && (p.s.bits & 1)) ? 100 : simt ? 128 : flat ? 116 : 100;
-    if (heaviest * here / 100 > (even > wait ? even : wait) + wait) return false;      // smaller clusters are heavier still
-    // a turn: every warp of the SM over one packed tile; even shares of the cost leave some warp up to a tile more
-    const long long turn = (long long)k.max_warps * kCostPacked;
-    if (flat && 2 * pairs <= sm_count && (t.pair_cost + kCostPacked * 3 / 2 + cs * turn - 1) / (cs * turn) > (even + turn - 1) / turn) return false;
+    const long long turn = (long long)cs * nw * t.cost_q;
+    if (kClusterBase[p.gqa > 4] + cluster_tile_us(p) * (float)(nw * ((t.pair_cost + turn - 1) / turn)) > limit) return false;    // smaller clusters are heavier still
     if (cs > 1 && clusters_at_once(k, cs, nw * 32, t.smem_bytes) < pairs) continue;
     // tiles are dealt to the cluster's warps by cost; every warp gets at most about one residual tile's cost more than its share
     if (cut(t, 1, (long long)cs * nw) != MZ_OK) return false;
@@ -329,8 +347,12 @@ int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slo
     return MZ_OK;
   }
   p.cluster = 0;
-  if (simt_is_faster(p)) return mz_plan_tiles(p, splits_request, sm_count, slots);
-  if (mz_decode_flat_supported(p)) return mz_plan_flat(p, splits_request, sm_count, slots);
+  describe_tiles(p.tp, p);
+  switch (choose_cut(p, tiles_per_sm(p, p.tp, sm_count))) {
+    case Cut::kUnrolled: return mz_plan_flat(p, splits_request, sm_count, slots);
+    case Cut::kSimt: return mz_plan_tiles(p, splits_request, sm_count, slots);
+    case Cut::kGeneral: break;
+  }
   take_lookup_entries(p);
   const long long pairs = (long long)s.batch * s.kv_heads;
   const int dense_tiles = (s.res_len + mzm::DT - 1) / mzm::DT;
