@@ -5,7 +5,7 @@
 // a histogram (65,536 samples at most by default): one launch instead of a gather, a radix sort and index arithmetic
 // in 64-bit tensors (25 launches).  The last CTA to finish walks the histogram and leaves it zeroed for the next call.
 // The anchor pass reads the block once and is bound by that; per-CTA sums are added in CTA order by the last CTA.
-// With the packed quantizer, a 2-bit prompt of 16 x 8 x 4096 tokens went from 2222 to 139 us (call included).
+// Taken for 1-, 3- and 8-bit caches only: the other widths have one alpha whatever the data is.
 #include "mz_common.cuh"
 
 namespace {

@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(Cfg<BITS, D_, G_, NT>::MAXW * 32, 1) decode_mm
     };
     float A[D / 32], sp[D / 32], bup[D / 32], bdn[D / 32];
     int zc[D / 32];
-    bool any = false, wild = false;
+    bool any = false, wild = msz == 4;        // fp32 metadata: see row_split
     float most = 0.f;
 #pragma unroll
     for (int i = 0; i < D / 32; ++i) {

@@ -194,10 +194,13 @@ __device__ __forceinline__ void row_constants(float lo, float span, int& zc, flo
 }
 // ---- row constants: Bdn = clamp(-lo, 0, span) is the part of the range below zero, Bup the part above, A the value of the
 // zero code (0 when the range straddles zero).  The zero code is rint(RN(RN(-lo / span) * TOP)) as the dequantizer has it.
-// The quotient is correctly rounded by Markstein's final step (IBM J. Res. Dev. 34(1), 1990: with y = RN(1/s) and q within
-// an ulp of b/s, q + (b - q s) y rounds to RN(b/s)); that is branch-free, where the IEEE division costs a range test and a
-// slow path per row.  Ties matter: 16-bit extremes often give a quotient that lies exactly on a code boundary.
-// Spans from 2^125 on would flush the reciprocal: `wild` asks for the division.
+// The quotient takes Markstein's final step (IBM J. Res. Dev. 34(1), 1990), q0 + (b - q0 s) y with y close to 1/s, which is
+// branch-free, where the IEEE division costs a range test and a slow path per row.  Ties matter: 16-bit extremes often give
+// a quotient that lies exactly on a code boundary.  For 16-bit metadata the step is correctly rounded whatever the last bits of
+// y: b and s have at most 11 significant bits, so b/s is at least 2^-13 ulp away from every rounding boundary (a quotient
+// with 25 bits would need a dividend of more than 11), and the step's value before rounding is within 2^-20 ulp of b/s.
+// fp32 metadata has no such gap: its rows, and spans from 2^125 on, which would flush the reciprocal, take the
+// division (`wild`).
 __device__ __forceinline__ void row_split(float lo, float span, float top, float& A, float& bup, float& bdn, int& zc, bool& wild) {
   span = fmaxf(span, 1e-8f);
   bdn = fminf(fmaxf(-lo, 0.0f), span);

@@ -4,7 +4,8 @@ Mirrors the public functions of the reference's ``muzero/quantizer.py``
 (``select_alpha`` :29-83, ``quantize_rows`` :119-158, ``dequantize_rows``
 :205-226, ``roundtrip`` :273-323).  The row kernels are the CUDA library's; there
 is no torch or Triton backend behind them, so CPU tensors raise.
-Alpha selection is a one-time statistic per layer and stays in torch.
+Alpha selection is a one-time statistic per layer, taken on the device (``mz_alpha_stats``) for 16-bit CUDA blocks and in
+torch otherwise; code widths with one alpha take none.
 """
 from __future__ import annotations
 

@@ -198,3 +198,22 @@ def test_scratch_buffers_stay_where_a_captured_graph_saw_them(monkeypatch):
     grown = A._workspace(cpu, (1 << 20) + 1)
     assert grown.numel() >= 2 << 20 and first in alive()
     assert sum(t.numel() for t in A._outgrown) < grown.numel()
+
+
+def test_final_quotient_step_rounds_correctly_for_half_precision_operands():
+    """The decode kernels' quotient q0 + (b - q0 s) y, q0 = b y: the IEEE quotient for every pair of 11-bit significands, with y up to
+    2 ulp off 1/s either way.  (numpy's extended precision stands in for the fused operations: the distance to a rounding
+    boundary, 2^-13 ulp, is far above its own rounding.)"""
+    import numpy as np
+    if np.finfo(np.longdouble).nmant < 63:
+        pytest.skip("no extended precision on this host")
+    sig = np.arange(1024, 2048, dtype=np.float32)
+    s = sig[None, :]
+    near = (np.float32(1) / sig)[None, :]
+    for ulps in (-2, -1, 0, 1, 2):
+        y = (near.view(np.int32) + np.int32(ulps)).view(np.float32)
+        for b in np.split(sig[:, None], 8):
+            q0 = b * y
+            rest = (b.astype(np.longdouble) - q0.astype(np.longdouble) * s).astype(np.float32)
+            q = (q0.astype(np.longdouble) + rest.astype(np.longdouble) * y).astype(np.float32)
+            assert np.array_equal(q, b / s), ulps
