@@ -108,6 +108,51 @@ def test_error_at_any_scale(oracle, bits, D, group, gqa, vs, ks, qs, meta):
             assert relative_error(got[..., part], want[..., part]) <= (FP32_ERROR if part.start or group == 32 else SHARED_GROUP_ERROR)
 
 
+@pytest.mark.parametrize("bits,D,group,gqa,B,S", [(4, 128, 64, 8, 12, 1777), (3, 128, 32, 8, 10, 725), (1, 128, 128, 2, 12, 1777), (8, 64, 32, 4, 18, 601),
+                                                  (4, 128, 32, 2, 16, 800), (4, 128, 64, 4, 18, 289), (2, 128, 64, 4, 1, 11213), (5, 128, 64, 1, 8, 1500)])
+def test_clusters_whose_warps_take_several_tiles(oracle, bits, D, group, gqa, B, S):
+    """Up to 148 pairs with more tiles than the pair's cluster has warps, on both sides of the choice between a cluster and an
+    even cut; the forced cut of the same call gives the same values."""
+    import muzero_b200 as mz
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = oracle.synth_kv(B, 8, S, D, 8 * gqa, seed=bits + S)
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=group, residual_length=128, alpha_key=2.0, alpha_value=2.0)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+    mask = torch.zeros(B, 1, 1, S)
+    mask[B - 1, ..., : S // 2] = torch.finfo(torch.bfloat16).min
+    got = decode_attention(layer, q.cuda(), D ** -0.5, mask.cuda(), out_dtype=torch.float32).cpu()
+    cut = decode_attention(layer, q.cuda(), D ** -0.5, mask.cuda(), out_dtype=torch.float32, splits=2).cpu()
+    unrolled = group == 64 and D == 128 and bits in (2, 4) and gqa <= 4         # its cut has the error pinned below
+    assert relative_error(got, cut.double()) <= (1.2e-4 if unrolled else 2 * FP32_ERROR)
+    for b in {0, B - 1}:
+        ref = oracle.OracleCacheLayer(bits=bits, group=group, residual=128, alpha_key=2.0, alpha_value=2.0)
+        ref.append(k[b:b + 1], v[b:b + 1])
+        want = attention64(oracle, ref, q[b:b + 1], D ** -0.5, mask[b:b + 1])
+        assert relative_error(got[b:b + 1], want) <= (1.2e-4 if unrolled else FP32_ERROR)
+
+
+@pytest.mark.parametrize("bits,D,group,gqa", [(3, 128, 64, 4), (4, 64, 32, 8), (8, 128, 64, 8)])
+def test_an_infinite_range_stays_in_its_group(oracle, bits, D, group, gqa):
+    """A value range that overflowed fp16 metadata makes its own channels non-finite, as the dequantizer does, and no others."""
+    import muzero_b200 as mz
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = oracle.synth_kv(2, 2, 500, D, 2 * gqa, seed=bits)
+    ref = oracle.OracleCacheLayer(bits=bits, group=group, residual=128, alpha_key=2.0, alpha_value=2.0)
+    ref.append(k, v)
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=group, residual_length=128, alpha_key=2.0, alpha_value=2.0)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+    layer._value_scale[0, 1, 5, 1] = float("inf")
+    got = decode_attention(layer, q.cuda(), D ** -0.5, out_dtype=torch.float32).cpu()
+    want = attention64(oracle, ref, q, D ** -0.5)
+    hit = torch.zeros(got.shape, dtype=torch.bool)
+    hit[0, :, gqa:, group:2 * group] = True
+    assert not bool(torch.isfinite(got[hit]).any()) and relative_error(got[~hit], want[~hit]) <= FP32_ERROR
+
+
 @pytest.mark.parametrize("bits,bound", [(2, 1.2e-4), (4, 5e-5)])
 def test_error_of_the_unrolled_kernel(oracle, bits, bound):
     """Head_dim 128, group 64, up to four heads, more pairs than SMs: the unrolled kernel's table keeps 11 bits and a nominal
