@@ -250,45 +250,54 @@ int clusters_at_once(const MzMmaKernel& k, int cs, int threads, unsigned smem) {
 
 // ---- choice between cluster mode and an even cut of the tiles over all SMs, and of the kernel for the cut, by measured
 // cost.  The constants are least-squares fits, in us, to device times of calls of 1..40 sequences x 2, 4 or 8 kv heads x
-// 260..40000 tokens (1060 shapes, each run in every form that serves it).  x = packed tiles per SM, a residual tile counted by
-// its cost.
-struct CutCost { float base, tile; };      // base + tile * x: launch, prologue, last turn and merge kernel; a tile's share of an SM
-// [group 32, 64, 128][codes up to 4 bits, wider][heads per kv head: 1 and 2, 4, 8]; the fits are within 10 to 19 % (rms)
-constexpr CutCost kSimtCost[3][2][3] = {{{{19.f, 0.59f}, {22.7f, 0.64f}, {24.8f, 1.05f}}, {{17.3f, 0.94f}, {19.4f, 1.03f}, {24.7f, 1.35f}}},
-                                        {{{23.2f, 0.87f}, {27.3f, 0.93f}, {35.3f, 1.62f}}, {{21.f, 1.54f}, {23.4f, 1.71f}, {32.7f, 2.40f}}},
-                                        {{{28.3f, 1.30f}, {33.3f, 1.61f}, {43.7f, 2.88f}}, {{25.3f, 2.97f}, {31.3f, 3.66f}, {43.2f, 4.75f}}}};
-constexpr CutCost kUnrolledCost = {18.f, 0.69f};
-// Cluster mode: base + tile * warps * turns, a turn being one packed tile for every warp of the cluster: [group][width][up to 4
-// heads, up to 8] (within 4 to 13 %, 22 % in groups of 128).  Tiles of head_dim 64 take 0.6 of it.
-constexpr float kClusterTile[3][2][2] = {{{0.57f, 1.03f}, {0.95f, 1.36f}}, {{0.83f, 1.47f}, {1.70f, 1.91f}}, {{1.40f, 2.10f}, {3.80f, 4.57f}}};
-constexpr float kClusterBase[2] = {10.5f, 13.5f};
+// 260..40000 tokens at head_dim 128 (1060 shapes, each run in every form that serves it).  x = packed tiles per SM, a residual
+// tile counted by its cost.
+// SIMT cut: base (launch, prologue, last turn, merge kernel) + tile * x; within 9 to 19 % (rms).  [group 32, 64, 128], then
+// [heads per kv head: 1 and 2, 4, 8] and [bits]
+constexpr float kSimtBase[3][3] = {{18.2f, 21.7f, 24.8f}, {22.4f, 26.1f, 34.6f}, {28.1f, 33.2f, 44.7f}};
+constexpr float kSimtTile[3][3][8] = {{{0.56f, 0.54f, 0.59f, 0.72f, 0.91f, 0.93f, 0.95f, 0.89f},
+                                       {0.60f, 0.57f, 0.67f, 0.80f, 1.02f, 0.98f, 0.99f, 0.95f},
+                                       {0.96f, 0.95f, 1.12f, 1.15f, 1.40f, 1.35f, 1.36f, 1.30f}},
+                                      {{0.85f, 0.88f, 1.01f, 0.90f, 1.36f, 1.43f, 1.72f, 1.53f},
+                                       {0.92f, 0.84f, 1.04f, 1.02f, 1.72f, 1.93f, 1.99f, 1.35f},
+                                       {1.57f, 1.51f, 1.65f, 1.76f, 2.50f, 2.46f, 2.25f, 2.22f}},
+                                      {{1.43f, 1.57f, 1.58f, 1.37f, 2.77f, 3.15f, 4.71f, 2.87f},
+                                       {1.71f, 1.58f, 2.09f, 1.84f, 3.42f, 3.67f, 6.23f, 3.81f},
+                                       {3.00f, 3.08f, 2.98f, 3.53f, 5.29f, 5.68f, 7.26f, 4.21f}}};
+constexpr float kUnrolledBase = 18.f, kUnrolledTile = 0.69f;      // 14 %
+// Cluster mode: base + tile * warps * turns, a turn being one packed tile for every warp of the cluster; within 5 to 10 %.
+// [group][up to 4 heads, up to 8][bits].  Tiles of head_dim 64 take 0.6 of it.
+constexpr float kClusterBase[2] = {10.5f, 13.f};
+constexpr float kClusterTile[3][2][8] = {{{0.60f, 0.57f, 0.61f, 0.59f, 1.01f, 1.00f, 1.00f, 0.89f}, {1.02f, 0.94f, 1.04f, 0.99f, 1.40f, 1.39f, 1.36f, 1.25f}},
+                                         {{0.77f, 0.88f, 0.89f, 0.88f, 1.50f, 1.86f, 1.85f, 1.69f}, {1.53f, 1.57f, 1.63f, 1.50f, 2.19f, 2.28f, 2.12f, 1.89f}},
+                                         {{1.44f, 1.49f, 2.20f, 1.95f, 4.20f, 4.88f, 4.78f, 4.36f}, {2.87f, 2.89f, 3.15f, 3.47f, 4.92f, 5.52f, 5.39f, 5.10f}}};
 // The general kernel's own cut: a tile costs 1.25 of the cluster's (its turns are not aligned), its base is 24 / 35 us.
 constexpr float kGeneralBase[2] = {24.f, 35.f}, kGeneralTile = 1.25f;
 
 int group_index(int group) { return group == 32 ? 0 : group == 64 ? 1 : 2; }
 float cluster_tile_us(const MzDecodeParams& p) {
-  return kClusterTile[group_index(p.s.group)][p.s.bits > 4][p.gqa > 4] * (p.s.head_dim == 64 ? 0.6f : 1.0f);
+  return kClusterTile[group_index(p.s.group)][p.gqa > 4][p.s.bits - 1] * (p.s.head_dim == 64 ? 0.6f : 1.0f);
 }
 
-// The kernel of an even cut: the unrolled kernel where it serves; else the SIMT kernel where it serves.  The general
-// kernel has a larger base and needs as much or more per tile (groups of 32, 4 heads: 0.75 against 0.64 us; 64, 8 heads: 1.70 against
-// 1.62; 128, 8 heads: 2.86 against 2.88; wide codes, 64, 4 heads: 2.16 against 1.71), except for codes of up to 4 bits in groups of 64 with 4 heads, where its smaller base (24.4 against
-// 27.3 us) and its separate residual CTAs win up to about 40 tiles per SM (3 bits: 24 x 8 x 1537 51 against 63 us, 16 x 8 x 4000 81 against 80,
-// 2 x 8 x 60000 144 against 127).
+// The kernel of an even cut: the unrolled kernel where it serves; else the SIMT kernel where it serves.  The general kernel's base is
+// larger and its tiles cost as much or more (3 bits, 4 heads, groups of 32: 0.81 against 0.67 us; 64: 1.09 against 1.04; 128: 2.7
+// against 2.1; 8 bits, 64: 2.4 against 1.35), but its residual tiles have CTAs of their own once every warp has two
+// packed tiles, which is worth a turn.  Codes of up to 4 bits in groups of 64 with 4 or 8 heads gain by that between about 28 and 52
+// tiles per SM (20 shapes: 0.79 to 1.06 of the SIMT kernel's time, 0.96 on average; 1 bit, 24 x 8 x 1537 48 against 62 us); below
+// (1.04 on average) and above (1.04; 3 bits, 2 x 8 x 60000 144 against 126) they don't.
 enum class Cut { kUnrolled, kSimt, kGeneral };
 Cut choose_cut(const MzDecodeParams& p, float x) {
   if (mz_decode_flat_supported(p)) return Cut::kUnrolled;
   if (!mz_decode_tiles_supported(p)) return Cut::kGeneral;
-  return p.s.bits <= 4 && p.s.group == 64 && p.gqa == 4 && x < 40.f ? Cut::kGeneral : Cut::kSimt;
+  return p.s.bits <= 4 && p.s.group == 64 && p.gqa >= 4 && x >= 28.f && x < 52.f ? Cut::kGeneral : Cut::kSimt;
 }
 float cut_us(const MzDecodeParams& p, float x) {
-  CutCost c = kUnrolledCost;
+  const int g = group_index(p.s.group), heads = p.gqa > 4 ? 2 : p.gqa == 4 ? 1 : 0;
   switch (choose_cut(p, x)) {
-    case Cut::kUnrolled: break;
-    case Cut::kSimt: c = kSimtCost[group_index(p.s.group)][p.s.bits > 4][p.gqa > 4 ? 2 : p.gqa == 4 ? 1 : 0]; break;
-    case Cut::kGeneral: c = {kGeneralBase[p.gqa > 4], kGeneralTile * cluster_tile_us(p)}; break;
+    case Cut::kUnrolled: return kUnrolledBase + kUnrolledTile * x;
+    case Cut::kSimt: return kSimtBase[g][heads] + kSimtTile[g][heads][p.s.bits - 1] * x;
+    default: return kGeneralBase[p.gqa > 4] + kGeneralTile * cluster_tile_us(p) * x;
   }
-  return c.base + c.tile * x;
 }
 float tiles_per_sm(const MzDecodeParams& p, const MzTilesPlan& t, int sm_count) {
   return (float)((double)p.s.batch * p.s.kv_heads * (double)t.pair_cost / t.cost_q / sm_count);
