@@ -80,7 +80,7 @@ int kernel_override() {
 
 using Plan = MzDecodePlan;
 
-int make_plan(const mz_decode_args* a, Plan* plan, bool need_tables) {
+int make_plan(const mz_decode_args* a, Plan* plan, bool need_tables, size_t scratch_limit = 0) {
   MZ_REQUIRE(a != nullptr, "args is NULL");
   const mz_kv_store* s = &a->store;
   int rc = mz_check_store_basic(s);
@@ -114,6 +114,7 @@ int make_plan(const mz_decode_args* a, Plan* plan, bool need_tables) {
   p.new_k = p.new_v = nullptr;
   p.new_sb = p.new_sh = 0;
   p.new_rows = 0;
+  p.scratch_limit = scratch_limit;
   const int force = kernel_override();
   // 1 = tcgen05, 2 = tensor cores (mma.sync), 3 = SIMT tiles, 0 = shape-generic
   const int which = force == 1 ? 0 : force == 4 && mz_decode_umma_supported(p) ? 1 : force != 2 && mz_decode_mma_supported(p) ? 2
@@ -183,24 +184,30 @@ int finish(const Plan& plan, const MzDecodeOut& o, cudaStream_t st) {
   return MZ_OK;
 }
 
-int run(const mz_decode_args* a, const MzDecodeOut& o, cudaStream_t st) {
+int run(const mz_decode_args* a, const MzDecodeOut& o, cudaStream_t st, size_t scratch_limit = 0) {
   Plan plan;
-  int rc = make_plan(a, &plan, true);
+  int rc = make_plan(a, &plan, true, scratch_limit);
   if (rc == MZ_OK) rc = launch_partials(a, &plan, o, st);
   return rc ? rc : finish(plan, o, st);
 }
 }  // namespace
 
-// Internal (used by the static-scratch entry point): scratch bytes a call needs and whether it
+// Internal (used by the static-scratch entry point): scratch bytes a call needs that should keep to `limit`, and whether it
 // would use the lazily allocated lookup tables.  Returns the validation status.
-int mz_decode_plan_info(const mz_decode_args* args, size_t* ws_bytes, int* needs_tables) {
+int mz_decode_plan_info(const mz_decode_args* args, size_t limit, size_t* ws_bytes, int* needs_tables) {
   Plan plan;
-  int rc = make_plan(args, &plan, false);
+  int rc = make_plan(args, &plan, false, limit);
   if (rc) return rc;
   *ws_bytes = plan.ws_bytes;
   // the promise is made for the shapes of the tiled kernels, whichever of them runs
   *needs_tables = plan.tiles && mz_decode_tiles_supported(plan.p) ? 0 : 1;
   return MZ_OK;
+}
+
+// Internal (used by the static-scratch entry point): the call that mz_decode_plan_info described.
+int mz_decode_attention_limited(const mz_decode_args* a, size_t limit, cudaStream_t st) {
+  MZ_REQUIRE(a != nullptr && a->out != nullptr && mz_dtype_ok(a->out_dtype), "bad output");
+  return run(a, {a->out, a->out_dtype, nullptr, nullptr, nullptr, 0, 0}, st, limit);
 }
 
 // Internal (used by mz_decode_step): validation and planning of a normalising call, then its launches.

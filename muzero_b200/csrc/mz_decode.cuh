@@ -96,6 +96,9 @@ struct MzDecodeParams {
   // uses it from there and stores it into the window
   const void* new_k; const void* new_v; long long new_sb, new_sh;
   int new_rows;      // rows of the window's buffer (read by the checked build only)
+  // bytes of scratch the plan should keep to (0: any): a cut whose records need more gives way to cluster mode, which
+  // needs none, where that serves
+  size_t scratch_limit;
 };
 
 // A validated call: which kernel runs, its parameters, the partial records and scratch bytes it needs.

@@ -304,14 +304,14 @@ float tiles_per_sm(const MzDecodeParams& p, const MzTilesPlan& t, int sm_count) 
 }
 
 // Cluster mode: one cluster per pair, no partial records in memory and no merge kernel; taken where the estimates above say that it
-// is not slower than the cut.
-bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count) {
+// is not slower than the cut, or at any cost.
+bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count, bool any_cost = false) {
   const long long pairs = (long long)p.s.batch * p.s.kv_heads;
   if (pairs > sm_count) return false;
   MzTilesPlan& t = p.tp;
   describe_tiles(t, p);
   const int T = t.tiles_per_pair;
-  const float limit = cut_us(p, tiles_per_sm(p, t, sm_count));
+  const float limit = any_cost ? INFINITY : cut_us(p, tiles_per_sm(p, t, sm_count));
   int cs = 1;
   while (cs < 8 && cs * 2 * pairs <= sm_count && cs * 4 < T) cs *= 2;
   const unsigned rec = (unsigned)(p.gqa * (p.s.head_dim + 4) * 4);
@@ -344,18 +344,9 @@ static void take_lookup_entries(MzDecodeParams& p) {
   p.lut = p.s.k_groups > 0 && p.s.bits <= 4 ? mz_mma_lookup_entries(p.s.bits, true, p.s.alpha_key, p.s.alpha_value) : nullptr;
 }
 
-int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slots) {
+// an even cut by the kernel that serves it best
+static int plan_cut(MzDecodeParams& p, const MzMmaKernel& k, int splits_request, int sm_count, size_t* slots) {
   const mz_kv_store& s = p.s;
-  p.hetero = 0;
-  p.cluster = 0;
-  MzMmaKernel k;
-  if (!find_kernel(p, &k)) return mz_fail(MZ_ERR_UNSUPPORTED, "no tensor-core kernel for this shape");
-  if (splits_request == 0 && plan_cluster(p, k, sm_count)) {
-    *slots = 4;                                   // no records; a workspace is still asked for, so that its size is never 0
-    take_lookup_entries(p);
-    return MZ_OK;
-  }
-  p.cluster = 0;
   describe_tiles(p.tp, p);
   switch (choose_cut(p, tiles_per_sm(p, p.tp, sm_count))) {
     case Cut::kUnrolled: return mz_plan_flat(p, splits_request, sm_count, slots);
@@ -392,6 +383,29 @@ int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slo
     }
   }
   return plan_single(p, k, splits_request, sm_count, slots);
+}
+
+int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slots) {
+  p.hetero = 0;
+  p.cluster = 0;
+  MzMmaKernel k;
+  if (!find_kernel(p, &k)) return mz_fail(MZ_ERR_UNSUPPORTED, "no tensor-core kernel for this shape");
+  auto clustered = [&](MzDecodeParams& q, bool any_cost) {
+    if (splits_request != 0 || !plan_cluster(q, k, sm_count, any_cost)) return false;
+    *slots = 4;                                   // no records; a workspace is still asked for, so that its size is never 0
+    take_lookup_entries(q);
+    return true;
+  };
+  if (clustered(p, false)) return MZ_OK;
+  p.cluster = 0;
+  MzDecodeParams other = p;
+  const int rc = plan_cut(p, k, splits_request, sm_count, slots);
+  if (rc == MZ_OK && p.scratch_limit > 0 && *slots * sizeof(float) * (2 + (size_t)p.s.head_dim) > p.scratch_limit) {
+    const size_t cut_slots = *slots;
+    if (clustered(other, true)) p = other;
+    else *slots = cut_slots;
+  }
+  return rc;
 }
 
 int mz_launch_decode_mma(const MzDecodeParams& p, cudaStream_t st) {

@@ -4,7 +4,8 @@
 
 #include "mz_decode.cuh"
 
-int mz_decode_plan_info(const mz_decode_args* args, size_t* ws_bytes, int* needs_tables);
+int mz_decode_plan_info(const mz_decode_args* args, size_t limit, size_t* ws_bytes, int* needs_tables);
+int mz_decode_attention_limited(const mz_decode_args* args, size_t limit, cudaStream_t st);
 
 // The scratch itself.  In host code this name is only a stand-in for the symbol: it is not a
 // device address and must never be handed to a kernel; the address comes from
@@ -39,7 +40,7 @@ extern "C" int mz_decode_attention_static(const mz_decode_args* args, void* stre
   MZ_REQUIRE(args != nullptr, "args is NULL");
   size_t need = 0;
   int needs_tables = 0;
-  int rc = mz_decode_plan_info(args, &need, &needs_tables);
+  int rc = mz_decode_plan_info(args, MZ_STATIC_SCRATCH_BYTES, &need, &needs_tables);
   if (rc) return rc;
   if (needs_tables)
     return mz_fail(MZ_ERR_UNSUPPORTED,
@@ -53,5 +54,5 @@ extern "C" int mz_decode_attention_static(const mz_decode_args* args, void* stre
   mz_decode_args local = *args;
   local.workspace = scratch;
   local.workspace_bytes = MZ_STATIC_SCRATCH_BYTES;
-  return mz_decode_attention(&local, stream);
+  return mz_decode_attention_limited(&local, MZ_STATIC_SCRATCH_BYTES, (cudaStream_t)stream);
 }

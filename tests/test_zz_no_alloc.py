@@ -79,3 +79,22 @@ def test_static_scratch_rejects_what_it_cannot_serve():
     args = build_decode_args(small, q64.cuda(), 0.125, None, out64)
     assert lib.mz_decode_attention_static(ctypes.byref(args), stream_ptr(q.device)) == 2
     assert "shape-generic" in last_error()
+
+
+@pytest.mark.parametrize("batch,seq,bits,group", [(37, 16100, 1, 32), (37, 1200, 4, 64), (20, 4000, 2, 64)])
+def test_static_scratch_with_eight_heads(batch, seq, bits, group):
+    """Eight heads per kv head over all SMs need more records than the array holds; the pairs of such a call run as clusters, which
+    need none, whatever the ordinary entry point prefers."""
+    import muzero_b200 as mz
+    from muzero_b200.cache.attention import build_decode_args, decode_attention
+    from muzero_b200.kernels._cabi import check, load_library, stream_ptr
+    gen = torch.Generator(device="cuda").manual_seed(seq)
+    k, v = (torch.randn(batch, 2, seq, 128, device="cuda", generator=gen, dtype=torch.bfloat16) for _ in range(2))
+    q = torch.randn(batch, 16, 1, 128, device="cuda", generator=gen, dtype=torch.bfloat16)
+    layer = mz.MuZeroCacheLayer(mz.MuZeroConfig(bits=bits, q_group_size=group, residual_length=128, alpha_key=2.0, alpha_value=2.0))
+    layer.update(k, v, {"materialize_full_kv": False})
+    out = torch.empty(batch, 1, 16, 128, dtype=torch.float32, device="cuda")
+    args = build_decode_args(layer, q, 0.088, None, out)
+    args.workspace, args.workspace_bytes = None, 0
+    check(load_library().mz_decode_attention_static(ctypes.byref(args), stream_ptr(q.device)), "mz_decode_attention_static")
+    assert (out - decode_attention(layer, q, 0.088, out_dtype=torch.float32)).abs().max().item() <= 1e-5
