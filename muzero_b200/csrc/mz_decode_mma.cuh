@@ -192,8 +192,8 @@ __device__ __forceinline__ void look_step(const Q& w, int h, uint32_t zz, uint32
 }
 
 // One step's product with M tile `m` of half a quad, added to c: the remainders first, then the rounded values, on a
-// fresh accumulator, so that the running sum is rounded to nearest (the tensor cores truncate theirs: over the 256 steps
-// of eight tiles that alone would be 1e-5).
+// fresh accumulator, so that the running sum is rounded to nearest.  The tensor cores truncate theirs: with the keys' sums left
+// on them the error against 64 bits is 2.0e-6 instead of 4.5e-7 (4 bits, head_dim 128), for 0 to 3 % of the time.
 template <bool SCALED = false>
 __device__ __forceinline__ void mma_step(float (&c)[4], const uint2 (&a)[8], int m, uint32_t b0, uint32_t b1, float unit = 1.0f) {
   float x[4];
