@@ -2,14 +2,12 @@
 #include "mz_decode.cuh"
 
 namespace {
-// ---- merge of the records of one (batch, kv head) pair: one CTA per pair, one group of D
-// threads per query head.  The warps of the main kernel that hold records of the pair are found from
+// ---- merge of the records of one (batch, kv head) pair and head: one CTA, whose groups of D threads each merge every n-th chunk
+// of records; their partial states are merged in a fixed order at the end.  The warps of the main kernel that hold records of the pair are found from
 // the partition functions the main kernel uses: warp g owns the tiles whose start cost lies in
 // [cost(g), cost(g+1)), and cost(g) is within [g*quot, g*(quot+1)), so every contributor lies in the
 // candidate range [c_lo/(quot+1) - 1, (c_hi-1)/quot + 1], c_lo..c_hi being the pair's cost interval.
 // All threads test candidates at once; the list keeps the candidates' order (a fixed merge order).
-// WIDE (many records per pair, few pairs): one CTA per (pair, head); its groups each merge every n-th chunk
-// of records and the partial states are merged in a fixed order at the end.
 constexpr int kMaxCombineSlots = 4096;
 // The workers of plan `tp` that can hold records of `pair` lie in [first, last] (a superset; see above).
 struct WorkerRange { long long first, last; };
@@ -33,13 +31,12 @@ __device__ __forceinline__ long long record_of(const MzTilesPlan& tp, long long 
   if (!(f0 < hi && f1 > lo && f0 < f1)) return -1;
   return first_record + gw * tp.max_segs + (pair - (int)((unsigned)f0 / (unsigned)T));
 }
-template <bool WIDE, int D>
-__global__ void __launch_bounds__(512, 4) combine_tiles_kernel(const MzDecodeParams p, const MzDecodeOut o) {
+template <int D>
+__global__ void __launch_bounds__(512, 3) combine_tiles_kernel(const MzDecodeParams p, const MzDecodeOut o) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a dependent waits for this grid's completion itself
   __shared__ int s_slot[kMaxCombineSlots];     // record of candidate i, or -1
-  __shared__ float s_part[WIDE ? 512 / D : 1][WIDE ? D + 2 : 1];
-  const int pair = WIDE ? blockIdx.x / p.gqa : blockIdx.x;
-  const int gqa = p.gqa;
+  __shared__ float s_part[512 / D][D + 2];
+  const int gqa = p.gqa, pair = blockIdx.x / gqa, h = blockIdx.x % gqa;
   // candidates of the main plan, then of the residual-tile plan of the tcgen05 route (its records follow)
   const WorkerRange ra = candidate_workers(p.tp, pair), rb = candidate_workers(p.tp2, pair);
   const long long cand_a = ra.last - ra.first + 1, cand_b = rb.last - rb.first + 1;
@@ -66,70 +63,64 @@ __global__ void __launch_bounds__(512, 4) combine_tiles_kernel(const MzDecodePar
       if (rec >= 0) fn(rec);
     }
   };
-  const int quad = threadIdx.x / D, quads = blockDim.x / D;
-  for (int h = WIDE ? blockIdx.x % gqa : quad; h < gqa; h += WIDE ? gqa : quads) {
-    const int d = threadIdx.x % D;
-    float mx = -INFINITY, lsum = 0.f, a = 0.f;
-    if (listed) {
-      // four records at a time: their loads are independent and in flight together; the running
-      // maximum is carried along (one pass)
-      for (int i0 = WIDE ? 4 * quad : 0; i0 < n; i0 += WIDE ? 4 * quads : 4) {
-        float mi[4], li[4], ai[4];
+  const int quad = threadIdx.x / D, quads = blockDim.x / D, d = threadIdx.x % D;
+  float mx = -INFINITY, lsum = 0.f, a = 0.f;
+  if (listed) {
+    // four records at a time: their loads are independent and in flight together; the running
+    // maximum is carried along (one pass)
+    for (int i0 = 4 * quad; i0 < n; i0 += 4 * quads) {
+      float mi[4], li[4], ai[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int sl = i0 + j < n ? s_slot[i0 + j] : -1;
-          const bool on = sl >= 0;
-          const long long slot = on ? (long long)sl * gqa + h : 0;
-          mi[j] = on ? p.part.m[slot] : -INFINITY;
-          li[j] = on ? p.part.l[slot] : 0.f;
-          ai[j] = on ? p.part.acc[slot * D + d] : 0.f;
-        }
-        const float m_new = fmaxf(fmaxf(mx, fmaxf(mi[0], mi[1])), fmaxf(mi[2], mi[3]));
-        const float keep = mx > -INFINITY ? __expf(mx - m_new) : 0.f;
-        lsum *= keep; a *= keep;
+      for (int j = 0; j < 4; ++j) {
+        const int sl = i0 + j < n ? s_slot[i0 + j] : -1;
+        const bool on = sl >= 0;
+        const long long slot = on ? (long long)sl * gqa + h : 0;
+        mi[j] = on ? p.part.m[slot] : -INFINITY;
+        li[j] = on ? p.part.l[slot] : 0.f;
+        ai[j] = on ? p.part.acc[slot * D + d] : 0.f;
+      }
+      const float m_new = fmaxf(fmaxf(mx, fmaxf(mi[0], mi[1])), fmaxf(mi[2], mi[3]));
+      const float keep = mx > -INFINITY ? __expf(mx - m_new) : 0.f;
+      lsum *= keep; a *= keep;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float wgt = mi[j] > -INFINITY ? __expf(mi[j] - m_new) : 0.f;
-          lsum = fmaf(li[j], wgt, lsum);
-          a = fmaf(ai[j], wgt, a);
-        }
-        mx = m_new;
+      for (int j = 0; j < 4; ++j) {
+        const float wgt = mi[j] > -INFINITY ? __expf(mi[j] - m_new) : 0.f;
+        lsum = fmaf(li[j], wgt, lsum);
+        a = fmaf(ai[j], wgt, a);
       }
-      if (WIDE) {
-        // the quads' states, merged in quad order by quad 0
-        s_part[quad][d] = a;
-        if (d == 0) { s_part[quad][D] = mx; s_part[quad][D + 1] = lsum; }
-        __syncthreads();
-        if (quad != 0) continue;      // WIDE visits one head per CTA: nothing follows for these threads
-        float m_all = -INFINITY;
-        for (int k = 0; k < quads; ++k) m_all = fmaxf(m_all, s_part[k][D]);
-        lsum = 0.f; a = 0.f;
-        for (int k = 0; k < quads; ++k) {
-          const float mk = s_part[k][D];
-          const float wgt = mk > -INFINITY ? __expf(mk - m_all) : 0.f;
-          lsum = fmaf(s_part[k][D + 1], wgt, lsum);
-          a = fmaf(s_part[k][d], wgt, a);
-        }
-        mx = m_all;
-      }
-    } else if (!WIDE || quad == 0) {
-      for_each_slot([&](long long sl) { mx = fmaxf(mx, p.part.m[sl * gqa + h]); });
-      for_each_slot([&](long long sl) {
-        const long long slot = sl * gqa + h;
-        const float mi = p.part.m[slot];
-        const float wgt = mi > -INFINITY ? __expf(mi - mx) : 0.f;
-        lsum = fmaf(p.part.l[slot], wgt, lsum);
-        a = fmaf(p.part.acc[slot * D + d], wgt, a);
-      });
-    } else {
-      continue;
+      mx = m_new;
     }
-    const long long row = (long long)pair * gqa + h;
-    if (o.out) mz_store_from_float(o.out, row * D + d, a / fmaxf(lsum, 1e-20f), o.out_dt);
-    else {
-      o.acc[row * o.acc_stride + d] = a;
-      if (d == 0) { o.m[row * o.ml_stride] = mx; o.l[row * o.ml_stride] = lsum; }
+    // the groups' states, merged in order by the first
+    s_part[quad][d] = a;
+    if (d == 0) { s_part[quad][D] = mx; s_part[quad][D + 1] = lsum; }
+    __syncthreads();
+    if (quad != 0) return;
+    float m_all = -INFINITY;
+    for (int k = 0; k < quads; ++k) m_all = fmaxf(m_all, s_part[k][D]);
+    lsum = 0.f; a = 0.f;
+    for (int k = 0; k < quads; ++k) {
+      const float mk = s_part[k][D];
+      const float wgt = mk > -INFINITY ? __expf(mk - m_all) : 0.f;
+      lsum = fmaf(s_part[k][D + 1], wgt, lsum);
+      a = fmaf(s_part[k][d], wgt, a);
     }
+    mx = m_all;
+  } else {
+    if (quad != 0) return;
+    for_each_slot([&](long long sl) { mx = fmaxf(mx, p.part.m[sl * gqa + h]); });
+    for_each_slot([&](long long sl) {
+      const long long slot = sl * gqa + h;
+      const float mi = p.part.m[slot];
+      const float wgt = mi > -INFINITY ? __expf(mi - mx) : 0.f;
+      lsum = fmaf(p.part.l[slot], wgt, lsum);
+      a = fmaf(p.part.acc[slot * D + d], wgt, a);
+    });
+  }
+  const long long row = (long long)pair * gqa + h;
+  if (o.out) mz_store_from_float(o.out, row * D + d, a / fmaxf(lsum, 1e-20f), o.out_dt);
+  else {
+    o.acc[row * o.acc_stride + d] = a;
+    if (d == 0) { o.m[row * o.ml_stride] = mx; o.l[row * o.ml_stride] = lsum; }
   }
 }
 
@@ -231,12 +222,15 @@ int mz_combine_tiles(const MzDecodeParams& p, const MzDecodeOut& o, cudaStream_t
   // programmatic dependent launch: the merge grid may start while the main kernel drains; it finds its
   // records (pure arithmetic) and then waits for the main grid's results (griddepcontrol.wait)
   cudaLaunchConfig_t cfg = {};
-  // many records per pair and few pairs: one CTA per (pair, head) with the records split over its quads
+  // A warp per (pair, head) takes eight records at a time and pays while that is about one turn: below eight workers per pair.  From there on a
+  // CTA per (pair, head) shares them (12 x 8 pairs x 3000 tokens at 4 bits, 19 workers per pair: 35.2 us per call with warps,
+  // 34.3 with CTAs; 16 x 8 x 4224, 13 per pair: 49.5 and 47.9; 48 x 8 x 2100, 4 per pair: 70.9 and 76.9; 64 pairs with 27 records
+  // 150 and 140).  One CTA per pair for all heads, which had served 8 to 24 workers per pair, took 22 us on its own: 48.2 and 58.2.
   const long long pairs = (long long)p.s.batch * p.s.kv_heads;
-  const bool wide = p.tp.total_warps / pairs >= 24 && pairs * p.gqa <= 4096;
-  cfg.gridDim = dim3((unsigned)(wide ? pairs * p.gqa : pairs));
+  const bool per_warp = p.tp.total_warps / pairs < 8;
   const int D = p.s.head_dim;
-  cfg.blockDim = dim3(wide ? 512 : D * (p.gqa < 4 ? p.gqa : 4));
+  cfg.gridDim = dim3((unsigned)(per_warp ? (pairs * p.gqa + 7) / 8 : pairs * p.gqa));
+  cfg.blockDim = dim3(per_warp ? 256 : 512);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -244,20 +238,12 @@ int mz_combine_tiles(const MzDecodeParams& p, const MzDecodeOut& o, cudaStream_t
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  // one plan and a few records per pair (workers per pair below 8): the warp-per-row kernel
-  const bool per_warp = !wide && (p.tp2.total_warps == 0 || p.hetero > 0) && p.tp.total_warps / pairs < 8;
-  if (per_warp) {
-    cfg.blockDim = dim3(256);
-    cfg.gridDim = dim3((unsigned)((pairs * p.gqa + 7) / 8));
-  }
   if (D == 128) {
     if (per_warp) MZ_CUDA(cudaLaunchKernelEx(&cfg, combine_tiles_warp_kernel<128>, p, o));
-    else if (wide) MZ_CUDA(cudaLaunchKernelEx(&cfg, combine_tiles_kernel<true, 128>, p, o));
-    else MZ_CUDA(cudaLaunchKernelEx(&cfg, combine_tiles_kernel<false, 128>, p, o));
+    else MZ_CUDA(cudaLaunchKernelEx(&cfg, combine_tiles_kernel<128>, p, o));
   } else {
     if (per_warp) MZ_CUDA(cudaLaunchKernelEx(&cfg, combine_tiles_warp_kernel<64>, p, o));
-    else if (wide) MZ_CUDA(cudaLaunchKernelEx(&cfg, combine_tiles_kernel<true, 64>, p, o));
-    else MZ_CUDA(cudaLaunchKernelEx(&cfg, combine_tiles_kernel<false, 64>, p, o));
+    else MZ_CUDA(cudaLaunchKernelEx(&cfg, combine_tiles_kernel<64>, p, o));
   }
   MZ_LAUNCH_CHECK("combine_tiles");
   return MZ_OK;

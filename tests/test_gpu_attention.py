@@ -257,6 +257,18 @@ def test_many_pairs_and_split_counts_beyond_16_bits(oracle):
         assert (again - got).abs().max().item() < SPLIT_TOL, splits
 
 
+@pytest.mark.parametrize("D,group", [(128, 64), (64, 32)])
+def test_merge_kernels_at_their_boundary(oracle, D, group):
+    """Up to seven workers per pair a warp merges a head's records, from eight on a CTA does: on both sides of the line, at the warp
+    kernel's largest turn, and at record counts that leave groups of the CTA without any."""
+    from muzero_b200.cache.attention import decode_attention
+    ref, layer, q = _oracle_and_gpu_layers(oracle, 2, 3, 6, 2500, D, 4, group, 128, seed=77, steps=1)
+    want = oracle.decode_attention_oracle(q, ref, 0.09, 2, compute_dtype=torch.float32)
+    for splits in (2, 7, 8, 9, 16, 17, 33):
+        got = decode_attention(layer, q.cuda(), 0.09, out_dtype=torch.float32, splits=splits)
+        assert (got.cpu() - want).abs().max().item() <= TOL, splits
+
+
 @pytest.mark.parametrize("which,name", [(1, "generic"), (2, "tiles"), (3, "mma"), (4, "umma")])
 def test_every_kernel_against_the_oracle(oracle, which, name):
     """The four decode kernels on the same caches (4- and 2-bit, group 64, a pair boundary inside a worker's range,
