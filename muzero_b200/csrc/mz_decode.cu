@@ -58,7 +58,7 @@ int sm_count() {
 
 // Which decode kernel serves a call.  0 = automatic (tensor-core mma.sync kernel where it applies, else the SIMT
 // tiled kernel, else the shape-generic kernel), 1 = generic, 2 = no tensor-core kernel, 3 = the same as 0,
-// 4 = the tcgen05 kernel where it applies (an opt-in: correct, but slower than the mma.sync kernel so far).
+// 4 = the tcgen05 kernel for every call that it serves, whatever the automatic choice would be.
 // MZ_DECODE_KERNEL = generic | tiles | mma | umma sets the initial value (read once, at the first call);
 // mz_debug_force_kernel changes it for later calls, so that tests can cross-check the kernels in one process.
 std::atomic<int> g_kernel_override{-1};
@@ -109,6 +109,7 @@ int make_plan(const mz_decode_args* a, Plan* plan, bool need_tables, size_t scra
   p.table_k = p.table_v = nullptr;
   p.lut = nullptr;
   p.hetero = 0;
+  p.planes = 0;
   p.cluster = 0;
   p.o = MzDecodeOut{};
   p.new_k = p.new_v = nullptr;
@@ -125,7 +126,7 @@ int make_plan(const mz_decode_args* a, Plan* plan, bool need_tables, size_t scra
   if (plan->tiles) {
     p.tp2 = MzTilesPlan{};
     p.slots_a = 0;
-    if (which == 1) rc = mz_plan_umma(p, a->splits, sm_count(), &plan->slots);
+    if (which == 1) rc = mz_plan_umma(p, false, a->splits, sm_count(), &plan->slots);
     else if (which == 2) rc = mz_plan_mma(p, a->splits, sm_count(), &plan->slots);
     else rc = mz_plan_tiles(p, a->splits, sm_count(), &plan->slots);
     if (rc) return rc;

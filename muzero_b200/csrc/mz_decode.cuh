@@ -79,16 +79,17 @@ struct MzDecodeParams {
   // window have their values in the packed store (rows k_groups*G ..), the rest in the dense window
   int v_lead;
   MzTilesPlan tp;
-  // tcgen05 route: the packed tiles run on plan `tp`, the residual tiles on plan `tp2` (mma.sync kernel,
-  // total_warps == 0 when there is no residual window); the records of tp2 start at record slots_a
+  // second plan of a launch over two plans (`hetero`), total_warps == 0: none; its records start at record slots_a
   MzTilesPlan tp2;
   long long slots_a;
   // tensor-core kernel: the lookup-table entries in global memory (built once per device and (bits, alphas));
   // nullptr = every CTA computes them itself
   const unsigned* lut;
-  // tensor-core kernel, one launch over two plans: CTAs [0, hetero) work on plan `tp` (packed tiles only), the
+  // tensor-core kernels, one launch over two plans: CTAs [0, hetero) work on plan `tp` (packed tiles only), the
   // rest on plan `tp2` (residual tiles only, records from slots_a on).  0 = one plan per launch.
   int hetero;
+  // tcgen05 kernel: bytes per value
+  int planes;
   // tensor-core kernel, cluster mode: CTAs per pair (0 = flat partition and merge kernel); the kernel writes `o` itself
   int cluster;
   MzDecodeOut o;
@@ -146,8 +147,8 @@ bool mz_mma_kernel_b4(int D, int G, int nt, MzMmaKernel* k);
 bool mz_mma_kernel_b8(int D, int G, int nt, MzMmaKernel* k);
 bool mz_mma_kernel_wide(int D, int G, int nt, MzMmaKernel* k);
 
-// tcgen05 kernel (A operand in tensor memory): the packed tiles of head_dim 128 / group 64 / 2- or 4-bit caches;
-// the residual tiles go to the mma.sync kernel in a companion launch
+// tcgen05 kernel: 1 to 3 bits, head_dim 128, group 64.  full_precision: that of the fp32 kernels also at 2 bits, where the call would
+// not have gone to the unrolled kernel
 bool mz_decode_umma_supported(const MzDecodeParams& p);
-int mz_plan_umma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slots);
+int mz_plan_umma(MzDecodeParams& p, bool full_precision, int splits_request, int sm_count, size_t* slots);
 int mz_launch_decode_umma(const MzDecodeParams& p, cudaStream_t st);

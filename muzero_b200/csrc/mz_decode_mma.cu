@@ -396,6 +396,21 @@ int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slo
     take_lookup_entries(q);
     return true;
   };
+  // The tcgen05 kernel takes what it serves: over 150 shapes of 0.1 to 210 tiles per SM it needs 0.55 (1 bit), 0.70 (3 bits) and 0.78 (2 bits)
+  // of the time of the best other form, and is nowhere behind it by more than the timing's spread (device time of the smallest
+  // calls: 0.51 to 0.92 of cluster mode).  At 2 bits it runs with two planes where the choice below would have been the
+  // unrolled kernel, whose precision that is, and with three where it would have been a cluster.
+  if (splits_request == 0 && mz_decode_umma_supported(p)) {
+    MzDecodeParams t = p, c = p;
+    size_t n = 0;
+    const bool full = p.s.bits == 2 && plan_cluster(c, k, sm_count);
+    const int rc = mz_plan_umma(t, full, 0, sm_count, &n);
+    if (rc == MZ_OK && (p.scratch_limit == 0 || n * sizeof(float) * (2 + (size_t)p.s.head_dim) <= p.scratch_limit)) {
+      p = t;
+      *slots = n;
+      return MZ_OK;
+    }
+  }
   if (clustered(p, false)) return MZ_OK;
   p.cluster = 0;
   MzDecodeParams other = p;

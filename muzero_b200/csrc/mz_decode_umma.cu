@@ -1,684 +1,922 @@
-// tcgen05 / TMEM decode attention over the packed tiles of a cache: head_dim 128, group 64, 2- or 4-bit codes,
-// 1/2/4 query heads per kv head (sm_100a).
+// tcgen05 decode attention over the packed tiles of a cache, on the integer tensor cores: head_dim 128, group 64, 1-, 2- or 3-bit codes,
+// 1 / 2 / 4 query heads per kv head (sm_100a).
 //
-// Same mathematics as the mma.sync kernel (mz_decode_mma.cu): the value of a code is
-// A + Bup * u+[zc][e] + Bdn * u-[zc][e], the per-row constants are folded into the other operand of each
-// contraction, and one 32-bit shared-memory lookup per code returns the fp16 pair (u+, u-).  What changes is
-// where the contractions run: the legacy mma.sync pipe of this GPU needs 32 cycles per m16n8k16, which bounds
-// that kernel; here they are tcgen05.mma instructions with the table values as the A operand in tensor memory:
-//   * a warpgroup (4 warps, 128 threads) is one worker; it takes two packed tiles (128 tokens) of a
-//     (batch, kv head) pair per step
-//   * keys: the 128 tokens are the 128 rows (TMEM lanes) of A, a reduction block is 8 channels x {above, below
-//     the zero code} = 16 fp16 = 8 TMEM columns; a thread looks up the codes of 4 tokens x 2 channels per block
-//     and writes them with tcgen05.st.16x128b.x2, whose register layout is the A fragment of mma.sync.  The B
-//     operand (folded query, N = 16: two tiles x 4 heads x {product, remainder}) is built in shared memory in
-//     the no-swizzle K-major layout; 16 MMAs of 128x16x16 produce the logits in TMEM
-//   * values: the 128 channels are the rows, a reduction block is 8 tokens; B holds the folded probabilities
-//     (N = 16: two channel groups x 4 heads x {product, remainder}); the output accumulates in TMEM across
-//     steps and is rescaled in place (tcgen05.ld / st) when the running maximum of a head grows
-//   * online softmax state, the exchange of maxima and probabilities between the four warps, and the fold go
-//     through shared memory and named barriers; MMA completion is tracked with mbarriers (tcgen05.commit), and
-//     every wait on one is bounded: when it runs out the worker poisons its records (the merged output
-//     becomes NaN) and carries on
-// Residual (un-quantized) tiles are not handled here: the mma.sync kernel runs them in a companion launch and the
-// merge kernel combines the records of both.
-#include <mutex>
-
-#include "mz_mma_common.cuh"
+// Both contractions reduce over the packed rows (keys: over channels, values: over tokens), and a row of 64 codes runs along the
+// dimension that is kept.  So one thread owns a row: it builds the row's book of dequantized values (fixed point, relative to the
+// row's larger side S) in registers, expands the codes four at a time with byte permutes, and stores the bytes of the values, each
+// in a plane of its own, as they stand into operands in shared memory that are major along the kept dimension.  The other operand is
+// the query (the probabilities) times S, as a fixed-point number in signed bytes, so that the products and their sums are exact integers:
+//   * a worker is two teams of four warps; a step is 128 tokens of a (batch, kv head) pair.  One team expands the keys (thread r = channel
+//     r of the step's two groups) one step ahead of the other, which finishes the logits, keeps the softmax and expands the values (thread
+//     r = token r with its two channel groups).  A CTA has two or three workers and a warp per worker that only issues MMAs: one
+//     thread needs 55 cycles for each
+//   * tcgen05.mma.kind::i8, M 128 x N 32 x K 32: M = 2 groups x 64 tokens (2 x 64 channels), N = 2 groups x 4 heads x 4 bytes; the
+//     group of a row of the result picks its half of the columns
+//   * the top byte is signed, the others unsigned; each plane has an accumulator of its own, and column_sum adds products of equal weight
+//   * online softmax with one thread per token, the running output in registers (thread = channel); MMA completion is tracked with
+//     mbarriers, every wait on one is bounded: when it runs out the worker poisons its records (the merged output becomes
+//     NaN), frees its tensor memory and returns
+//   * the residual window is un-quantized: its tiles have CTAs of their own (mz_dense_tiles.cuh)
+//
+// What bounds it: issue (58 % of the cycles; per row of 64 two-bit codes about 230 instructions, of which 32 permutes) and the logic pipe
+// (48 %, two cycles per instruction); integer MMAs take 40 cycles each, all of it reading their operands, 41 %.  A thread that spills
+// is dear: 227 KB of shared memory leave 28 KB of L1, and 20 bytes of spill per thread cost 10 %.  Hence the register split.
+// 64 x 8 pairs x 4224 tokens, 4 heads, us per call: 1 bit 202 -> 93 (before: SIMT kernel), 2 bits 148 -> 120 (before: unrolled mma.sync
+// kernel), 3 bits 230 -> 180 (SIMT); 24 x 8 x 1537, 3 bits: 53 -> 37; one sequence of 1300 tokens, device time: 15 -> 8 to 11.
+//
+// Precision: three planes hold a value to 2^-22 of its row's larger side and the fold to 2^-31 of the step's largest product, which is that of the
+// fp32 kernels (relative error against 64 bits 2e-7 to 9e-7; 1 bit is exact in one plane).  Two planes (2 bits, calls that the
+// unrolled kernel served with 9e-5): 2^-15 and 2^-22, 2e-5 to 6e-5.  Any range is served: sides and query are scaled by powers of two.
+#include "mz_dense_tiles.cuh"
 
 namespace mzu {
 using namespace mzm;
 
-constexpr int WGS = 3;                     // warpgroups (workers) per CTA
-constexpr int THREADS = WGS * 128;
-constexpr int TM_PER_WG = 160;             // TMEM columns of a worker: A operand 128, logits 16, output 16
-constexpr int TM_A = 0, TM_L = 128, TM_O = 144;
-// B operands in shared memory: per reduction block the four 8x8 core matrices (k chunk kc, n block nb) of 128
-// bytes sit at kc*LBO + nb*SBO; the strides carry a skew of 16 / 32 / 64 bytes so that the folding threads' stores
-// of one instruction fall into 32 different banks
-constexpr int KOP_BLOCK = 544, KOP_LBO = 272, KOP_SBO = 128;
-constexpr int VOP_BLOCK = 576, VOP_LBO = 288, VOP_SBO = 144;
-constexpr int KOP_BYTES = 16 * KOP_BLOCK, VOP_BYTES = 16 * VOP_BLOCK;
-constexpr int ZK_BYTES = 2 * 128, ZV_BYTES = 2 * 2 * 64;
-constexpr int PB_HEAD = 65;                // probabilities [tile][head][65]: the odd stride spreads the softmax lanes' stores
-constexpr int PB_BYTES = 2 * 4 * PB_HEAD * 4;
-constexpr int RED_BYTES = 768;             // reductions between the four warps, and the two mbarriers
-constexpr int SPIN_LIMIT = 4000000;
+constexpr int STEP_GROUPS = 2;                   // groups of 64 tokens per step
+constexpr int SPIN_LIMIT = 1000000;
+constexpr int PLANE_BYTES = 16384;               // [16-byte chunk of the kept dimension, 8][row 128][16]
+constexpr int FOLD_BYTES = 4096;                 // [group 2][row 128][4 heads x 4 bytes]
+constexpr float MAGIC = 12582912.0f;             // 1.5 * 2^23: adding it rounds to an integer that stands in the low mantissa bits
 
-__host__ __device__ constexpr unsigned wg_bytes(unsigned stage) {
-  return 4 * stage + KOP_BYTES + VOP_BYTES + ZK_BYTES + ZV_BYTES + ((PB_BYTES + 127) / 128) * 128 + RED_BYTES;
-}
+constexpr int DENSE_WARPS = 12, DENSE_REGS = 128;          // of a CTA that has residual tiles
 
-// ---- tcgen05 / mbarrier wrappers --------------------------------------------------------------------------------
-__device__ __forceinline__ void tm_st4(uint32_t taddr, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
-  asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(a0), "r"(a1), "r"(a2), "r"(a3) : "memory");
+// How a code width is run.  A CTA has WORKERS workers, each with four warps for the keys and four for softmax and values, and one more group
+// of four warps that issue the workers' MMAs (one each).  The registers that the warps are launched with (LAUNCH each) are
+// redistributed: KEY * 4 W + VALUE * 4 W + ISSUE * 4 <= LAUNCH * (8 W + 4).
+template <int BITS, int P>
+struct Cfg {
+  static constexpr int NE = 1 << BITS, TOP = NE - 1, ZC = NE / 2;
+  static constexpr int PLANES = P;                                       // bytes per value
+  static constexpr int WORKERS = PLANES == 3 ? 2 : 3;
+  static constexpr int WARPS = 8 * WORKERS + 4, THREADS = 32 * WARPS;
+  static constexpr int LAUNCH = WORKERS == 3 ? 72 : 96, KEY = WORKERS == 3 ? 56 : 88, VALUE = WORKERS == 3 ? 104 : 136, ISSUE = 24;
+  static_assert(DENSE_REGS * DENSE_WARPS + 24 * (WARPS - DENSE_WARPS) <= LAUNCH * WARPS, "register split of a residual CTA");
+  static_assert(KEY * 4 * WORKERS + VALUE * 4 * WORKERS + ISSUE * 4 <= LAUNCH * WARPS, "register split");
+  static constexpr bool BOOKS = BITS <= 3;                               // wider codes are expanded by arithmetic
+  // book table: per zero code up to the middle (rows above are mirrored) slopes and offsets of the entries
+  static constexpr int BOOK_ROW = 8 * NE, BOOK_BYTES = BITS == 2 || BITS == 3 ? ZC * BOOK_ROW : 128;
+  static constexpr float FULL = PLANES == 1 ? 1.0f : PLANES == 2 ? 32766.0f : 4194000.0f;      // fixed-point value of S
+  // fixed-point value of 1 in the folded operand (two planes: half of it; else its upper half), and what a unit of column_sum is worth
+  static constexpr float FOLD_FULL = PLANES == 2 ? 4161536.0f : 32000.0f;
+  static constexpr float UNIT = (PLANES == 1 ? 1.0f / 65536.0f : PLANES == 2 ? 128.0f : 256.0f) / (FULL * FOLD_FULL);
+  static constexpr int TM_SIDE = 32 * PLANES, TM_WORKER = 2 * TM_SIDE;   // tensor-memory columns: one accumulator per plane
+  static constexpr int TM_ALLOC = WORKERS * TM_WORKER <= 256 ? 256 : 512;
+  static constexpr int OFF_FOLD = PLANES * PLANE_BYTES, SIDE_BYTES = OFF_FOLD + FOLD_BYTES;      // operands of one side
+  static constexpr int OFF_RED = 2 * SIDE_BYTES, WORKER_BYTES = OFF_RED + 896;
+  static constexpr int BOOKS_BYTES = (2 * BOOK_BYTES + 127) / 128 * 128;
+  static constexpr int SMEM = BOOKS_BYTES + WORKERS * WORKER_BYTES;
+};
+// exchange between a worker's warps, doubled by the step's parity where a fast warp may be a step ahead
+constexpr int RED_SK = 0;                        // [parity][warp] largest |S| of the keys
+constexpr int RED_SV = 32;                       // [parity][group][warp] of the values: what is not finite stays in its group
+constexpr int RED_MAX = 96;                      // [parity][warp][4] largest logit
+constexpr int RED_EX = 224, RED_FLAG = 240, RED_CA = 272;  // [parity] exponent of the keys; [parity][warp] whether there is a constant term; [parity][warp][group][4] its parts
+constexpr int RED_QS = RED_CA + 256;             // [4] logit per unit of column_sum
+constexpr int RED_END = RED_QS + 16;             // [warp][16]: constant terms of the output [group][4], sum of probabilities [4]
+constexpr int RED_BARS = RED_END + 256, BAR_KDONE = RED_BARS, BAR_KFREE = RED_BARS + 8, BAR_VDONE = RED_BARS + 16, RED_TMEM = RED_BARS + 24;
+
+// ---- tcgen05 / mbarrier wrappers
+// this lane's row of every plane's accumulator: the 8 columns of two heads
+template <int P>
+__device__ __forceinline__ void tm_ld8(uint32_t taddr, int (&c)[P][8]) {
+#define MZ_LD8(q) \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" \
+               : "=r"(c[q][0]), "=r"(c[q][1]), "=r"(c[q][2]), "=r"(c[q][3]), "=r"(c[q][4]), "=r"(c[q][5]), "=r"(c[q][6]), "=r"(c[q][7]) \
+               : "r"(taddr + 32 * (q)) : "memory")
+  MZ_LD8(0);
+  if (P > 1) MZ_LD8(P > 1 ? 1 : 0);
+  if (P > 2) MZ_LD8(P > 2 ? 2 : 0);
+#undef MZ_LD8
+  // the wait names the registers, so that nothing reads them above it
+#pragma unroll
+  for (int q = 0; q < P; ++q)
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(c[q][0]), "+r"(c[q][1]), "+r"(c[q][2]), "+r"(c[q][3]), "+r"(c[q][4]), "+r"(c[q][5]), "+r"(c[q][6]), "+r"(c[q][7]) :: "memory");
 }
-__device__ __forceinline__ void tm_ld_frag(uint32_t taddr, float (&c)[4]) {      // 16 lanes x 8 columns, mma.sync C-fragment layout
-  uint32_t r0, r1, r2, r3;
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(taddr));
-  c[0] = __uint_as_float(r0); c[1] = __uint_as_float(r1); c[2] = __uint_as_float(r2); c[3] = __uint_as_float(r3);
-}
-__device__ __forceinline__ void tm_ld_row8(uint32_t taddr, uint32_t (&v)[8]) {    // this lane's row, 8 columns
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
-}
-__device__ __forceinline__ void tm_st_row8(uint32_t taddr, const uint32_t (&v)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
-}
-__device__ __forceinline__ void tm_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tm_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tm_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void wg_barrier(int wg) { asm volatile("bar.sync %0, 128;" ::"r"(wg + 1) : "memory"); }
-
-// D[128 x 16] (+)= A[128 x 16] (TMEM) * B[16 x 16]^T (shared memory descriptor), fp16 operands, fp32 accumulate
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t accumulate) {
-  const uint32_t idesc = (1u << 4) | (2u << 17) | (8u << 24);     // D fp32; A, B fp16, K-major; N = 16; M = 128
+// among the four warps of a team
+__device__ __forceinline__ void team_barrier(int team) { asm volatile("bar.sync %0, 128;" ::"r"(team + 1) : "memory"); }
+// from a team to its issuing warp
+__device__ __forceinline__ void team_ready(int team) { asm volatile("bar.arrive %0, 160;" ::"r"(team + 7) : "memory"); }
+__device__ __forceinline__ void join_team(int team) { asm volatile("bar.sync %0, 160;" ::"r"(team + 7) : "memory"); }
+template <int N>
+__device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+  return p != 0;
+}
+// table reads: constant after the set-up, so they may be moved and merged
+__device__ __forceinline__ uint4 book128(uint32_t a) {
+  uint4 v;
+  asm("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+// shared-memory operand, not swizzled, major along the kept dimension: core matrices of 8 rows x 16 bytes, 128 bytes apart along the
+// reduction (leading offset), 2048 bytes along the kept dimension (stride offset)
+__device__ __forceinline__ uint64_t descriptor(uint32_t sa) {
+  return (uint64_t)((sa >> 4) & 0x3FFF) | (128ull >> 4) << 16 | (2048ull >> 4) << 32 | 1ull << 46;
+}
+// D[128 x 32] (+)= A[128 x 32] * B[32 x 32], 8-bit integers into 32-bit
+template <bool SIGNED_A>
+__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+  const uint32_t idesc = (2u << 4) | ((SIGNED_A ? 1u : 0u) << 7) | (1u << 10) | (1u << 15) | (1u << 16) | (4u << 17) | (8u << 24);
   const uint32_t zero = 0;
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}\n"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(zero), "r"(zero), "r"(zero), "r"(zero) : "memory");
-}
-__device__ __forceinline__ uint64_t b_descriptor(uint32_t sa, int lbo, int sbo) {
-  return (uint64_t)((sa >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) | ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(zero), "r"(zero), "r"(zero), "r"(zero) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// waits for phase `parity` of an mbarrier with a limit; false = gave up
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-  for (int it = 0; it < SPIN_LIMIT; ++it) {
+// the products of a side: its 128 rows in four slices, each plane on an accumulator of its own
+template <int BITS, int P>
+__device__ __forceinline__ void umma_side(uint32_t d_tmem, uint64_t values, uint64_t folds) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int q = 0; q < Cfg<BITS, P>::PLANES; ++q) {
+      const uint64_t a = values + ((q * PLANE_BYTES + j * 512) >> 4), b = folds + j * (512 >> 4);
+      if (q == 0) umma<true>(d_tmem, a, b, j > 0);
+      else umma<false>(d_tmem + 32 * q, a, b, j > 0);
+    }
+}
+__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(uint32_t bar) {
+  asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}\n" ::"r"(bar) : "memory");
+}
+// waits for phase `parity` of an mbarrier with a limit; `failed` is set when it gives up, and makes later waits short.  SLEEP: ns between
+// looks, for a team that is ahead anyway
+template <int SLEEP = 0>
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, bool& failed) {
+  const int limit = failed ? 1 : SPIN_LIMIT;
+  for (int it = 0; it < limit; ++it) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}\n"
                  : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done) return true;
+    if (done) return;
+    if (SLEEP > 0) __nanosleep(SLEEP);
   }
-  return false;
+  failed = true;
 }
 
-// ---- codes of one reduction block for this thread: two rows (slot 0 / 1) x four positions (4g .. 4g+3 inside the
-// warp's 32), as bytes (zc << BITS | code).  4-bit: r[0] / r[1] = even / odd positions, byte = 2*slot + (pos >> 1).
-// 2-bit: r[pos], byte = slot.
-template <int BITS>
-struct Codes4 { uint32_t r[4]; };
-template <int BITS>
-__device__ __forceinline__ Codes4<BITS> spread4(uint32_t x0, uint32_t x1, uint32_t z) {
-  Codes4<BITS> c;
-  if (BITS == 4) {
-    const uint32_t w = prmt(x0, x1, 0x5410u);              // 16 bits of row 0, 16 bits of row 1
-    c.r[0] = (w & 0x0F0F0F0Fu) | z;
-    c.r[1] = ((w >> 4) & 0x0F0F0F0Fu) | z;
-    c.r[2] = c.r[3] = 0;
-  } else {
-    const uint32_t w = prmt(x0, x1, 0x4440u);              // byte 0 = row 0, byte 1 = row 1
+// ---- books.  A row's zero code is brought to the lower half by mirroring (code -> TOP - code, S -> -S): then the side above it is the
+// larger one, its fixed-point values FULL * u are the same for every row with that zero code, and the values below are FULL * u *
+// (smaller / larger side).
+__device__ __forceinline__ float unit_value(float alpha, int e, int zc, int top) {
+  const int room = max(e >= zc ? top - zc : zc, 1), n = min(abs(e - zc), room);
+  const float grow = expm1f((float)n / (float)room * log1pf(alpha)) / alpha;
+  return e >= zc ? grow : -grow;
+}
+template <int BITS, int P>
+__device__ __forceinline__ void fill_books(uint32_t table, float alpha, int first, int n) {
+  using C = Cfg<BITS, P>;
+  for (int i = first; C::BOOKS && BITS > 1 && i < C::ZC * C::NE; i += n) {
+    const int zc = i / C::NE, e = i % C::NE;
+    const float u = C::FULL * unit_value(alpha, e, zc, C::TOP);
+    const uint32_t row = table + zc * C::BOOK_ROW;
+    stsf(row + e * 4, e < zc ? u : 0.0f);
+    stsf(row + C::NE * 4 + e * 4, e < zc ? MAGIC : MAGIC + rintf(u));
+  }
+}
+
+// constants of one row: signed scale, ratio of the smaller to the larger side, value of the zero code, mirrored zero code
+// (codes wider than 3 bits: sides are not mirrored, ratio is the lower side over the larger, zc the zero code + 2^23 as a float)
+struct Row { float s, ratio, A; uint32_t zc; };
+template <int BITS, int P, bool EXACT>
+__device__ __forceinline__ Row prepare_row(float lo, float span) {
+  constexpr int TOP = Cfg<BITS, P>::TOP;
+  Row r;
+  float bup, bdn;
+  int zc;
+  bool wild = false;       // never with 16-bit floats of 5 exponent bits
+  row_split(lo, span, (float)TOP, r.A, bup, bdn, zc, wild);
+  if (EXACT) zc = exact_zero_code(lo, span, (float)TOP);
+  if (!Cfg<BITS, P>::BOOKS) {
+    r.s = fmaxf(bup, bdn);
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r.s));
+    // the ratio of the side below zero to the one above, as one number: |ratio| <= 1 is the smaller side, its sign says which side it is
+    r.ratio = bup >= bdn ? bdn * y : -bup * y;
+    r.zc = 0x4B000000u | (uint32_t)zc;
+    return r;
+  }
+  const bool mirrored = zc > TOP / 2 && bup < INFINITY;              // an infinite range has no zero code; it stays S = inf
+  const float big = mirrored ? bdn : bup, small = mirrored ? bup : bdn;
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(big));
+  r.ratio = small * y;
+  r.s = mirrored ? -big : big;
+  r.zc = min((uint32_t)(mirrored ? TOP - zc : zc), (uint32_t)(TOP / 2));
+  return r;
+}
+// four fixed-point values (low mantissa bits) -> their bytes, plane by plane, top byte first
+template <int P>
+__device__ __forceinline__ void pack4(const uint32_t* v, uint32_t* plane) {
+  const uint32_t a = prmt(v[0], v[1], 0x5140u), b = prmt(v[2], v[3], 0x5140u);
+  plane[P - 1] = prmt(a, b, 0x5410u);
+  plane[P - 2] = prmt(a, b, 0x7632u);
+  // three planes: the third byte is 64 + the top digit; a byte of its own each, so nothing carries
+  if (P == 3) plane[0] = (prmt(prmt(v[0], v[1], 0x0062u), prmt(v[2], v[3], 0x0062u), 0x5410u) + 0x40404040u) ^ 0x80808080u;
+}
+// the alphas' constants of the arithmetic expansion, per CTA: log2(1 + alpha) and 1 / alpha
+struct Compand { float log2base, inv_alpha; };
+// expands the 64 codes of one row: `dst` is the row's 16 bytes in the first chunk of its group's half of the first plane.  The permutes
+// take their selector from the low half of a register; `two16` is 2^16 as a run-time value, so that the multiplier brings the
+// upper half down: the logic pipe is the busy one
+template <int BITS, int P, int NW>
+__device__ __forceinline__ void expand_row(const uint32_t (&w)[NW], const Row& r, uint32_t table, const Compand& cp, uint32_t dst, uint32_t two16) {
+  using C = Cfg<BITS, P>;
+  const uint32_t flip = (uint32_t)(__float_as_int(r.s) >> 31);       // mirrored rows: TOP - code is the complement
+  if constexpr (BITS == 1) {
+    // the zero code is the first (mirrored: the last) code, so a value is S times the (complemented) code
 #pragma unroll
-    for (int k = 0; k < 4; ++k) c.r[k] = ((w >> (2 * k)) & 0x0303u) | z;
+    for (int q = 0; q < 4; ++q) {
+      // 16 codes: four nibble fields of one bit; position 4 k + j of the chunk is code k + 4 j
+      const uint32_t c = (q & 1) ? __umulhi(w[q >> 1] ^ flip, two16) : w[q >> 1] ^ flip;
+      sts128(dst + q * 2048, make_uint4(prmt(0x00000100u, 0u, c & 0x1111u), prmt(0x00000100u, 0u, c >> 1 & 0x1111u),
+                                        prmt(0x00000100u, 0u, c >> 2 & 0x1111u), prmt(0x00000100u, 0u, c >> 3 & 0x1111u)));
+    }
+  } else if constexpr (C::BOOKS) {
+    const uint32_t row = table + r.zc * C::BOOK_ROW;
+    constexpr int Q = C::NE / 4;
+    uint32_t book[P][Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const uint4 t = book128(row + 16 * q), c = book128(row + C::NE * 4 + 16 * q);
+      uint32_t v[4], b[P];
+      v[0] = __float_as_uint(fmaf(__uint_as_float(t.x), r.ratio, __uint_as_float(c.x)));
+      v[1] = __float_as_uint(fmaf(__uint_as_float(t.y), r.ratio, __uint_as_float(c.y)));
+      v[2] = __float_as_uint(fmaf(__uint_as_float(t.z), r.ratio, __uint_as_float(c.z)));
+      v[3] = __float_as_uint(fmaf(__uint_as_float(t.w), r.ratio, __uint_as_float(c.w)));
+      pack4<P>(v, b);
+#pragma unroll
+      for (int k = 0; k < P; ++k) book[k][q] = b[k];
+    }
+    if constexpr (BITS == 2) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t even = (w[q] ^ flip) & 0x33333333u, odd = ((w[q] >> 2) ^ flip) & 0x33333333u;
+        const uint32_t even2 = __umulhi(even, two16), odd2 = __umulhi(odd, two16);
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+          sts128(dst + k * PLANE_BYTES + q * 2048, make_uint4(prmt(book[k][0], 0u, even), prmt(book[k][0], 0u, even2), prmt(book[k][0], 0u, odd), prmt(book[k][0], 0u, odd2)));
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t o[P][4];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          // 24 bits from bit 24 (2 q + k) on, spread to eight nibbles: the multiplier adds what has to move
+          constexpr uint32_t M12 = 0x00FFF000u, M6 = 0x0FC00FC0u, M3 = 0x38383838u;
+          const int bit = 24 * (2 * q + k), word = bit >> 5, sh = bit & 31;
+          uint32_t x = sh == 0 ? w[word] : sh <= 8 ? w[word] >> sh : __funnelshift_r(w[word], w[(word + 1) % NW], sh);
+          x = (x ^ flip) & 0x00FFFFFFu;
+          x = (x & M12) * 15u + x;
+          x = (x & M6) * 3u + x;
+          x = (x & M3) * 1u + x;
+          const uint32_t x2 = __umulhi(x, two16);
+#pragma unroll
+          for (int b = 0; b < P; ++b) { o[b][2 * k] = prmt(book[b][0], book[b][Q - 1], x); o[b][2 * k + 1] = prmt(book[b][0], book[b][Q - 1], x2); }
+        }
+#pragma unroll
+        for (int b = 0; b < P; ++b) sts128(dst + b * PLANE_BYTES + q * 2048, make_uint4(o[b][0], o[b][1], o[b][2], o[b][3]));
+      }
+    }
+  } else {
+    // value = +-side * (base^(|n| / room) - 1) / alpha, n = code - zero code; the exponent is the larger of the two sides' candidates
+    const float zc = __uint_as_float(r.zc), z = zc - 8388608.0f;
+    const float kup = __fdividef(cp.log2base, fmaxf((float)C::TOP - z, 1.0f)), kdn = __fdividef(cp.log2base, fmaxf(z, 1.0f));
+    const float big = C::FULL * cp.inv_alpha, small = big * fabsf(r.ratio);
+    const bool up = __float_as_int(r.ratio) >= 0;                       // -0 is negative
+    const float cup = up ? big : small, cdn = up ? -small : -big;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint32_t o[P][4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        uint32_t v[4], b[P];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int code = 16 * q + 4 * k + j, bit = code * BITS, word = bit >> 5, sh = bit & 31;
+          uint32_t f;                                                 // 2^23 + code as a float
+          if (BITS == 8) f = prmt(w[word], 0x4B000000u, 0x7440u | (uint32_t)j);
+          else f = ((sh + BITS <= 32 ? w[word] >> sh : __funnelshift_r(w[word], w[(word + 1) % NW], sh)) & (uint32_t)C::TOP) | 0x4B000000u;
+          const float n = __uint_as_float(f) - zc;
+          const float grow = ex2f(fmaxf(n * kup, n * -kdn)) - 1.0f;
+          v[j] = __float_as_uint(fmaf(grow, n >= 0.0f ? cup : cdn, MAGIC));
+        }
+        pack4<P>(v, b);
+#pragma unroll
+        for (int p = 0; p < P; ++p) o[p][k] = b[p];
+      }
+#pragma unroll
+      for (int b = 0; b < P; ++b) sts128(dst + b * PLANE_BYTES + q * 2048, make_uint4(o[b][0], o[b][1], o[b][2], o[b][3]));
+    }
   }
-  return c;
 }
-// table value of (slot, position 2h + r): the A-fragment register (M tile h, row half r, column half = slot)
+// position inside a 16-byte chunk of the kept dimension -> code of the row
 template <int BITS>
-__device__ __forceinline__ uint32_t look(const Codes4<BITS>& c, uint32_t lane_base, int slot, int h, int r) {
-  if (BITS == 4) return lds32(prmt(c.r[r], lane_base, 0x7604u | (uint32_t)((2 * slot + h) << 4)));
-  return lds32(prmt(c.r[2 * h + r], lane_base, 0x7604u | (uint32_t)(slot << 4)));
-}
-// zero-code bytes of slot 0 / 1 (bytes b0, b0 + 1 of zreg) in the form spread4 wants
-template <int BITS>
-__device__ __forceinline__ uint32_t zero_bytes(uint32_t zreg, int b0) {
-  if (BITS == 4) return prmt(zreg, 0u, (uint32_t)(b0 * 0x0011 + (b0 + 1) * 0x1100));   // (z0, z0, z1, z1)
-  return prmt(zreg, 0u, (uint32_t)(b0 + ((b0 + 1) << 4)) | 0x4400u);                   // (z0, z1, 0, 0)
+__device__ __forceinline__ int chunk_code(int i) {
+  if (BITS == 1) return (i >> 2) + 4 * (i & 3);
+  if (BITS > 2) return i;
+  return (i & 8) ? 2 * (i & 7) + 1 : 2 * (i & 7);
 }
 
-template <int BITS, int GQA>
-__global__ void __launch_bounds__(THREADS, 1) decode_umma_kernel(const MzDecodeParams p) {
-  constexpr int QB = G * BITS / 8;            // bytes of a packed key row (64 tokens)
+// fold value x * s, |x| <= FOLD_FULL, |s| < 1, in signed base-256 digits, low digit first.  Two planes: 2 x s rounded (24 bits) in three
+// digits, the top byte is of no use (its columns of the result are not read).  Else 2^16 x s rounded (31 bits) in four: the upper half is
+// rounded off by one magic addition, what is left by another, and the constants add up to 0x80808080.
+template <int P>
+__device__ __forceinline__ uint32_t fold_digits(float x, float s) {
+  if (P == 2) return (__float_as_uint(fmaf(x, s, MAGIC + 16448.0f)) << 1) ^ 0x00808080u;
+  constexpr float HIGH = MAGIC + 13632.0f, LOW = MAGIC + 32896.0f;
+  const float h = fmaf(x, s, HIGH), rest = fmaf(x, s, -(h - HIGH));
+  return (__float_as_uint(h) * 65536u + __float_as_uint(fmaf(rest, 65536.0f, LOW))) ^ 0x80808080u;
+}
+// a result row's accumulators of one head -> sum of value * fold in units of UNIT.  Column k of plane q counts digit k of the fold with byte
+// q of the values; products of equal weight are added, the largest three weights (and for three planes the fourth) count.
+template <int P>
+__device__ __forceinline__ float column_sum(const int (&c)[P][8], int at) {
+  const int* a = c[0] + at;
+  if (P == 1) return fmaf((float)a[3], 16777216.0f, fmaf((float)a[2], 65536.0f, (float)(a[0] + a[1] * 256)));
+  const int* b = c[P > 1 ? 1 : 0] + at;
+  if (P == 2) return fmaf((float)a[2], 65536.0f, (float)(a[0] + b[1] + 256 * (a[1] + b[2])));
+  const int* d = c[P > 2 ? 2 : 0] + at;
+  return fmaf((float)a[3], 65536.0f, (float)(a[1] + b[2] + d[3] + 256 * (a[2] + b[3]) + ((a[0] + b[1] + d[2]) >> 8)));
+}
+
+// power of two that brings a positive number of exponent field `ex` into [0.5, 1), and its inverse
+__device__ __forceinline__ float scale_down(uint32_t ex) {
+  return __uint_as_float(ex <= 252u ? (253u - max(ex, 1u)) << 23 : 0x00800000u >> (ex - 252u));
+}
+__device__ __forceinline__ float scale_up(uint32_t ex) { return __uint_as_float(min(max(ex, 1u) + 1u, 255u) << 23); }
+// exponent field of the largest magnitude of a head's query (128 elements of 16 bits)
+__device__ __forceinline__ uint32_t query_exponent(const uint16_t* q, int lane, int dtype) {
+  const uint32_t a = *((const uint32_t*)q + lane), b = *((const uint32_t*)q + 32 + lane);
+  const uint32_t mx = __reduce_max_sync(0xffffffffu, max(max(a & 0x7FFFu, a >> 16 & 0x7FFFu), max(b & 0x7FFFu, b >> 16 & 0x7FFFu)));
+  return __float_as_uint(mz_u16_to_float((uint16_t)mx, dtype)) >> 23;
+}
+
+
+struct Place { int pair, step, b, kvh; };
+
+template <int BITS, int P, int GQA, bool HALF_META>
+__global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(const MzDecodeParams p, const uint32_t two16) {
+  using C = Cfg<BITS, P>;
+  constexpr int WORKERS = C::WORKERS;
+  constexpr int QB = G * BITS / 8;            // bytes of a packed row of 64 codes
+  constexpr int NW = QB / 4;                  // words of it
   constexpr int CODE_BYTES = D * QB;          // packed bytes of one tile side
-  constexpr int VROW = 16 * BITS;             // bytes of one token's 128 value codes
-  constexpr int QUAD = BITS / 2;              // bytes holding a thread's 4 codes of one row
+  constexpr int VROW = 2 * QB;                // bytes of one token's 128 value codes
   extern __shared__ __align__(128) uint8_t smem[];
   const mz_kv_store& s = p.s;
-  const int wg = threadIdx.x >> 7, tid = threadIdx.x & 127, w = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t0 = lane & 3;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);            // uniform: the descriptors stay in uniform registers
+  const bool issuer = warp >= 8 * WORKERS;
+  const int lane = threadIdx.x & 31, w = warp & 3, team = warp >> 2, wk = issuer ? min(w, WORKERS - 1) : warp >> 3;
+  const bool keys = (team & 1) == 0;
+  const int r = w * 32 + lane;                                                    // row of the operands and of the results
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (p.hetero > 0 && (int)blockIdx.x >= p.hetero) {
+    // ================= a CTA of the residual tiles: twelve warps of its own plan =================
+    if (warp >= DENSE_WARPS) {
+      fewer_registers<24>();
+      return;
+    }
+    more_registers<DENSE_REGS>();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    mzd::dense_tiles<GQA>(p, p.tp2, p.slots_a, ((int)blockIdx.x - p.hetero) * DENSE_WARPS + warp,
+                          (uint32_t)__cvta_generic_to_shared(smem) + warp * mzd::WARP_BYTES);
+    return;
+  }
 
-  // ---- shared-memory layout of this worker (absolute shared-window addresses, sized by the planner)
-  const int msz = s.meta_dtype == MZ_F32 ? 4 : 2;
-  const uint32_t SB = p.tp.stage_bytes;
-  const uint32_t base = wg == 0 ? p.tp.low_base : p.tp.high_base + (wg - 1) * wg_bytes(SB);
-  const uint32_t kbuf0 = base, vbuf0 = base + 2 * SB;
-  const uint32_t kop = base + 4 * SB, vop = kop + KOP_BYTES;
-  const uint32_t zK = vop + VOP_BYTES, zV = zK + ZK_BYTES, pbuf = zV + ZV_BYTES;
-  const uint32_t red = pbuf + ((PB_BYTES + 127) / 128) * 128;
-  // the TMEM base address is kept right behind worker 0's block (the kernel has no static shared memory: its
-  // buffers are addressed absolutely from the start of the dynamic region)
-  const uint32_t s_tmem = p.tp.low_base + wg_bytes(SB);
-  const uint32_t r_max = red, r_ca = red + 64, r_l = red + 192, r_base = red + 256, r_q = red + 384, bar_k = red + 512, bar_v = red + 520;
-
-  if (threadIdx.x < 32) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(512));
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+  const uint32_t book = base + (keys ? 0 : C::BOOK_BYTES);
+  const uint32_t worker = base + C::BOOKS_BYTES + wk * C::WORKER_BYTES;
+  const uint32_t side = worker + (keys ? 0 : C::SIDE_BYTES), red = worker + C::OFF_RED;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(red + RED_TMEM), "r"(C::TM_ALLOC));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_k), "r"(1));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_v), "r"(1));
+  if (!issuer && keys && r == 0) {
+    bar_init(red + BAR_KDONE, 2); bar_init(red + BAR_KFREE, 4); bar_init(red + BAR_VDONE, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  fill_lookup_table<BITS>(s.alpha_key, s.alpha_value);
+  fill_books<BITS, P>(base, s.alpha_key, threadIdx.x, C::THREADS);
+  fill_books<BITS, P>(base + C::BOOK_BYTES, s.alpha_value, threadIdx.x, C::THREADS);
   tm_fence_before();
   __syncthreads();
   tm_fence_after();
-  const uint32_t tm_base = lds32(s_tmem);
-  const uint32_t tm = tm_base + wg * TM_PER_WG;      // column base of this worker (lane field 0)
-  const uint32_t tm_warp = tm + ((uint32_t)(32 * w) << 16);
+  const uint32_t tm_base = lds32(red - wk * C::WORKER_BYTES + RED_TMEM);             // kept by worker 0
+  const uint32_t tm_k = tm_base + wk * C::TM_WORKER, tm_v = tm_k + C::TM_SIDE;
 
-  const int T = p.tp.tiles_per_pair;                  // packed tiles per (batch, kv head) pair
-  const int gwg = blockIdx.x * WGS + wg;
+  const int T = p.tp.tiles_per_pair;          // steps per (batch, kv head) pair
+  const int kt = s.k_groups;
+  const int gwk = blockIdx.x * WORKERS + wk;
   long long f0 = 0, f1 = 0;
-  if (gwg < p.tp.total_warps) mz_warp_tiles(p.tp, gwg, &f0, &f1);
-
-  const uint32_t lbK = TBL + lane * 4, lbV = TBL + 128 + lane * 4;
-  const bool bf = s.kv_dtype == MZ_BF16;
-  (void)bf;
-
-  // ---- state of the current (batch, kv head) segment
-  float m_run[GQA];          // running maximum per head (base-2 logits), identical in all threads of the worker
-  float l_part = 0.f;        // sum of probabilities of this thread's tokens for head t0
-  float base_part[GQA];      // sum p * A of this thread's value rows (its channel group is tid & 1)
-  float qn[GQA];             // query of row d = tid, scaled by a power of two per head into [0.5, 1)
-  float qs[GQA];             // logit scale per head: 2^k * scaling * log2(e)
-  float qraw[GQA];           // the unscaled query values (for the constant term)
-  int cur_pair = -1, seg = 0;
-  uint32_t ph_k = 0, ph_v = 0;
-  bool v_pending = false, first_step = true, failed = false;
-#pragma unroll
-  for (int h = 0; h < GQA; ++h) { m_run[h] = -INFINITY; base_part[h] = 0.f; qn[h] = qs[h] = qraw[h] = 0.f; }
-
-  // position of a flat tile index
-  auto stage_tiles = [&](long long f, int n, bool keys) {
-    // n tiles starting at flat index f (same pair): codes + metadata of the keys (or values) into buffers 0 .. n-1
-    const int pair = (int)(f / T), tile = (int)(f % T);
-    const int b = pair / s.kv_heads, kvh = pair % s.kv_heads;
-    const uint8_t* codes = keys ? s.packed_k + b * s.pk_stride_b + kvh * s.pk_stride_h : s.packed_v + b * s.pv_stride_b + kvh * s.pv_stride_h;
-    const long long mbase = keys ? b * s.km_stride_b + kvh * s.km_stride_h : b * s.vm_stride_b + kvh * s.vm_stride_h;
-    const uint8_t* mn = (const uint8_t*)(keys ? s.k_mn : s.v_mn);
-    const uint8_t* sc = (const uint8_t*)(keys ? s.k_scale : s.v_scale);
-    for (int x = 0; x < n; ++x) {
-      const uint32_t dst = (keys ? kbuf0 : vbuf0) + x * SB;
-      const uint8_t* src = codes + (long long)(tile + x) * CODE_BYTES;
-      for (int i = tid; i < CODE_BYTES / 16; i += 128) {
-        // 4-bit values: a token's row is 64 bytes; its two 32-byte halves are swapped for tokens with bit 1 set so
-        // that the four tokens one load instruction touches fall into different banks
-        const int di = (!keys && BITS == 4) ? (i ^ ((i >> 2) & 2)) : i;
-        cp16(dst + di * 16, src + i * 16);
-      }
-      const long long m0 = (mbase + (long long)(tile + x) * D) * msz;
-      for (int off = tid * 16; off < D * msz; off += 128 * 16) {
-        cp16(dst + CODE_BYTES + off, mn + m0 + off);
-        cp16(dst + CODE_BYTES + D * msz + off, sc + m0 + off);
-      }
+  if (gwk < p.tp.total_warps) mz_warp_tiles(p.tp, gwk, &f0, &f1);
+  const int steps = (int)(f1 - f0);
+  Place cur;
+  cur.pair = (int)((unsigned)f0 / (unsigned)T); cur.step = (int)((unsigned)f0 % (unsigned)T);
+  cur.b = cur.pair / s.kv_heads; cur.kvh = cur.pair % s.kv_heads;
+  auto advance = [&](Place& c) {
+    if (++c.step == T) {
+      c.step = 0; ++c.pair;
+      if (++c.kvh == s.kv_heads) { c.kvh = 0; ++c.b; }
     }
   };
-  auto tiles_of_step = [&](long long f) -> int {       // two tiles when the next one is in the same pair and in range
-    return (f + 1 < f1 && (int)((f + 1) % T) != 0) ? 2 : 1;
+  bool failed = false;
+  Compand compand;
+  compand.inv_alpha = 1.0f / (keys ? s.alpha_key : s.alpha_value);
+  compand.log2base = log1pf(keys ? s.alpha_key : s.alpha_value) * LOG2E;
+  const bool meta32 = s.meta_dtype == MZ_F32;
+  // everything above reads kernel parameters only and may run while the grid before drains
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  // rows in flight, one of either group: codes and metadata as loaded (16-bit metadata in the low half)
+  uint32_t code[2][NW], lo[2], span[2];
+  const int half = r >> 6;                                            // values: group of this thread's token; also of its row of the results
+  const int spot = (r & 0x70) + chunk_code<BITS>(r & 15);             // values: its token of a step, and its channel of the output
+  // Keys: channel r of the step's two groups (a last half step reads its group twice); values: token `spot` with its two channel groups (in a
+  // last half step the tokens of the first group twice, the second time with probability zero).
+  // The cursor of the loads runs ahead: pointers of the step `ahead`, advanced with it.
+  Place ahead = cur;
+  const int msz = HALF_META ? 2 : meta32 ? 4 : 2;
+  const uint8_t *code_at, *mn_at, *span_at;
+  auto point = [&]() {
+    const long long tile = STEP_GROUPS * ahead.step;
+    const long long row = keys ? r : half * G + (spot & 63);
+    const long long m = keys ? ahead.b * s.km_stride_b + ahead.kvh * s.km_stride_h + tile * D + row : ahead.b * s.vm_stride_b + ahead.kvh * s.vm_stride_h + (tile * G + row) * 2;
+    code_at = keys ? s.packed_k + ahead.b * s.pk_stride_b + ahead.kvh * s.pk_stride_h + tile * CODE_BYTES + row * QB
+                   : s.packed_v + ahead.b * s.pv_stride_b + ahead.kvh * s.pv_stride_h + (tile * G + row) * VROW;
+    mn_at = (const uint8_t*)(keys ? s.k_mn : s.v_mn) + m * msz;
+    span_at = (const uint8_t*)(keys ? s.k_scale : s.v_scale) + m * msz;
   };
-  auto meta_at = [&](uint32_t buf, int r, float& lo, float& span) {
-    if (msz == 4) {
-      lo = ldsf(buf + CODE_BYTES + r * 4);
-      span = ldsf(buf + CODE_BYTES + D * 4 + r * 4);
+  auto move_ahead = [&]() {
+    if (++ahead.step == T) {
+      ahead.step = 0; ++ahead.pair;
+      if (++ahead.kvh == s.kv_heads) { ahead.kvh = 0; ++ahead.b; }
+      point();
     } else {
-      lo = mz_u16_to_float((uint16_t)lds16(buf + CODE_BYTES + r * 2), s.meta_dtype);
-      span = mz_u16_to_float((uint16_t)lds16(buf + CODE_BYTES + D * 2 + r * 2), s.meta_dtype);
+      code_at += STEP_GROUPS * CODE_BYTES;
+      mn_at += STEP_GROUPS * D * msz;
+      span_at += STEP_GROUPS * D * msz;
+    }
+  };
+  // bytes (codes) / elements (metadata) from the first row's to this thread's row of either group
+  const int x_codes = keys ? CODE_BYTES : QB, x_meta = keys ? D : 1;
+  const uint8_t* code_next;                                           // codes of the step that comes next
+  int code_second;
+  auto load_meta = [&]() {                                            // and keeps where the codes are
+    int back = 0, second = x_meta;                                    // tokens back from the first row, elements on to the second
+    code_next = code_at; code_second = x_codes;
+    if (STEP_GROUPS * ahead.step + 1 >= kt) {                         // a last half step
+      if (keys) second = code_second = 0;
+      else if (half) back = -G;
+      code_next += back * VROW;
+    }
+    const uint8_t* a = mn_at + back * 2 * msz;
+    const uint8_t* b = span_at + back * 2 * msz;
+    if (HALF_META || !meta32) {
+      lo[0] = __ldg((const uint16_t*)a); lo[1] = __ldg((const uint16_t*)a + second);
+      span[0] = __ldg((const uint16_t*)b); span[1] = __ldg((const uint16_t*)b + second);
+    } else {
+      lo[0] = __ldg((const uint32_t*)a); lo[1] = __ldg((const uint32_t*)a + second);
+      span[0] = __ldg((const uint32_t*)b); span[1] = __ldg((const uint32_t*)b + second);
+    }
+  };
+  auto load_codes = [&](int x) {
+    if constexpr (QB % 16 == 0) {
+      const uint4* src = (const uint4*)(code_next + (x ? code_second : 0));
+#pragma unroll
+      for (int i = 0; i < NW / 4; ++i) {
+        const uint4 v = __ldg(src + i);
+        code[x][4 * i] = v.x; code[x][4 * i + 1] = v.y; code[x][4 * i + 2] = v.z; code[x][4 * i + 3] = v.w;
+      }
+    } else {
+      const uint2* src = (const uint2*)(code_next + (x ? code_second : 0));
+#pragma unroll
+      for (int i = 0; i < NW / 2; ++i) {
+        const uint2 v = __ldg(src + i);
+        code[x][2 * i] = v.x; code[x][2 * i + 1] = v.y;
+      }
+    }
+  };
+  Row rows[2];
+  // row constants from the metadata in flight
+  auto prepare = [&]() {
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+      rows[x] = HALF_META ? prepare_row<BITS, P, false>(mz_u16_to_float((uint16_t)lo[x], MZ_F16), mz_u16_to_float((uint16_t)span[x], MZ_F16))
+                : meta32  ? prepare_row<BITS, P, true>(__uint_as_float(lo[x]), __uint_as_float(span[x]))
+                          : prepare_row<BITS, P, true>(mz_u16_to_float((uint16_t)lo[x], s.meta_dtype), mz_u16_to_float((uint16_t)span[x], s.meta_dtype));
+  };
+  auto magnitude = [&](int x) { return __float_as_uint(rows[x].s) & 0x7FFFFFFFu; };
+  // the largest of a side: per warp here, over the four warps behind the next barrier
+  auto publish_largest = [&](uint32_t at, uint32_t v) {
+    v = __reduce_max_sync(0xffffffffu, v);
+    if (lane == 0) sts32(at + 4 * w, v);
+  };
+  auto exponent_of_largest = [&](uint32_t at) {
+    const uint4 v = lds128(at);
+    return max(max(v.x, v.y), max(v.z, v.w)) >> 23;
+  };
+  auto put_folds = [&](const float (&x)[GQA], float down0, float down1) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float sx = rows[k].s * (k ? down1 : down0);
+      uint32_t d[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int g = 0; g < GQA; ++g) d[g] = fold_digits<P>(x[g], sx);
+      sts128(side + C::OFF_FOLD + k * 2048 + r * 16, make_uint4(d[0], d[1], d[2], d[3]));
     }
   };
 
-  // ---- end of a segment: the partial record (m, l, acc) of this worker for the pair it just left
-  auto write_partial = [&]() {
-    if (v_pending) { failed |= !bar_wait(bar_v, ph_v); ph_v ^= 1; v_pending = false; }
-    tm_fence_after();
-    // l: over the g lanes of a warp, then over the warps
-    float lsum = l_part;
-#pragma unroll
-    for (int off = 4; off < 32; off <<= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
-    if (g == 0 && t0 < GQA) stsf(r_l + (w * 4 + t0) * 4, lsum);
-    // constant term of the values: over the lanes of the same channel group (lane parity), then over the warps
-#pragma unroll
-    for (int h = 0; h < GQA; ++h) {
-      float bsum = base_part[h];
-#pragma unroll
-      for (int off = 2; off < 32; off <<= 1) bsum += __shfl_xor_sync(0xffffffffu, bsum, off);
-      if (lane < 2) stsf(r_base + ((w * 2 + lane) * 4 + h) * 4, bsum);
-    }
-    wg_barrier(wg);
-    const int grp = w >> 1;
-    uint32_t v[8];
-    tm_ld_row8(tm_warp + TM_O + 8 * grp, v);
-    tm_wait_ld();
-    // TMEM lane 16h' + 8r + g' of this warp holds channel 32w + 4g' + 2h' + r
-    const int chan = 32 * w + 4 * (lane & 7) + 2 * (lane >> 4) + ((lane >> 3) & 1);
-    const long long slot0 = ((long long)gwg * p.tp.max_segs + seg) * GQA;
-    const bool in_range = MZ_IN_BOUNDS(slot0 + GQA - 1, p.part.slots, 12);   // always true outside the checked build
-#pragma unroll
-    for (int h = 0; h < GQA && in_range; ++h) {
-      const float bs = ldsf(r_base + ((0 * 2 + grp) * 4 + h) * 4) + ldsf(r_base + ((1 * 2 + grp) * 4 + h) * 4) +
-                       ldsf(r_base + ((2 * 2 + grp) * 4 + h) * 4) + ldsf(r_base + ((3 * 2 + grp) * 4 + h) * 4);
-      p.part.acc[(slot0 + h) * D + chan] = __uint_as_float(v[2 * h]) + __uint_as_float(v[2 * h + 1]) + bs;
-    }
-    if (tid < GQA && in_range) {
-      const float lt = ldsf(r_l + (0 * 4 + tid) * 4) + ldsf(r_l + (1 * 4 + tid) * 4) + ldsf(r_l + (2 * 4 + tid) * 4) + ldsf(r_l + (3 * 4 + tid) * 4);
-      float mv = -INFINITY;
-#pragma unroll
-      for (int h = 0; h < GQA; ++h) if (h == tid) mv = m_run[h];
-      p.part.m[slot0 + tid] = failed ? INFINITY : mv * (1.0f / LOG2E);   // a wait ran out: +inf turns the merged output into NaN
-      p.part.l[slot0 + tid] = lt;
-    }
-    tm_fence_before();
-    wg_barrier(wg);
-  };
-
-  if (f0 < f1) {
-    long long f = f0;
-    int n_cur = tiles_of_step(f);
-    stage_tiles(f, n_cur, true);
-    cp_async_commit();
-    stage_tiles(f, n_cur, false);
-    cp_async_commit();
-    while (f < f1) {
-      const int ntile = n_cur;
-      const int pair = (int)(f / T), tile = (int)(f % T);
-      const int b = pair / s.kv_heads, kvh = pair % s.kv_heads;
-      const long long fn = f + ntile;
-      const int n_next = fn < f1 ? tiles_of_step(fn) : 0;
-      if (pair != cur_pair) {
-        if (cur_pair >= 0) { write_partial(); ++seg; }
-        cur_pair = pair;
-        first_step = true;
-        l_part = 0.f;
-#pragma unroll
-        for (int h = 0; h < GQA; ++h) { m_run[h] = -INFINITY; base_part[h] = 0.f; }
-        // query of row d = tid for every head; per head a power of two brings max |q| into [0.5, 1) so that the
-        // folded query fits fp16 whatever the row constants (<= 65504) are
-        float amax[GQA];
-#pragma unroll
-        for (int h = 0; h < GQA; ++h) {
-          qraw[h] = mz_load_as_float(p.query, b * p.q_stride_b + (long long)(kvh * GQA + h) * p.q_stride_h + tid, s.kv_dtype);
-          amax[h] = fabsf(qraw[h]);
-#pragma unroll
-          for (int off = 1; off < 32; off <<= 1) amax[h] = fmaxf(amax[h], __shfl_xor_sync(0xffffffffu, amax[h], off));
-          if (lane == 0) stsf(r_q + (w * 4 + h) * 4, amax[h]);
+  if (issuer) {
+    // ================= the issuing warps: keys of step i + 1, then values of step i =================
+    fewer_registers<C::ISSUE>();
+    if (w < WORKERS) {
+      const uint64_t key_values = descriptor(worker), key_folds = descriptor(worker + C::OFF_FOLD);
+      const uint64_t value_values = descriptor(worker + C::SIDE_BYTES), value_folds = descriptor(worker + C::SIDE_BYTES + C::OFF_FOLD);
+      for (int i = -1; i < steps; ++i) {
+        if (i + 1 < steps) {
+          join_team(2 * wk);
+          if (i >= 0) bar_wait(red + BAR_KFREE, (uint32_t)i & 1, failed);        // the logits before have been read
+          tm_fence_after();
+          if (elect_one()) {
+            bar_arrive(red + BAR_KDONE);                              // hands on what the team has noted
+            umma_side<BITS, P>(tm_k, key_values, key_folds);
+            umma_commit(red + BAR_KDONE);
+          }
+          __syncwarp();
         }
-        wg_barrier(wg);
-#pragma unroll
-        for (int h = 0; h < GQA; ++h) {
-          const float am = fmaxf(fmaxf(ldsf(r_q + h * 4), ldsf(r_q + (4 + h) * 4)), fmaxf(ldsf(r_q + (8 + h) * 4), ldsf(r_q + (12 + h) * 4)));
-          int ex = (__float_as_int(am) >> 23) & 0xff;
-          ex = min(max(ex, 1), 253);
-          qn[h] = qraw[h] * __int_as_float((253 - ex) << 23);
-          qs[h] = __int_as_float((ex + 1) << 23) * p.scaling * LOG2E;
+        if (i >= 0) {
+          join_team(2 * wk + 1);
+          tm_fence_after();
+          if (elect_one()) {
+            umma_side<BITS, P>(tm_v, value_values, value_folds);
+            umma_commit(red + BAR_VDONE);
+          }
+          __syncwarp();
         }
       }
-      // ================= keys: row constants and folded query of row d = tid of each tile =================
-      cp_async_wait<1>();                     // this step's key tiles have landed (the value tiles may still be in flight)
-      wg_barrier(wg);
-      {
-        float ca[2][GQA];
-        bool any = false;
+    }
+  } else if (keys) {
+    fewer_registers<C::KEY>();
+    if (steps > 0) {
+    // ================= keys: channel r of the step's groups, one step ahead of the values =================
+    float qn[GQA];                                                    // query of this channel, scaled per head into (-C::FOLD_FULL, C::FOLD_FULL)
+    int q_pair = -1;
+    point();
+    load_meta();
+    load_codes(0);
+    load_codes(1);
+    prepare();
+    publish_largest(red + RED_SK, max(magnitude(0), magnitude(1)));
+    if (steps > 1) { move_ahead(); load_meta(); }
+    team_barrier(team);
+    for (int i = 0; i < steps; ++i) {
+      const int par = i & 1;
+      const bool more = i + 1 < steps;
+      if (cur.pair != q_pair) {
+        q_pair = cur.pair;
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
+        for (int g = 0; g < GQA; ++g) {
+          const uint16_t* q = (const uint16_t*)p.query + cur.b * p.q_stride_b + (long long)(cur.kvh * GQA + g) * p.q_stride_h;
+          qn[g] = mz_u16_to_float(q[r], s.kv_dtype) * (scale_down(query_exponent(q, lane, s.kv_dtype)) * C::FOLD_FULL);
+        }
+      }
+      const uint32_t ex = exponent_of_largest(red + RED_SK + 16 * par);
+      if (i > 0) bar_wait<64>(red + BAR_KDONE, (uint32_t)(i - 1) & 1, failed);       // the operands have been read
+      expand_row<BITS, P, NW>(code[0], rows[0], book, compand, side + r * 16, two16);
+      if (more) load_codes(0);
+      expand_row<BITS, P, NW>(code[1], rows[1], book, compand, side + 8192 + r * 16, two16);
+      if (more) load_codes(1);
+      const float down = scale_down(ex);
+      put_folds(qn, down, down);
+      // constant term sum_d q[h][d] A_d per group and head (rows whose range does not straddle zero): this warp's part
+      const bool any = __any_sync(0xffffffffu, rows[0].A != 0.0f || rows[1].A != 0.0f);
+      if (any) {
 #pragma unroll
-          for (int h = 0; h < GQA; ++h) ca[x][h] = 0.f;
-          if (x < ntile) {
-            float lo, span, A, Bup, Bdn;
-            int zc;
-            meta_at(kbuf0 + x * SB, tid, lo, span);
-            row_constants<BITS>(lo, span, zc, A, Bup, Bdn);
-            sts8(zK + x * 128 + (tid & 3) * 32 + (tid >> 2), (uint32_t)(zc << BITS));
-            any |= A != 0.0f;
-            const uint32_t dst = kop + (tid >> 3) * KOP_BLOCK + ((tid >> 2) & 1) * KOP_LBO + x * KOP_SBO + (tid & 3) * 4;
+        for (int x = 0; x < 2; ++x)
 #pragma unroll
-            for (int h = 0; h < GQA; ++h) {
-              const float wu = qn[h] * Bup, wd = qn[h] * Bdn;
-              const __half2 hi = __floats2half2_rn(wu, wd);
-              const float2 hf = __half22float2(hi);
-              sts32(dst + (2 * h) * 16, h2_bits(hi));
-              sts32(dst + (2 * h + 1) * 16, h2_bits(__floats2half2_rn(wu - hf.x, wd - hf.y)));
-              ca[x][h] = qraw[h] * A;
-            }
+          for (int g = 0; g < GQA; ++g) {
+            float v = qn[g] * rows[x].A;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+            if (lane == 0) stsf(red + RED_CA + par * 128 + ((w * 2 + x) * 4 + g) * 4, v);
+          }
+      }
+      if (lane == 0) {
+        sts32(red + RED_FLAG + par * 16 + 4 * w, any ? 1u : 0u);
+        if (w == 0) sts32(red + RED_EX + 4 * par, ex);
+      }
+      if (more) {
+        prepare();
+        publish_largest(red + RED_SK + 16 * (par ^ 1), max(magnitude(0), magnitude(1)));
+      }
+      advance(cur);
+      if (i + 2 < steps) { move_ahead(); load_meta(); }
+      proxy_fence();
+      team_ready(team);
+      team_barrier(team);
+    }
+    }
+  } else {
+    more_registers<C::VALUE>();
+    if (steps > 0) {
+    // ================= softmax and values: thread r has row r of the results =================
+    const uint32_t tm_mine = ((uint32_t)(32 * w) << 16) + 16 * half;
+    float m_run[GQA], l_part[GQA], out[GQA];                          // running maximum (base-2 logits), this thread's sum of probabilities, output
+    float base_sum = 0.f;                                             // lane 4 x + g: sum p * A of the warp's tokens, channel group x and head g
+    bool has_base = false;
+    float up_v = 0.f;
+    int seg = 0;
+    auto start_pair = [&](const Place& c) {
+#pragma unroll
+      for (int g = 0; g < GQA; ++g) {
+        m_run[g] = -INFINITY; l_part[g] = out[g] = 0.f;
+        const uint16_t* q = (const uint16_t*)p.query + c.b * p.q_stride_b + (long long)(c.kvh * GQA + g) * p.q_stride_h;
+        const uint32_t ex = query_exponent(q, lane, s.kv_dtype);
+        if (r == 0) stsf(red + RED_QS + 4 * g, scale_up(ex) * p.scaling * (LOG2E * C::UNIT));     // read behind the next barrier but one
+      }
+      base_sum = 0.f; has_base = false;
+      team_barrier(team);
+    };
+    // adds the products of step v's values to the output
+    auto drain = [&](int v) {
+      bar_wait(red + BAR_VDONE, (uint32_t)v & 1, failed);
+      tm_fence_after();
+#pragma unroll
+      for (int g = 0; g < GQA; g += 2) {
+        int c[P][8];
+        tm_ld8<P>(tm_v + tm_mine + 4 * g, c);
+        out[g] = fmaf(column_sum<P>(c, 0), up_v, out[g]);
+        if (g + 1 < GQA) out[(g + 1) % GQA] = fmaf(column_sum<P>(c, 4), up_v, out[(g + 1) % GQA]);
+      }
+      tm_fence_before();
+    };
+    // ---- end of a segment: the partial record (m, l, acc) of this worker for the pair it just left
+    auto write_partial = [&]() {
+#pragma unroll
+      for (int g = 0; g < GQA; ++g) {
+        float lsum = l_part[g];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
+        if (lane == 0) stsf(red + RED_END + w * 64 + 32 + 4 * g, lsum);
+      }
+      if (lane < 8) stsf(red + RED_END + w * 64 + 4 * lane, base_sum);
+      team_barrier(team);
+      const long long slot0 = ((long long)gwk * p.tp.max_segs + seg) * GQA;
+      if (MZ_IN_BOUNDS(slot0 + GQA - 1, p.part.slots, 12)) {          // always true outside the checked build
+#pragma unroll
+        for (int g = 0; g < GQA; ++g) {
+          float bs = 0.f, lt = 0.f;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            bs += ldsf(red + RED_END + k * 64 + 16 * half + 4 * g);
+            lt += ldsf(red + RED_END + k * 64 + 32 + 4 * g);
+          }
+          p.part.acc[(slot0 + g) * D + spot] = out[g] + bs;
+          if (r == 0) {
+            p.part.m[slot0 + g] = failed ? INFINITY : m_run[g] * (1.0f / LOG2E);   // a wait ran out: +inf turns the merged output into NaN
+            p.part.l[slot0 + g] = lt;
           }
         }
-        // constant term sum_d q[h][d] A_d per tile and head (rows whose range does not straddle zero)
-        if (__any_sync(0xffffffffu, any)) {
+      }
+      team_barrier(team);
+    };
+    point();
+    load_meta();
+    load_codes(0);
+    load_codes(1);
+    start_pair(cur);
+    bool pending = false;                                             // the last step's values are not in the output yet
+    for (int i = 0; i < steps; ++i) {
+      const int par = i & 1;
+      Place nxt = cur;
+      advance(nxt);
+      prepare();
+      publish_largest(red + RED_SV + 32 * par, magnitude(0));
+      publish_largest(red + RED_SV + 32 * par + 16, magnitude(1));
+      const bool more = i + 1 < steps;
+      if (more) { move_ahead(); load_meta(); }
+      const bool live = STEP_GROUPS * cur.step + half < kt;
+      float mask = 0.f;
+      if (p.mask && live)
+        mask = mz_load_as_float(p.mask, cur.b * p.mask_stride_b + (long long)cur.step * (STEP_GROUPS * G) + spot, p.mask_dtype) * LOG2E;
+      // ================= logits of token `spot` =================
+      bar_wait(red + BAR_KDONE, (uint32_t)par, failed);
+      tm_fence_after();
+      float lg[GQA];
+      {
+#pragma unroll
+        for (int g = 0; g < GQA; g += 2) {
+          int c[P][8];
+          tm_ld8<P>(tm_k + tm_mine + 4 * g, c);
+          lg[g] = column_sum<P>(c, 0);
+          if (g + 1 < GQA) lg[(g + 1) % GQA] = column_sum<P>(c, 4);
+        }
+        const float up_k = scale_up(lds32(red + RED_EX + 4 * par));
+        const uint4 fl = lds128(red + RED_FLAG + 16 * par);
+        float ca[GQA];
+#pragma unroll
+        for (int g = 0; g < GQA; ++g) ca[g] = 0.f;
+        if (fl.x | fl.y | fl.z | fl.w) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const bool on = (k == 0 ? fl.x : k == 1 ? fl.y : k == 2 ? fl.z : fl.w) != 0;
+#pragma unroll
+            for (int g = 0; g < GQA; ++g) ca[g] += on ? ldsf(red + RED_CA + par * 128 + ((k * 2 + half) * 4 + g) * 4) : 0.f;
+          }
+        }
+        tm_fence_before();
+        __syncwarp();
+        if (lane == 0) bar_arrive(red + BAR_KFREE);
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        const uint4 qs = lds128(red + RED_QS);
+#pragma unroll
+        for (int g = 0; g < GQA; ++g) {
+          const float v = fmaf(lg[g], up_k, ca[g] * (1.0f / (C::FOLD_FULL * C::UNIT)));
+          lg[g] = live ? fmaf(v, __uint_as_float(g == 0 ? qs.x : g == 1 ? qs.y : g == 2 ? qs.z : qs.w), mask) : -INFINITY;
+          asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(mx[g]) : "f"(lg[g]));
+        }
+        if (lane == 0) sts128(red + RED_MAX + par * 64 + w * 16, make_uint4(__float_as_uint(mx[0]), __float_as_uint(mx[1]), __float_as_uint(mx[2]), __float_as_uint(mx[3])));
+      }
+      team_barrier(team);
+      if (pending) drain(i - 1);                                      // and its operands have been read
+      // ================= softmax =================
+      {
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint4 a = lds128(red + RED_MAX + par * 64 + k * 16);
+          mx[0] = fmaxf(mx[0], __uint_as_float(a.x)); mx[1] = fmaxf(mx[1], __uint_as_float(a.y));
+          mx[2] = fmaxf(mx[2], __uint_as_float(a.z)); mx[3] = fmaxf(mx[3], __uint_as_float(a.w));
+        }
+#pragma unroll
+        for (int g = 0; g < GQA; ++g) {
+          const float m_new = fmaxf(m_run[g], mx[g]);
+          const float top = fmaxf(m_new, -3.0e38f);                  // -inf as long as every token is masked: then the probabilities are 0
+          const float c = ex2f(m_run[g] - top);
+          m_run[g] = m_new;
+          lg[g] = ex2f(lg[g] - top);
+          l_part[g] = fmaf(l_part[g], c, lg[g]);
+          out[g] *= c;
+          if (has_base && (lane & 3) == g) base_sum *= c;
+        }
+        // constant terms of the output (rows whose range does not straddle zero)
+        has_base |= __any_sync(0xffffffffu, rows[0].A != 0.0f || rows[1].A != 0.0f);
+        if (has_base) {
 #pragma unroll
           for (int x = 0; x < 2; ++x)
 #pragma unroll
-            for (int h = 0; h < GQA; ++h) {
-              float v = ca[x][h];
+            for (int g = 0; g < GQA; ++g) {
+              float v = lg[g] * rows[x].A;
 #pragma unroll
               for (int off = 1; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-              if (lane == 0) stsf(r_ca + ((w * 2 + x) * 4 + h) * 4, v);
+              if (lane == 4 * x + g) base_sum += v;
             }
-        } else if (lane < 2 * GQA) {
-          stsf(r_ca + ((w * 2 + lane / GQA) * 4 + lane % GQA) * 4, 0.f);
         }
+#pragma unroll
+        for (int g = 0; g < GQA; ++g) lg[g] *= C::FOLD_FULL;
       }
+      // ================= values: token `spot`, its two channel groups =================
+      const uint32_t ex0 = exponent_of_largest(red + RED_SV + 32 * par), ex1 = exponent_of_largest(red + RED_SV + 32 * par + 16);
+      up_v = scale_up(half ? ex1 : ex0) * C::UNIT;
+      put_folds(lg, scale_down(ex0), scale_down(ex1));
+      expand_row<BITS, P, NW>(code[0], rows[0], book, compand, side + r * 16, two16);
+      if (more) load_codes(0);
+      expand_row<BITS, P, NW>(code[1], rows[1], book, compand, side + 8192 + r * 16, two16);
+      if (more) load_codes(1);
       proxy_fence();
-      if (v_pending) { failed |= !bar_wait(bar_v, ph_v); ph_v ^= 1; v_pending = false; }   // the A operand region is free again
-      tm_fence_after();
-      wg_barrier(wg);
-      // ================= keys: table values of this warp's 32 tokens -> A operand =================
-      {
-        const int x = w >> 1, wh = w & 1;            // tile and half of the tile this warp covers
-        if (x < ntile) {
-          uint32_t zr[8];
-          {
-            const uint4 za = lds128(zK + x * 128 + t0 * 32), zb = lds128(zK + x * 128 + t0 * 32 + 16);
-            zr[0] = za.x; zr[1] = za.y; zr[2] = za.z; zr[3] = za.w; zr[4] = zb.x; zr[5] = zb.y; zr[6] = zb.z; zr[7] = zb.w;
-          }
-          const uint32_t kb = kbuf0 + x * SB + 4 * BITS * wh + QUAD * g;
-          auto load_codes = [&](int j, uint32_t& x0, uint32_t& x1) {
-            if (BITS == 4) { x0 = lds16(kb + (8 * j + t0) * QB); x1 = lds16(kb + (8 * j + 4 + t0) * QB); }
-            else { x0 = lds8(kb + (8 * j + t0) * QB); x1 = lds8(kb + (8 * j + 4 + t0) * QB); }
-          };
-          uint32_t c0, c1, n0 = 0, n1 = 0;
-          load_codes(0, c0, c1);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            if (j + 1 < 16) load_codes(j + 1, n0, n1);
-            const Codes4<BITS> c = spread4<BITS>(c0, c1, zero_bytes<BITS>(zr[j >> 1], 2 * (j & 1)));
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-              tm_st4(tm_warp + ((uint32_t)(16 * h) << 16) + TM_A + 8 * j, look<BITS>(c, lbK, 0, h, 0), look<BITS>(c, lbK, 0, h, 1),
-                     look<BITS>(c, lbK, 1, h, 0), look<BITS>(c, lbK, 1, h, 1));
-            c0 = n0; c1 = n1;
-          }
-        }
-      }
-      tm_wait_st();
-      cp_async_wait<0>();                     // this step's value tiles have landed
       tm_fence_before();
-      wg_barrier(wg);
-      if (tid == 0) {
-        tm_fence_after();
-#pragma unroll 1
-        for (int j = 0; j < 16; ++j) umma(tm + TM_L, tm + TM_A + 8 * j, b_descriptor(kop + j * KOP_BLOCK, KOP_LBO, KOP_SBO), j > 0);
-        umma_commit(bar_k);
+      team_ready(team);
+      pending = true;
+      if (!more || nxt.pair != cur.pair) {
+        drain(i);
+        write_partial();
+        ++seg;
+        pending = false;
+        if (more) start_pair(nxt);
       }
-      if (n_next > 0) stage_tiles(fn, n_next, true);
-      cp_async_commit();
-      // ================= values: row constants of row (token, group) = (tid / 2, tid % 2) of each tile =================
-      float vA[2], vBu[2], vBd[2];
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        vA[x] = vBu[x] = vBd[x] = 0.f;
-        if (x < ntile) {
-          float lo, span;
-          int zc;
-          meta_at(vbuf0 + x * SB, tid, lo, span);
-          row_constants<BITS>(lo, span, zc, vA[x], vBu[x], vBd[x]);
-          const int tok = tid >> 1;
-          sts8(zV + x * 128 + (tid & 1) * 64 + (tok & 3) * 16 + (tok >> 2), (uint32_t)(zc << BITS));
-        }
-      }
-      // ================= logits of this warp's 32 tokens, softmax across the worker =================
-      failed |= !bar_wait(bar_k, ph_k);
-      ph_k ^= 1;
-      tm_fence_after();
-      float sv[4];                            // head t0; positions 2h + r of the thread's four tokens
-      {
-        const int x = w >> 1;
-        if (x < ntile) {
-          float c[2][4];
-          tm_ld_frag(tm_warp + TM_L + 8 * x, c[0]);
-          tm_ld_frag(tm_warp + ((uint32_t)16 << 16) + TM_L + 8 * x, c[1]);
-          tm_wait_ld();
-          float q_scale = 0.f;
-#pragma unroll
-          for (int h = 0; h < GQA; ++h) if (h == t0) q_scale = qs[h];
-          const float cterm = t0 < GQA ? (ldsf(r_ca + ((0 * 2 + x) * 4 + t0) * 4) + ldsf(r_ca + ((1 * 2 + x) * 4 + t0) * 4) +
-                                          ldsf(r_ca + ((2 * 2 + x) * 4 + t0) * 4) + ldsf(r_ca + ((3 * 2 + x) * 4 + t0) * 4)) * p.scaling * LOG2E
-                                       : 0.f;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            sv[2 * h] = fmaf(c[h][0] + c[h][1], q_scale, cterm);
-            sv[2 * h + 1] = fmaf(c[h][2] + c[h][3], q_scale, cterm);
-          }
-          if (p.mask) {
-            const long long m0 = b * p.mask_stride_b + (long long)(tile + x) * G + 32 * (w & 1) + 4 * g;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) sv[i] += mz_load_as_float(p.mask, m0 + i, p.mask_dtype) * LOG2E;
-          }
-        } else {
-          sv[0] = sv[1] = sv[2] = sv[3] = -INFINITY;
-        }
-        float mx = fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]));
-#pragma unroll
-        for (int off = 4; off < 32; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        if (g == 0) stsf(r_max + (w * 4 + t0) * 4, mx);
-      }
-      tm_fence_before();
-      wg_barrier(wg);
-      float corr[GQA];
-      bool grow = false;
-#pragma unroll
-      for (int h = 0; h < GQA; ++h) {
-        const float mx = fmaxf(fmaxf(ldsf(r_max + h * 4), ldsf(r_max + (4 + h) * 4)), fmaxf(ldsf(r_max + (8 + h) * 4), ldsf(r_max + (12 + h) * 4)));
-        const float m_new = fmaxf(m_run[h], mx);
-        corr[h] = (m_new > -INFINITY) ? ex2f(m_run[h] - m_new) : 1.0f;     // m_run = -inf -> 0
-        grow |= m_new > m_run[h];
-        m_run[h] = m_new;
-      }
-      {
-        float m_mine = -INFINITY, c_mine = 1.0f;
-#pragma unroll
-        for (int h = 0; h < GQA; ++h) if (h == t0) { m_mine = m_run[h]; c_mine = corr[h]; }
-        const bool dead = !(m_mine > -INFINITY);
-        float sum = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          sv[i] = dead ? 0.f : ex2f(sv[i] - m_mine);
-          sum += sv[i];
-        }
-        l_part = l_part * c_mine + sum;
-        const int x = w >> 1;
-        if (t0 < GQA && x < ntile) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) stsf(pbuf + ((x * 4 + t0) * PB_HEAD + 32 * (w & 1) + 4 * g + i) * 4, sv[i]);
-        }
-      }
-      // the output so far belongs to the old maxima: rescale it in place (all earlier value MMAs have completed: the
-      // wait before the key lookups).  Nothing to do in the first step of a segment, where the accumulator is unset.
-      if (grow && !first_step) {
-        tm_fence_after();
-        uint32_t v[8];
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          tm_ld_row8(tm_warp + TM_O + 8 * half, v);
-          tm_wait_ld();
-#pragma unroll
-          for (int c = 0; c < 8; ++c) v[c] = c / 2 < GQA ? __float_as_uint(__uint_as_float(v[c]) * corr[c / 2 < GQA ? c / 2 : 0]) : v[c];
-          tm_st_row8(tm_warp + TM_O + 8 * half, v);
-        }
-        tm_wait_st();
-      }
-#pragma unroll
-      for (int h = 0; h < GQA; ++h) base_part[h] *= corr[h];
-      tm_fence_before();
-      wg_barrier(wg);
-      // ================= values: folded probabilities of row (token, group) -> B operand =================
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        if (x < ntile) {
-          const int tok = tid >> 1, grp = tid & 1;
-          const uint32_t dst = vop + (x * 8 + (tok >> 3)) * VOP_BLOCK + ((tok >> 2) & 1) * VOP_LBO + grp * VOP_SBO + (tok & 3) * 4;
-#pragma unroll
-          for (int h = 0; h < GQA; ++h) {
-            const float pr = ldsf(pbuf + ((x * 4 + h) * PB_HEAD + tok) * 4);
-            const float wu = pr * vBu[x], wd = pr * vBd[x];
-            const __half2 hi = __floats2half2_rn(wu, wd);
-            const float2 hf = __half22float2(hi);
-            sts32(dst + (2 * h) * 16, h2_bits(hi));
-            sts32(dst + (2 * h + 1) * 16, h2_bits(__floats2half2_rn(wu - hf.x, wd - hf.y)));
-            base_part[h] = fmaf(pr, vA[x], base_part[h]);
-          }
-        }
-      }
-      proxy_fence();
-      // ================= values: table values of this warp's 32 channels -> A operand =================
-      {
-        const int grp = w >> 1;
-#pragma unroll 1
-        for (int x = 0; x < ntile; ++x) {
-          const uint4 zr4 = lds128(zV + x * 128 + grp * 64 + t0 * 16);
-          const uint32_t zr[4] = {zr4.x, zr4.y, zr4.z, zr4.w};
-          // 4-bit: the warp's 16 bytes of a token row sit in 16-byte chunk w, swapped with chunk w ^ 2 for tokens with bit 1 set
-          const uint32_t vb = vbuf0 + x * SB + (BITS == 4 ? ((w ^ (2 * (t0 >> 1))) * 16) : 4 * BITS * w) + QUAD * g;
-          auto load_codes = [&](int j, uint32_t& x0, uint32_t& x1) {
-            if (BITS == 4) { x0 = lds16(vb + (8 * j + t0) * VROW); x1 = lds16(vb + (8 * j + 4 + t0) * VROW); }
-            else { x0 = lds8(vb + (8 * j + t0) * VROW); x1 = lds8(vb + (8 * j + 4 + t0) * VROW); }
-          };
-          uint32_t c0, c1, n0 = 0, n1 = 0;
-          load_codes(0, c0, c1);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            if (j + 1 < 8) load_codes(j + 1, n0, n1);
-            const Codes4<BITS> c = spread4<BITS>(c0, c1, zero_bytes<BITS>(zr[j >> 1], 2 * (j & 1)));
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-              tm_st4(tm_warp + ((uint32_t)(16 * h) << 16) + TM_A + 64 * x + 8 * j, look<BITS>(c, lbV, 0, h, 0), look<BITS>(c, lbV, 0, h, 1),
-                     look<BITS>(c, lbV, 1, h, 0), look<BITS>(c, lbV, 1, h, 1));
-            c0 = n0; c1 = n1;
-          }
-        }
-      }
-      tm_wait_st();
-      tm_fence_before();
-      wg_barrier(wg);
-      if (tid == 0) {
-        tm_fence_after();
-#pragma unroll 1
-        for (int blk = 0; blk < 8 * ntile; ++blk)
-          umma(tm + TM_O, tm + TM_A + 8 * blk, b_descriptor(vop + blk * VOP_BLOCK, VOP_LBO, VOP_SBO), !(first_step && blk == 0));
-        umma_commit(bar_v);
-      }
-      v_pending = true;
-      first_step = false;
-      if (n_next > 0) stage_tiles(fn, n_next, false);
-      cp_async_commit();
-      f = fn;
-      n_cur = n_next;
+      cur = nxt;
     }
-    cp_async_wait<0>();
-    write_partial();
+    }
   }
   tm_fence_before();
   __syncthreads();
-  if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(512));
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(C::TM_ALLOC));
 }
 
-template <int BITS, int GQA>
+template <int BITS, int P, int GQA, bool HALF_META>
 int launch_one(const MzDecodeParams& p, cudaStream_t st) {
-  auto kern = decode_umma_kernel<BITS, GQA>;
-  MZ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.tp.smem_bytes));
-  kern<<<(unsigned)p.tp.ctas, THREADS, p.tp.smem_bytes, st>>>(p);
+  auto kern = decode_umma_kernel<BITS, P, GQA, HALF_META>;
+  MZ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BITS, P>::SMEM));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.hetero > 0 ? p.tp.ctas + p.tp2.ctas : p.tp.ctas));
+  cfg.blockDim = dim3(Cfg<BITS, P>::THREADS);
+  cfg.dynamicSmemBytes = Cfg<BITS, P>::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MZ_CUDA(cudaLaunchKernelEx(&cfg, kern, p, 65536u));
   MZ_LAUNCH_CHECK("decode_umma");
   return MZ_OK;
 }
-template <int BITS>
+template <int BITS, int P>
 int launch_gqa(const MzDecodeParams& p, cudaStream_t st) {
+  const bool half = p.s.meta_dtype == MZ_F16;
   switch (p.gqa) {
-    case 1: return launch_one<BITS, 1>(p, st);
-    case 2: return launch_one<BITS, 2>(p, st);
-    case 4: return launch_one<BITS, 4>(p, st);
+    case 1: return half ? launch_one<BITS, P, 1, true>(p, st) : launch_one<BITS, P, 1, false>(p, st);
+    case 2: return half ? launch_one<BITS, P, 2, true>(p, st) : launch_one<BITS, P, 2, false>(p, st);
+    case 4: return half ? launch_one<BITS, P, 4, true>(p, st) : launch_one<BITS, P, 4, false>(p, st);
   }
   return mz_fail(MZ_ERR_UNSUPPORTED, "gqa %d", p.gqa);
 }
 }  // namespace mzu
 
-
 bool mz_decode_umma_supported(const MzDecodeParams& p) {
-  return mz_decode_mma_supported(p) && p.s.head_dim == 128 && p.s.group == 64 && (p.s.bits == 2 || p.s.bits == 4) &&
+  return mz_decode_mma_supported(p) && p.s.head_dim == 128 && p.s.group == 64 && p.s.bits <= 3 &&
          (p.gqa == 1 || p.gqa == 2 || p.gqa == 4) && p.s.k_groups > 0;
 }
 
-// Plan of the packed tiles for the tcgen05 kernel (p.tp, workers = warpgroups) and, when there is a residual
-// window, of the residual tiles for the companion launch of the mma.sync kernel (p.tp2); the records of the
-// second plan follow those of the first in the workspace.
-int mz_plan_umma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slots) {
-  const mz_kv_store& s = p.s;
-  MzTilesPlan& t = p.tp;
-  const int msz = s.meta_dtype == MZ_F32 ? 4 : 2;
-  unsigned sb = mzm::D * (mzm::G * s.bits / 8) + 2 * mzm::D * msz;
-  sb = (sb + 127u) & ~127u;
-  const unsigned table_bytes = (1u << (2 * s.bits)) * 256u;
-  const unsigned wb = (unsigned)mz_smem_window_base();
-  const unsigned wgb = mzu::wg_bytes(sb);
+// us of one residual tile in a CTA of residual tiles (12 warps, 2.4 us each), and of a step of 128 packed tokens on an SM: [bits][planes]
+constexpr float kDenseTileUs = 0.2f;
+constexpr float step_us(int bits, int planes) { return bits == 1 ? 0.55f : planes == 2 ? 0.88f : 1.35f; }
+
+namespace {
+// even cut of `tiles` tiles per pair over W workers
+int cut(MzTilesPlan& t, long long pairs, int tiles, long long W) {
   t = MzTilesPlan{};
   t.kind = 2;
-  t.stage_bytes = sb;
-  t.low_base = (wb + 127u) & ~127u;
-  t.high_base = mzm::TBL + table_bytes;
-  if (t.low_base + wgb + 16 > mzm::TBL || t.high_base + 2 * wgb > wb + 227u * 1024u)
-    return mz_fail(MZ_ERR_UNSUPPORTED, "tile does not fit shared memory");
-  t.packed_tiles = s.k_groups;
-  t.dense_tokens = 0;
-  t.tiles_per_pair = s.k_groups;
-  t.cost_q = 1;
-  t.cost_d = 1;
-  const long long pairs = (long long)s.batch * s.kv_heads;
-  t.total_tiles = pairs * t.tiles_per_pair;
-  t.pair_cost = t.tiles_per_pair;
-  t.total_cost = t.total_tiles;
+  t.tiles_per_pair = tiles;
+  // in 64ths of a tile, so that the merge kernel finds a pair's workers within a narrow range (it divides by the whole units per worker)
+  t.cost_q = t.cost_d = 64;
+  t.pair_cost = 64LL * tiles;
+  t.total_tiles = pairs * tiles;
+  t.total_cost = pairs * t.pair_cost;
   if (t.total_cost >= (1LL << 31)) return mz_fail(MZ_ERR_UNSUPPORTED, "cache too large for the tiled kernel");
-  long long W;
-  if (splits_request > 0) {
-    W = pairs * splits_request;
-  } else {
-    W = (long long)sm_count * mzu::WGS;             // one resident CTA per SM
-    const long long steps = (t.total_tiles + 1) / 2;  // at least one step of two tiles per worker
-    if (W > steps) W = steps;
-    if (W < 1) W = 1;
-  }
+  if (W > t.total_tiles) W = t.total_tiles;
+  if (W < 1) W = 1;
   if (W > (1LL << 30)) return mz_fail(MZ_ERR_ARG, "too many splits");
   t.total_warps = (int)W;
   t.cost_quot = (unsigned)(t.total_cost / W);
   t.cost_rem = (unsigned)(t.total_cost % W);
-  t.warps_per_cta = mzu::WGS * 4;
-  t.smem_per_warp = wgb / 4;
-  t.smem_bytes = t.high_base + 2 * wgb - wb;
-  t.ctas = (int)((W + mzu::WGS - 1) / mzu::WGS);
   const long long len = t.total_cost / W + 2;
   t.max_segs = (int)((len - 1) / t.pair_cost + 2);
-  size_t slots_a = (size_t)W * t.max_segs * p.gqa;
-  p.slots_a = (long long)slots_a;
-  p.tp2 = MzTilesPlan{};
-  size_t slots_b = 0;
-  if (s.res_len > 0) {
-    // the residual tiles alone, as a plan of the mma.sync kernel: the same arithmetic with zero packed tiles
-    MzDecodeParams q = p;
-    q.s.k_groups = 0;
-    int rc = mz_plan_mma(q, splits_request > 0 ? splits_request : -1, sm_count, &slots_b);
-    if (rc) return rc;
-    p.tp2 = q.tp;
+  return MZ_OK;
+}
+}  // namespace
+
+// One launch over two plans: the packed tiles (p.tp, workers = warp groups, tiles = steps of 128 tokens) and, when there is a residual
+// window, its tiles on CTAs of their own (p.tp2, workers = warps); the records of the second plan follow those of the first.
+int mz_plan_umma(MzDecodeParams& p, bool full_precision, int splits_request, int sm_count, size_t* slots) {
+  const mz_kv_store& s = p.s;
+  p.planes = s.bits == 1 ? 1 : s.bits == 2 && !full_precision ? 2 : 3;
+  const int workers = p.planes == 3 ? mzu::Cfg<3, 3>::WORKERS : mzu::Cfg<2, 2>::WORKERS;
+  const int steps = (s.k_groups + mzu::STEP_GROUPS - 1) / mzu::STEP_GROUPS;
+  const long long pairs = (long long)s.batch * s.kv_heads;
+  const int dense_tiles = (s.res_len + mzd::DT - 1) / mzd::DT;
+  int n_d = 0;
+  if (dense_tiles > 0) {
+    const float dense = (float)dense_tiles * kDenseTileUs, packed = (float)steps * step_us(s.bits, p.planes);
+    n_d = (int)((float)sm_count * dense / (dense + packed) + 0.5f);
+    if (n_d < 1) n_d = 1;
+    if (n_d > sm_count / 2) n_d = sm_count / 2;
   }
-  *slots = slots_a + slots_b;
+  p.cluster = 0;
+  p.hetero = 0;
+  int rc = cut(p.tp, pairs, steps, splits_request > 0 ? pairs * splits_request : (long long)(sm_count - n_d) * workers);
+  if (rc) return rc;
+  p.tp.packed_tiles = steps;
+  p.tp.ctas = (p.tp.total_warps + workers - 1) / workers;
+  *slots = (size_t)p.tp.total_warps * p.tp.max_segs * p.gqa;
+  p.slots_a = (long long)*slots;
+  p.tp2 = MzTilesPlan{};
+  if (dense_tiles > 0) {
+    if ((rc = cut(p.tp2, pairs, dense_tiles, splits_request > 0 ? pairs * splits_request : (long long)n_d * mzu::DENSE_WARPS))) return rc;
+    p.tp2.ctas = (p.tp2.total_warps + mzu::DENSE_WARPS - 1) / mzu::DENSE_WARPS;
+    p.hetero = p.tp.ctas;
+    *slots += (size_t)p.tp2.total_warps * p.tp2.max_segs * p.gqa;
+  }
   return MZ_OK;
 }
 
 int mz_launch_decode_umma(const MzDecodeParams& p, cudaStream_t st) {
-  if (p.tp2.total_warps > 0) {
-    // residual tiles: the mma.sync kernel on its own plan, records behind those of the packed tiles
-    MzDecodeParams q = p;
-    q.tp = p.tp2;
-    q.part.m = p.part.m + p.slots_a;
-    q.part.l = p.part.l + p.slots_a;
-    q.part.acc = p.part.acc + p.slots_a * p.s.head_dim;
-    q.part.slots = p.part.slots - (long long)p.slots_a;
-    int rc = mz_launch_decode_mma(q, st);
-    if (rc) return rc;
+  switch (p.s.bits * 16 + p.planes) {
+    case 0x11: return mzu::launch_gqa<1, 1>(p, st);
+    case 0x22: return mzu::launch_gqa<2, 2>(p, st);
+    case 0x23: return mzu::launch_gqa<2, 3>(p, st);
+    case 0x33: return mzu::launch_gqa<3, 3>(p, st);
   }
-  if (p.s.bits == 4) return mzu::launch_gqa<4>(p, st);
-  if (p.s.bits == 2) return mzu::launch_gqa<2>(p, st);
-  return mz_fail(MZ_ERR_UNSUPPORTED, "bits %d", p.s.bits);
+  return mz_fail(MZ_ERR_UNSUPPORTED, "bits %d, %d planes", p.s.bits, p.planes);
 }

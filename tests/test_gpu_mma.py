@@ -153,6 +153,33 @@ def test_an_infinite_range_stays_in_its_group(oracle, bits, D, group, gqa):
     assert not bool(torch.isfinite(got[hit]).any()) and relative_error(got[~hit], want[~hit]) <= FP32_ERROR
 
 
+@pytest.mark.parametrize("meta", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("bits,gqa,B,S", [(1, 4, 3, 128 + 64), (1, 2, 2, 128 + 5 * 64 + 63), (2, 4, 3, 128 + 128), (2, 1, 2, 128 + 3 * 64 + 1), (2, 4, 24, 1111),
+                                          (3, 4, 3, 128 + 64 + 17), (3, 1, 2, 128 + 128 + 1), (3, 4, 20, 128 + 9 * 64), (1, 4, 40, 700), (3, 2, 2, 5000)])
+def test_tcgen05_kernel(oracle, bits, gqa, B, S, meta):
+    """One group, whole and half steps, one tile and many in the residual window, a worker's range over several pairs, ranges that do not
+    straddle zero, symmetric ones, masked tokens and sequences.  Two-plane calls round a value to 2^-15 of its side:
+    2^-16 / sqrt(3) over a value of 0.4 sides, times a logit of about 3, once for keys and once for values: 6e-5, bounded by twice that."""
+    import muzero_b200 as mz
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = oracle.synth_kv(B, 8 if B > 3 else 2, S, 128, (8 if B > 3 else 2) * gqa, seed=bits * 100 + S)
+    k[:, :, :, :3] += 4.0
+    v[0] -= 3.0
+    k[0, 0, 0::2, 5], k[0, 0, 1::2, 5] = 1.5, -1.5
+    ref = oracle.OracleCacheLayer(bits=bits, group=64, residual=128, meta_dtype=meta, alpha_key=2.0, alpha_value=4.0)
+    ref.append(k, v)
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=64, residual_length=128, amax_dtype=str(meta)[6:], alpha_key=2.0, alpha_value=4.0)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+    mask = torch.zeros(B, 1, 1, S)
+    mask[1, ..., : S - 130] = torch.finfo(torch.bfloat16).min
+    for m in (None, mask):
+        want = attention64(oracle, ref, q, 128 ** -0.5, m)
+        got = decode_attention(layer, q.cuda(), 128 ** -0.5, None if m is None else m.cuda(), out_dtype=torch.float32)
+        assert bool(torch.isfinite(got).all()) and relative_error(got, want) <= (1.2e-4 if bits == 2 and B > 3 else FP32_ERROR)
+
+
 @pytest.mark.parametrize("bits,bound", [(2, 1.2e-4), (4, 5e-5)])
 def test_error_of_the_unrolled_kernel(oracle, bits, bound):
     """Head_dim 128, group 64, up to four heads, more pairs than SMs: the unrolled kernel's table keeps 11 bits and a nominal
