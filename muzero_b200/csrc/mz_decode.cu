@@ -109,7 +109,7 @@ int make_plan(const mz_decode_args* a, Plan* plan, bool need_tables, size_t scra
   p.table_k = p.table_v = nullptr;
   p.lut = nullptr;
   p.hetero = 0;
-  p.planes = 0;
+  p.planes = p.kv_share = 0;
   p.cluster = 0;
   p.o = MzDecodeOut{};
   p.new_k = p.new_v = nullptr;
@@ -217,7 +217,7 @@ int mz_decode_plan(const mz_decode_args* a, MzDecodePlan* plan) {
   return make_plan(a, plan, true);
 }
 bool mz_decode_takes_new_token(const MzDecodePlan& plan, const void* k_new, const void* v_new, long long nsb, long long nsh) {
-  return plan.tiles && plan.p.tp.kind == 1 && (((uintptr_t)k_new | (uintptr_t)v_new) & 15) == 0 && ((nsb | nsh) & 7) == 0;
+  return plan.tiles && (plan.p.tp.kind == 1 || plan.p.tp.kind == 2) && (((uintptr_t)k_new | (uintptr_t)v_new) & 15) == 0 && ((nsb | nsh) & 7) == 0;
 }
 int mz_decode_run_plan(const mz_decode_args* a, MzDecodePlan* plan, const void* k_new, const void* v_new, long long nsb, long long nsh,
                        int rows, cudaStream_t st) {

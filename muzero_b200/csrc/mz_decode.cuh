@@ -88,8 +88,9 @@ struct MzDecodeParams {
   // tensor-core kernels, one launch over two plans: CTAs [0, hetero) work on plan `tp` (packed tiles only), the
   // rest on plan `tp2` (residual tiles only, records from slots_a on).  0 = one plan per launch.
   int hetero;
-  // tcgen05 kernel: bytes per value
-  int planes;
+  // tcgen05 kernel: bytes per value; log2 of the kv heads of the plan that share one of the store (8 query heads per kv head are
+  // planned as two kv heads with 4)
+  int planes, kv_share;
   // tensor-core kernel, cluster mode: CTAs per pair (0 = flat partition and merge kernel); the kernel writes `o` itself
   int cluster;
   MzDecodeOut o;
@@ -147,7 +148,7 @@ bool mz_mma_kernel_b4(int D, int G, int nt, MzMmaKernel* k);
 bool mz_mma_kernel_b8(int D, int G, int nt, MzMmaKernel* k);
 bool mz_mma_kernel_wide(int D, int G, int nt, MzMmaKernel* k);
 
-// tcgen05 kernel: 1 to 3 bits, head_dim 128, group 64.  full_precision: that of the fp32 kernels also at 2 bits, where the call would
+// tcgen05 kernel: 1 to 4 bits, head_dim 128, group 64, 1 / 2 / 4 / 8 query heads per kv head.  full_precision: that of the fp32 kernels also at 2 bits, where the call would
 // not have gone to the unrolled kernel
 bool mz_decode_umma_supported(const MzDecodeParams& p);
 int mz_plan_umma(MzDecodeParams& p, bool full_precision, int splits_request, int sm_count, size_t* slots);

@@ -303,6 +303,13 @@ float tiles_per_sm(const MzDecodeParams& p, const MzTilesPlan& t, int sm_count) 
   return (float)((double)p.s.batch * p.s.kv_heads * (double)t.pair_cost / t.cost_q / sm_count);
 }
 
+// estimate for clusters of `cs` CTAs of `nw` warps
+float cluster_us(const MzDecodeParams& p, const MzTilesPlan& t, int cs, int nw) {
+  const long long turn = (long long)cs * nw * t.cost_q, pair_cost = (long long)t.packed_tiles * t.cost_q + (long long)(t.tiles_per_pair - t.packed_tiles) * t.cost_d;
+  return kClusterBase[p.gqa > 4] + cluster_tile_us(p) * (float)(nw * ((pair_cost + turn - 1) / turn));
+}
+float cluster_us(const MzDecodeParams& c) { return cluster_us(c, c.tp, c.cluster, c.tp.warps_per_cta); }
+
 // Cluster mode: one cluster per pair, no partial records in memory and no merge kernel; taken where the estimates above say that it
 // is not slower than the cut, or at any cost.
 bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count, bool any_cost = false) {
@@ -321,8 +328,7 @@ bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count, bool an
     if (want < 4) want = 4;
     const int nw = layout(t, p, k, want, rec);
     if (nw < 1) return false;
-    const long long turn = (long long)cs * nw * t.cost_q;
-    if (kClusterBase[p.gqa > 4] + cluster_tile_us(p) * (float)(nw * ((t.pair_cost + turn - 1) / turn)) > limit) return false;    // smaller clusters are heavier still
+    if (cluster_us(p, t, cs, nw) > limit) return false;    // smaller clusters are heavier still
     if (cs > 1 && clusters_at_once(k, cs, nw * 32, t.smem_bytes) < pairs) continue;
     // tiles are dealt to the cluster's warps by cost; every warp gets at most about one residual tile's cost more than its share
     if (cut(t, 1, (long long)cs * nw) != MZ_OK) return false;
@@ -333,6 +339,23 @@ bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count, bool an
   }
   return false;
 }
+// Whether the tcgen05 kernel takes a call that it serves; `clusters`: the choice without it is cluster mode, planned in `c`.
+// 1 to 3 bits: always.  Over 150 shapes of 0.1 to 210 tiles per SM it needs 0.55 (1 bit), 0.70 (3 bits) and 0.78 (2 bits) of the time of the
+// best other form, and is nowhere behind it by more than the timing's spread (device time of 90 calls below 12 tiles per
+// SM: 0.49 to 0.92 of cluster mode).
+// 4 bits need two lookups per code, and three planes because the unrolled kernel's error (3e-5) is out of reach of two (4e-5 to 6e-5).
+// With up to four heads the unrolled kernel keeps its calls (64 x 8 pairs x 4224 tokens 149 us; 28 x 8 x 9800 49.9 against 72.7); cluster mode's
+// go by cost (1 x 8 x 17879 54 -> 30 us, 5 x 4 x 4988 30 -> 22; 15 x 8 x 459 would be 17.2 -> 19.5).  Eight heads run as two times four.
+constexpr float kUmmaBase = 14.5f, kUmmaBase8 = 15.0f, kUmmaTile4 = 1.0f;       // us, and us per packed tile on an SM; 8 %, 70 shapes
+bool choose_umma(const MzDecodeParams& p, const MzDecodeParams& c, bool clusters, int sm_count) {
+  if (p.s.bits < 4) return true;
+  if (!clusters && p.gqa <= 4) return false;
+  MzTilesPlan t = {};
+  describe_tiles(t, p);
+  const float x = tiles_per_sm(p, t, sm_count), us = p.gqa > 4 ? kUmmaBase8 + 2.0f * kUmmaTile4 * x : kUmmaBase + kUmmaTile4 * x;
+  return us < (clusters ? cluster_us(c) : cut_us(p, x));
+}
+
 }  // namespace
 
 // Cost of a residual tile in CTAs that hold residual tiles only, in units of a packed tile among busy warps.  Such a
@@ -396,16 +419,12 @@ int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slo
     take_lookup_entries(q);
     return true;
   };
-  // The tcgen05 kernel takes what it serves: over 150 shapes of 0.1 to 210 tiles per SM it needs 0.55 (1 bit), 0.70 (3 bits) and 0.78 (2 bits)
-  // of the time of the best other form, and is nowhere behind it by more than the timing's spread (device time of the smallest
-  // calls: 0.51 to 0.92 of cluster mode).  At 2 bits it runs with two planes where the choice below would have been the
-  // unrolled kernel, whose precision that is, and with three where it would have been a cluster.
   if (splits_request == 0 && mz_decode_umma_supported(p)) {
-    MzDecodeParams t = p, c = p;
+    MzDecodeParams c = p, t = p;
+    const bool clusters = plan_cluster(c, k, sm_count), flat = mz_decode_flat_supported(p);
     size_t n = 0;
-    const bool full = p.s.bits == 2 && plan_cluster(c, k, sm_count);
-    const int rc = mz_plan_umma(t, full, 0, sm_count, &n);
-    if (rc == MZ_OK && (p.scratch_limit == 0 || n * sizeof(float) * (2 + (size_t)p.s.head_dim) <= p.scratch_limit)) {
+    if (choose_umma(p, c, clusters, sm_count) && mz_plan_umma(t, clusters || !flat, 0, sm_count, &n) == MZ_OK &&
+        (p.scratch_limit == 0 || n * sizeof(float) * (2 + (size_t)p.s.head_dim) <= p.scratch_limit)) {
       p = t;
       *slots = n;
       return MZ_OK;

@@ -1,5 +1,5 @@
-// tcgen05 decode attention over the packed tiles of a cache, on the integer tensor cores: head_dim 128, group 64, 1-, 2- or 3-bit codes,
-// 1 / 2 / 4 query heads per kv head (sm_100a).
+// tcgen05 decode attention over the packed tiles of a cache, on the integer tensor cores: head_dim 128, group 64, 1- to 4-bit codes,
+// 1 / 2 / 4 / 8 query heads per kv head (sm_100a).
 //
 // Both contractions reduce over the packed rows (keys: over channels, values: over tokens), and a row of 64 codes runs along the
 // dimension that is kept.  So one thread owns a row: it builds the row's book of dequantized values (fixed point, relative to the
@@ -24,7 +24,7 @@
 // 64 x 8 pairs x 4224 tokens, 4 heads, us per call: 1 bit 202 -> 93 (before: SIMT kernel), 2 bits 148 -> 120 (before: unrolled mma.sync
 // kernel), 3 bits 230 -> 180 (SIMT); 24 x 8 x 1537, 3 bits: 53 -> 37; one sequence of 1300 tokens, device time: 15 -> 8 to 11.
 //
-// Precision: three planes hold a value to 2^-22 of its row's larger side and the fold to 2^-31 of the step's largest product, which is that of the
+// Precision: three planes hold a value to 2^-24 of its row's larger side and the fold to 2^-31 of the step's largest product, which is that of the
 // fp32 kernels (relative error against 64 bits 2e-7 to 9e-7; 1 bit is exact in one plane).  Two planes (2 bits, calls that the
 // unrolled kernel served with 9e-5): 2^-15 and 2^-22, 2e-5 to 6e-5.  Any range is served: sides and query are scaled by powers of two.
 #include "mz_dense_tiles.cuh"
@@ -49,13 +49,13 @@ struct Cfg {
   static constexpr int PLANES = P;                                       // bytes per value
   static constexpr int WORKERS = PLANES == 3 ? 2 : 3;
   static constexpr int WARPS = 8 * WORKERS + 4, THREADS = 32 * WARPS;
-  static constexpr int LAUNCH = WORKERS == 3 ? 72 : 96, KEY = WORKERS == 3 ? 56 : 88, VALUE = WORKERS == 3 ? 104 : 136, ISSUE = 24;
+  static constexpr int LAUNCH = WORKERS == 3 ? 72 : 96, KEY = WORKERS == 3 ? 56 : BITS == 4 ? 96 : 88, VALUE = WORKERS == 3 ? 104 : BITS == 4 ? 128 : 136, ISSUE = 24;
   static_assert(DENSE_REGS * DENSE_WARPS + 24 * (WARPS - DENSE_WARPS) <= LAUNCH * WARPS, "register split of a residual CTA");
   static_assert(KEY * 4 * WORKERS + VALUE * 4 * WORKERS + ISSUE * 4 <= LAUNCH * WARPS, "register split");
-  static constexpr bool BOOKS = BITS <= 3;                               // wider codes are expanded by arithmetic
-  // book table: per zero code up to the middle (rows above are mirrored) slopes and offsets of the entries
-  static constexpr int BOOK_ROW = 8 * NE, BOOK_BYTES = BITS == 2 || BITS == 3 ? ZC * BOOK_ROW : 128;
-  static constexpr float FULL = PLANES == 1 ? 1.0f : PLANES == 2 ? 32766.0f : 4194000.0f;      // fixed-point value of S
+  // book table: per zero code up to the middle (rows above are mirrored) slopes and offsets of the entries that may lie on the row's
+  // smaller side, and for 4 bits the bytes of the upper eight entries, plane by plane
+  static constexpr int MIXED = NE < 8 ? NE : 8, BOOK_ROW = BITS == 4 ? 96 : 8 * NE, BOOK_BYTES = ZC * BOOK_ROW;
+  static constexpr float FULL = PLANES == 1 ? 1.0f : PLANES == 2 ? 32766.0f : 8388600.0f;      // fixed-point value of S
   // fixed-point value of 1 in the folded operand (two planes: half of it; else its upper half), and what a unit of column_sum is worth
   static constexpr float FOLD_FULL = PLANES == 2 ? 4161536.0f : 32000.0f;
   static constexpr float UNIT = (PLANES == 1 ? 1.0f / 65536.0f : PLANES == 2 ? 128.0f : 256.0f) / (FULL * FOLD_FULL);
@@ -72,7 +72,8 @@ constexpr int RED_SV = 32;                       // [parity][group][warp] of the
 constexpr int RED_MAX = 96;                      // [parity][warp][4] largest logit
 constexpr int RED_EX = 224, RED_FLAG = 240, RED_CA = 272;  // [parity] exponent of the keys; [parity][warp] whether there is a constant term; [parity][warp][group][4] its parts
 constexpr int RED_QS = RED_CA + 256;             // [4] logit per unit of column_sum
-constexpr int RED_END = RED_QS + 16;             // [warp][16]: constant terms of the output [group][4], sum of probabilities [4]
+constexpr int RED_RUN = RED_QS + 16;            // [parity][4] running maximum of the logits (base 2)
+constexpr int RED_END = RED_RUN + 32;             // [warp][16]: constant terms of the output [group][4], sum of probabilities [4]
 constexpr int RED_BARS = RED_END + 256, BAR_KDONE = RED_BARS, BAR_KFREE = RED_BARS + 8, BAR_VDONE = RED_BARS + 16, RED_TMEM = RED_BARS + 24;
 
 // ---- tcgen05 / mbarrier wrappers
@@ -176,17 +177,20 @@ __device__ __forceinline__ float unit_value(float alpha, int e, int zc, int top)
 template <int BITS, int P>
 __device__ __forceinline__ void fill_books(uint32_t table, float alpha, int first, int n) {
   using C = Cfg<BITS, P>;
-  for (int i = first; C::BOOKS && BITS > 1 && i < C::ZC * C::NE; i += n) {
+  for (int i = first; BITS > 1 && i < C::ZC * C::NE; i += n) {
     const int zc = i / C::NE, e = i % C::NE;
     const float u = C::FULL * unit_value(alpha, e, zc, C::TOP);
     const uint32_t row = table + zc * C::BOOK_ROW;
-    stsf(row + e * 4, e < zc ? u : 0.0f);
-    stsf(row + C::NE * 4 + e * 4, e < zc ? MAGIC : MAGIC + rintf(u));
+    if (e < C::MIXED) {
+      stsf(row + e * 4, e < zc ? u : 0.0f);
+      stsf(row + C::MIXED * 4 + e * 4, (P == 2 ? MAGIC : 0.0f) + (e < zc ? 0.0f : rintf(u)));
+    } else {
+      for (int q = 0; q < P; ++q) sts8(row + 64 + 8 * q + (e - 8), (uint32_t)(__float2int_rn(u) >> (8 * (P - 1 - q))) & 0xff);
+    }
   }
 }
 
 // constants of one row: signed scale, ratio of the smaller to the larger side, value of the zero code, mirrored zero code
-// (codes wider than 3 bits: sides are not mirrored, ratio is the lower side over the larger, zc the zero code + 2^23 as a float)
 struct Row { float s, ratio, A; uint32_t zc; };
 template <int BITS, int P, bool EXACT>
 __device__ __forceinline__ Row prepare_row(float lo, float span) {
@@ -197,15 +201,6 @@ __device__ __forceinline__ Row prepare_row(float lo, float span) {
   bool wild = false;       // never with 16-bit floats of 5 exponent bits
   row_split(lo, span, (float)TOP, r.A, bup, bdn, zc, wild);
   if (EXACT) zc = exact_zero_code(lo, span, (float)TOP);
-  if (!Cfg<BITS, P>::BOOKS) {
-    r.s = fmaxf(bup, bdn);
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r.s));
-    // the ratio of the side below zero to the one above, as one number: |ratio| <= 1 is the smaller side, its sign says which side it is
-    r.ratio = bup >= bdn ? bdn * y : -bup * y;
-    r.zc = 0x4B000000u | (uint32_t)zc;
-    return r;
-  }
   const bool mirrored = zc > TOP / 2 && bup < INFINITY;              // an infinite range has no zero code; it stays S = inf
   const float big = mirrored ? bdn : bup, small = mirrored ? bup : bdn;
   float y;
@@ -215,22 +210,25 @@ __device__ __forceinline__ Row prepare_row(float lo, float span) {
   r.zc = min((uint32_t)(mirrored ? TOP - zc : zc), (uint32_t)(TOP / 2));
   return r;
 }
-// four fixed-point values (low mantissa bits) -> their bytes, plane by plane, top byte first
+// a book entry: offset + slope * ratio as an integer.  Two planes: in the low mantissa bits, by magic addition in the offset; three: 24 bits
+template <int P>
+__device__ __forceinline__ uint32_t book_entry(uint32_t slope, float ratio, uint32_t offset) {
+  const float v = fmaf(__uint_as_float(slope), ratio, __uint_as_float(offset));
+  return P == 2 ? __float_as_uint(v) : (uint32_t)__float2int_rn(v);
+}
+// four book entries -> their bytes, plane by plane, top byte first
 template <int P>
 __device__ __forceinline__ void pack4(const uint32_t* v, uint32_t* plane) {
   const uint32_t a = prmt(v[0], v[1], 0x5140u), b = prmt(v[2], v[3], 0x5140u);
   plane[P - 1] = prmt(a, b, 0x5410u);
   plane[P - 2] = prmt(a, b, 0x7632u);
-  // three planes: the third byte is 64 + the top digit; a byte of its own each, so nothing carries
-  if (P == 3) plane[0] = (prmt(prmt(v[0], v[1], 0x0062u), prmt(v[2], v[3], 0x0062u), 0x5410u) + 0x40404040u) ^ 0x80808080u;
+  if (P == 3) plane[0] = prmt(prmt(v[0], v[1], 0x0062u), prmt(v[2], v[3], 0x0062u), 0x5410u);
 }
-// the alphas' constants of the arithmetic expansion, per CTA: log2(1 + alpha) and 1 / alpha
-struct Compand { float log2base, inv_alpha; };
 // expands the 64 codes of one row: `dst` is the row's 16 bytes in the first chunk of its group's half of the first plane.  The permutes
 // take their selector from the low half of a register; `two16` is 2^16 as a run-time value, so that the multiplier brings the
 // upper half down: the logic pipe is the busy one
 template <int BITS, int P, int NW>
-__device__ __forceinline__ void expand_row(const uint32_t (&w)[NW], const Row& r, uint32_t table, const Compand& cp, uint32_t dst, uint32_t two16) {
+__device__ __forceinline__ void expand_row(const uint32_t (&w)[NW], const Row& r, uint32_t table, uint32_t dst, uint32_t two16) {
   using C = Cfg<BITS, P>;
   const uint32_t flip = (uint32_t)(__float_as_int(r.s) >> 31);       // mirrored rows: TOP - code is the complement
   if constexpr (BITS == 1) {
@@ -242,18 +240,18 @@ __device__ __forceinline__ void expand_row(const uint32_t (&w)[NW], const Row& r
       sts128(dst + q * 2048, make_uint4(prmt(0x00000100u, 0u, c & 0x1111u), prmt(0x00000100u, 0u, c >> 1 & 0x1111u),
                                         prmt(0x00000100u, 0u, c >> 2 & 0x1111u), prmt(0x00000100u, 0u, c >> 3 & 0x1111u)));
     }
-  } else if constexpr (C::BOOKS) {
+  } else {
     const uint32_t row = table + r.zc * C::BOOK_ROW;
-    constexpr int Q = C::NE / 4;
+    constexpr int Q = C::MIXED / 4;
     uint32_t book[P][Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-      const uint4 t = book128(row + 16 * q), c = book128(row + C::NE * 4 + 16 * q);
+      const uint4 t = book128(row + 16 * q), c = book128(row + C::MIXED * 4 + 16 * q);
       uint32_t v[4], b[P];
-      v[0] = __float_as_uint(fmaf(__uint_as_float(t.x), r.ratio, __uint_as_float(c.x)));
-      v[1] = __float_as_uint(fmaf(__uint_as_float(t.y), r.ratio, __uint_as_float(c.y)));
-      v[2] = __float_as_uint(fmaf(__uint_as_float(t.z), r.ratio, __uint_as_float(c.z)));
-      v[3] = __float_as_uint(fmaf(__uint_as_float(t.w), r.ratio, __uint_as_float(c.w)));
+      v[0] = book_entry<P>(t.x, r.ratio, c.x);
+      v[1] = book_entry<P>(t.y, r.ratio, c.y);
+      v[2] = book_entry<P>(t.z, r.ratio, c.z);
+      v[3] = book_entry<P>(t.w, r.ratio, c.w);
       pack4<P>(v, b);
 #pragma unroll
       for (int k = 0; k < P; ++k) book[k][q] = b[k];
@@ -266,6 +264,26 @@ __device__ __forceinline__ void expand_row(const uint32_t (&w)[NW], const Row& r
 #pragma unroll
         for (int k = 0; k < P; ++k)
           sts128(dst + k * PLANE_BYTES + q * 2048, make_uint4(prmt(book[k][0], 0u, even), prmt(book[k][0], 0u, even2), prmt(book[k][0], 0u, odd), prmt(book[k][0], 0u, odd2)));
+      }
+    } else if constexpr (BITS == 4) {
+      // lower eight entries from the registers, upper eight from the table; a code's top bit says which
+      const uint4 a = book128(row + 64), b = book128(row + 80);
+      const uint32_t up[3][2] = {{a.x, a.y}, {a.z, a.w}, {b.x, b.y}};
+      const uint32_t flip4 = flip & 0x44444444u;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t o[P][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t c = w[2 * q + (k >> 1)];
+          uint32_t sel = (c ^ flip) & 0x77777777u, top = ((c >> 1) & 0x44444444u) ^ flip4;
+          if (k & 1) { sel = __umulhi(sel, two16); top = __umulhi(top, two16); }
+          const uint32_t m = prmt(0u, 0xFFFFFFFFu, top);
+#pragma unroll
+          for (int p = 0; p < P; ++p) o[p][k] = (prmt(book[p][0], book[p][Q - 1], sel) & ~m) | (prmt(up[p][0], up[p][1], sel) & m);
+        }
+#pragma unroll
+        for (int p = 0; p < P; ++p) sts128(dst + p * PLANE_BYTES + q * 2048, make_uint4(o[p][0], o[p][1], o[p][2], o[p][3]));
       }
     } else {
 #pragma unroll
@@ -288,36 +306,6 @@ __device__ __forceinline__ void expand_row(const uint32_t (&w)[NW], const Row& r
 #pragma unroll
         for (int b = 0; b < P; ++b) sts128(dst + b * PLANE_BYTES + q * 2048, make_uint4(o[b][0], o[b][1], o[b][2], o[b][3]));
       }
-    }
-  } else {
-    // value = +-side * (base^(|n| / room) - 1) / alpha, n = code - zero code; the exponent is the larger of the two sides' candidates
-    const float zc = __uint_as_float(r.zc), z = zc - 8388608.0f;
-    const float kup = __fdividef(cp.log2base, fmaxf((float)C::TOP - z, 1.0f)), kdn = __fdividef(cp.log2base, fmaxf(z, 1.0f));
-    const float big = C::FULL * cp.inv_alpha, small = big * fabsf(r.ratio);
-    const bool up = __float_as_int(r.ratio) >= 0;                       // -0 is negative
-    const float cup = up ? big : small, cdn = up ? -small : -big;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      uint32_t o[P][4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        uint32_t v[4], b[P];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int code = 16 * q + 4 * k + j, bit = code * BITS, word = bit >> 5, sh = bit & 31;
-          uint32_t f;                                                 // 2^23 + code as a float
-          if (BITS == 8) f = prmt(w[word], 0x4B000000u, 0x7440u | (uint32_t)j);
-          else f = ((sh + BITS <= 32 ? w[word] >> sh : __funnelshift_r(w[word], w[(word + 1) % NW], sh)) & (uint32_t)C::TOP) | 0x4B000000u;
-          const float n = __uint_as_float(f) - zc;
-          const float grow = ex2f(fmaxf(n * kup, n * -kdn)) - 1.0f;
-          v[j] = __float_as_uint(fmaf(grow, n >= 0.0f ? cup : cdn, MAGIC));
-        }
-        pack4<P>(v, b);
-#pragma unroll
-        for (int p = 0; p < P; ++p) o[p][k] = b[p];
-      }
-#pragma unroll
-      for (int b = 0; b < P; ++b) sts128(dst + b * PLANE_BYTES + q * 2048, make_uint4(o[b][0], o[b][1], o[b][2], o[b][3]));
     }
   }
 }
@@ -431,9 +419,6 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
     }
   };
   bool failed = false;
-  Compand compand;
-  compand.inv_alpha = 1.0f / (keys ? s.alpha_key : s.alpha_value);
-  compand.log2base = log1pf(keys ? s.alpha_key : s.alpha_value) * LOG2E;
   const bool meta32 = s.meta_dtype == MZ_F32;
   // everything above reads kernel parameters only and may run while the grid before drains
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -449,11 +434,12 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
   const int msz = HALF_META ? 2 : meta32 ? 4 : 2;
   const uint8_t *code_at, *mn_at, *span_at;
   auto point = [&]() {
+    const int kvh = ahead.kvh >> p.kv_share;
     const long long tile = STEP_GROUPS * ahead.step;
     const long long row = keys ? r : half * G + (spot & 63);
-    const long long m = keys ? ahead.b * s.km_stride_b + ahead.kvh * s.km_stride_h + tile * D + row : ahead.b * s.vm_stride_b + ahead.kvh * s.vm_stride_h + (tile * G + row) * 2;
-    code_at = keys ? s.packed_k + ahead.b * s.pk_stride_b + ahead.kvh * s.pk_stride_h + tile * CODE_BYTES + row * QB
-                   : s.packed_v + ahead.b * s.pv_stride_b + ahead.kvh * s.pv_stride_h + (tile * G + row) * VROW;
+    const long long m = keys ? ahead.b * s.km_stride_b + kvh * s.km_stride_h + tile * D + row : ahead.b * s.vm_stride_b + kvh * s.vm_stride_h + (tile * G + row) * 2;
+    code_at = keys ? s.packed_k + ahead.b * s.pk_stride_b + kvh * s.pk_stride_h + tile * CODE_BYTES + row * QB
+                   : s.packed_v + ahead.b * s.pv_stride_b + kvh * s.pv_stride_h + (tile * G + row) * VROW;
     mn_at = (const uint8_t*)(keys ? s.k_mn : s.v_mn) + m * msz;
     span_at = (const uint8_t*)(keys ? s.k_scale : s.v_scale) + m * msz;
   };
@@ -593,9 +579,9 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       }
       const uint32_t ex = exponent_of_largest(red + RED_SK + 16 * par);
       if (i > 0) bar_wait<64>(red + BAR_KDONE, (uint32_t)(i - 1) & 1, failed);       // the operands have been read
-      expand_row<BITS, P, NW>(code[0], rows[0], book, compand, side + r * 16, two16);
+      expand_row<BITS, P, NW>(code[0], rows[0], book, side + r * 16, two16);
       if (more) load_codes(0);
-      expand_row<BITS, P, NW>(code[1], rows[1], book, compand, side + 8192 + r * 16, two16);
+      expand_row<BITS, P, NW>(code[1], rows[1], book, side + 8192 + r * 16, two16);
       if (more) load_codes(1);
       const float down = scale_down(ex);
       put_folds(qn, down, down);
@@ -632,7 +618,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
     if (steps > 0) {
     // ================= softmax and values: thread r has row r of the results =================
     const uint32_t tm_mine = ((uint32_t)(32 * w) << 16) + 16 * half;
-    float m_run[GQA], l_part[GQA], out[GQA];                          // running maximum (base-2 logits), this thread's sum of probabilities, output
+    float l_part[GQA], out[GQA];                                      // this thread's sum of probabilities, output
     float base_sum = 0.f;                                             // lane 4 x + g: sum p * A of the warp's tokens, channel group x and head g
     bool has_base = false;
     float up_v = 0.f;
@@ -640,11 +626,12 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
     auto start_pair = [&](const Place& c) {
 #pragma unroll
       for (int g = 0; g < GQA; ++g) {
-        m_run[g] = -INFINITY; l_part[g] = out[g] = 0.f;
+        l_part[g] = out[g] = 0.f;
         const uint16_t* q = (const uint16_t*)p.query + c.b * p.q_stride_b + (long long)(c.kvh * GQA + g) * p.q_stride_h;
         const uint32_t ex = query_exponent(q, lane, s.kv_dtype);
         if (r == 0) stsf(red + RED_QS + 4 * g, scale_up(ex) * p.scaling * (LOG2E * C::UNIT));     // read behind the next barrier but one
       }
+      if (r < 2) sts128(red + RED_RUN + 16 * r, make_uint4(0xFF800000u, 0xFF800000u, 0xFF800000u, 0xFF800000u));
       base_sum = 0.f; has_base = false;
       team_barrier(team);
     };
@@ -662,7 +649,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       tm_fence_before();
     };
     // ---- end of a segment: the partial record (m, l, acc) of this worker for the pair it just left
-    auto write_partial = [&]() {
+    auto write_partial = [&](int par) {
 #pragma unroll
       for (int g = 0; g < GQA; ++g) {
         float lsum = l_part[g];
@@ -684,7 +671,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
           }
           p.part.acc[(slot0 + g) * D + spot] = out[g] + bs;
           if (r == 0) {
-            p.part.m[slot0 + g] = failed ? INFINITY : m_run[g] * (1.0f / LOG2E);   // a wait ran out: +inf turns the merged output into NaN
+            p.part.m[slot0 + g] = failed ? INFINITY : ldsf(red + RED_RUN + 16 * par + 4 * g) * (1.0f / LOG2E);   // a wait ran out: +inf turns the merged output into NaN
             p.part.l[slot0 + g] = lt;
           }
         }
@@ -759,12 +746,15 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
           mx[0] = fmaxf(mx[0], __uint_as_float(a.x)); mx[1] = fmaxf(mx[1], __uint_as_float(a.y));
           mx[2] = fmaxf(mx[2], __uint_as_float(a.z)); mx[3] = fmaxf(mx[3], __uint_as_float(a.w));
         }
+        const uint4 run = lds128(red + RED_RUN + 16 * (par ^ 1));
+        const float before[4] = {__uint_as_float(run.x), __uint_as_float(run.y), __uint_as_float(run.z), __uint_as_float(run.w)};
+#pragma unroll
+        for (int g = 0; g < 4; ++g) mx[g] = fmaxf(mx[g], before[g]);
+        if (r == 0) sts128(red + RED_RUN + 16 * par, make_uint4(__float_as_uint(mx[0]), __float_as_uint(mx[1]), __float_as_uint(mx[2]), __float_as_uint(mx[3])));
 #pragma unroll
         for (int g = 0; g < GQA; ++g) {
-          const float m_new = fmaxf(m_run[g], mx[g]);
-          const float top = fmaxf(m_new, -3.0e38f);                  // -inf as long as every token is masked: then the probabilities are 0
-          const float c = ex2f(m_run[g] - top);
-          m_run[g] = m_new;
+          const float top = fmaxf(mx[g], -3.0e38f);                  // -inf as long as every token is masked: then the probabilities are 0
+          const float c = ex2f(before[g] - top);
           lg[g] = ex2f(lg[g] - top);
           l_part[g] = fmaf(l_part[g], c, lg[g]);
           out[g] *= c;
@@ -790,9 +780,9 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       const uint32_t ex0 = exponent_of_largest(red + RED_SV + 32 * par), ex1 = exponent_of_largest(red + RED_SV + 32 * par + 16);
       up_v = scale_up(half ? ex1 : ex0) * C::UNIT;
       put_folds(lg, scale_down(ex0), scale_down(ex1));
-      expand_row<BITS, P, NW>(code[0], rows[0], book, compand, side + r * 16, two16);
+      expand_row<BITS, P, NW>(code[0], rows[0], book, side + r * 16, two16);
       if (more) load_codes(0);
-      expand_row<BITS, P, NW>(code[1], rows[1], book, compand, side + 8192 + r * 16, two16);
+      expand_row<BITS, P, NW>(code[1], rows[1], book, side + 8192 + r * 16, two16);
       if (more) load_codes(1);
       proxy_fence();
       tm_fence_before();
@@ -800,7 +790,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       pending = true;
       if (!more || nxt.pair != cur.pair) {
         drain(i);
-        write_partial();
+        write_partial(par);
         ++seg;
         pending = false;
         if (more) start_pair(nxt);
@@ -845,13 +835,14 @@ int launch_gqa(const MzDecodeParams& p, cudaStream_t st) {
 }  // namespace mzu
 
 bool mz_decode_umma_supported(const MzDecodeParams& p) {
-  return mz_decode_mma_supported(p) && p.s.head_dim == 128 && p.s.group == 64 && p.s.bits <= 3 &&
-         (p.gqa == 1 || p.gqa == 2 || p.gqa == 4) && p.s.k_groups > 0;
+  return mz_decode_mma_supported(p) && p.s.head_dim == 128 && p.s.group == 64 && p.s.bits <= 4 &&
+         (p.gqa == 1 || p.gqa == 2 || p.gqa == 4 || p.gqa == 8) && p.s.k_groups > 0;
 }
 
-// us of one residual tile in a CTA of residual tiles (12 warps, 2.4 us each), and of a step of 128 packed tokens on an SM: [bits][planes]
-constexpr float kDenseTileUs = 0.2f;
-constexpr float step_us(int bits, int planes) { return bits == 1 ? 0.55f : planes == 2 ? 0.88f : 1.35f; }
+// us of one residual tile in a CTA of residual tiles (12 warps, 3 us each; swept 0.20 .. 0.36: 64 x 8 pairs x 4224 tokens at 3 bits 215, 186, 186,
+// 185, 187 us), and of a step of 128 packed tokens on an SM: [bits][planes]
+constexpr float kDenseTileUs = 0.26f;
+constexpr float step_us(int bits, int planes) { return bits == 1 ? 0.55f : planes == 2 ? 0.88f : bits < 4 ? 1.35f : 1.7f; }
 
 namespace {
 // even cut of `tiles` tiles per pair over W workers
@@ -881,6 +872,11 @@ int cut(MzTilesPlan& t, long long pairs, int tiles, long long W) {
 // window, its tiles on CTAs of their own (p.tp2, workers = warps); the records of the second plan follow those of the first.
 int mz_plan_umma(MzDecodeParams& p, bool full_precision, int splits_request, int sm_count, size_t* slots) {
   const mz_kv_store& s = p.s;
+  if (p.gqa == 8) {       // eight heads are two times four, each with the kv head to itself
+    p.gqa = 4;
+    p.s.kv_heads *= 2;
+    p.kv_share = 1;
+  }
   p.planes = s.bits == 1 ? 1 : s.bits == 2 && !full_precision ? 2 : 3;
   const int workers = p.planes == 3 ? mzu::Cfg<3, 3>::WORKERS : mzu::Cfg<2, 2>::WORKERS;
   const int steps = (s.k_groups + mzu::STEP_GROUPS - 1) / mzu::STEP_GROUPS;
@@ -917,6 +913,7 @@ int mz_launch_decode_umma(const MzDecodeParams& p, cudaStream_t st) {
     case 0x22: return mzu::launch_gqa<2, 2>(p, st);
     case 0x23: return mzu::launch_gqa<2, 3>(p, st);
     case 0x33: return mzu::launch_gqa<3, 3>(p, st);
+    case 0x43: return mzu::launch_gqa<4, 3>(p, st);
   }
   return mz_fail(MZ_ERR_UNSUPPORTED, "bits %d, %d planes", p.s.bits, p.planes);
 }

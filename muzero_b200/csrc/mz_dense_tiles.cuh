@@ -1,9 +1,10 @@
 // Residual (un-quantized) tiles of 16 tokens on mma.sync, head_dim 128: one warp walks the tiles of a plan that has no packed
-// tiles and leaves a partial record per (batch, kv head) pair.  A tile is a short latency-bound chain (2.4 us), so a launch
+// tiles and leaves a partial record per (batch, kv head) pair.  A tile is a short latency-bound chain (3 us), so a launch
 // gives these warps CTAs of their own beside the packed tiles'.
 //
 // M rows are tokens (keys) / channels (values); B columns are 4 heads x {query or probability rounded to 16 bits, remainder}.  A bf16
-// probability has a third part, so that no more is lost than to fp32.
+// probability has a third part, and products go to a fresh accumulator that is added in round-to-nearest (the tensor cores truncate their
+// running sums), so that no more is lost than to fp32.
 #pragma once
 #include "mz_mma_common.cuh"
 
@@ -36,15 +37,24 @@ __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTil
       if (++c.kvh == s.kv_heads) { c.kvh = 0; ++c.b; }
     }
   };
-  // up to 16 rows of 128 elements; rows past the end are zeroed (they meet probability 0, which must not meet a NaN bit pattern)
-  auto stage = [&](uint32_t dst, const uint16_t* res, const Cursor& c, bool valid) {
+  // up to 16 rows of 128 elements; rows past the end are zeroed (they meet probability 0, which must not meet a NaN bit pattern).  The
+  // newest token may still be in the caller's tensors (p.new_k / new_v): it is staged from there, and stored into the window
+  auto stage = [&](uint32_t dst, void* window, const void* fresh, const Cursor& c, bool valid) {
     if (valid) {
-      const int tok0 = c.tile * DT, ntok = min(DT, s.res_len - tok0);
-      const uint16_t* src = res + c.b * s.res_stride_b + c.kvh * s.res_stride_h + (long long)(s.res_start + tok0) * s.res_stride_t;
+      const int tok0 = c.tile * DT, ntok = min(DT, s.res_len - tok0), kvh = c.kvh >> p.kv_share;
+      const int newest = fresh != nullptr ? s.res_len - 1 - tok0 : -1;
+      uint16_t* src = (uint16_t*)window + c.b * s.res_stride_b + kvh * s.res_stride_h + (long long)(s.res_start + tok0) * s.res_stride_t;
       for (int i = lane; i < DT * 16; i += 32) {
         const int row = i >> 4, k = i & 15;
-        if (row < ntok) cp16(dst + row * STRIDE + k * 16, src + (long long)row * s.res_stride_t + k * 8);
-        else sts128(dst + row * STRIDE + k * 16, make_uint4(0, 0, 0, 0));
+        if (row < ntok) {
+          const uint16_t* from = src + (long long)row * s.res_stride_t + k * 8;
+          if (row == newest) {
+            from = (const uint16_t*)fresh + c.b * p.new_sb + kvh * p.new_sh + k * 8;
+            if (kvh << p.kv_share == c.kvh && MZ_IN_BOUNDS(s.res_start + tok0 + row, p.new_rows, 15))
+              *(uint4*)(src + (long long)row * s.res_stride_t + k * 8) = *(const uint4*)from;
+          }
+          cp16(dst + row * STRIDE + k * 16, from);
+        } else sts128(dst + row * STRIDE + k * 16, make_uint4(0, 0, 0, 0));
       }
     }
     cp_async_commit();
@@ -83,8 +93,8 @@ __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTil
   cur.pair = (int)((unsigned)f0 / (unsigned)T); cur.tile = (int)((unsigned)f0 % (unsigned)T);
   cur.b = cur.pair / s.kv_heads; cur.kvh = cur.pair % s.kv_heads;
   Cursor nxt = cur;
-  stage(kbuf, (const uint16_t*)s.res_k, cur, true);
-  stage(vbuf, (const uint16_t*)s.res_v, cur, true);
+  stage(kbuf, s.res_k, p.new_k, cur, true);
+  stage(vbuf, s.res_v, p.new_v, cur, true);
   reset();
   const uint16_t* qrow = nullptr;
   for (int left = (int)(f1 - f0); left > 0; --left, cur = nxt) {
@@ -107,11 +117,13 @@ __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTil
       const uint32_t a0 = lds32(ka), a1 = lds32(ka + 8 * STRIDE), a2 = lds32(ka + 16), a3 = lds32(ka + 8 * STRIDE + 16);
       const uint32_t b0 = fold_lane ? *(const uint32_t*)(qrow + 16 * j + 2 * t) : 0u;
       const uint32_t b1 = fold_lane ? *(const uint32_t*)(qrow + 16 * j + 8 + 2 * t) : 0u;
-      if (bf) mma_bf16(acc, a0, a1, a2, a3, b0, b1);
-      else mma_f16(acc, a0, a1, a2, a3, b0, b1);
+      float part[4];
+      if (bf) mma_bf16_first(part, a0, a1, a2, a3, b0, b1);
+      else mma_f16_first(part, a0, a1, a2, a3, b0, b1);
+      add4(acc, part);
     }
     warp_sync();
-    stage(kbuf, (const uint16_t*)s.res_k, nxt, left > 1);
+    stage(kbuf, s.res_k, p.new_k, nxt, left > 1);
     // ---- softmax: this lane has head t, tokens g and g + 8
     float sv[2] = {acc[0] * p.scaling * LOG2E, acc[2] * p.scaling * LOG2E};
 #pragma unroll
@@ -174,14 +186,18 @@ __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTil
         // rows g / g + 8 = channels 8g + 2m / 8g + 2m + 1; columns = tokens (2t, 2t + 1) and (2t + 8, 2t + 9)
         const uint32_t a0 = prmt(c0[m], c1[m], 0x5410u), a1 = prmt(c0[m], c1[m], 0x7632u);
         const uint32_t a2 = prmt(c2[m], c3[m], 0x5410u), a3 = prmt(c2[m], c3[m], 0x7632u);
+        float part[4];
         if (bf) {
-          mma_bf16(out[grp * 4 + m], a0, a1, a2, a3, bb[0], bb[1]);
-          mma_bf16(out[grp * 4 + m], a0, a1, a2, a3, b3[0], b3[1]);
-        } else mma_f16(out[grp * 4 + m], a0, a1, a2, a3, bb[0], bb[1]);
+          mma_bf16_first(part, a0, a1, a2, a3, b3[0], b3[1]);
+          mma_bf16(part, a0, a1, a2, a3, bb[0], bb[1]);
+        } else {
+          mma_f16_first(part, a0, a1, a2, a3, bb[0], bb[1]);
+        }
+        add4(out[grp * 4 + m], part);
       }
     }
     warp_sync();
-    stage(vbuf, (const uint16_t*)s.res_v, nxt, left > 1);
+    stage(vbuf, s.res_v, p.new_v, nxt, left > 1);
   }
   cp_async_wait<0>();
   write_partial();
