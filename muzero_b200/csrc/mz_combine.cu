@@ -32,7 +32,7 @@ __device__ __forceinline__ long long record_of(const MzTilesPlan& tp, long long 
   return first_record + gw * tp.max_segs + (pair - (int)((unsigned)f0 / (unsigned)T));
 }
 template <int D>
-__global__ void __launch_bounds__(512, 3) combine_tiles_kernel(const MzDecodeParams p, const MzDecodeOut o) {
+__global__ void __launch_bounds__(512, 4) combine_tiles_kernel(const MzDecodeParams p, const MzDecodeOut o) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a dependent waits for this grid's completion itself
   __shared__ int s_slot[kMaxCombineSlots];     // record of candidate i, or -1
   __shared__ float s_part[512 / D][D + 2];

@@ -1,4 +1,4 @@
-// tcgen05 decode attention over the packed tiles of a cache, on the integer tensor cores: head_dim 128, group 64, 1- to 4-bit codes,
+// tcgen05 decode attention over the packed tiles of a cache, on the integer tensor cores: head_dim 64 or 128, group 64, 1- to 4-bit codes,
 // 1 / 2 / 4 / 8 query heads per kv head (sm_100a).
 //
 // Both contractions reduce over the packed rows (keys: over channels, values: over tokens), and a row of 64 codes runs along the
@@ -135,11 +135,11 @@ __device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a_desc, uint64_t 
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// the products of a side: its 128 rows in four slices, each plane on an accumulator of its own
-template <int BITS, int P>
+// the products of a side: its rows in slices of 32, each plane on an accumulator of its own
+template <int BITS, int P, int SLICES>
 __device__ __forceinline__ void umma_side(uint32_t d_tmem, uint64_t values, uint64_t folds) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
+  for (int j = 0; j < SLICES; ++j)
 #pragma unroll
     for (int q = 0; q < Cfg<BITS, P>::PLANES; ++q) {
       const uint64_t a = values + ((q * PLANE_BYTES + j * 512) >> 4), b = folds + j * (512 >> 4);
@@ -344,9 +344,10 @@ __device__ __forceinline__ float scale_down(uint32_t ex) {
   return __uint_as_float(ex <= 252u ? (253u - max(ex, 1u)) << 23 : 0x00800000u >> (ex - 252u));
 }
 __device__ __forceinline__ float scale_up(uint32_t ex) { return __uint_as_float(min(max(ex, 1u) + 1u, 255u) << 23); }
-// exponent field of the largest magnitude of a head's query (128 elements of 16 bits)
+// exponent field of the largest magnitude of a head's query (HD elements of 16 bits)
+template <int HD>
 __device__ __forceinline__ uint32_t query_exponent(const uint16_t* q, int lane, int dtype) {
-  const uint32_t a = *((const uint32_t*)q + lane), b = *((const uint32_t*)q + 32 + lane);
+  const uint32_t a = *((const uint32_t*)q + lane), b = HD == 128 ? *((const uint32_t*)q + 32 + lane) : 0u;
   const uint32_t mx = __reduce_max_sync(0xffffffffu, max(max(a & 0x7FFFu, a >> 16 & 0x7FFFu), max(b & 0x7FFFu, b >> 16 & 0x7FFFu)));
   return __float_as_uint(mz_u16_to_float((uint16_t)mx, dtype)) >> 23;
 }
@@ -354,14 +355,15 @@ __device__ __forceinline__ uint32_t query_exponent(const uint16_t* q, int lane, 
 
 struct Place { int pair, step, b, kvh; };
 
-template <int BITS, int P, int GQA, bool HALF_META>
+template <int BITS, int P, int HD, int GQA, bool HALF_META>
 __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(const MzDecodeParams p, const uint32_t two16) {
   using C = Cfg<BITS, P>;
   constexpr int WORKERS = C::WORKERS;
   constexpr int QB = G * BITS / 8;            // bytes of a packed row of 64 codes
   constexpr int NW = QB / 4;                  // words of it
-  constexpr int CODE_BYTES = D * QB;          // packed bytes of one tile side
-  constexpr int VROW = 2 * QB;                // bytes of one token's 128 value codes
+  constexpr int NG = HD / G;                  // channel groups of a token
+  constexpr int CODE_BYTES = HD * QB;         // packed bytes of one tile side
+  constexpr int VROW = NG * QB;               // bytes of one token's value codes
   extern __shared__ __align__(128) uint8_t smem[];
   const mz_kv_store& s = p.s;
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);            // uniform: the descriptors stay in uniform registers
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
     }
     more_registers<DENSE_REGS>();
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    mzd::dense_tiles<GQA>(p, p.tp2, p.slots_a, ((int)blockIdx.x - p.hetero) * DENSE_WARPS + warp,
+    mzd::dense_tiles<HD, GQA>(p, p.tp2, p.slots_a, ((int)blockIdx.x - p.hetero) * DENSE_WARPS + warp,
                           (uint32_t)__cvta_generic_to_shared(smem) + warp * mzd::WARP_BYTES);
     return;
   }
@@ -425,6 +427,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
 
   // rows in flight, one of either group: codes and metadata as loaded (16-bit metadata in the low half)
   uint32_t code[2][NW], lo[2], span[2];
+  const int channel = r & (HD - 1);                                   // keys: its channel (64 of them: the other threads have no rows)
   const int half = r >> 6;                                            // values: group of this thread's token; also of its row of the results
   const int spot = (r & 0x70) + chunk_code<BITS>(r & 15);             // values: its token of a step, and its channel of the output
   // Keys: channel r of the step's two groups (a last half step reads its group twice); values: token `spot` with its two channel groups (in a
@@ -436,8 +439,8 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
   auto point = [&]() {
     const int kvh = ahead.kvh >> p.kv_share;
     const long long tile = STEP_GROUPS * ahead.step;
-    const long long row = keys ? r : half * G + (spot & 63);
-    const long long m = keys ? ahead.b * s.km_stride_b + kvh * s.km_stride_h + tile * D + row : ahead.b * s.vm_stride_b + kvh * s.vm_stride_h + (tile * G + row) * 2;
+    const long long row = keys ? channel : half * G + (spot & 63);
+    const long long m = keys ? ahead.b * s.km_stride_b + kvh * s.km_stride_h + tile * HD + row : ahead.b * s.vm_stride_b + kvh * s.vm_stride_h + (tile * G + row) * NG;
     code_at = keys ? s.packed_k + ahead.b * s.pk_stride_b + kvh * s.pk_stride_h + tile * CODE_BYTES + row * QB
                    : s.packed_v + ahead.b * s.pv_stride_b + kvh * s.pv_stride_h + (tile * G + row) * VROW;
     mn_at = (const uint8_t*)(keys ? s.k_mn : s.v_mn) + m * msz;
@@ -450,12 +453,12 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       point();
     } else {
       code_at += STEP_GROUPS * CODE_BYTES;
-      mn_at += STEP_GROUPS * D * msz;
-      span_at += STEP_GROUPS * D * msz;
+      mn_at += STEP_GROUPS * HD * msz;
+      span_at += STEP_GROUPS * HD * msz;
     }
   };
   // bytes (codes) / elements (metadata) from the first row's to this thread's row of either group
-  const int x_codes = keys ? CODE_BYTES : QB, x_meta = keys ? D : 1;
+  const int x_codes = keys ? CODE_BYTES : (NG - 1) * QB, x_meta = keys ? HD : NG - 1;     // (one channel group: the row twice, not used)
   const uint8_t* code_next;                                           // codes of the step that comes next
   int code_second;
   auto load_meta = [&]() {                                            // and keeps where the codes are
@@ -466,8 +469,8 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       else if (half) back = -G;
       code_next += back * VROW;
     }
-    const uint8_t* a = mn_at + back * 2 * msz;
-    const uint8_t* b = span_at + back * 2 * msz;
+    const uint8_t* a = mn_at + back * NG * msz;
+    const uint8_t* b = span_at + back * NG * msz;
     if (HALF_META || !meta32) {
       lo[0] = __ldg((const uint16_t*)a); lo[1] = __ldg((const uint16_t*)a + second);
       span[0] = __ldg((const uint16_t*)b); span[1] = __ldg((const uint16_t*)b + second);
@@ -512,9 +515,10 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
     const uint4 v = lds128(at);
     return max(max(v.x, v.y), max(v.z, v.w)) >> 23;
   };
-  auto put_folds = [&](const float (&x)[GQA], float down0, float down1) {
+  auto put_folds = [&](const float (&x)[GQA], float down0, float down1, int groups) {
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
+      if (k >= groups) break;
       const float sx = rows[k].s * (k ? down1 : down0);
       uint32_t d[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -536,7 +540,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
           tm_fence_after();
           if (elect_one()) {
             bar_arrive(red + BAR_KDONE);                              // hands on what the team has noted
-            umma_side<BITS, P>(tm_k, key_values, key_folds);
+            umma_side<BITS, P, HD / 32>(tm_k, key_values, key_folds);
             umma_commit(red + BAR_KDONE);
           }
           __syncwarp();
@@ -545,7 +549,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
           join_team(2 * wk + 1);
           tm_fence_after();
           if (elect_one()) {
-            umma_side<BITS, P>(tm_v, value_values, value_folds);
+            umma_side<BITS, P, 4>(tm_v, value_values, value_folds);
             umma_commit(red + BAR_VDONE);
           }
           __syncwarp();
@@ -574,19 +578,20 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
 #pragma unroll
         for (int g = 0; g < GQA; ++g) {
           const uint16_t* q = (const uint16_t*)p.query + cur.b * p.q_stride_b + (long long)(cur.kvh * GQA + g) * p.q_stride_h;
-          qn[g] = mz_u16_to_float(q[r], s.kv_dtype) * (scale_down(query_exponent(q, lane, s.kv_dtype)) * C::FOLD_FULL);
+          qn[g] = mz_u16_to_float(q[channel], s.kv_dtype) * (scale_down(query_exponent<HD>(q, lane, s.kv_dtype)) * C::FOLD_FULL);
         }
       }
       const uint32_t ex = exponent_of_largest(red + RED_SK + 16 * par);
       if (i > 0) bar_wait<64>(red + BAR_KDONE, (uint32_t)(i - 1) & 1, failed);       // the operands have been read
-      expand_row<BITS, P, NW>(code[0], rows[0], book, side + r * 16, two16);
+      const bool own = HD == 128 || w < 2;                            // this warp has rows
+      if (own) expand_row<BITS, P, NW>(code[0], rows[0], book, side + r * 16, two16);
       if (more) load_codes(0);
-      expand_row<BITS, P, NW>(code[1], rows[1], book, side + 8192 + r * 16, two16);
+      if (own) expand_row<BITS, P, NW>(code[1], rows[1], book, side + 8192 + r * 16, two16);
       if (more) load_codes(1);
       const float down = scale_down(ex);
-      put_folds(qn, down, down);
+      if (own) put_folds(qn, down, down, 2);
       // constant term sum_d q[h][d] A_d per group and head (rows whose range does not straddle zero): this warp's part
-      const bool any = __any_sync(0xffffffffu, rows[0].A != 0.0f || rows[1].A != 0.0f);
+      const bool any = own && __any_sync(0xffffffffu, rows[0].A != 0.0f || rows[1].A != 0.0f);
       if (any) {
 #pragma unroll
         for (int x = 0; x < 2; ++x)
@@ -628,7 +633,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       for (int g = 0; g < GQA; ++g) {
         l_part[g] = out[g] = 0.f;
         const uint16_t* q = (const uint16_t*)p.query + c.b * p.q_stride_b + (long long)(c.kvh * GQA + g) * p.q_stride_h;
-        const uint32_t ex = query_exponent(q, lane, s.kv_dtype);
+        const uint32_t ex = query_exponent<HD>(q, lane, s.kv_dtype);
         if (r == 0) stsf(red + RED_QS + 4 * g, scale_up(ex) * p.scaling * (LOG2E * C::UNIT));     // read behind the next barrier but one
       }
       if (r < 2) sts128(red + RED_RUN + 16 * r, make_uint4(0xFF800000u, 0xFF800000u, 0xFF800000u, 0xFF800000u));
@@ -669,7 +674,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
             bs += ldsf(red + RED_END + k * 64 + 16 * half + 4 * g);
             lt += ldsf(red + RED_END + k * 64 + 32 + 4 * g);
           }
-          p.part.acc[(slot0 + g) * D + spot] = out[g] + bs;
+          if (HD == 128 || r < HD) p.part.acc[(slot0 + g) * HD + spot] = out[g] + bs;
           if (r == 0) {
             p.part.m[slot0 + g] = failed ? INFINITY : ldsf(red + RED_RUN + 16 * par + 4 * g) * (1.0f / LOG2E);   // a wait ran out: +inf turns the merged output into NaN
             p.part.l[slot0 + g] = lt;
@@ -690,7 +695,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       advance(nxt);
       prepare();
       publish_largest(red + RED_SV + 32 * par, magnitude(0));
-      publish_largest(red + RED_SV + 32 * par + 16, magnitude(1));
+      if (NG == 2) publish_largest(red + RED_SV + 32 * par + 16, magnitude(1));
       const bool more = i + 1 < steps;
       if (more) { move_ahead(); load_meta(); }
       const bool live = STEP_GROUPS * cur.step + half < kt;
@@ -761,10 +766,10 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
           if (has_base && (lane & 3) == g) base_sum *= c;
         }
         // constant terms of the output (rows whose range does not straddle zero)
-        has_base |= __any_sync(0xffffffffu, rows[0].A != 0.0f || rows[1].A != 0.0f);
+        has_base |= __any_sync(0xffffffffu, rows[0].A != 0.0f || (NG == 2 && rows[1].A != 0.0f));
         if (has_base) {
 #pragma unroll
-          for (int x = 0; x < 2; ++x)
+          for (int x = 0; x < NG; ++x)
 #pragma unroll
             for (int g = 0; g < GQA; ++g) {
               float v = lg[g] * rows[x].A;
@@ -777,13 +782,15 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
         for (int g = 0; g < GQA; ++g) lg[g] *= C::FOLD_FULL;
       }
       // ================= values: token `spot`, its two channel groups =================
-      const uint32_t ex0 = exponent_of_largest(red + RED_SV + 32 * par), ex1 = exponent_of_largest(red + RED_SV + 32 * par + 16);
+      const uint32_t ex0 = exponent_of_largest(red + RED_SV + 32 * par), ex1 = NG == 2 ? exponent_of_largest(red + RED_SV + 32 * par + 16) : ex0;
       up_v = scale_up(half ? ex1 : ex0) * C::UNIT;
-      put_folds(lg, scale_down(ex0), scale_down(ex1));
+      put_folds(lg, scale_down(ex0), scale_down(ex1), NG);
       expand_row<BITS, P, NW>(code[0], rows[0], book, side + r * 16, two16);
       if (more) load_codes(0);
-      expand_row<BITS, P, NW>(code[1], rows[1], book, side + 8192 + r * 16, two16);
-      if (more) load_codes(1);
+      if (NG == 2) {
+        expand_row<BITS, P, NW>(code[1], rows[1], book, side + 8192 + r * 16, two16);
+        if (more) load_codes(1);
+      }
       proxy_fence();
       tm_fence_before();
       team_ready(team);
@@ -804,9 +811,9 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(C::TM_ALLOC));
 }
 
-template <int BITS, int P, int GQA, bool HALF_META>
+template <int BITS, int P, int HD, int GQA, bool HALF_META>
 int launch_one(const MzDecodeParams& p, cudaStream_t st) {
-  auto kern = decode_umma_kernel<BITS, P, GQA, HALF_META>;
+  auto kern = decode_umma_kernel<BITS, P, HD, GQA, HALF_META>;
   MZ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BITS, P>::SMEM));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.hetero > 0 ? p.tp.ctas + p.tp2.ctas : p.tp.ctas));
@@ -822,20 +829,20 @@ int launch_one(const MzDecodeParams& p, cudaStream_t st) {
   MZ_LAUNCH_CHECK("decode_umma");
   return MZ_OK;
 }
-template <int BITS, int P>
+template <int BITS, int P, int HD>
 int launch_gqa(const MzDecodeParams& p, cudaStream_t st) {
   const bool half = p.s.meta_dtype == MZ_F16;
   switch (p.gqa) {
-    case 1: return half ? launch_one<BITS, P, 1, true>(p, st) : launch_one<BITS, P, 1, false>(p, st);
-    case 2: return half ? launch_one<BITS, P, 2, true>(p, st) : launch_one<BITS, P, 2, false>(p, st);
-    case 4: return half ? launch_one<BITS, P, 4, true>(p, st) : launch_one<BITS, P, 4, false>(p, st);
+    case 1: return half ? launch_one<BITS, P, HD, 1, true>(p, st) : launch_one<BITS, P, HD, 1, false>(p, st);
+    case 2: return half ? launch_one<BITS, P, HD, 2, true>(p, st) : launch_one<BITS, P, HD, 2, false>(p, st);
+    case 4: return half ? launch_one<BITS, P, HD, 4, true>(p, st) : launch_one<BITS, P, HD, 4, false>(p, st);
   }
   return mz_fail(MZ_ERR_UNSUPPORTED, "gqa %d", p.gqa);
 }
 }  // namespace mzu
 
 bool mz_decode_umma_supported(const MzDecodeParams& p) {
-  return mz_decode_mma_supported(p) && p.s.head_dim == 128 && p.s.group == 64 && p.s.bits <= 4 &&
+  return mz_decode_mma_supported(p) && (p.s.head_dim == 64 || p.s.head_dim == 128) && p.s.group == 64 && p.s.bits <= 4 &&
          (p.gqa == 1 || p.gqa == 2 || p.gqa == 4 || p.gqa == 8) && p.s.k_groups > 0;
 }
 
@@ -877,14 +884,14 @@ int mz_plan_umma(MzDecodeParams& p, bool full_precision, int splits_request, int
     p.s.kv_heads *= 2;
     p.kv_share = 1;
   }
-  p.planes = s.bits == 1 ? 1 : s.bits == 2 && !full_precision ? 2 : 3;
+  p.planes = s.bits == 1 ? 1 : s.bits == 2 && s.head_dim == 128 && !full_precision ? 2 : 3;
   const int workers = p.planes == 3 ? mzu::Cfg<3, 3>::WORKERS : mzu::Cfg<2, 2>::WORKERS;
   const int steps = (s.k_groups + mzu::STEP_GROUPS - 1) / mzu::STEP_GROUPS;
   const long long pairs = (long long)s.batch * s.kv_heads;
   const int dense_tiles = (s.res_len + mzd::DT - 1) / mzd::DT;
   int n_d = 0;
   if (dense_tiles > 0) {
-    const float dense = (float)dense_tiles * kDenseTileUs, packed = (float)steps * step_us(s.bits, p.planes);
+    const float dense = (float)dense_tiles * kDenseTileUs, packed = (float)steps * step_us(s.bits, p.planes) * (s.head_dim == 64 ? 0.6f : 1.0f);
     n_d = (int)((float)sm_count * dense / (dense + packed) + 0.5f);
     if (n_d < 1) n_d = 1;
     if (n_d > sm_count / 2) n_d = sm_count / 2;
@@ -908,12 +915,22 @@ int mz_plan_umma(MzDecodeParams& p, bool full_precision, int splits_request, int
 }
 
 int mz_launch_decode_umma(const MzDecodeParams& p, cudaStream_t st) {
-  switch (p.s.bits * 16 + p.planes) {
-    case 0x11: return mzu::launch_gqa<1, 1>(p, st);
-    case 0x22: return mzu::launch_gqa<2, 2>(p, st);
-    case 0x23: return mzu::launch_gqa<2, 3>(p, st);
-    case 0x33: return mzu::launch_gqa<3, 3>(p, st);
-    case 0x43: return mzu::launch_gqa<4, 3>(p, st);
+  const int which = p.s.bits * 16 + p.planes;
+  if (p.s.head_dim == 64) {
+    switch (which) {
+      case 0x11: return mzu::launch_gqa<1, 1, 64>(p, st);
+      case 0x23: return mzu::launch_gqa<2, 3, 64>(p, st);
+      case 0x33: return mzu::launch_gqa<3, 3, 64>(p, st);
+      case 0x43: return mzu::launch_gqa<4, 3, 64>(p, st);
+    }
+  } else {
+    switch (which) {
+      case 0x11: return mzu::launch_gqa<1, 1, 128>(p, st);
+      case 0x22: return mzu::launch_gqa<2, 2, 128>(p, st);
+      case 0x23: return mzu::launch_gqa<2, 3, 128>(p, st);
+      case 0x33: return mzu::launch_gqa<3, 3, 128>(p, st);
+      case 0x43: return mzu::launch_gqa<4, 3, 128>(p, st);
+    }
   }
   return mz_fail(MZ_ERR_UNSUPPORTED, "bits %d, %d planes", p.s.bits, p.planes);
 }

@@ -1,4 +1,4 @@
-// Residual (un-quantized) tiles of 16 tokens on mma.sync, head_dim 128: one warp walks the tiles of a plan that has no packed
+// Residual (un-quantized) tiles of 16 tokens on mma.sync, head_dim HD (64 or 128): one warp walks the tiles of a plan that has no packed
 // tiles and leaves a partial record per (batch, kv head) pair.  A tile is a short latency-bound chain (3 us), so a launch
 // gives these warps CTAs of their own beside the packed tiles'.
 //
@@ -11,14 +11,14 @@
 namespace mzd {
 using namespace mzm;
 constexpr int DT = 16;                      // tokens per tile
-constexpr int STRIDE = 2 * D + 16;          // padded row of a staged tile (bank spread)
-constexpr int TILE_BYTES = DT * STRIDE;
+constexpr int TILE_BYTES = DT * (2 * 128 + 16);            // rows are padded (bank spread)
 constexpr int PROB_BYTES = DT * 16;         // probabilities [16 tokens][4 heads]
 constexpr int WARP_BYTES = 2 * TILE_BYTES + PROB_BYTES;
 
 // warp `gw` of plan `tp`; `buf` is the shared-window address of its WARP_BYTES, records from `first_record` (in records of one head) on
-template <int GQA>
+template <int HD, int GQA>
 __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTilesPlan& tp, long long first_record, int gw, uint32_t buf) {
+  constexpr int STRIDE = 2 * HD + 16, PIECES = HD / 8;
   const mz_kv_store& s = p.s;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int hq = g >> 1;                    // head whose query and probabilities this lane supplies (B column g)
@@ -37,15 +37,15 @@ __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTil
       if (++c.kvh == s.kv_heads) { c.kvh = 0; ++c.b; }
     }
   };
-  // up to 16 rows of 128 elements; rows past the end are zeroed (they meet probability 0, which must not meet a NaN bit pattern).  The
+  // up to 16 rows of HD elements; rows past the end are zeroed (they meet probability 0, which must not meet a NaN bit pattern).  The
   // newest token may still be in the caller's tensors (p.new_k / new_v): it is staged from there, and stored into the window
   auto stage = [&](uint32_t dst, void* window, const void* fresh, const Cursor& c, bool valid) {
     if (valid) {
       const int tok0 = c.tile * DT, ntok = min(DT, s.res_len - tok0), kvh = c.kvh >> p.kv_share;
       const int newest = fresh != nullptr ? s.res_len - 1 - tok0 : -1;
       uint16_t* src = (uint16_t*)window + c.b * s.res_stride_b + kvh * s.res_stride_h + (long long)(s.res_start + tok0) * s.res_stride_t;
-      for (int i = lane; i < DT * 16; i += 32) {
-        const int row = i >> 4, k = i & 15;
+      for (int i = lane; i < DT * PIECES; i += 32) {
+        const int row = i / PIECES, k = i % PIECES;
         if (row < ntok) {
           const uint16_t* from = src + (long long)row * s.res_stride_t + k * 8;
           if (row == newest) {
@@ -60,12 +60,12 @@ __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTil
     cp_async_commit();
   };
 
-  float out[8][4];          // M tile m: channels (m < 4 ? 0 : 64) + 8g + 2(m%4) + {0,1}, head t, columns {value, remainder}
+  float out[HD / 16][4];    // M tile m: channels (m < 4 ? 0 : 64) + 8g + 2(m%4) + {0,1}, head t, columns {value, remainder}
   float m_st = -INFINITY, l_st = 0.f;       // softmax state of head t (l: this lane's tokens only)
   int cur_pair = -1, seg = 0;
   auto reset = [&]() {
 #pragma unroll
-    for (int m = 0; m < 8; ++m)
+    for (int m = 0; m < HD / 16; ++m)
 #pragma unroll
       for (int k = 0; k < 4; ++k) out[m][k] = 0.f;
     m_st = -INFINITY; l_st = 0.f;
@@ -77,9 +77,9 @@ __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTil
     if (t < GQA) {
       const long long slot = first_record + ((long long)gw * tp.max_segs + seg) * GQA + t;
       if (!MZ_IN_BOUNDS(slot, p.part.slots, 10)) return;
-      float* dst = p.part.acc + slot * D + 8 * g;
+      float* dst = p.part.acc + slot * HD + 8 * g;
 #pragma unroll
-      for (int h = 0; h < 4; ++h)           // channels 0..3, 4..7 of the lower and of the upper half
+      for (int h = 0; h < HD / 32; ++h)     // channels 0..3, 4..7 of the lower and of the upper half
         *(float4*)(dst + (h >> 1) * 64 + (h & 1) * 4) = make_float4(out[2 * h][0] + out[2 * h][1], out[2 * h][2] + out[2 * h][3],
                                                                     out[2 * h + 1][0] + out[2 * h + 1][1], out[2 * h + 1][2] + out[2 * h + 1][3]);
       if (g == 0) {
@@ -112,7 +112,7 @@ __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTil
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     const bool fold_lane = (g & 1) == 0 && hq < GQA;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < HD / 16; ++j) {
       const uint32_t ka = kbuf + g * STRIDE + (16 * j + 2 * t) * 2;
       const uint32_t a0 = lds32(ka), a1 = lds32(ka + 8 * STRIDE), a2 = lds32(ka + 16), a3 = lds32(ka + 8 * STRIDE + 16);
       const uint32_t b0 = fold_lane ? *(const uint32_t*)(qrow + 16 * j + 2 * t) : 0u;
@@ -143,7 +143,7 @@ __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTil
     m_st = m_new;
     if (__any_sync(0xffffffffu, c != 1.0f)) {
 #pragma unroll
-      for (int m = 0; m < 8; ++m)
+      for (int m = 0; m < HD / 16; ++m)
 #pragma unroll
         for (int k = 0; k < 4; ++k) out[m][k] *= c;
     }
@@ -176,7 +176,7 @@ __device__ __forceinline__ void dense_tiles(const MzDecodeParams& p, const MzTil
       }
     }
 #pragma unroll
-    for (int grp = 0; grp < 2; ++grp) {
+    for (int grp = 0; grp < HD / 64; ++grp) {
       const uint32_t va = vbuf + (2 * t) * STRIDE + (grp * 64 + 8 * g) * 2;
       const uint4 x0 = lds128(va), x1 = lds128(va + STRIDE), x2 = lds128(va + 8 * STRIDE), x3 = lds128(va + 9 * STRIDE);
       const uint32_t c0[4] = {x0.x, x0.y, x0.z, x0.w}, c1[4] = {x1.x, x1.y, x1.z, x1.w};
