@@ -1,14 +1,15 @@
 // Store -> dense keys and values: a range of the packed prefix, optionally followed by the residual window, in one
 // launch.  Bit-exact with the reference's fp32 dequantizer (muzero/quantizer.py:229-266).
 // Measured (8 x 8 x 4224 tokens, head_dim 128, 4 bits, call included): 721 us as two dequantizers, conversions and
-// concatenations, 65.6 us now (0.42 of the copy rate).
+// concatenations, 65.6 us with every value evaluated, 61.0 us now (0.45 of the copy rate).
 //
 // head_dim 64 / 128, groups of 32 / 64 / 128 that divide it, 16-bit output: bound by HBM (the output is 4 to 16 times
 // the packed input).  Keys are packed along tokens and written along channels, so a key tile is staged in shared
 // memory and a thread takes two neighbouring channels of 16 tokens (one 4-byte store per token, 128 bytes per warp
 // row); with codes of up to 4 bits each channel gets a 2^bits-entry book of finished 16-bit values, laid out entry-major
 // so that the 32 lanes of a lookup always hit 32 different half-bank pairs.  Values are packed the way they are
-// written; a thread takes 16 channels of a row and evaluates them directly.
+// written; a thread takes 16 channels of a row.  Up to 4 bits the row's lanes share out the evaluation of its 2^bits entries and look
+// them up by byte permute; wider codes are evaluated one by one.
 #include "mz_quant_math.cuh"
 #include "mz_store.cuh"
 
@@ -143,6 +144,52 @@ __device__ __forceinline__ void dense_keys(const DenseParams& p, uint8_t* smem) 
   }
 }
 
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
+// eight codes (LSB first) in the nibbles of a word
+template <int BITS>
+__device__ __forceinline__ uint32_t nibbles(uint32_t x) {
+  if (BITS == 4) return x;
+  if (BITS == 3) {
+    x = (x & 0x00FFF000u) * 15u + x;
+    x = (x & 0x0FC00FC0u) * 3u + x;
+    return (x & 0x38383838u) + x;
+  }
+  if (BITS == 2) {
+    x = (x | x << 8) & 0x00FF00FFu;
+    x = (x | x << 4) & 0x0F0F0F0Fu;
+    return (x | x << 2) & 0x33333333u;
+  }
+  x = (x | x << 12) & 0x000F000Fu;
+  x = (x | x << 6) & 0x03030303u;
+  return (x | x << 3) & 0x11111111u;
+}
+// eight codes -> eight 16-bit values, out of a book in registers (low and high bytes of its entries, four to a word)
+template <int BITS, int N>
+__device__ __forceinline__ uint4 book_values(uint32_t codes, const uint32_t (&lo)[N], const uint32_t (&hi)[N]) {
+  const uint32_t x = nibbles<BITS>(codes);
+  uint32_t v[4];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    uint32_t l, h;
+    if (BITS == 4) {
+      const uint32_t sel = (x >> (16 * k)) & 0x7777u, m = prmt(0u, 0xFFFFFFFFu, (x >> (16 * k + 1)) & 0x4444u);
+      l = (prmt(lo[0], lo[1 % N], sel) & ~m) | (prmt(lo[N / 2], lo[N - 1], sel) & m);
+      h = (prmt(hi[0], hi[1 % N], sel) & ~m) | (prmt(hi[N / 2], hi[N - 1], sel) & m);
+    } else {
+      const uint32_t sel = x >> (16 * k);
+      l = prmt(lo[0], lo[N - 1], sel);
+      h = prmt(hi[0], hi[N - 1], sel);
+    }
+    v[2 * k] = prmt(l, h, 0x5140u);
+    v[2 * k + 1] = prmt(l, h, 0x7362u);
+  }
+  return make_uint4(v[0], v[1], v[2], v[3]);
+}
+
 // A CTA takes kValChunks x 256 / lanes-per-row rows; the codes and metadata of all of a thread's rows are in flight before the
 // table is staged (one chunk per CTA spent most of its life in those two latencies).
 constexpr int kValChunks = 4;
@@ -182,14 +229,47 @@ __device__ __forceinline__ void dense_values(const DenseParams& p, unsigned blk,
     const long long at = (long long)pair * p.sv * D + (long long)row * G;
     if (!MZ_IN_BOUNDS(at + G - 1, (long long)s.batch * s.kv_heads * p.sv * D, 19)) continue;
     uint16_t* dst = (uint16_t*)p.out_v + at;
+    if constexpr (BITS <= 4) {
+      // the row's book of finished values, four entries to a word; its lanes (2, 4 or 8) share the words out.  16 codes per lane took 16
+      // evaluations of the exact chain, 4 (4 bits in groups of 32: 8) and a permute lookup are what is left
+      constexpr int N = NE < 4 ? 1 : NE / 4;
+      const int share = min(lpr, N), lane = threadIdx.x & 31;
+      uint32_t lo_own[2] = {0, 0}, hi_own[2] = {0, 0}, blo[N], bhi[N];
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      uint32_t v[4];
+      for (int c = 0; c < (N == 4 ? 2 : 1); ++c) {
+        const int word = sub % share + c * share;
+        if (word >= N) break;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        v[i] = pack16<DT>(mz_dequant_exact(r, (int)(w[k][c] >> (2 * i * BITS)) & top, table, NE),
-                          mz_dequant_exact(r, (int)(w[k][c] >> ((2 * i + 1) * BITS)) & top, table, NE));
-      *(uint4*)(dst + (sub + c * lpr) * 8) = make_uint4(v[0], v[1], v[2], v[3]);
+        for (int e = 0; e < 4 && e < NE; ++e) {
+          const uint32_t v = to16<DT>(mz_dequant_exact(r, 4 * word + e, table, NE));
+          lo_own[c] |= (v & 0xff) << (8 * e);
+          hi_own[c] |= (v >> 8) << (8 * e);
+        }
+      }
+      if (N == 1) {
+        blo[0] = lo_own[0]; bhi[0] = hi_own[0];
+      } else {
+        const unsigned row_lanes = ((1u << lpr) - 1u) << (lane & ~(lpr - 1));
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          const int from = (lane & ~(lpr - 1)) | (j % share);
+          const bool second = j >= share;
+          blo[j] = __shfl_sync(row_lanes, second ? lo_own[1] : lo_own[0], from);
+          bhi[j] = __shfl_sync(row_lanes, second ? hi_own[1] : hi_own[0], from);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) *(uint4*)(dst + (sub + c * lpr) * 8) = book_values<BITS, N>((uint32_t)w[k][c], blo, bhi);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          v[i] = pack16<DT>(mz_dequant_exact(r, (int)(w[k][c] >> (2 * i * BITS)) & top, table, NE),
+                            mz_dequant_exact(r, (int)(w[k][c] >> ((2 * i + 1) * BITS)) & top, table, NE));
+        *(uint4*)(dst + (sub + c * lpr) * 8) = make_uint4(v[0], v[1], v[2], v[3]);
+      }
     }
   }
 }

@@ -289,3 +289,26 @@ def test_logq_layout_matches_reference(oracle, golden, name, hf_strides, monkeyp
     assert (out.cpu() - ref).abs().max().item() <= 2e-3
     k_full, v_full = layer._full_kv()
     assert k_full.shape == v_full.shape and k_full.shape[2] == meta["S"] + meta["steps"]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D,group", [(128, 32), (128, 64), (128, 128), (64, 32), (64, 64)])
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 5])
+def test_dense_values_from_books(oracle, bits, D, group, dtype):
+    """The values of a dense read-back, bit for bit: books shared by 2, 4 and 8 lanes and the widths without one; rows that do not fill the last
+    chunk, one-sided and symmetric rows."""
+    import muzero_b200 as mz
+    S = 128 + 3 * group + 11
+    k, v, _ = oracle.synth_kv(2, 3, S, D, 3, seed=bits + group, dtype=dtype)
+    v[0] -= 3.0
+    v[1, 0, :, :group:2], v[1, 0, :, 1:group:2] = 1.5, -1.5
+    ref = oracle.OracleCacheLayer(bits=bits, group=group, residual=128)
+    ref.append(k, v)
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=group, residual_length=128)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+    keys, values = layer._full_kv()
+    kp, vp = ref.key_prefix(dtype), ref.value_prefix(dtype)
+    assert np.array_equal(bits16(keys[:, :, :kp.shape[2]].contiguous()), bits16(kp))
+    assert np.array_equal(bits16(values[:, :, :vp.shape[2]].contiguous()), bits16(vp))
