@@ -423,18 +423,29 @@ int mz_plan_mma(MzDecodeParams& p, int splits_request, int sm_count, size_t* slo
     take_lookup_entries(q);
     return true;
   };
+  bool decided = false;                           // cluster mode has been planned already, and does not pay
   if (splits_request == 0 && mz_decode_umma_supported(p)) {
-    MzDecodeParams c = p, t = p;
-    const bool clusters = plan_cluster(c, k, sm_count), flat = mz_decode_flat_supported(p);
-    size_t n = 0;
-    if (choose_umma(p, c, clusters, sm_count) && mz_plan_umma(t, clusters || !flat, 0, sm_count, &n) == MZ_OK &&
-        (p.scratch_limit == 0 || n * sizeof(float) * (2 + (size_t)p.s.head_dim) <= p.scratch_limit)) {
-      p = t;
-      *slots = n;
+    MzDecodeParams c = p;
+    const bool clusters = plan_cluster(c, k, sm_count);
+    if (choose_umma(p, c, clusters, sm_count)) {
+      MzDecodeParams t = p;
+      size_t n = 0;
+      if (mz_plan_umma(t, clusters || !mz_decode_flat_supported(p), 0, sm_count, &n) == MZ_OK &&
+          (p.scratch_limit == 0 || n * sizeof(float) * (2 + (size_t)p.s.head_dim) <= p.scratch_limit)) {
+        p = t;
+        *slots = n;
+        return MZ_OK;
+      }
+    }
+    if (clusters) {
+      p = c;
+      *slots = 4;
+      take_lookup_entries(p);
       return MZ_OK;
     }
+    decided = true;
   }
-  if (clustered(p, false)) return MZ_OK;
+  if (!decided && clustered(p, false)) return MZ_OK;
   p.cluster = 0;
   MzDecodeParams other = p;
   const int rc = plan_cut(p, k, splits_request, sm_count, slots);
