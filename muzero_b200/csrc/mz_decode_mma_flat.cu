@@ -1,5 +1,5 @@
 // Tensor-core decode attention, one fully unrolled instance family: head_dim 128, group 64, 2- and 4-bit codes, 1 / 2 / 4
-// query heads per kv head, on a machine-filling grid.
+// query heads per kv head, on a machine-filling grid (2 bits: with explicit splits; else the tcgen05 kernel has them).
 //
 // The mathematics is that of mz_decode_mma.cuh.  This variant keeps the query and the zero codes of all 16 reduction blocks in
 // registers and the blocks unrolled, so a block costs fewer shared-memory wavefronts (4 instead of 7 besides its

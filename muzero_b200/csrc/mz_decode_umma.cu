@@ -21,8 +21,8 @@
 // What bounds it: issue (58 % of the cycles; per row of 64 two-bit codes about 230 instructions, of which 32 permutes) and the logic pipe
 // (48 %, two cycles per instruction); integer MMAs take 40 cycles each, all of it reading their operands, 41 %.  A thread that spills
 // is dear: 227 KB of shared memory leave 28 KB of L1, and 20 bytes of spill per thread cost 10 %.  Hence the register split.
-// 64 x 8 pairs x 4224 tokens, 4 heads, us per call: 1 bit 202 -> 93 (before: SIMT kernel), 2 bits 148 -> 120 (before: unrolled mma.sync
-// kernel), 3 bits 230 -> 180 (SIMT); 24 x 8 x 1537, 3 bits: 53 -> 37; one sequence of 1300 tokens, device time: 15 -> 8 to 11.
+// 64 x 8 pairs x 4224 tokens, 4 heads, us per call: 1 bit 202 -> 97 (before: SIMT kernel), 2 bits 148 -> 125 (before: unrolled mma.sync
+// kernel), 3 bits 230 -> 186 (SIMT); 24 x 8 x 1537, 3 bits: 53 -> 39; one sequence of 1300 tokens, device time: 15 -> 8 to 11.
 //
 // Precision: three planes hold a value to 2^-24 of its row's larger side and the fold to 2^-31 of the step's largest product, which is that of the
 // fp32 kernels (relative error against 64 bits 2e-7 to 9e-7; 1 bit is exact in one plane).  Two planes (2 bits, calls that the

@@ -272,8 +272,8 @@ def test_merge_kernels_at_their_boundary(oracle, D, group):
 @pytest.mark.parametrize("which,name", [(1, "generic"), (2, "tiles"), (3, "mma"), (4, "umma")])
 def test_every_kernel_against_the_oracle(oracle, which, name):
     """The four decode kernels on the same caches (4- and 2-bit, group 64, a pair boundary inside a worker's range,
-    an odd number of tiles, a mask): each within 2e-3 of the oracle.  `umma` is the tcgen05 / tensor-memory kernel,
-    which the automatic selection does not use yet."""
+    an odd number of tiles, a mask): each within 2e-3 of the oracle.  `umma` is the tcgen05 / tensor-memory kernel
+    for every call that it serves."""
     from muzero_b200.cache.attention import decode_attention
     from muzero_b200.kernels._cabi import load_library
     lib = load_library()
