@@ -340,17 +340,23 @@ bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count, bool an
   return false;
 }
 // Whether the tcgen05 kernel takes a call that it serves; `clusters`: the choice without it is cluster mode, planned in `c`.
-// head_dim 128, 1 to 3 bits: always.  Over 150 shapes of 0.1 to 210 tiles per SM it needs 0.55 (1 bit), 0.70 (3 bits) and 0.78 (2 bits) of the
-// time of the best other form, and is nowhere behind it by more than the timing's spread (device time of 90 calls below 12
+// head_dim 128, 1 to 3 bits: always but for the smallest calls (kOneLaunchTiles).  On the device, over 150 shapes of 0.1 to 210 tiles per SM it needs 0.55 (1 bit), 0.70 (3 bits) and 0.78 (2 bits) of the
+// time of the best other form, and is nowhere behind it by more than the timing's spread (90 calls below 12
 // tiles per SM: 0.49 to 0.92 of cluster mode).
 // 4 bits need two lookups per code, and three planes because the unrolled kernel's error (3e-5) is out of reach of two (4e-5 to 6e-5).
 // With up to four heads the unrolled kernel keeps its calls (64 x 8 pairs x 4224 tokens 149 us; 28 x 8 x 9800 49.9 against 72.7); cluster mode's
 // go by cost (1 x 8 x 17879 54 -> 30 us, 5 x 4 x 4988 30 -> 22; 15 x 8 x 459 would be 17.2 -> 19.5).  Eight heads run as two times four.
 // head_dim 64 halves the expansion and not the softmax, and cluster mode has less to gain from (48 shapes: 0.40 to 0.9 from about 8 tiles per
 // SM on, up to 1.5 below): by cost at every width.
+// One launch against two (kernel and merge): a small call takes less time on the device than the host needs for it, and there the second
+// launch costs about 2 us whatever the kernel does.  Drawn by packed tiles per SM (cluster mode's estimate does not tell these apart):
+// 16 steps of a generation at 2 bits in cluster mode and here, 0.3 tiles per SM (1 x 8 x 500 tokens) 361 and 389 us, 2.6 (4 x 8 x 900) 333 and
+// 370, 4.0 (2 x 8 x 2500) 405 and 366; one call at 3.1 (2 x 8 x 2000) 18.9 and 15.1.
+constexpr float kOneLaunchTiles = 3.f;
 constexpr float kUmmaBase = 14.5f, kUmmaBase8 = 15.0f;                          // us
 constexpr float kUmmaTile[4] = {0.30f, 0.55f, 0.72f, 1.0f}, kUmmaTile64 = 0.9f;  // us per packed tile on an SM [bits]; at head_dim 64 of it
 bool choose_umma(const MzDecodeParams& p, const MzDecodeParams& c, bool clusters, int sm_count) {
+  if (clusters && (float)((long long)p.s.batch * p.s.kv_heads * p.s.k_groups) < kOneLaunchTiles * (float)sm_count) return false;
   if (p.s.head_dim == 128 && p.s.bits < 4) return true;
   if (!clusters && mz_decode_flat_supported(p)) return false;
   MzTilesPlan t = {};

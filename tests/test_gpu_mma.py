@@ -157,7 +157,9 @@ def test_an_infinite_range_stays_in_its_group(oracle, bits, D, group, gqa):
 @pytest.mark.parametrize("bits,D,gqa,B,S", [(1, 128, 4, 3, 128 + 64), (1, 128, 2, 2, 128 + 5 * 64 + 63), (2, 128, 4, 3, 128 + 128), (2, 128, 1, 2, 128 + 3 * 64 + 1), (2, 128, 4, 24, 1111),
                                           (3, 128, 4, 3, 128 + 64 + 17), (3, 128, 1, 2, 128 + 128 + 1), (3, 128, 4, 20, 128 + 9 * 64), (1, 128, 4, 40, 700), (3, 128, 2, 2, 5000),
                                           (4, 128, 4, 3, 128 + 64 + 5), (4, 128, 1, 3, 2500), (4, 128, 8, 3, 700), (4, 128, 8, 20, 1000), (1, 128, 8, 2, 900), (2, 128, 8, 12, 777), (3, 128, 8, 3, 200), (1, 64, 4, 3, 330), (2, 64, 4, 3, 128 + 64 + 9), (2, 64, 2, 24, 600),
-                                            (3, 64, 1, 2, 1500), (4, 64, 4, 3, 700), (4, 64, 8, 2, 128 + 128), (3, 64, 4, 20, 900)])
+                                            (3, 64, 1, 2, 1500), (4, 64, 4, 3, 700), (4, 64, 8, 2, 128 + 128), (3, 64, 4, 20, 900),
+                                          # too many pairs or tiles for cluster mode, which takes calls below three tiles per SM
+                                          (1, 128, 4, 20, 128 + 64), (2, 128, 4, 20, 128 + 128), (3, 128, 4, 20, 128 + 64 + 17), (1, 128, 2, 2, 128 + 112 * 64 + 63)])
 def test_tcgen05_kernel(oracle, bits, D, gqa, B, S, meta):
     """One group, whole and half steps, one tile and many in the residual window, a worker's range over several pairs, ranges that do not
     straddle zero, symmetric ones, masked tokens and sequences.  Two-plane calls round a value to 2^-15 of its side:
