@@ -339,11 +339,12 @@ __device__ __forceinline__ float column_sum(const int (&c)[P][8], int at) {
   return fmaf((float)a[3], 65536.0f, (float)(a[1] + b[2] + d[3] + 256 * (a[2] + b[3]) + ((a[0] + b[1] + d[2]) >> 8)));
 }
 
-// power of two that brings a positive number of exponent field `ex` into [0.5, 1), and its inverse
+// power of two that brings a positive number of exponent field `ex` into [0.5, 1), and its inverse.  What is not finite has no digits: its
+// inverse is NaN, and so is every sum that it has a part in
 __device__ __forceinline__ float scale_down(uint32_t ex) {
   return __uint_as_float(ex <= 252u ? (253u - max(ex, 1u)) << 23 : 0x00800000u >> (ex - 252u));
 }
-__device__ __forceinline__ float scale_up(uint32_t ex) { return __uint_as_float(min(max(ex, 1u) + 1u, 255u) << 23); }
+__device__ __forceinline__ float scale_up(uint32_t ex) { return __uint_as_float(ex < 255u ? (max(ex, 1u) + 1u) << 23 : 0x7FFFFFFFu); }
 // exponent field of the largest magnitude of a head's query (HD elements of 16 bits)
 template <int HD>
 __device__ __forceinline__ uint32_t query_exponent(const uint16_t* q, int lane, int dtype) {
@@ -674,7 +675,8 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
             bs += ldsf(red + RED_END + k * 64 + 16 * half + 4 * g);
             lt += ldsf(red + RED_END + k * 64 + 32 + 4 * g);
           }
-          if (HD == 128 || r < HD) p.part.acc[(slot0 + g) * HD + spot] = out[g] + bs;
+          // a NaN probability has no digits either: what shows it is their sum
+          if (HD == 128 || r < HD) p.part.acc[(slot0 + g) * HD + spot] = lt == lt ? out[g] + bs : lt;
           if (r == 0) {
             p.part.m[slot0 + g] = failed ? INFINITY : ldsf(red + RED_RUN + 16 * par + 4 * g) * (1.0f / LOG2E);   // a wait ran out: +inf turns the merged output into NaN
             p.part.l[slot0 + g] = lt;

@@ -1,10 +1,24 @@
 """GPU: the tensor-core decode kernel at the edges of its tiles, widths and head sets, in its cluster and flat forms."""
+from contextlib import contextmanager
+
 import pytest
 import torch
 
 from test_gpu_attention import SPLIT_TOL, check_output
 
 pytestmark = pytest.mark.gpu
+
+
+@contextmanager
+def kernel(which):
+    """Decode calls inside go to one kernel (4: the tcgen05 kernel for all that it serves)."""
+    from muzero_b200.kernels._cabi import load_library
+    lib = load_library()
+    before = lib.mz_debug_force_kernel(which)
+    try:
+        yield
+    finally:
+        lib.mz_debug_force_kernel(before)
 
 
 @pytest.mark.parametrize("gqa,S,residual", [(1, 65, 64), (3, 300, 64), (4, 129 + 128, 128), (5, 450, 64), (8, 1000, 128), (7, 40, 64)])
@@ -151,6 +165,30 @@ def test_an_infinite_range_stays_in_its_group(oracle, bits, D, group, gqa):
     hit = torch.zeros(got.shape, dtype=torch.bool)
     hit[0, :, gqa:, group:2 * group] = True
     assert not bool(torch.isfinite(got[hit]).any()) and relative_error(got[~hit], want[~hit]) <= FP32_ERROR
+
+
+@pytest.mark.parametrize("bits,D,gqa", [(1, 128, 4), (2, 128, 2), (2, 128, 8), (3, 128, 4), (4, 128, 4), (4, 64, 8), (2, 64, 1)])
+def test_nan_stays_nan(oracle, bits, D, gqa):
+    """tcgen05 kernel: a NaN in the mask or in a query and an infinite key range make the heads that meet them NaN, as a floating-point
+    evaluation does, and no others (integer products have no NaN of their own)."""
+    import muzero_b200 as mz
+    from muzero_b200.cache.attention import decode_attention, decode_attention_partial
+    k, v, q = oracle.synth_kv(3, 2, 500, D, 2 * gqa, seed=bits)
+    q[1, gqa, 0, 3] = float("nan")
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=64, residual_length=128, alpha_key=2.0, alpha_value=2.0)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+    layer._key_scale[2, 0, 1, 5] = float("inf")
+    mask = torch.zeros(3, 1, 1, 500)
+    mask[0, ..., 70] = float("nan")
+    hit = torch.zeros(3, 1, 2 * gqa, D, dtype=torch.bool)
+    hit[0], hit[1, :, gqa], hit[2, :, :gqa] = True, True, True
+    with kernel(4):
+        got = decode_attention(layer, q.cuda(), D ** -0.5, mask.cuda(), out_dtype=torch.float32).cpu()
+        acc = decode_attention_partial(layer, q.cuda(), D ** -0.5, mask.cuda())[2].cpu().reshape(got.shape)
+    for out in (got, acc):
+        assert torch.equal(torch.isnan(out), hit) and bool(torch.isfinite(out[~hit]).all())
 
 
 @pytest.mark.parametrize("meta", [torch.float16, torch.bfloat16, torch.float32])
