@@ -24,9 +24,10 @@
 // 64 x 8 pairs x 4224 tokens, 4 heads, us per call: 1 bit 202 -> 97 (before: SIMT kernel), 2 bits 148 -> 125 (before: unrolled mma.sync
 // kernel), 3 bits 230 -> 186 (SIMT); 24 x 8 x 1537, 3 bits: 53 -> 39; one sequence of 1300 tokens, device time: 15 -> 8 to 11.
 //
-// Precision: three planes hold a value to 2^-24 of its row's larger side and the fold to 2^-31 of the step's largest product, which is that of the
-// fp32 kernels (relative error against 64 bits 2e-7 to 9e-7; 1 bit is exact in one plane).  Two planes (2 bits, calls that the
-// unrolled kernel served with 9e-5): 2^-15 and 2^-22, 2e-5 to 6e-5.  Any range is served: sides and query are scaled by powers of two.
+// Precision: three planes hold a value to 2^-24 of its row's larger side and a product to 4e-9 of the step's largest for its head and group, which
+// is no worse than the fp32 kernels (relative error against 64 bits 2e-7 to 7e-7 where those have 2e-7 to 1.1e-6, attention sinks, outlier
+// channels and tokens of unlike range included; 1 bit is exact in one plane).  Two planes (2 bits, calls that the unrolled kernel served): 2^-15
+// and 1e-6, 1e-5 to 4e-5 where the unrolled kernel has 5e-5 to 2e-4.  Any range is served: folds and query are scaled by powers of two.
 #include "mz_dense_tiles.cuh"
 
 namespace mzu {
@@ -56,25 +57,30 @@ struct Cfg {
   // smaller side, and for 4 bits the bytes of the upper eight entries, plane by plane
   static constexpr int MIXED = NE < 8 ? NE : 8, BOOK_ROW = BITS == 4 ? 96 : 8 * NE, BOOK_BYTES = ZC * BOOK_ROW;
   static constexpr float FULL = PLANES == 1 ? 1.0f : PLANES == 2 ? 32766.0f : 8388600.0f;      // fixed-point value of S
-  // fixed-point value of 1 in the folded operand (two planes: half of it; else its upper half), and what a unit of column_sum is worth
-  static constexpr float FOLD_FULL = PLANES == 2 ? 4161536.0f : 32000.0f;
+  // fixed-point value of 1 in the folded operand (two planes: half of it; else its upper half), and what a unit of column_sum is worth.  The
+  // largest number that the digits hold is 1.129 (two planes) or 1.125 of it: scales are powers of two, found to within a factor of 1.125
+  static constexpr float FOLD_FULL = PLANES == 2 ? 3700000.0f : 29000.0f;
   static constexpr float UNIT = (PLANES == 1 ? 1.0f / 65536.0f : PLANES == 2 ? 128.0f : 256.0f) / (FULL * FOLD_FULL);
   static constexpr int TM_SIDE = 32 * PLANES, TM_WORKER = 2 * TM_SIDE;   // tensor-memory columns: one accumulator per plane
   static constexpr int TM_ALLOC = WORKERS * TM_WORKER <= 256 ? 256 : 512;
   static constexpr int OFF_FOLD = PLANES * PLANE_BYTES, SIDE_BYTES = OFF_FOLD + FOLD_BYTES;      // operands of one side
-  static constexpr int OFF_RED = 2 * SIDE_BYTES, WORKER_BYTES = OFF_RED + 896;
+  static constexpr int OFF_RED = 2 * SIDE_BYTES, WORKER_BYTES = OFF_RED + 1792;
   static constexpr int BOOKS_BYTES = (2 * BOOK_BYTES + 127) / 128 * 128;
   static constexpr int SMEM = BOOKS_BYTES + WORKERS * WORKER_BYTES;
 };
 // exchange between a worker's warps, doubled by the step's parity where a fast warp may be a step ahead
-constexpr int RED_SK = 0;                        // [parity][warp] largest |S| of the keys
-constexpr int RED_SV = 32;                       // [parity][group][warp] of the values: what is not finite stays in its group
-constexpr int RED_MAX = 96;                      // [parity][warp][4] largest logit
-constexpr int RED_EX = 224, RED_FLAG = 240, RED_CA = 272;  // [parity] exponent of the keys; [parity][warp] whether there is a constant term; [parity][warp][group][4] its parts
-constexpr int RED_QS = RED_CA + 256;             // [4] logit per unit of column_sum
-constexpr int RED_RUN = RED_QS + 16;            // [parity][4] running maximum of the logits (base 2)
-constexpr int RED_END = RED_RUN + 32;             // [warp][16]: constant terms of the output [group][4], sum of probabilities [4]
-constexpr int RED_BARS = RED_END + 256, BAR_KDONE = RED_BARS, BAR_KFREE = RED_BARS + 8, BAR_VDONE = RED_BARS + 16, RED_TMEM = RED_BARS + 24;
+constexpr int RED_SK = 0;                        // [parity][warp][group][4] largest |query * S| of the keys, as the sum of the two bit patterns
+constexpr int RED_SV = RED_SK + 256;             // [parity][warp][group][4] largest log2 (probability * |S|) of the values, before the maximum is taken off
+constexpr int RED_MAX = RED_SV + 256;            // [parity][warp][4] largest logit
+constexpr int RED_EX = RED_MAX + 128;            // [parity][group][4] what a unit of the keys' column_sum is worth
+constexpr int RED_FLAG = RED_EX + 64, RED_CA = RED_FLAG + 32;      // [parity][warp] whether there is a constant term; [parity][warp][group][4] its parts
+constexpr int RED_QS = RED_CA + 256;             // [4] logit (base 2) per unit of the scaled query times a key
+constexpr int RED_RUN = RED_QS + 16;             // [parity][4] running maximum of the logits (base 2)
+constexpr int RED_END = RED_RUN + 32;            // [warp][16]: constant terms of the output [group][4], sum of probabilities [4]
+constexpr int RED_KFOLD = RED_END + 256;         // [warp of the keys][group][4] factors of the step's folds
+constexpr int RED_VFOLD = RED_KFOLD + 128;       // [warp of the values]: factors of the step's folds [group][4], worth of a unit of their column_sum [group][4]
+constexpr int RED_BARS = RED_VFOLD + 256, BAR_KDONE = RED_BARS, BAR_KFREE = RED_BARS + 8, BAR_VDONE = RED_BARS + 16, RED_TMEM = RED_BARS + 24;
+static_assert(RED_TMEM + 4 <= 1792, "exchange area");
 
 // ---- tcgen05 / mbarrier wrappers
 // this lane's row of every plane's accumulator: the 8 columns of two heads
@@ -339,12 +345,28 @@ __device__ __forceinline__ float column_sum(const int (&c)[P][8], int at) {
   return fmaf((float)a[3], 65536.0f, (float)(a[1] + b[2] + d[3] + 256 * (a[2] + b[3]) + ((a[0] + b[1] + d[2]) >> 8)));
 }
 
-// power of two that brings a positive number of exponent field `ex` into [0.5, 1), and its inverse.  What is not finite has no digits: its
-// inverse is NaN, and so is every sum that it has a part in
+// power of two that brings a positive number of exponent field `ex` (up to 255) into [0.5, 1), and half its inverse.  What is not finite has no
+// digits: its inverse is NaN, and so is every sum that it has a part in
 __device__ __forceinline__ float scale_down(uint32_t ex) {
   return __uint_as_float(ex <= 252u ? (253u - max(ex, 1u)) << 23 : 0x00800000u >> (ex - 252u));
 }
-__device__ __forceinline__ float scale_up(uint32_t ex) { return __uint_as_float(ex < 255u ? (max(ex, 1u) + 1u) << 23 : 0x7FFFFFFFu); }
+__device__ __forceinline__ float half_scale_up(uint32_t ex) { return __uint_as_float(ex < 255u ? max(ex, 1u) << 23 : 0x7FFFFFFFu); }
+__device__ __forceinline__ float lg2f(float x) {
+  float y;
+  asm("lg2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// maxima that keep a NaN
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+__device__ __forceinline__ float warp_max_nan(float a) {
+  float y;
+  asm("redux.sync.max.NaN.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(a));
+  return y;
+}
 // exponent field of the largest magnitude of a head's query (HD elements of 16 bits)
 template <int HD>
 __device__ __forceinline__ uint32_t query_exponent(const uint16_t* q, int lane, int dtype) {
@@ -507,23 +529,20 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
                           : prepare_row<BITS, P, true>(mz_u16_to_float((uint16_t)lo[x], s.meta_dtype), mz_u16_to_float((uint16_t)span[x], s.meta_dtype));
   };
   auto magnitude = [&](int x) { return __float_as_uint(rows[x].s) & 0x7FFFFFFFu; };
-  // the largest of a side: per warp here, over the four warps behind the next barrier
-  auto publish_largest = [&](uint32_t at, uint32_t v) {
-    v = __reduce_max_sync(0xffffffffu, v);
-    if (lane == 0) sts32(at + 4 * w, v);
-  };
-  auto exponent_of_largest = [&](uint32_t at) {
-    const uint4 v = lds128(at);
-    return max(max(v.x, v.y), max(v.z, v.w)) >> 23;
-  };
-  auto put_folds = [&](const float (&x)[GQA], float down0, float down1, int groups) {
+  // Folds are scaled by their largest product, per head and group of the step: rounding and dropped low products of digits then come to 1e-6 (two
+  // planes) or 4e-9 of the largest addend of a sum (rms), whatever the sides and queries or probabilities beside it.  (One scale for the largest side times the
+  // largest query or probability lost 2 to 40 times the fp32 kernels' error where these do not meet: a token that
+  // dominates and has a small value, an outlier channel with a small query.  Finding the products costs 7 % of a call: 8 x 8 pairs x 131072
+  // tokens at 2 bits 408 -> 437 us.  Their factors before the output of the step before, instead of behind it: 444.)  They are kept per
+  // warp at `factors`.
+  auto put_folds = [&](const float (&x)[GQA], uint32_t factors, int groups) {
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       if (k >= groups) break;
-      const float sx = rows[k].s * (k ? down1 : down0);
+      const uint4 f = lds128(factors + 16 * k);
       uint32_t d[4] = {0, 0, 0, 0};
 #pragma unroll
-      for (int g = 0; g < GQA; ++g) d[g] = fold_digits<P>(x[g], sx);
+      for (int g = 0; g < GQA; ++g) d[g] = fold_digits<P>(x[g] * __uint_as_float(g == 0 ? f.x : g == 1 ? f.y : g == 2 ? f.z : f.w), rows[k].s);
       sts128(side + C::OFF_FOLD + k * 2048 + r * 16, make_uint4(d[0], d[1], d[2], d[3]));
     }
   };
@@ -561,36 +580,55 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
     fewer_registers<C::KEY>();
     if (steps > 0) {
     // ================= keys: channel r of the step's groups, one step ahead of the values =================
-    float qn[GQA];                                                    // query of this channel, scaled per head into (-C::FOLD_FULL, C::FOLD_FULL)
-    int q_pair = -1;
+    float qn[GQA];                                                    // query of this channel, scaled per head into (-1, 1)
+    auto load_query = [&](const Place& c) {
+#pragma unroll
+      for (int g = 0; g < GQA; ++g) {
+        const uint16_t* q = (const uint16_t*)p.query + c.b * p.q_stride_b + (long long)(c.kvh * GQA + g) * p.q_stride_h;
+        qn[g] = mz_u16_to_float(q[channel], s.kv_dtype) * scale_down(query_exponent<HD>(q, lane, s.kv_dtype));
+      }
+    };
+    // the warp's largest products: bit patterns of positive numbers add up to that of their product but for a factor in [8/9, 1].  A side
+    // that is not finite outweighs every finite product
+    auto publish_products = [&](uint32_t at) {
+      uint32_t m[2][4];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const uint32_t a = magnitude(x) < 0x7F800000u ? magnitude(x) : 0xC0000000u;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) m[x][g] = g < GQA ? __reduce_max_sync(0xffffffffu, a + (__float_as_uint(qn[g % GQA]) & 0x7FFFFFFFu)) : 0u;
+      }
+      if (lane == 0) {
+        sts128(at + 32 * w, make_uint4(m[0][0], m[0][1], m[0][2], m[0][3]));
+        sts128(at + 32 * w + 16, make_uint4(m[1][0], m[1][1], m[1][2], m[1][3]));
+      }
+    };
     point();
     load_meta();
     load_codes(0);
     load_codes(1);
+    load_query(cur);
     prepare();
-    publish_largest(red + RED_SK, max(magnitude(0), magnitude(1)));
+    publish_products(red + RED_SK);
     if (steps > 1) { move_ahead(); load_meta(); }
     team_barrier(team);
     for (int i = 0; i < steps; ++i) {
       const int par = i & 1;
       const bool more = i + 1 < steps;
-      if (cur.pair != q_pair) {
-        q_pair = cur.pair;
-#pragma unroll
-        for (int g = 0; g < GQA; ++g) {
-          const uint16_t* q = (const uint16_t*)p.query + cur.b * p.q_stride_b + (long long)(cur.kvh * GQA + g) * p.q_stride_h;
-          qn[g] = mz_u16_to_float(q[channel], s.kv_dtype) * (scale_down(query_exponent<HD>(q, lane, s.kv_dtype)) * C::FOLD_FULL);
-        }
-      }
-      const uint32_t ex = exponent_of_largest(red + RED_SK + 16 * par);
+      // lane l has group and head l mod 8
+      uint32_t most = lds32(red + RED_SK + 128 * par + 4 * lane);
+      most = max(most, __shfl_xor_sync(0xffffffffu, most, 8));
+      most = max(most, __shfl_xor_sync(0xffffffffu, most, 16));
+      const uint32_t ex = (uint32_t)min(max((int)(most >> 23) - 127, 1), 255);
+      if (lane < 8) stsf(red + RED_KFOLD + 32 * w + 4 * lane, scale_down(ex) * C::FOLD_FULL);
+      __syncwarp();
       if (i > 0) bar_wait<64>(red + BAR_KDONE, (uint32_t)(i - 1) & 1, failed);       // the operands have been read
       const bool own = HD == 128 || w < 2;                            // this warp has rows
       if (own) expand_row<BITS, P, NW>(code[0], rows[0], book, side + r * 16, two16);
       if (more) load_codes(0);
       if (own) expand_row<BITS, P, NW>(code[1], rows[1], book, side + 8192 + r * 16, two16);
       if (more) load_codes(1);
-      const float down = scale_down(ex);
-      if (own) put_folds(qn, down, down, 2);
+      if (own) put_folds(qn, red + RED_KFOLD + 32 * w, 2);
       // constant term sum_d q[h][d] A_d per group and head (rows whose range does not straddle zero): this warp's part
       const bool any = own && __any_sync(0xffffffffu, rows[0].A != 0.0f || rows[1].A != 0.0f);
       if (any) {
@@ -604,15 +642,15 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
             if (lane == 0) stsf(red + RED_CA + par * 128 + ((w * 2 + x) * 4 + g) * 4, v);
           }
       }
-      if (lane == 0) {
-        sts32(red + RED_FLAG + par * 16 + 4 * w, any ? 1u : 0u);
-        if (w == 0) sts32(red + RED_EX + 4 * par, ex);
-      }
+      if (lane == 0) sts32(red + RED_FLAG + par * 16 + 4 * w, any ? 1u : 0u);
+      if (w == 0 && lane < 8) stsf(red + RED_EX + 32 * par + 4 * lane, half_scale_up(ex) * (2.0f * C::UNIT));
+      const int pair = cur.pair;
+      advance(cur);
       if (more) {
         prepare();
-        publish_largest(red + RED_SK + 16 * (par ^ 1), max(magnitude(0), magnitude(1)));
+        if (cur.pair != pair) load_query(cur);
+        publish_products(red + RED_SK + 128 * (par ^ 1));
       }
-      advance(cur);
       if (i + 2 < steps) { move_ahead(); load_meta(); }
       proxy_fence();
       team_ready(team);
@@ -627,7 +665,6 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
     float l_part[GQA], out[GQA];                                      // this thread's sum of probabilities, output
     float base_sum = 0.f;                                             // lane 4 x + g: sum p * A of the warp's tokens, channel group x and head g
     bool has_base = false;
-    float up_v = 0.f;
     int seg = 0;
     auto start_pair = [&](const Place& c) {
 #pragma unroll
@@ -635,7 +672,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
         l_part[g] = out[g] = 0.f;
         const uint16_t* q = (const uint16_t*)p.query + c.b * p.q_stride_b + (long long)(c.kvh * GQA + g) * p.q_stride_h;
         const uint32_t ex = query_exponent<HD>(q, lane, s.kv_dtype);
-        if (r == 0) stsf(red + RED_QS + 4 * g, scale_up(ex) * p.scaling * (LOG2E * C::UNIT));     // read behind the next barrier but one
+        if (r == 0) stsf(red + RED_QS + 4 * g, half_scale_up(ex) * p.scaling * (2.0f * LOG2E));     // read behind the next barrier but one
       }
       if (r < 2) sts128(red + RED_RUN + 16 * r, make_uint4(0xFF800000u, 0xFF800000u, 0xFF800000u, 0xFF800000u));
       base_sum = 0.f; has_base = false;
@@ -649,8 +686,9 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       for (int g = 0; g < GQA; g += 2) {
         int c[P][8];
         tm_ld8<P>(tm_v + tm_mine + 4 * g, c);
-        out[g] = fmaf(column_sum<P>(c, 0), up_v, out[g]);
-        if (g + 1 < GQA) out[(g + 1) % GQA] = fmaf(column_sum<P>(c, 4), up_v, out[(g + 1) % GQA]);
+        const uint2 up = lds64(red + RED_VFOLD + 64 * w + 32 + 16 * half + 4 * g);
+        out[g] = fmaf(column_sum<P>(c, 0), __uint_as_float(up.x), out[g]);
+        if (g + 1 < GQA) out[(g + 1) % GQA] = fmaf(column_sum<P>(c, 4), __uint_as_float(up.y), out[(g + 1) % GQA]);
       }
       tm_fence_before();
     };
@@ -696,8 +734,6 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       Place nxt = cur;
       advance(nxt);
       prepare();
-      publish_largest(red + RED_SV + 32 * par, magnitude(0));
-      if (NG == 2) publish_largest(red + RED_SV + 32 * par + 16, magnitude(1));
       const bool more = i + 1 < steps;
       if (more) { move_ahead(); load_meta(); }
       const bool live = STEP_GROUPS * cur.step + half < kt;
@@ -716,7 +752,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
           lg[g] = column_sum<P>(c, 0);
           if (g + 1 < GQA) lg[(g + 1) % GQA] = column_sum<P>(c, 4);
         }
-        const float up_k = scale_up(lds32(red + RED_EX + 4 * par));
+        const uint4 up = lds128(red + RED_EX + 32 * par + 16 * half);
         const uint4 fl = lds128(red + RED_FLAG + 16 * par);
         float ca[GQA];
 #pragma unroll
@@ -736,13 +772,23 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
         const uint4 qs = lds128(red + RED_QS);
 #pragma unroll
         for (int g = 0; g < GQA; ++g) {
-          const float v = fmaf(lg[g], up_k, ca[g] * (1.0f / (C::FOLD_FULL * C::UNIT)));
+          const float v = fmaf(lg[g], __uint_as_float(g == 0 ? up.x : g == 1 ? up.y : g == 2 ? up.z : up.w), ca[g]);
           lg[g] = live ? fmaf(v, __uint_as_float(g == 0 ? qs.x : g == 1 ? qs.y : g == 2 ? qs.z : qs.w), mask) : -INFINITY;
           asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(mx[g]) : "f"(lg[g]));
         }
         if (lane == 0) sts128(red + RED_MAX + par * 64 + w * 16, make_uint4(__float_as_uint(mx[0]), __float_as_uint(mx[1]), __float_as_uint(mx[2]), __float_as_uint(mx[3])));
+        // the warp's largest products of a probability and a side, in logarithms
+#pragma unroll
+        for (int x = 0; x < NG; ++x) {
+          const float a = lg2f(fabsf(rows[x].s));
+          float m[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int g = 0; g < GQA; ++g) m[g] = warp_max_nan(lg[g] + a);
+          if (lane == 0) sts128(red + RED_SV + par * 128 + w * 32 + x * 16, make_uint4(__float_as_uint(m[0]), __float_as_uint(m[1]), __float_as_uint(m[2]), __float_as_uint(m[3])));
+        }
       }
       team_barrier(team);
+      float most = ldsf(red + RED_SV + 128 * par + 4 * lane);         // lane l has group and head l mod 8
       if (pending) drain(i - 1);                                      // and its operands have been read
       // ================= softmax =================
       {
@@ -757,6 +803,15 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
         const float before[4] = {__uint_as_float(run.x), __uint_as_float(run.y), __uint_as_float(run.z), __uint_as_float(run.w)};
 #pragma unroll
         for (int g = 0; g < 4; ++g) mx[g] = fmaxf(mx[g], before[g]);
+        // scale of the folds: the power of two above the largest product; the logits' own rounding (a logit of 2^20 has steps of 1/8) is
+        // made up for
+        most = max_nan(most, __shfl_xor_sync(0xffffffffu, most, 8));
+        most = max_nan(most, __shfl_xor_sync(0xffffffffu, most, 16));
+        const float high = fmaxf((lane & 2) ? ((lane & 1) ? mx[3] : mx[2]) : ((lane & 1) ? mx[1] : mx[0]), -3.0e38f);
+        most = fmaf(fabsf(high), 2.4e-7f, most - high);
+        const uint32_t ex = most < 200.0f ? (uint32_t)(min(max(__float2int_ru(most), -100), 128) + 126) : 255u;      // (a NaN has none)
+        if (lane < 16) stsf(red + RED_VFOLD + 64 * w + 4 * lane, lane < 8 ? scale_down(ex) * C::FOLD_FULL : half_scale_up(ex) * (2.0f * C::UNIT));
+        __syncwarp();
         if (r == 0) sts128(red + RED_RUN + 16 * par, make_uint4(__float_as_uint(mx[0]), __float_as_uint(mx[1]), __float_as_uint(mx[2]), __float_as_uint(mx[3])));
 #pragma unroll
         for (int g = 0; g < GQA; ++g) {
@@ -780,13 +835,9 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
               if (lane == 4 * x + g) base_sum += v;
             }
         }
-#pragma unroll
-        for (int g = 0; g < GQA; ++g) lg[g] *= C::FOLD_FULL;
       }
       // ================= values: token `spot`, its two channel groups =================
-      const uint32_t ex0 = exponent_of_largest(red + RED_SV + 32 * par), ex1 = NG == 2 ? exponent_of_largest(red + RED_SV + 32 * par + 16) : ex0;
-      up_v = scale_up(half ? ex1 : ex0) * C::UNIT;
-      put_folds(lg, scale_down(ex0), scale_down(ex1), NG);
+      put_folds(lg, red + RED_VFOLD + 64 * w, NG);
       expand_row<BITS, P, NW>(code[0], rows[0], book, side + r * 16, two16);
       if (more) load_codes(0);
       if (NG == 2) {

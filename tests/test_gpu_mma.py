@@ -167,6 +167,52 @@ def test_an_infinite_range_stays_in_its_group(oracle, bits, D, group, gqa):
     assert not bool(torch.isfinite(got[hit]).any()) and relative_error(got[~hit], want[~hit]) <= FP32_ERROR
 
 
+def unlike_tokens(oracle, kind, batch, kv_heads, tokens, head_dim, gqa, seed):
+    """Keys, values and queries whose largest factors do not meet in one product.  sink: one token dominates by 8 or 12 nats and has values a
+    hundredth or a thousandth of the others' (early: in the first step of a range; late: behind others).  outlier: a key channel a thousand or
+    ten thousand times the others' under a query as much smaller.  spread: tokens' values over a factor of 400."""
+    k, v, q = (t.float() for t in oracle.synth_kv(batch, kv_heads, tokens, head_dim, kv_heads * gqa, seed=seed))
+    gen = torch.Generator().manual_seed(seed)
+    if kind.startswith("sink"):
+        nats = 8.0 if "8" in kind else 12.0
+        at = tokens - 300 if kind.endswith("late") else 5
+        base = torch.randn(1, kv_heads, 1, 1, head_dim, generator=gen).sign()
+        q = (base + 0.3 * torch.randn(batch, kv_heads, gqa, 1, head_dim, generator=gen)).reshape(batch, kv_heads * gqa, 1, head_dim)
+        k = 0.3 * torch.randn(batch, kv_heads, tokens, head_dim, generator=gen)
+        k[:, :, at] = base[:, :, 0, 0] * (nats + 1.5) / head_dim ** 0.5
+        v[:, :, at] *= 0.01 if nats < 10 else 0.001
+    elif kind == "outlier1e3":
+        k[..., 7] *= 1e3
+        q[..., 7] *= 1e-4
+    elif kind == "outlier1e4":
+        k[..., 7] = k[..., 7].clamp(-3, 3) * 1e4
+        q[..., 7] *= 1e-5
+    else:
+        v *= torch.exp(2 * torch.randn(1, 1, tokens, 1, generator=gen).clamp(-1.5, 1.5))
+    return [t.to(torch.bfloat16) for t in (k, v, q)]
+
+
+@pytest.mark.parametrize("kind", ["sink8", "sink12", "sink8late", "outlier1e3", "outlier1e4", "spread"])
+@pytest.mark.parametrize("bits,D,gqa,B,KVH,S", [(1, 128, 4, 2, 2, 1500), (2, 128, 4, 40, 4, 700), (2, 64, 2, 2, 2, 900), (3, 128, 4, 2, 2, 1500), (3, 128, 4, 20, 8, 500),
+                                                (4, 128, 4, 2, 2, 1500), (4, 128, 8, 2, 2, 1500), (4, 64, 1, 2, 2, 1500)])
+def test_error_where_large_factors_do_not_meet(oracle, bits, D, gqa, B, KVH, S, kind):
+    """tcgen05 kernel: its fixed-point operands are scaled by the largest products of a step, so that rows as models have them (attention sinks,
+    outlier channels) keep the error of an fp32 evaluation, or with two planes that of their values (test_tcgen05_kernel).  Two planes:
+    2 bits, head_dim 128, more pairs than SMs."""
+    import muzero_b200 as mz
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = unlike_tokens(oracle, kind, B, KVH, S, D, gqa, bits + 10)
+    ref = oracle.OracleCacheLayer(bits=bits, group=64, residual=128, alpha_key=2.0, alpha_value=4.0)
+    ref.append(k, v)
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=64, residual_length=128, alpha_key=2.0, alpha_value=4.0)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+    with kernel(4):
+        got = decode_attention(layer, q.cuda(), D ** -0.5, out_dtype=torch.float32)
+    assert relative_error(got, attention64(oracle, ref, q, D ** -0.5)) <= (1.2e-4 if bits == 2 and D == 128 else FP32_ERROR)
+
+
 @pytest.mark.parametrize("bits,D,gqa", [(1, 128, 4), (2, 128, 2), (2, 128, 8), (3, 128, 4), (4, 128, 4), (4, 64, 8), (2, 64, 1)])
 def test_nan_stays_nan(oracle, bits, D, gqa):
     """tcgen05 kernel: a NaN in the mask or in a query and an infinite key range make the heads that meet them NaN, as a floating-point
