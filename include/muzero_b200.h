@@ -226,6 +226,13 @@ typedef struct mz_decode_args {
 int mz_debug_force_kernel(int which);
 
 /*
+ * Testing aid of the checked build (-DMZ_BOUNDS): on != 0 makes every wait of later calls of the tcgen05 kernel in this process run out at once, 0
+ * gives them their limit back; returns what was set before.  The output of such a call is NaN, and the context stays usable.  Returns -1
+ * from a library built without the flag.
+ */
+int mz_debug_fail_waits(int on);
+
+/*
  * Testing aid of the checked build (library compiled with -DMZ_BOUNDS): the number of guarded global
  * accesses on the current device that fell outside the extent the host passed and were skipped; the
  * index, extent and site number of the first one go to the optional pointers; `reset` != 0 clears the

@@ -109,7 +109,7 @@ int make_plan(const mz_decode_args* a, Plan* plan, bool need_tables, size_t scra
   p.table_k = p.table_v = nullptr;
   p.lut = nullptr;
   p.hetero = 0;
-  p.planes = p.kv_share = 0;
+  p.planes = p.kv_share = p.fail_waits = 0;
   p.cluster = 0;
   p.o = MzDecodeOut{};
   p.new_k = p.new_v = nullptr;

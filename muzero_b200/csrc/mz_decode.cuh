@@ -91,6 +91,7 @@ struct MzDecodeParams {
   // tcgen05 kernel: bytes per value; log2 of the kv heads of the plan that share one of the store (8 query heads per kv head are
   // planned as two kv heads with 4)
   int planes, kv_share;
+  int fail_waits;                           // checked build: not 0 = its waits run out at once
   // tensor-core kernel, cluster mode: CTAs per pair (0 = flat partition and merge kernel); the kernel writes `o` itself
   int cluster;
   MzDecodeOut o;

@@ -14,8 +14,9 @@
 //     group of a row of the result picks its half of the columns
 //   * the top byte is signed, the others unsigned; each plane has an accumulator of its own, and column_sum adds products of equal weight
 //   * online softmax with one thread per token, the running output in registers (thread = channel); MMA completion is tracked with
-//     mbarriers, every wait on one is bounded: when it runs out the worker poisons its records (the merged output becomes
-//     NaN), frees its tensor memory and returns
+//     mbarriers, and so is what the teams hand to their issuing warp.  Every wait on one is bounded: whichever warp's runs out tells its worker,
+//     which poisons its records from then on (the merged output becomes NaN), issues no more products, waits for those in flight, frees its
+//     tensor memory and returns.  (The named barriers left are within a team, whose warps keep step whatever runs out.)
 //   * the residual window is un-quantized: its tiles have CTAs of their own (mz_dense_tiles.cuh)
 //
 // What bounds it: issue (58 % of the cycles; per row of 64 two-bit codes about 230 instructions, of which 32 permutes) and the logic pipe
@@ -28,13 +29,20 @@
 // is no worse than the fp32 kernels (relative error against 64 bits 2e-7 to 7e-7 where those have 2e-7 to 1.1e-6, attention sinks, outlier
 // channels and tokens of unlike range included; 1 bit is exact in one plane).  Two planes (2 bits, calls that the unrolled kernel served): 2^-15
 // and 1e-6, 1e-5 to 4e-5 where the unrolled kernel has 5e-5 to 2e-4.  Any range is served: folds and query are scaled by powers of two.
+#include <atomic>
+
 #include "mz_dense_tiles.cuh"
 
 namespace mzu {
 using namespace mzm;
 
 constexpr int STEP_GROUPS = 2;                   // groups of 64 tokens per step
-constexpr int SPIN_LIMIT = 1000000;
+constexpr int SPIN_LIMIT = 1000000;              // looks of a wait before it gives up
+#ifdef MZ_BOUNDS
+constexpr int SHORT_LIMIT = 0;                   // and once one has: none, so that a test fails every wait
+#else
+constexpr int SHORT_LIMIT = 1;
+#endif
 constexpr int PLANE_BYTES = 16384;               // [16-byte chunk of the kept dimension, 8][row 128][16]
 constexpr int FOLD_BYTES = 4096;                 // [group 2][row 128][4 heads x 4 bytes]
 constexpr float MAGIC = 12582912.0f;             // 1.5 * 2^23: adding it rounds to an integer that stands in the low mantissa bits
@@ -79,8 +87,12 @@ constexpr int RED_RUN = RED_QS + 16;             // [parity][4] running maximum 
 constexpr int RED_END = RED_RUN + 32;            // [warp][16]: constant terms of the output [group][4], sum of probabilities [4]
 constexpr int RED_KFOLD = RED_END + 256;         // [warp of the keys][group][4] factors of the step's folds
 constexpr int RED_VFOLD = RED_KFOLD + 128;       // [warp of the values]: factors of the step's folds [group][4], worth of a unit of their column_sum [group][4]
-constexpr int RED_BARS = RED_VFOLD + 256, BAR_KDONE = RED_BARS, BAR_KFREE = RED_BARS + 8, BAR_VDONE = RED_BARS + 16, RED_TMEM = RED_BARS + 24;
-static_assert(RED_TMEM + 4 <= 1792, "exchange area");
+// mbarriers: products of the keys / values are done, the keys' accumulators have been read, the operands of the keys / values are written, no
+// product of this worker is in flight
+constexpr int RED_BARS = RED_VFOLD + 256, BAR_KDONE = RED_BARS, BAR_KFREE = RED_BARS + 8, BAR_VDONE = RED_BARS + 16, BAR_KREADY = RED_BARS + 24,
+              BAR_VREADY = RED_BARS + 32, BAR_END = RED_BARS + 40, RED_TMEM = RED_BARS + 48;
+constexpr int RED_FAILED = RED_TMEM + 4;         // not 0: a wait of this worker has run out
+static_assert(RED_FAILED + 4 <= 1792, "exchange area");
 
 // ---- tcgen05 / mbarrier wrappers
 // this lane's row of every plane's accumulator: the 8 columns of two heads
@@ -105,9 +117,6 @@ __device__ __forceinline__ void tm_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // among the four warps of a team
 __device__ __forceinline__ void team_barrier(int team) { asm volatile("bar.sync %0, 128;" ::"r"(team + 1) : "memory"); }
-// from a team to its issuing warp
-__device__ __forceinline__ void team_ready(int team) { asm volatile("bar.arrive %0, 160;" ::"r"(team + 7) : "memory"); }
-__device__ __forceinline__ void join_team(int team) { asm volatile("bar.sync %0, 160;" ::"r"(team + 7) : "memory"); }
 template <int N>
 __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
@@ -157,11 +166,12 @@ __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t n) { asm volatil
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
   asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}\n" ::"r"(bar) : "memory");
 }
-// waits for phase `parity` of an mbarrier with a limit; `failed` is set when it gives up, and makes later waits short.  SLEEP: ns between
-// looks, for a team that is ahead anyway
+// waits for phase `parity` of an mbarrier with a limit.  Who gives up says so to the whole worker before it goes on, so that what it spoils
+// from then on is in a record that is poisoned; its later waits are short.  SLEEP: ns between looks, for a team that is ahead anyway.  (What
+// stands here is dear: a limit or first value of `failed` that only the launch knows costs 2 to 15 % of a call.)
 template <int SLEEP = 0>
-__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, bool& failed) {
-  const int limit = failed ? 1 : SPIN_LIMIT;
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, uint32_t red, bool& failed) {
+  const int limit = failed ? SHORT_LIMIT : SPIN_LIMIT;
   for (int it = 0; it < limit; ++it) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}\n"
@@ -170,6 +180,7 @@ __device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, bool& fa
     if (SLEEP > 0) __nanosleep(SLEEP);
   }
   failed = true;
+  sts32(red + RED_FAILED, 1u);
 }
 
 // ---- books.  A row's zero code is brought to the lower half by mirroring (code -> TOP - code, S -> -S): then the side above it is the
@@ -377,6 +388,7 @@ __device__ __forceinline__ uint32_t query_exponent(const uint16_t* q, int lane, 
 
 
 struct Place { int pair, step, b, kvh; };
+std::atomic<int> g_fail_waits{0};                // mz_debug_fail_waits (checked build)
 
 template <int BITS, int P, int HD, int GQA, bool HALF_META>
 __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(const MzDecodeParams p, const uint32_t two16) {
@@ -418,6 +430,8 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
   }
   if (!issuer && keys && r == 0) {
     bar_init(red + BAR_KDONE, 2); bar_init(red + BAR_KFREE, 4); bar_init(red + BAR_VDONE, 1);
+    bar_init(red + BAR_KREADY, 4); bar_init(red + BAR_VREADY, 4); bar_init(red + BAR_END, 1);
+    sts32(red + RED_FAILED, 0u);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   fill_books<BITS, P>(base, s.alpha_key, threadIdx.x, C::THREADS);
@@ -443,7 +457,11 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       if (++c.kvh == s.kv_heads) { c.kvh = 0; ++c.b; }
     }
   };
+#ifdef MZ_BOUNDS
+  bool failed = p.fail_waits != 0;
+#else
   bool failed = false;
+#endif
   const bool meta32 = s.meta_dtype == MZ_F32;
   // everything above reads kernel parameters only and may run while the grid before drains
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -555,26 +573,31 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       const uint64_t value_values = descriptor(worker + C::SIDE_BYTES), value_folds = descriptor(worker + C::SIDE_BYTES + C::OFF_FOLD);
       for (int i = -1; i < steps; ++i) {
         if (i + 1 < steps) {
-          join_team(2 * wk);
-          if (i >= 0) bar_wait(red + BAR_KFREE, (uint32_t)i & 1, failed);        // the logits before have been read
+          bar_wait(red + BAR_KREADY, (uint32_t)(i + 1) & 1, red, failed);
+          if (i >= 0) bar_wait(red + BAR_KFREE, (uint32_t)i & 1, red, failed);        // the logits before have been read
           tm_fence_after();
           if (elect_one()) {
             bar_arrive(red + BAR_KDONE);                              // hands on what the team has noted
-            umma_side<BITS, P, HD / 32>(tm_k, key_values, key_folds);
+            if (!failed) umma_side<BITS, P, HD / 32>(tm_k, key_values, key_folds);
             umma_commit(red + BAR_KDONE);
           }
           __syncwarp();
         }
         if (i >= 0) {
-          join_team(2 * wk + 1);
+          bar_wait(red + BAR_VREADY, (uint32_t)i & 1, red, failed);
           tm_fence_after();
           if (elect_one()) {
-            umma_side<BITS, P, 4>(tm_v, value_values, value_folds);
+            if (!failed) umma_side<BITS, P, 4>(tm_v, value_values, value_folds);
             umma_commit(red + BAR_VDONE);
           }
           __syncwarp();
         }
       }
+      // no product may be in flight when the tensor memory goes back, whoever has given up before
+      if (elect_one()) umma_commit(red + BAR_END);
+      __syncwarp();
+      bool given_up = false;
+      bar_wait(red + BAR_END, 0, red, given_up);
     }
   } else if (keys) {
     fewer_registers<C::KEY>();
@@ -622,7 +645,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       const uint32_t ex = (uint32_t)min(max((int)(most >> 23) - 127, 1), 255);
       if (lane < 8) stsf(red + RED_KFOLD + 32 * w + 4 * lane, scale_down(ex) * C::FOLD_FULL);
       __syncwarp();
-      if (i > 0) bar_wait<64>(red + BAR_KDONE, (uint32_t)(i - 1) & 1, failed);       // the operands have been read
+      if (i > 0) bar_wait<64>(red + BAR_KDONE, (uint32_t)(i - 1) & 1, red, failed);       // the operands have been read
       const bool own = HD == 128 || w < 2;                            // this warp has rows
       if (own) expand_row<BITS, P, NW>(code[0], rows[0], book, side + r * 16, two16);
       if (more) load_codes(0);
@@ -653,7 +676,8 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       }
       if (i + 2 < steps) { move_ahead(); load_meta(); }
       proxy_fence();
-      team_ready(team);
+      __syncwarp();
+      if (lane == 0) bar_arrive(red + BAR_KREADY);
       team_barrier(team);
     }
     }
@@ -680,7 +704,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
     };
     // adds the products of step v's values to the output
     auto drain = [&](int v) {
-      bar_wait(red + BAR_VDONE, (uint32_t)v & 1, failed);
+      bar_wait(red + BAR_VDONE, (uint32_t)v & 1, red, failed);
       tm_fence_after();
 #pragma unroll
       for (int g = 0; g < GQA; g += 2) {
@@ -716,7 +740,8 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
           // a NaN probability has no digits either: what shows it is their sum
           if (HD == 128 || r < HD) p.part.acc[(slot0 + g) * HD + spot] = lt == lt ? out[g] + bs : lt;
           if (r == 0) {
-            p.part.m[slot0 + g] = failed ? INFINITY : ldsf(red + RED_RUN + 16 * par + 4 * g) * (1.0f / LOG2E);   // a wait ran out: +inf turns the merged output into NaN
+            // a wait of any of the worker's warps ran out: +inf turns the merged output into NaN
+            p.part.m[slot0 + g] = lds32(red + RED_FAILED) != 0 ? INFINITY : ldsf(red + RED_RUN + 16 * par + 4 * g) * (1.0f / LOG2E);
             p.part.l[slot0 + g] = lt;
           }
         }
@@ -741,7 +766,7 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       if (p.mask && live)
         mask = mz_load_as_float(p.mask, cur.b * p.mask_stride_b + (long long)cur.step * (STEP_GROUPS * G) + spot, p.mask_dtype) * LOG2E;
       // ================= logits of token `spot` =================
-      bar_wait(red + BAR_KDONE, (uint32_t)par, failed);
+      bar_wait(red + BAR_KDONE, (uint32_t)par, red, failed);
       tm_fence_after();
       float lg[GQA];
       {
@@ -846,7 +871,8 @@ __global__ void __launch_bounds__(Cfg<BITS, P>::THREADS, 1) decode_umma_kernel(c
       }
       proxy_fence();
       tm_fence_before();
-      team_ready(team);
+      __syncwarp();
+      if (lane == 0) bar_arrive(red + BAR_VREADY);
       pending = true;
       if (!more || nxt.pair != cur.pair) {
         drain(i);
@@ -951,6 +977,7 @@ int mz_plan_umma(MzDecodeParams& p, bool full_precision, int splits_request, int
   }
   p.cluster = 0;
   p.hetero = 0;
+  p.fail_waits = mzu::g_fail_waits.load(std::memory_order_relaxed);
   int rc = cut(p.tp, pairs, steps, splits_request > 0 ? pairs * splits_request : (long long)(sm_count - n_d) * workers);
   if (rc) return rc;
   p.tp.packed_tiles = steps;
@@ -986,4 +1013,13 @@ int mz_launch_decode_umma(const MzDecodeParams& p, cudaStream_t st) {
     }
   }
   return mz_fail(MZ_ERR_UNSUPPORTED, "bits %d, %d planes", p.s.bits, p.planes);
+}
+
+extern "C" int mz_debug_fail_waits(int on) {
+#ifdef MZ_BOUNDS
+  return mzu::g_fail_waits.exchange(on != 0);
+#else
+  (void)on;
+  return -1;
+#endif
 }

@@ -106,3 +106,41 @@ def test_checked_build_small_shapes():
     env = dict(os.environ, MUZERO_B200_LIB=CHECKED_LIB)
     res = subprocess.run([sys.executable, "-c", CHILD.format(root=ROOT)], env=env, capture_output=True, text=True, timeout=900)
     assert res.returncode == 0 and "CHECKED-BUILD-OK" in res.stdout, res.stdout[-2000:] + res.stderr[-4000:]
+
+
+WAITS_CHILD = r"""
+import sys, torch
+sys.path.insert(0, {root!r}); sys.path.insert(0, {root!r} + "/tests")
+from conftest import load_oracle
+import muzero_b200 as mz
+from muzero_b200.cache.attention import decode_attention
+from muzero_b200.kernels._cabi import load_library
+lib, orc = load_library(), load_oracle()
+lib.mz_debug_force_kernel(4)
+for bits, D, gqa, B, S in ((1, 128, 4, 2, 500), (2, 128, 2, 20, 500), (3, 64, 1, 2, 500), (4, 128, 8, 2, 500), (3, 128, 4, 20, 1000)):
+    k, v, q = orc.synth_kv(B, 8, S, D, 8 * gqa, seed=bits)
+    ref = orc.OracleCacheLayer(bits=bits, group=64, residual=128, alpha_key=2.0, alpha_value=4.0)
+    ref.append(k, v)
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=64, residual_length=128, alpha_key=2.0, alpha_value=4.0)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda(), v.cuda(), {{"materialize_full_kv": False}})
+    assert lib.mz_debug_fail_waits(1) == 0
+    got = decode_attention(layer, q.cuda(), D ** -0.5, out_dtype=torch.float32).cpu()
+    assert lib.mz_debug_fail_waits(0) == 1
+    assert bool(torch.isnan(got).all()), (bits, D, gqa)
+    got = decode_attention(layer, q.cuda(), D ** -0.5, out_dtype=torch.float32).cpu()
+    want = orc.decode_attention_oracle(q, ref, D ** -0.5, gqa, compute_dtype=torch.float32)
+    assert (got - want).abs().max().item() <= 2e-3, (bits, D, gqa)
+assert lib.mz_bounds_violations(None, None, None, 0) == 0
+print("WAITS-OK")
+"""
+
+
+def test_a_wait_that_runs_out_gives_nan():
+    """tcgen05 kernel, every wait run out at once: every worker gives up, and the output says so; the next call is right again."""
+    if not os.path.exists(CHECKED_LIB):
+        pytest.skip("checked library not built (python -m muzero_b200.build --bounds)")
+    env = dict(os.environ, MUZERO_B200_LIB=CHECKED_LIB)
+    res = subprocess.run([sys.executable, "-c", WAITS_CHILD.format(root=ROOT)], env=env, capture_output=True, text=True, timeout=120)
+    assert res.returncode == 0 and "WAITS-OK" in res.stdout, res.stdout[-2000:] + res.stderr[-4000:]
