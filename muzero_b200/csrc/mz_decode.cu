@@ -244,8 +244,8 @@ extern "C" size_t mz_decode_workspace_bound(const mz_decode_args* a) {
   const long long pairs = (long long)s.batch * s.kv_heads, gqa = a->q_heads / s.kv_heads;
   const long long sms = sm_count();
   // tiled kernels: slots = W * max_segs * gqa <= gqa * (pairs + 3 W) per plan; at most two plans (packed and
-  // residual tiles) with W <= 3 + 12 workers per SM (or pairs * splits + pairs)
-  const long long w_max = a->splits > 0 ? pairs * (a->splits + 1) : sms * 15;
+  // residual tiles) with W <= 3 + 12 workers per SM together (or pairs * splits each)
+  const long long w_max = a->splits > 0 ? pairs * (2LL * a->splits + 1) : sms * 15;
   const long long tiled = gqa * (2 * pairs + 3 * w_max);
   // generic kernel: one slot per (batch, head, split)
   const long long splits = a->splits > 0 ? a->splits : (2 * sms * 4 + pairs - 1) / pairs;

@@ -291,3 +291,24 @@ def test_error_of_the_unrolled_kernel(oracle, bits, bound):
     layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
     got = decode_attention(layer, q.cuda(), 128 ** -0.5, out_dtype=torch.float32)
     assert relative_error(got, attention64(oracle, ref, q, 128 ** -0.5)) <= bound
+
+
+@pytest.mark.parametrize("which", [0, 4])
+@pytest.mark.parametrize("bits,D,gqa,B,S,residual", [(4, 128, 8, 2, 1200, 128), (2, 128, 4, 2, 1200, 256), (3, 64, 1, 3, 700, 256), (4, 128, 8, 20, 400, 128)])
+def test_workspace_bound_covers_every_split_count(oracle, bits, D, gqa, B, S, residual, which):
+    """The bound that holds for any token count also holds for two plans of as many workers as explicit splits ask for."""
+    import ctypes
+    import muzero_b200 as mz
+    from muzero_b200.cache.attention import build_decode_args
+    from muzero_b200.kernels._cabi import load_library
+    k, v, q = oracle.synth_kv(B, 4, S, D, 4 * gqa, seed=bits)
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=64, residual_length=residual, alpha_key=2.0, alpha_value=2.0)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+    lib = load_library()
+    with kernel(which):
+        a = build_decode_args(layer, q.cuda(), D ** -0.5, None, None)
+        for a.splits in range(0, 40):
+            need, bound = lib.mz_decode_workspace_bytes(ctypes.byref(a)), lib.mz_decode_workspace_bound(ctypes.byref(a))
+            assert 0 < need <= bound, (a.splits, need, bound)
