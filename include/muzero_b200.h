@@ -242,6 +242,13 @@ int mz_debug_fail_waits(int on);
  */
 long long mz_bounds_violations(long long* first_index, long long* first_extent, int* first_site, int reset);
 
+/*
+ * Testing aid: the kernel that mz_decode_attention would take for these arguments.  0 = shape-generic, 1 = SIMT tiles, 2 = general tensor-core
+ * kernel in clusters, 3 = the same over an even cut, 4 = unrolled tensor-core kernel, 5 / 6 / 7 = tcgen05 kernel with one, two or
+ * three bytes per value; -1 = bad arguments.
+ */
+int mz_debug_decode_kernel(const mz_decode_args* args);
+
 /* Bytes of workspace mz_decode_attention needs for these arguments (splits resolved as the call would). */
 size_t mz_decode_workspace_bytes(const mz_decode_args* args);
 

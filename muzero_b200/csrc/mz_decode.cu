@@ -234,6 +234,14 @@ extern "C" int mz_debug_force_kernel(int which) {
   return before;
 }
 
+extern "C" int mz_debug_decode_kernel(const mz_decode_args* a) {
+  Plan plan;
+  if (make_plan(a, &plan, false) != MZ_OK) return -1;
+  const MzDecodeParams& p = plan.p;
+  if (!plan.tiles) return 0;
+  return p.tp.kind == 0 ? 1 : p.tp.kind == 1 ? (p.cluster > 0 ? 2 : 3) : p.tp.kind == 3 ? 4 : 4 + p.planes;
+}
+
 extern "C" size_t mz_decode_workspace_bound(const mz_decode_args* a) {
   if (a == nullptr || mz_check_store_basic(&a->store) != MZ_OK) return 0;
   const mz_kv_store& s = a->store;

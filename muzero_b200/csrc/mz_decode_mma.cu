@@ -352,6 +352,9 @@ bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count, bool an
 // launch costs about 2 us whatever the kernel does.  Drawn by packed tiles per SM (cluster mode's estimate does not tell these apart):
 // 16 steps of a generation at 2 bits in cluster mode and here, 0.3 tiles per SM (1 x 8 x 500 tokens) 361 and 389 us, 2.6 (4 x 8 x 900) 333 and
 // 370, 4.0 (2 x 8 x 2500) 405 and 366; one call at 3.1 (2 x 8 x 2000) 18.9 and 15.1.
+// Bytes per value (planes) at 2 bits, head_dim 128 and up to four heads: three where cluster mode was the choice without this kernel, whose error is that of
+// an fp32 evaluation, two where the unrolled kernel was (5e-5 to 2e-4 there, 1e-5 to 4e-5 with two planes).  So no call is less precise than by
+// the choice between those two, and the line between the two errors is theirs (3 x 2 pairs: 4928 tokens two planes, 4992 three).
 constexpr float kOneLaunchTiles = 3.f;
 constexpr float kUmmaBase = 14.5f, kUmmaBase8 = 15.0f;                          // us
 constexpr float kUmmaTile[4] = {0.30f, 0.55f, 0.72f, 1.0f}, kUmmaTile64 = 0.9f;  // us per packed tile on an SM [bits]; at head_dim 64 of it

@@ -22,7 +22,7 @@ EXPORTS = (
     "mz_version", "mz_last_error", "mz_set_expand_table", "mz_quantize_rows", "mz_dequantize_rows",
     "mz_flush_kv", "mz_append_kv", "mz_dequantize_kv", "mz_decode_workspace_bytes", "mz_decode_attention",
     "mz_decode_attention_partial", "mz_lse_merge", "mz_qk_logits", "mz_av_output", "mz_decode_attention_static",
-    "mz_decode_step", "mz_decode_step_workspace_bytes", "mz_flush_kv_parts", "mz_decode_workspace_bound", "mz_decode_attention_partial_packed", "mz_lse_merge_packed", "mz_store_gather_batch", "mz_debug_force_kernel", "mz_debug_fail_waits", "mz_bounds_violations",
+    "mz_decode_step", "mz_decode_step_workspace_bytes", "mz_flush_kv_parts", "mz_decode_workspace_bound", "mz_decode_attention_partial_packed", "mz_lse_merge_packed", "mz_store_gather_batch", "mz_debug_force_kernel", "mz_debug_fail_waits", "mz_debug_decode_kernel", "mz_bounds_violations",
     "mz_alpha_stats", "mz_alpha_stats_workspace_bytes", "mz_materialize_kv", "mz_roundtrip_kv", "mz_flush_kv_move",
 )
 
@@ -113,6 +113,8 @@ def load_library() -> ctypes.CDLL:
     lib.mz_debug_force_kernel.restype = c_int
     lib.mz_debug_fail_waits.argtypes = [c_int]
     lib.mz_debug_fail_waits.restype = c_int
+    lib.mz_debug_decode_kernel.argtypes = [POINTER(DecodeArgs)]
+    lib.mz_debug_decode_kernel.restype = c_int
     lib.mz_bounds_violations.argtypes = [ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(c_int), c_int]
     lib.mz_bounds_violations.restype = ctypes.c_longlong
     lib.mz_materialize_kv.argtypes = [POINTER(KVStore), c_void_p, c_void_p, c_int, c_float, c_void_p]

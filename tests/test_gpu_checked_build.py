@@ -132,6 +132,11 @@ for bits, D, gqa, B, S in ((1, 128, 4, 2, 500), (2, 128, 2, 20, 500), (3, 64, 1,
     got = decode_attention(layer, q.cuda(), D ** -0.5, out_dtype=torch.float32).cpu()
     want = orc.decode_attention_oracle(q, ref, D ** -0.5, gqa, compute_dtype=torch.float32)
     assert (got - want).abs().max().item() <= 2e-3, (bits, D, gqa)
+    # and its stores of the newest token, across a flush
+    for step in range(66):
+        kn, vn, qn = orc.synth_kv(B, 8, 1, D, 8 * gqa, seed=5000 + step)
+        layer.decode_step(kn.cuda(), vn.cuda(), qn.cuda(), D ** -0.5)
+    assert torch.equal(layer.keys[:, :, -1:].cpu(), kn) and torch.equal(layer.values[:, :, -1:].cpu(), vn)
 assert lib.mz_bounds_violations(None, None, None, 0) == 0
 print("WAITS-OK")
 """

@@ -312,3 +312,117 @@ def test_workspace_bound_covers_every_split_count(oracle, bits, D, gqa, B, S, re
         for a.splits in range(0, 40):
             need, bound = lib.mz_decode_workspace_bytes(ctypes.byref(a)), lib.mz_decode_workspace_bound(ctypes.byref(a))
             assert 0 < need <= bound, (a.splits, need, bound)
+
+
+def planned_kernel(layer, q, splits=0):
+    """mz_debug_decode_kernel of a call: 2 general kernel in clusters, 4 unrolled kernel, 4 + n tcgen05 kernel with n bytes per value."""
+    import ctypes
+    from muzero_b200.cache.attention import build_decode_args
+    from muzero_b200.kernels._cabi import load_library
+    return load_library().mz_debug_decode_kernel(ctypes.byref(build_decode_args(layer, q, 1.0, None, None, splits=splits)))
+
+
+def caches(oracle, k, v, bits, **kw):
+    """The same keys and values in the oracle's cache and on the GPU, group 64 and a residual window of 128."""
+    import muzero_b200 as mz
+    meta = kw.pop("meta", torch.float16)
+    ref = oracle.OracleCacheLayer(bits=bits, group=64, residual=128, meta_dtype=meta, **kw)
+    ref.append(k, v)
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=64, residual_length=128, amax_dtype=str(meta)[6:], **kw)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    layer.update(k.cuda(), v.cuda(), {"materialize_full_kv": False})
+    return ref, layer
+
+
+# two planes: see test_tcgen05_kernel
+TWO_PLANE_ERROR = 1.2e-4
+
+
+@pytest.mark.parametrize("meta", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("bits,D,gqa,B,S", [(1, 128, 1, 2, 128 + 64), (1, 128, 8, 3, 700), (1, 64, 2, 2, 128 + 128), (2, 128, 4, 3, 128 + 64 + 63), (2, 128, 1, 2, 900), (2, 128, 8, 2, 330),
+                                            (2, 64, 4, 3, 1111), (2, 64, 8, 2, 200), (3, 128, 1, 2, 128 + 128 + 1), (3, 128, 2, 3, 777), (3, 128, 8, 2, 600), (3, 64, 8, 3, 300),
+                                            (4, 128, 1, 3, 128 + 64 + 5), (4, 128, 2, 2, 500), (4, 128, 4, 3, 2500), (4, 128, 8, 3, 1000), (4, 64, 1, 2, 330), (4, 64, 8, 3, 640)])
+def test_tcgen05_kernel_takes_the_new_token(oracle, bits, D, gqa, B, S, meta):
+    """Every width, head set and head_dim on the tcgen05 kernel itself, whatever the automatic choice: decode steps whose new token the kernel
+    stores (eight heads: two workers read it and one stores it), across a flush."""
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = oracle.synth_kv(B, 2, S, D, 2 * gqa, seed=bits * 100 + S)
+    k[:, :, :, :3] += 4.0
+    v[0] -= 3.0
+    ref, layer = caches(oracle, k, v, bits, alpha_key=2.0, alpha_value=4.0, meta=meta)
+    two = bits == 2 and D == 128
+    bound = TWO_PLANE_ERROR if two else FP32_ERROR
+    with kernel(4):
+        assert planned_kernel(layer, q.cuda()) == 4 + (1 if bits == 1 else 2 if two else 3)
+        for i in range(66):
+            kn, vn, qn = oracle.synth_kv(B, 2, 1, D, 2 * gqa, seed=9000 + i)
+            ref.append(kn, vn)
+            got = layer.decode_step(kn.cuda(), vn.cuda(), qn.cuda(), D ** -0.5)
+            if i in (0, 65):
+                want = attention64(oracle, ref, qn, D ** -0.5)
+                assert relative_error(got.float(), want) <= 2.0 ** -8      # bf16 output
+                assert relative_error(decode_attention(layer, qn.cuda(), D ** -0.5, out_dtype=torch.float32), want) <= bound
+    assert torch.equal(layer.keys.cpu(), ref.keys) and torch.equal(layer.values.cpu(), ref.values)
+
+
+@pytest.mark.parametrize("vs,ks,qs,meta", [(1e-4, 1.0, 1.0, torch.float16), (1e-6, 1.0, 1.0, torch.float32), (1e5, 1.0, 1.0, torch.float32),
+                                           (1e5, 1.0, 1.0, torch.bfloat16), (1.0, 1e-4, 1e4, torch.float16), (1.0, 1e5, 1e-5, torch.float32)])
+@pytest.mark.parametrize("bits,D,gqa", [(1, 128, 2), (2, 64, 4), (3, 128, 4), (4, 128, 8), (4, 64, 1)])
+def test_tcgen05_error_at_any_scale(oracle, bits, D, gqa, vs, ks, qs, meta):
+    """test_error_at_any_scale on the tcgen05 kernel."""
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = (t.float() for t in oracle.synth_kv(2, 2, 700, D, 2 * gqa, seed=bits))
+    v[..., :32] *= 1e-3
+    k, v, q = ((t * f).to(torch.bfloat16) for t, f in ((k, ks), (v, vs), (q, qs)))
+    ref, layer = caches(oracle, k, v, bits, alpha_key=2.0, alpha_value=2.0, meta=meta)
+    want = attention64(oracle, ref, q, D ** -0.5)
+    with kernel(4):
+        got = decode_attention(layer, q.cuda(), D ** -0.5, out_dtype=torch.float32)
+    assert bool(torch.isfinite(got).all())
+    for part in (slice(0, 32), slice(32, D)):
+        assert relative_error(got[..., part], want[..., part]) <= (FP32_ERROR if part.start else SHARED_GROUP_ERROR)
+
+
+@pytest.mark.parametrize("bits,D,gqa", [(1, 128, 4), (2, 128, 2), (3, 128, 4), (4, 64, 8), (4, 128, 8)])
+def test_tcgen05_infinite_range_stays_in_its_group(oracle, bits, D, gqa):
+    """test_an_infinite_range_stays_in_its_group on the tcgen05 kernel."""
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = oracle.synth_kv(2, 2, 500, D, 2 * gqa, seed=bits)
+    ref, layer = caches(oracle, k, v, bits, alpha_key=2.0, alpha_value=2.0)
+    want = attention64(oracle, ref, q, D ** -0.5)
+    last = D // 64 - 1
+    layer._value_scale[0, 1, 5, last] = float("inf")
+    with kernel(4):
+        got = decode_attention(layer, q.cuda(), D ** -0.5, out_dtype=torch.float32).cpu()
+    hit = torch.zeros(got.shape, dtype=torch.bool)
+    hit[0, :, gqa:, 64 * last:64 * last + 64] = True
+    assert not bool(torch.isfinite(got[hit]).any())
+    assert relative_error(got[~hit], want[~hit]) <= (TWO_PLANE_ERROR if bits == 2 else FP32_ERROR)
+
+
+@pytest.mark.parametrize("B,KVH,S,planned", [(1, 8, 3900, 7), (3, 2, 4992, 7), (3, 2, 4928, 6), (3, 2, 4864, 6), (20, 8, 400, 6), (1, 8, 1500, 2)])
+def test_bytes_per_value_at_2_bits(oracle, B, KVH, S, planned):
+    """Calls that cluster mode would serve keep the error of its fp32 evaluation on the tcgen05 kernel too (three planes); those that the unrolled
+    kernel would serve take two planes, whose error is below that kernel's.  On both sides of the line; the call's own choice."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the line is drawn per SM")
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = oracle.synth_kv(B, KVH, S, 128, 4 * KVH, seed=S)
+    ref, layer = caches(oracle, k, v, 2, alpha_key=2.0, alpha_value=2.0)
+    assert planned_kernel(layer, q.cuda()) == planned
+    got = decode_attention(layer, q.cuda(), 128 ** -0.5, out_dtype=torch.float32)
+    assert relative_error(got, attention64(oracle, ref, q, 128 ** -0.5)) <= (TWO_PLANE_ERROR if planned == 6 else FP32_ERROR)
+
+
+@pytest.mark.parametrize("gqa", [1, 2, 4])
+def test_unrolled_kernel_at_2_bits_with_splits(oracle, gqa):
+    """Explicit splits are what the unrolled kernel's 2-bit instances serve; the bound is that of test_error_of_the_unrolled_kernel."""
+    from muzero_b200.cache.attention import decode_attention
+    k, v, q = oracle.synth_kv(20, 8, 400, 128, 8 * gqa, seed=2)
+    ref, layer = caches(oracle, k, v, 2, alpha_key=2.0, alpha_value=2.0)
+    want = attention64(oracle, ref, q, 128 ** -0.5)
+    for splits in (1, 3):
+        assert planned_kernel(layer, q.cuda(), splits) == 4
+        got = decode_attention(layer, q.cuda(), 128 ** -0.5, out_dtype=torch.float32, splits=splits)
+        assert relative_error(got, want) <= 1.2e-4
