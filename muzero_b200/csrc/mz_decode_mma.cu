@@ -358,6 +358,13 @@ bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count, bool an
 constexpr float kOneLaunchTiles = 3.f;
 constexpr float kUmmaBase = 14.5f, kUmmaBase8 = 15.0f;                          // us
 constexpr float kUmmaTile[4] = {0.30f, 0.55f, 0.72f, 1.0f}, kUmmaTile64 = 0.9f;  // us per packed tile on an SM [bits]; at head_dim 64 of it
+// At head_dim 64 a residual tile weighs more than the 0.31 of a packed one that it counts for everywhere (33 x 8 x 592 at 4 bits has 16 of them on an SM
+// beside 12 packed ones: 31.9 us here and 22.0 by the general kernel's cut), and the estimates of that cut and of clusters are high there (1.0 to 1.7 of
+// the device time), as this kernel's is (1.0 to 1.4).  Over 190 calls that go by cost the choice without this weight and these margins was slower than the
+// other kernel by more than 3 % in 25 (up to 1.45), with them in 6 (up to 1.11); what both lose to the better of the two is 2.4 % on average.
+// Of 195 other calls it gives 76 to this kernel, at 0.73 of the other's time on average, 7 of them slower by more than 3 % (up to 1.28).
+constexpr float kUmmaDense64 = 0.6f;                                            // us per residual tile on an SM, besides
+constexpr float kUmmaMargin = 0.95f, kUmmaMarginCut64 = 0.9f;
 bool choose_umma(const MzDecodeParams& p, const MzDecodeParams& c, bool clusters, int sm_count) {
   if (clusters && (float)((long long)p.s.batch * p.s.kv_heads * p.s.k_groups) < kOneLaunchTiles * (float)sm_count) return false;
   if (p.s.head_dim == 128 && p.s.bits < 4) return true;
@@ -365,8 +372,9 @@ bool choose_umma(const MzDecodeParams& p, const MzDecodeParams& c, bool clusters
   MzTilesPlan t = {};
   describe_tiles(t, p);
   const float x = tiles_per_sm(p, t, sm_count), tile = kUmmaTile[p.s.bits - 1] * (p.s.head_dim == 64 ? kUmmaTile64 : 1.0f);
-  const float us = p.gqa > 4 ? kUmmaBase8 + 2.0f * tile * x : kUmmaBase + tile * x;
-  return us < (clusters ? cluster_us(c) : cut_us(p, x));
+  float us = p.gqa > 4 ? kUmmaBase8 + 2.0f * tile * x : kUmmaBase + tile * x;
+  if (p.s.head_dim == 64) us += kUmmaDense64 * (float)((double)p.s.batch * p.s.kv_heads * (t.tiles_per_pair - t.packed_tiles) / sm_count);
+  return us < (!clusters && p.s.head_dim == 64 ? kUmmaMarginCut64 : kUmmaMargin) * (clusters ? cluster_us(c) : cut_us(p, x));
 }
 
 }  // namespace

@@ -426,3 +426,18 @@ def test_unrolled_kernel_at_2_bits_with_splits(oracle, gqa):
         assert planned_kernel(layer, q.cuda(), splits) == 4
         got = decode_attention(layer, q.cuda(), 128 ** -0.5, out_dtype=torch.float32, splits=splits)
         assert relative_error(got, want) <= 1.2e-4
+
+
+@pytest.mark.parametrize("bits,gqa,B,KVH,S,planned", [(4, 4, 33, 8, 592, 3), (4, 4, 21, 8, 946, 3), (2, 4, 29, 4, 733, 2), (4, 8, 2, 8, 16198, 3), (4, 4, 40, 4, 3000, 3), (4, 2, 1, 4, 34849, 7)])
+def test_residual_tiles_weigh_in_the_choice_at_head_dim_64(oracle, bits, gqa, B, KVH, S, planned):
+    """Calls with about as many residual as packed tiles stay with the general kernel (20 to 45 % faster there), a long one goes to the tcgen05
+    kernel (twice as fast there)."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the line is drawn per SM")
+    import muzero_b200 as mz
+    cfg = mz.MuZeroConfig(bits=4, q_group_size=64, residual_length=128, alpha_key=2.0, alpha_value=2.0)
+    cfg.bits = bits
+    layer = mz.MuZeroCacheLayer(cfg)
+    k = torch.randn(B, KVH, S, 64, device="cuda", dtype=torch.bfloat16)
+    layer.update(k, k.clone(), {"materialize_full_kv": False})
+    assert planned_kernel(layer, k.new_zeros(B, KVH * gqa, 1, 64)) == planned
