@@ -56,8 +56,8 @@ int sm_count() {
   return g_sm_count[dev];
 }
 
-// Which decode kernel serves a call.  0 = automatic (tensor-core mma.sync kernel where it applies, else the SIMT
-// tiled kernel, else the shape-generic kernel), 1 = generic, 2 = no tensor-core kernel, 3 = the same as 0,
+// Which decode kernel serves a call.  0 = automatic (tcgen05 kernel where it serves and pays, else the tensor-core
+// mma.sync kernels, the SIMT tiled kernel, the shape-generic kernel), 1 = generic, 2 = no tensor-core kernel, 3 = the same as 0,
 // 4 = the tcgen05 kernel for every call that it serves, whatever the automatic choice would be.
 // MZ_DECODE_KERNEL = generic | tiles | mma | umma sets the initial value (read once, at the first call);
 // mz_debug_force_kernel changes it for later calls, so that tests can cross-check the kernels in one process.

@@ -149,7 +149,7 @@ bool mz_mma_kernel_b4(int D, int G, int nt, MzMmaKernel* k);
 bool mz_mma_kernel_b8(int D, int G, int nt, MzMmaKernel* k);
 bool mz_mma_kernel_wide(int D, int G, int nt, MzMmaKernel* k);
 
-// tcgen05 kernel: 1 to 4 bits, head_dim 128, group 64, 1 / 2 / 4 / 8 query heads per kv head.  full_precision: that of the fp32 kernels also at 2 bits, where the call would
+// tcgen05 kernel: 1 to 4 bits, head_dim 64 or 128, group 64, 1 / 2 / 4 / 8 query heads per kv head.  full_precision: that of the fp32 kernels also at 2 bits, where the call would
 // not have gone to the unrolled kernel
 bool mz_decode_umma_supported(const MzDecodeParams& p);
 int mz_plan_umma(MzDecodeParams& p, bool full_precision, int splits_request, int sm_count, size_t* slots);

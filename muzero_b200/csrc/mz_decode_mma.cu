@@ -284,7 +284,8 @@ float cluster_tile_us(const MzDecodeParams& p) {
 // against 2.1; 8 bits, 64: 2.4 against 1.35), but its residual tiles have CTAs of their own once every warp has two
 // packed tiles, which is worth a turn.  Codes of up to 4 bits in groups of 64 with 4 or 8 heads gain by that between about 28 and 52
 // tiles per SM (20 shapes: 0.79 to 1.06 of the SIMT kernel's time, 0.96 on average; 1 bit, 24 x 8 x 1537 48 against 62 us); below
-// (1.04 on average) and above (1.04; 3 bits, 2 x 8 x 60000 144 against 126) they don't.
+// (1.04 on average) and above (1.04; 3 bits, 2 x 8 x 60000 144 against 126) they don't.  (1 to 3 bits at head_dim 128 come here with explicit splits or under a
+// scratch limit only, 4 bits with 8 heads also where choose_umma leaves them; the other calls of this family are the tcgen05 kernel's.)
 enum class Cut { kUnrolled, kSimt, kGeneral };
 Cut choose_cut(const MzDecodeParams& p, float x) {
   if (mz_decode_flat_supported(p)) return Cut::kUnrolled;
@@ -340,18 +341,19 @@ bool plan_cluster(MzDecodeParams& p, const MzMmaKernel& k, int sm_count, bool an
   return false;
 }
 // Whether the tcgen05 kernel takes a call that it serves; `clusters`: the choice without it is cluster mode, planned in `c`.
-// head_dim 128, 1 to 3 bits: always but for the smallest calls (kOneLaunchTiles).  On the device, over 150 shapes of 0.1 to 210 tiles per SM it needs 0.55 (1 bit), 0.70 (3 bits) and 0.78 (2 bits) of the
-// time of the best other form, and is nowhere behind it by more than the timing's spread (90 calls below 12
-// tiles per SM: 0.49 to 0.92 of cluster mode).
+// head_dim 128, 1 to 3 bits: always but for the smallest calls (kOneLaunchTiles).  On the device, over 51 shapes of 3 to 120 tiles per SM it needs 0.56 (1 bit), 0.68 (2 bits) and
+// 0.62 (3 bits) of the time of the other choice, and was behind it in one (34 x 4 x 673 at 1 bit: 19.5 against 17.8 us).
 // 4 bits need two lookups per code, and three planes because the unrolled kernel's error (3e-5) is out of reach of two (4e-5 to 6e-5).
 // With up to four heads the unrolled kernel keeps its calls (64 x 8 pairs x 4224 tokens 149 us; 28 x 8 x 9800 49.9 against 72.7); cluster mode's
-// go by cost (1 x 8 x 17879 54 -> 30 us, 5 x 4 x 4988 30 -> 22; 15 x 8 x 459 would be 17.2 -> 19.5).  Eight heads run as two times four.
+// go by cost (1 x 8 x 17879 54 -> 30 us, 5 x 4 x 4988 30 -> 22; 15 x 8 x 459 would be 17.2 -> 19.5; all before the folds had scales of their own, which
+// cost this kernel 7 %).  Eight heads run as two times four.
 // head_dim 64 halves the expansion and not the softmax, and cluster mode has less to gain from (48 shapes: 0.40 to 0.9 from about 8 tiles per
 // SM on, up to 1.5 below): by cost at every width.
 // One launch against two (kernel and merge): a small call takes less time on the device than the host needs for it, and there the second
 // launch costs about 2 us whatever the kernel does.  Drawn by packed tiles per SM (cluster mode's estimate does not tell these apart):
 // 16 steps of a generation at 2 bits in cluster mode and here, 0.3 tiles per SM (1 x 8 x 500 tokens) 361 and 389 us, 2.6 (4 x 8 x 900) 333 and
-// 370, 4.0 (2 x 8 x 2500) 405 and 366; one call at 3.1 (2 x 8 x 2000) 18.9 and 15.1.
+// 370, 4.0 (2 x 8 x 2500) 405 and 366; one call at 3.1 (2 x 8 x 2000) 18.9 and 15.1.  These are eager loops at 2 bits; a captured graph, where the host is
+// not the limit, would gain by this kernel below the line too.
 // Bytes per value (planes) at 2 bits, head_dim 128 and up to four heads: three where cluster mode was the choice without this kernel, whose error is that of
 // an fp32 evaluation, two where the unrolled kernel was (5e-5 to 2e-4 there, 1e-5 to 4e-5 with two planes).  So no call is less precise than by
 // the choice between those two, and the line between the two errors is theirs (3 x 2 pairs: 4928 tokens two planes, 4992 three).

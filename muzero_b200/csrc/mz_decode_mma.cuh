@@ -33,7 +33,8 @@
 // tiles is cut by cost into one contiguous range per warp of a machine-filling grid and a merge kernel combines the
 // partial records, or (few pairs) a cluster of CTAs owns a pair and merges through distributed shared memory.
 // Measured (8 kv heads, call included): one sequence of 500 tokens, 4 bits 27.8 us as cut + merge on the unrolled kernel, 14.5 us
-// here; 6 x 1777 with 8 heads per kv head under a mask 43.0 us on the SIMT kernel, 38.1 us here; head_dim 64, 16 x 2050 333 us on the
+// here; 6 x 1777 with 8 heads per kv head under a mask 43.0 us on the SIMT kernel, 38.1 us here (and 32.8 on the tcgen05
+// kernel, which has that call now); head_dim 64, 16 x 2050 333 us on the
 // shape-generic kernel, 23.8 us here.  Without the second product (error 1e-5 instead of 5e-7): 13.8, 32.7 and 19.9 us.
 // Bound by the latency of a tile's chain: no unit is busy (issue 30 to 51 %, shared-memory pipe 17 to 39 %).
 #pragma once

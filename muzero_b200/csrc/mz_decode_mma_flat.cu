@@ -115,8 +115,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) decode_mma_kernel(const MzD
   const int g = lane >> 2, t = lane & 3;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-  // tiles 0 .. kt-1 of a pair are packed groups, the rest residual tiles; a plan without packed tiles (the
-  // residual-only companion launch of the tcgen05 kernel) needs no table
+  // tiles 0 .. kt-1 of a pair are packed groups, the rest residual tiles; a plan without packed tiles needs no table
   // one launch may carry two plans: the first p.hetero CTAs take the packed tiles, the others the residual tiles
   // (a residual tile is a short latency-bound chain; kept apart it no longer sits in the packed tiles' warps)
   const bool second = p.hetero > 0 && (int)blockIdx.x >= p.hetero;

@@ -19,11 +19,11 @@
 //     tensor memory and returns.  (The named barriers left are within a team, whose warps keep step whatever runs out.)
 //   * the residual window is un-quantized: its tiles have CTAs of their own (mz_dense_tiles.cuh)
 //
-// What bounds it: issue (58 % of the cycles; per row of 64 two-bit codes about 230 instructions, of which 32 permutes) and the logic pipe
-// (48 %, two cycles per instruction); integer MMAs take 40 cycles each, all of it reading their operands, 41 %.  A thread that spills
+// What bounds it: issue (58 % of the cycles; per row of 64 two-bit codes about 290 instructions, residual tiles included) and the logic pipe
+// (47 %, two cycles per instruction); integer MMAs take 40 cycles each, all of it reading their operands, 31 %.  A thread that spills
 // is dear: 227 KB of shared memory leave 28 KB of L1, and 20 bytes of spill per thread cost 10 %.  Hence the register split.
-// 64 x 8 pairs x 4224 tokens, 4 heads, us per call: 1 bit 202 -> 97 (before: SIMT kernel), 2 bits 148 -> 125 (before: unrolled mma.sync
-// kernel), 3 bits 230 -> 186 (SIMT); 24 x 8 x 1537, 3 bits: 53 -> 39; one sequence of 1300 tokens, device time: 15 -> 8 to 11.
+// 64 x 8 pairs x 4224 tokens, 4 heads, us per call: 1 bit 202 -> 108 (before: SIMT kernel), 2 bits 148 -> 134 (before: unrolled mma.sync
+// kernel), 3 bits 230 -> 208 (SIMT); 24 x 8 x 1537, 3 bits: 53 -> 41.  About 7 % of these are the folds' own scales (put_folds).
 //
 // Precision: three planes hold a value to 2^-24 of its row's larger side and a product to 4e-9 of the step's largest for its head and group, which
 // is no worse than the fp32 kernels (relative error against 64 bits 2e-7 to 7e-7 where those have 2e-7 to 1.1e-6, attention sinks, outlier
